@@ -102,6 +102,28 @@ def test_transcode_round_trip_random(g):
         assert ((host[li >> 5] >> (31 - (li & 31))) & 1) == ((mh[mi >> 5] >> (31 - (mi & 31))) & 1)
 
 
+@pytest.mark.parametrize("g", [4, 16, 32, 64, 128, 256, 512])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_transcode_every_bit_against_numpy(g, offset):
+    """Each grid's column layout (words per row 1 .. 16) and both store widths: a table that begins
+    4 bytes after a 16-byte boundary takes the scalar one."""
+    n = g ** 3 // 32
+    gen = torch.Generator(device="cuda").manual_seed(g + offset)
+    t = torch.randint(-2 ** 31, 2 ** 31 - 1, (n + offset,), dtype=torch.int32, device="cuda", generator=gen)[offset:]
+    c = np.arange(g, dtype=np.int64)
+    s = sum(((c >> i) & 1) << (3 * i) for i in range(10))  # the coordinate's bits, three apart
+    code = s[None, None, :] | s[None, :, None] << 1 | s[:, None, None] << 2
+    bits = np.unpackbits(t.cpu().numpy().view(np.uint32).byteswap().view(np.uint8))
+    want = np.empty_like(bits)
+    want[code.reshape(-1)] = bits
+    want = np.packbits(want).view(np.uint32).byteswap()
+    m = cv.transcode(t, g, True)
+    assert np.array_equal(m.cpu().numpy().view(np.uint32), want)
+    back = torch.empty(n + offset, dtype=torch.int32, device="cuda")[offset:]
+    back.copy_(m)
+    assert torch.equal(cv.transcode(back, g, False), t)
+
+
 @pytest.mark.parametrize("mesh", ["torus", "ico", "soup"])
 def test_device_bbox_and_voxinfo_equal_host_setup(mesh):
     tris = {"torus": lambda: meshgen.torus(3), "ico": lambda: meshgen.icosphere(1, level=7),
