@@ -301,16 +301,14 @@ struct Group {
 	std::vector<JobDesc> jobs;
 	uint64_t tris = 0;
 	uint32_t tiles = 0, units = 0;
-	uint64_t mwords = 0, mbricks = 0, mslabs = 0;
-	uint32_t slab_smem = 0;
+	uint64_t mwords = 0, mwarps = 0;
 	uint32_t bricks = 0;  // 64^3 bricks of the group's JOB_BRICKS jobs
 };
 
 void finish_group(Group& g, bool solid) {
 	uint32_t tile = 0, unit = 0, brick = 0;
-	uint64_t mw = 0, mb = 0, ms = 0;
+	uint64_t mw = 0, mc = 0;
 	g.tris = 0;
-	g.slab_smem = 0;
 	for (JobDesc& j : g.jobs) {
 		j.tile_begin = tile;
 		tile += tiles_of(j.n_tri);
@@ -319,33 +317,19 @@ void finish_group(Group& g, bool solid) {
 		if (!solid && (j.flags & JOB_BRICKS)) brick += bricks_of(j.grid);
 		if (solid) {
 			j.unit_begin = unit;
-			// Morton slab grids are resolved by solid_morton_slab alone: no resolve units
-			if (!((j.flags & JOB_MORTON) && morton_slab_grid(j.grid[0]))) unit += (uint32_t)solid_units(j.grid).units;
+			const uint64_t mwarps = (j.flags & JOB_MORTON) ? morton_warps(j.grid[0]) : 0;
+			if (!mwarps) unit += (uint32_t)solid_units(j.grid).units;  // solid_morton_cols resolves its rows itself
 			j.mword_begin = mw;
-			j.mbrick_begin = mb;
-			j.mslab_begin = ms;
-			const uint64_t vox = (uint64_t)j.grid[0] * j.grid[1] * j.grid[2];
-			if (j.flags & JOB_MORTON) {
-				const uint64_t gx = j.grid[0];
-				if (morton_slab_grid(gx)) {
-					ms += (gx / 16) * (gx / 16);  // slabs of 16 x 16 rows
-					const uint32_t stride = (uint32_t)(gx / 32) | 1u;
-					g.slab_smem = std::max(g.slab_smem, (256u * stride + kSlabSkewWords) * 4u);
-				} else if (gx >= 32) {
-					const uint64_t w = gx >= 128 ? 4 : gx / 32;  // x-adjacent 32^3 bricks per CTA
-					mb += (vox >> 15) / w;
-				} else {
-					mw += (vox + 31) / 32;
-				}
-			}
+			j.mwarp_begin = mc;
+			mc += mwarps;
+			if ((j.flags & JOB_MORTON) && !mwarps) mw += ((uint64_t)j.grid[0] * j.grid[1] * j.grid[2] + 31) / 32;
 		}
 	}
 	g.tiles = tile;
 	g.units = unit;
 	g.bricks = brick;
 	g.mwords = mw;
-	g.mbricks = mb;
-	g.mslabs = ms;
+	g.mwarps = mc;
 }
 
 // Split jobs of one mode into launch groups of fewer than kMaxTriPerLaunch triangles.  A job above
@@ -414,9 +398,7 @@ struct Runner {
 		L.n_tiles = g.tiles;
 		L.n_units = g.units;
 		L.n_mwords = g.mwords;
-		L.n_mbricks = g.mbricks;
-		L.n_mslabs = g.mslabs;
-		L.slab_smem = g.slab_smem;
+		L.n_mwarps = g.mwarps;
 		if (g.bricks > bricks) return fail(CVX_ERR_INVALID_VALUE, "brick scratch too small");
 		L.n_bricks = g.bricks;
 		bind_scratch(L, rec, cap, bricks, dev.tune);
@@ -842,9 +824,7 @@ static cudaError_t capture_group(const Group& g, bool solid, bool resolve, void*
 	L.n_tiles = g.tiles;
 	L.n_units = g.units;
 	L.n_mwords = g.mwords;
-	L.n_mbricks = g.mbricks;
-	L.n_mslabs = g.mslabs;
-	L.slab_smem = g.slab_smem;
+	L.n_mwarps = g.mwarps;
 	L.n_bricks = g.bricks;
 	bind_scratch(L, static_cast<char*>(rec), cap, bricks, dev.tune);
 	if (g.jobs.size() == 1)

@@ -96,8 +96,7 @@ struct JobDesc {
 	uint32_t tile_begin;   // first triangle tile of this job in the launch's tile space
 	uint32_t unit_begin;   // solid: first resolve unit of this job in the launch's unit space
 	uint64_t mword_begin;  // solid Morton, g < 32: first Morton word in the launch's word space
-	uint64_t mbrick_begin; // solid Morton, g > 1024: first group of x-adjacent 32^3 bricks in the launch
-	uint64_t mslab_begin;  // solid Morton, 32 <= g <= 1024: first 16x16-row slab in the launch
+	uint64_t mwarp_begin;  // solid Morton, g >= 32: first warp of solid_morton_cols in the launch
 	uint32_t brick_begin;  // JOB_BRICKS: first 32^3 brick of this job in the launch's brick space
 	uint32_t pad;
 };
@@ -201,9 +200,7 @@ struct LaunchDesc {
 	uint32_t n_tiles;      // total triangle tiles over all jobs
 	uint32_t n_units;      // solid resolve units over all jobs
 	uint64_t n_mwords;     // Morton words of solid Morton jobs with g < 32
-	uint64_t n_mbricks;    // groups of x-adjacent 32^3 bricks of solid Morton jobs with g > 1024
-	uint64_t n_mslabs;     // 16x16-row slabs of solid Morton jobs with 32 <= g <= 1024
-	uint32_t slab_smem;    // dynamic shared memory of the slab kernel (largest slab of the launch)
+	uint64_t n_mwarps;     // warps of solid_morton_cols: solid Morton jobs with g >= 32
 	uint32_t n_bricks;     // 32^3 bricks of the launch's JOB_BRICKS jobs
 	Scratch scr;
 };
@@ -256,13 +253,6 @@ __device__ __forceinline__ uint64_t morton3(uint32_t x, uint32_t y, uint32_t z) 
 }
 
 __device__ __forceinline__ uint64_t umin64(uint64_t a, uint64_t b) { return a < b ? a : b; }
-
-// Shared-memory slab of 256 rows (16 z-slices x 16 rows) of `stride` (odd) words: row r starts at
-// r * stride + r / 32.  The odd stride spreads consecutive rows over the banks; the skew of one word
-// per 32 rows does the same for rows 32 apart, which a Morton gather reads together (a word of a
-// 16^3 block touches rows (2Z + dz) * 16 + 4Y + dy).
-__host__ __device__ __forceinline__ uint32_t slab_row(uint32_t r, uint32_t stride) { return r * stride + (r >> 5); }
-constexpr uint32_t kSlabSkewWords = 256 / 32;  // extra words of a 256-row slab
 
 // Inverse of spread3: the bits at positions 0, 3, 6, ... of v, packed.
 __device__ __forceinline__ uint32_t compact3(uint64_t v) {

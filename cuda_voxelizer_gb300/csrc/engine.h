@@ -89,8 +89,9 @@ cudaError_t launch_solid(const LaunchDesc& L, const Tune& tune, int cols_grid, c
                          const Prof* prof);
 int solid_cols_blocks_per_sm();
 
-// Morton grids that solid_morton_slab resolves and transcodes in one pass.
-inline bool morton_slab_grid(uint64_t g) { return g >= 32 && g <= 1024; }
+// Warps of solid_morton_cols for a Morton job (g >= 32; its g < 32 jobs go through solid_morton_small):
+// (g / 4)^2 row groups, 32 / min(8, g / 32) of them per warp.
+inline uint64_t morton_warps(uint64_t g) { return g < 32 ? 0 : (g / 4) * (g / 4) * (g < 256 ? g / 32 : 8) / 32; }
 
 // Resolve-unit bookkeeping of a solid job: rows per unit and units per job.
 struct SolidUnits {

@@ -77,14 +77,18 @@ __host__ __device__ __forceinline__ MortonCols morton_cols(uint32_t lg) {
 	return m;
 }
 
+// Row group number q (of (g / 4)^2) -> (Y, Z) = (y / 4, z / 4), in the order y2, z2, the rest of y, the rest of z.
+__device__ __forceinline__ void morton_row_group(const MortonCols& m, uint64_t q, uint32_t& Y, uint32_t& Z) {
+	const uint64_t rest = q >> 2;
+	Y = ((uint32_t)q & 1u) | ((uint32_t)rest & ((1u << (m.lg - 3)) - 1u)) << 1;
+	Z = ((uint32_t)(q >> 1) & 1u) | (uint32_t)(rest >> (m.lg - 3)) << 1;
+}
+
 // Column t (of (g / 4)^2 * (g / 32)): its linear word w and row group (Y, Z) = (y / 4, z / 4).
 __device__ __forceinline__ void morton_column(const MortonCols& m, uint64_t t, uint32_t& w, uint32_t& Y, uint32_t& Z) {
-	const uint32_t yz = (uint32_t)(t >> m.lgc) & 3u;
 	const uint32_t whi = (uint32_t)(t >> (m.lgc + 2)) & ((1u << (m.lgw - m.lgc)) - 1u);
-	const uint64_t rest = t >> (m.lgw + 2);
 	w = ((uint32_t)t & ((1u << m.lgc) - 1u)) | whi << m.lgc;
-	Y = (yz & 1u) | ((uint32_t)rest & ((1u << (m.lg - 3)) - 1u)) << 1;
-	Z = (yz >> 1) | (uint32_t)(rest >> (m.lg - 3)) << 1;
+	morton_row_group(m, ((t >> m.lgc) & 3u) | (t >> (m.lgw + 2)) << 2, Y, Z);
 }
 
 // First Morton word of the column at linear word w of row group (Y, Z); its 16 words are base + c +

@@ -227,15 +227,10 @@ extern "C" cvx_status cvx_voxelize_solid_noalloc(const cvx_voxinfo* info, const 
 	L.n_tiles = 0;
 	L.n_units = (uint32_t)su.units;
 	if (morton) {
-		if (morton_slab_grid(g0)) {
-			L.n_units = 0;  // solid_morton_slab resolves these grids alone
-			L.n_mslabs = (g0 / 16) * (g0 / 16);
-			L.slab_smem = (256u * ((uint32_t)(g0 / 32) | 1u) + kSlabSkewWords) * 4u;
-		} else if (g0 >= 32) {
-			L.n_mbricks = ((g0 * g1 * g2) >> 15) / (g0 >= 128 ? 4 : g0 / 32);
-		} else {
+		if ((L.n_mwarps = morton_warps(g0)) != 0)
+			L.n_units = 0;  // solid_morton_cols resolves these grids alone
+		else
 			L.n_mwords = words;
-		}
 	}
 	return cuda_status(launch_solid(L, tune, cols_grid, s, kSolidResolve, nullptr), "solid resolve");
 }

@@ -17,12 +17,12 @@
 //   solid_resolve       linear jobs: one thread per row run (whole rows; 16-byte words where rows
 //                       are aligned): prefix XOR along x, XORed into the linear table (every word
 //                       stored, for JOB_TABLE_OVERWRITE jobs), flip table cleared.
-//   solid_morton_slab   Morton jobs with 32 <= g <= 1024: a CTA resolves a 16 x 16-row slab in
-//                       shared memory and writes it as 16^3 Morton blocks (128 contiguous words).
-//   solid_morton_brick  Morton jobs with g > 1024: groups of x-adjacent 32^3 bricks.
+//   solid_morton_cols   Morton jobs with g >= 32: a warp resolves row groups of 4 x 4 rows along x and
+//                       converts them to Morton words in registers.
 //   solid_morton_small  Morton jobs with g < 32 (one word at a time), then solid_zero clears the
 //                       flip table.
 #include "engine.h"
+#include "morton_block.cuh"
 
 namespace cvx {
 
@@ -473,9 +473,6 @@ __device__ __forceinline__ uint32_t prefix_xor_msb(uint32_t t) {
 	return t;
 }
 
-// Morton grids resolved and transcoded in one pass by solid_morton_slab (cubic powers of two).
-__host__ __device__ __forceinline__ bool slab_grid(uint64_t g) { return g >= 32 && g <= 1024; }
-
 // Resolve one word: toggles t (MSB first) plus the parity carried in from the row's earlier words.
 __device__ __forceinline__ uint32_t resolve_word(uint32_t t, uint32_t& carry) {
 	const uint32_t res = prefix_xor_msb(t) ^ (carry ? 0xFFFFFFFFu : 0u);
@@ -483,8 +480,8 @@ __device__ __forceinline__ uint32_t resolve_word(uint32_t t, uint32_t& carry) {
 	return res;
 }
 
-// Linear jobs: table ^= resolved, toggles cleared.  Morton jobs: toggles replaced by the resolved
-// bits for solid_morton_* to gather.
+// Linear jobs: table ^= resolved, toggles cleared.  Morton jobs (g < 32): toggles replaced by the
+// resolved bits for solid_morton_small to gather.
 // XOR a resolved word into the table (the reference's semantics: the caller's table is XORed), or
 // store it, zero or not, when the engine owns the table's content (JOB_TABLE_OVERWRITE).
 __device__ __forceinline__ void xor_out(uint32_t* dest, uint64_t w, uint32_t v, bool overwrite) {
@@ -517,7 +514,6 @@ __global__ void __launch_bounds__(256) solid_resolve(const __grid_constant__ Lau
 	uint32_t* flips = J.flips;
 	uint32_t* dest = J.table;
 	const uint64_t u = unit_id - J.unit_begin;
-	if (morton && slab_grid(gx)) return;  // solid_morton_slab resolves these jobs itself
 	if (gx % 32 == 0) {
 		const uint32_t wpr = (uint32_t)(gx >> 5);
 		const uint64_t w0 = u * wpr;
@@ -581,127 +577,93 @@ __global__ void __launch_bounds__(256) solid_resolve(const __grid_constant__ Lau
 	}
 }
 
+// Morton jobs with g >= 32: resolve, convert and clear in one pass, in registers.  A thread holds one
+// linear word of 16 rows (4 y x 4 z: 16 Morton words, morton_block.cuh); the C = min(8, g / 32) lowest
+// lane bits take neighbouring words of the rows, the others neighbouring 4 x 4 row groups, and the
+// warp walks along x, C words at a time.  A word's incoming parity is the XOR of its row's earlier
+// words' parities: the 16 rows' parities of a lane are one 16-bit mask, scanned over the C lanes with
+// log2(C) shuffles.  Where no lane's words hold a toggle -- most of the inside and the outside of a
+// solid -- every word is all zeros or all ones and nothing is scanned.  Bound by memory latency (the
+// flip table read, the table read and written); the filled icosphere at 512^3 takes 12.6 us, 4.2 M
+// warp instructions, where resolving 16 x 16-row slabs in shared memory and assembling words from
+// their eight row pieces took 27.8 us and 19.2 M.  72 registers keep 512^3's 1,024 CTAs in one wave
+// (7 per SM); at 64 (8 per SM) the kernel spills and takes 16 us.
+constexpr uint32_t kMortonThreads = 128;
 
-
-// Morton jobs with g >= 32: one CTA per group of W = min(4, g/32) x-adjacent Morton-aligned 32^3
-// bricks.  Each brick is 1,024 consecutive Morton words; the group's 32 x 32 rows of W*32 x-bits are
-// staged in shared memory (16-byte accesses when W = 4) and cleared in the flip table (this CTA is
-// their only reader), then each Morton word is assembled from eight 4-bit row nibbles and XORed into
-// the table with coalesced accesses.
-__global__ void __launch_bounds__(256) solid_morton_brick(const __grid_constant__ LaunchDesc L) {
-	__shared__ __align__(16) uint32_t s_rows[32 * 32 * 4];  // [z][y][W] words of x-bits
-	const uint64_t group = blockIdx.x;
-	const uint32_t j = job_search(L, group, [](const JobDesc& d) { return d.mbrick_begin; });
+__global__ void __launch_bounds__(kMortonThreads, 7) solid_morton_cols(const __grid_constant__ LaunchDesc L) {
+	const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+	if (warp >= L.n_mwarps) return;
+	const uint32_t lane = threadIdx.x & 31u;
+	const uint32_t j = job_search(L, warp, [](const JobDesc& d) { return d.mwarp_begin; });
 	const JobDesc& J = job_at(L, j);
-	const uint64_t g = J.grid[0];
-	const uint32_t W = g >= 128 ? 4u : (uint32_t)(g >> 5);       // bricks per group
-	const uint64_t gi = group - J.mbrick_begin;                  // group index within the job
-	// groups are numbered x-fastest over (g/32/W) x (g/32) x (g/32); group gi covers the bricks
-	// (W*Bx + k, by, bz), k < W (g is a power of two: the divisions are shifts)
-	const uint32_t lg_nb = 31u - __clz((uint32_t)(g >> 5));      // log2(bricks per axis)
-	const uint32_t lg_w = W == 4 ? 2u : (W == 2 ? 1u : 0u);
-	const uint64_t Bx = gi & ((1ull << (lg_nb - lg_w)) - 1ull);
-	const uint64_t by = (gi >> (lg_nb - lg_w)) & ((1ull << lg_nb) - 1ull);
-	const uint64_t bz = gi >> (2 * lg_nb - lg_w);
-	const uint64_t bx = Bx * W;
-	uint32_t* flips = J.flips;
-	const uint64_t wpr = g >> 5;
-	for (uint32_t i = threadIdx.x; i < 1024; i += 256) {
-		const uint64_t z = bz * 32 + (i >> 5), y = by * 32 + (i & 31);
-		const uint64_t w = (z * g + y) * wpr + bx;
-		if (W == 4 && ((reinterpret_cast<uintptr_t>(flips + w) & 15u) == 0)) {
-			const uint4 v = *reinterpret_cast<const uint4*>(flips + w);
-			*reinterpret_cast<uint4*>(s_rows + i * 4) = v;
-			if (v.x | v.y | v.z | v.w) *reinterpret_cast<uint4*>(flips + w) = make_uint4(0u, 0u, 0u, 0u);
+	const uint32_t lg = 31u - __clz(J.grid[0]);
+	const MortonCols m = morton_cols(lg);
+	const uint32_t C = 1u << m.lgc, col = lane & (C - 1u);
+	uint32_t w, Y, Z;  // this lane's first word (w = col) and its row group
+	morton_row_group(m, ((warp - J.mwarp_begin) << (5 - m.lgc)) + (lane >> m.lgc), Y, Z);
+	uint32_t* flips = J.flips + ((((uint64_t)Z << (lg + 2)) + (Y << 2)) << m.lgw);
+	uint32_t* table = J.table;
+	const bool overwrite = (J.flags & JOB_TABLE_OVERWRITE) != 0;
+	const bool vec = (reinterpret_cast<uintptr_t>(table) & 15u) == 0;
+	uint32_t carry = 0;  // bit i: parity of row i = 4 * dz + dy before this chunk of words
+	for (w = col; w < (1u << m.lgw); w += C) {
+		uint32_t* src = flips + w;
+		uint32_t t[16], any = 0;
+#pragma unroll
+		for (uint32_t i = 0; i < 16; i++) {
+			t[i] = src[(((uint64_t)(i >> 2) << lg) + (i & 3u)) << m.lgw];
+			any |= t[i];
+		}
+		uint32_t v[2][8];  // the resolved rows as rows_to_morton takes them
+		if (__any_sync(FULL, any != 0u)) {
+			uint32_t par = 0;  // bit i: parity of row i's word
+#pragma unroll
+			for (uint32_t i = 0; i < 16; i++) {
+				if (t[i]) src[(((uint64_t)(i >> 2) << lg) + (i & 3u)) << m.lgw] = 0u;
+				t[i] = prefix_xor_msb(t[i]);
+				par = __funnelshift_r(par, t[i], 1);  // its last bit in at the top
+			}
+			par >>= 16;
+			uint32_t incl = par;
+			for (uint32_t d = 1; d < C; d <<= 1) {
+				const uint32_t u = __shfl_up_sync(FULL, incl, d, C);
+				if (col >= d) incl ^= u;
+			}
+			const uint32_t in = carry ^ incl ^ par;
+			carry ^= __shfl_sync(FULL, incl, C - 1u, C);
+#pragma unroll
+			for (uint32_t i = 0; i < 16; i++)
+				v[i >> 3][7 - (2 * (i & 3u) + ((i >> 2) & 1u))] = t[i] ^ (uint32_t)((int)(in << (31 - i)) >> 31);
+		} else if (__any_sync(FULL, carry != 0u)) {
+#pragma unroll
+			for (uint32_t i = 0; i < 16; i++)
+				v[i >> 3][7 - (2 * (i & 3u) + ((i >> 2) & 1u))] = (uint32_t)((int)(carry << (31 - i)) >> 31);
 		} else {
-			for (uint32_t k = 0; k < W; k++) {
-				const uint32_t v = flips[w + k];
-				s_rows[i * 4 + k] = v;
-				if (v) flips[w + k] = 0u;
-			}
+			if (!overwrite) continue;
+#pragma unroll
+			for (uint32_t i = 0; i < 16; i++) v[i >> 3][i & 7u] = 0u;
 		}
-	}
-	__syncthreads();
-	for (uint32_t xk = 0; xk < W; xk++) {
-		// brick (bx + xk, by, bz): its Morton words are the 1,024 starting at its Morton index * 1024
-		const uint64_t brick = spread3((uint32_t)(bx + xk)) | (spread3((uint32_t)by) << 1) | (spread3((uint32_t)bz) << 2);
-		uint32_t* dest = J.table + (brick << 10);
-		for (uint32_t m = threadIdx.x; m < 1024; m += 256) {
-			const uint32_t X = compact3(m >> 1), Y = compact3(m >> 2), Z = compact3(m);
-			uint32_t out = 0;
+		rows_to_morton(v[0]);
+		rows_to_morton(v[1]);
+		uint32_t* dst = table + morton_col_base(w, Y, Z);
 #pragma unroll
-			for (uint32_t dz = 0; dz < 2; dz++)
-#pragma unroll
-				for (uint32_t dy = 0; dy < 4; dy++) {
-					const uint32_t row = s_rows[((2 * Z + dz) * 32 + 4 * Y + dy) * 4 + xk];
-					const uint32_t nib = (row >> (28u - 4u * X)) & 0xFu;
-					out |= nibble_mask(nib) >> (2u * (dy & 1u) + 4u * dz + 16u * (dy >> 1));
+		for (uint32_t k = 0; k < 8; k += 2) {  // x groups k and k + 1: x3 = k bit 1, x4 = k bit 2
+			uint4 o = make_uint4(v[0][7 - k], v[1][7 - k], v[0][6 - k], v[1][6 - k]);
+			uint32_t* d = dst + 8 * (k & 2) + 32 * (k & 4);
+			if (!overwrite && (o.x | o.y | o.z | o.w) == 0u) continue;
+			if (vec) {
+				if (!overwrite) {
+					const uint4 q = *reinterpret_cast<const uint4*>(d);
+					o = make_uint4(o.x ^ q.x, o.y ^ q.y, o.z ^ q.z, o.w ^ q.w);
 				}
-			xor_out(dest, m, out, (J.flags & JOB_TABLE_OVERWRITE) != 0);
-		}
-	}
-}
-
-// Morton jobs with 32 <= g <= 1024: resolve, transcode and clear in one pass.  One CTA per slab of
-// 16 x 16 rows (y block by, z block bz, 16 each): for each of its 16 z-slices the slab's 16 rows are
-// contiguous in the flip table, so they are loaded with coalesced 16-byte accesses into shared
-// memory (rows padded to an odd word count: no bank conflicts below) and cleared; each thread
-// resolves one whole row (prefix XOR along x); then every 16^3 block along x -- 128 consecutive
-// Morton words -- is gathered from 4-bit row nibbles and XORed into the table.
-__global__ void __launch_bounds__(256) solid_morton_slab(const __grid_constant__ LaunchDesc L) {
-	extern __shared__ __align__(16) uint32_t s_slab[];  // row zi*16 + yi at slab_row(row, stride)
-	const uint64_t slab = blockIdx.x;
-	const uint32_t j = job_search(L, slab, [](const JobDesc& d) { return d.mslab_begin; });
-	const JobDesc& J = job_at(L, j);
-	const uint64_t g = J.grid[0];
-	const uint32_t wpr = (uint32_t)(g >> 5);           // words per row
-	const uint32_t stride = wpr | 1u;
-	const uint32_t lgw = 31u - __clz(wpr);
-	const uint32_t nb = (uint32_t)(g >> 4);            // 16-blocks per axis
-	const uint32_t lgb = 31u - __clz(nb);
-	const uint64_t si = slab - J.mslab_begin;
-	const uint64_t by = si & (nb - 1u), bz = si >> lgb;
-	uint32_t* flips = J.flips;
-	const uint32_t chunk = 16u * wpr;                   // words of the slab in one z-slice
-	for (uint32_t i = threadIdx.x; i < 16u * (chunk / 4u); i += 256) {
-		const uint32_t zi = i / (chunk / 4u), q = i % (chunk / 4u);
-		uint4* src = reinterpret_cast<uint4*>(flips + ((bz * 16 + zi) * g + by * 16) * wpr) + q;
-		const uint4 v = *src;
-		const uint32_t vv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-		for (int k = 0; k < 4; k++) {
-			const uint32_t idx = 4 * q + k;
-			s_slab[slab_row(zi * 16 + (idx >> lgw), stride) + (idx & (wpr - 1u))] = vv[k];
-		}
-		if (v.x | v.y | v.z | v.w) *src = make_uint4(0u, 0u, 0u, 0u);
-	}
-	__syncthreads();
-	{
-		uint32_t* row = s_slab + slab_row(threadIdx.x, stride);  // 256 rows, one per thread
-		uint32_t carry = 0;
-		for (uint32_t w = 0; w < wpr; w++) {
-			const uint32_t t = row[w];
-			if (t == 0u && carry == 0u) continue;
-			row[w] = resolve_word(t, carry);
-		}
-	}
-	__syncthreads();
-	// 16^3 blocks along x: two per pass (128 Morton words each, one per thread)
-	const uint32_t half = threadIdx.x >> 7, m = threadIdx.x & 127u;
-	const uint32_t X = compact3(m >> 1), Y = compact3(m >> 2), Z = compact3(m);  // 2, 2, 3 bits
-	for (uint32_t bx = half; bx < nb; bx += 2) {
-		const uint64_t blk = spread3(bx) | (spread3((uint32_t)by) << 1) | (spread3((uint32_t)bz) << 2);
-		const uint32_t wsel = bx >> 1, xoff = (bx & 1u) * 16u + 4u * X;  // word, first x bit in it
-		uint32_t out = 0;
-#pragma unroll
-		for (uint32_t dz = 0; dz < 2; dz++)
-#pragma unroll
-			for (uint32_t dy = 0; dy < 4; dy++) {
-				const uint32_t rw = s_slab[slab_row((2 * Z + dz) * 16 + 4 * Y + dy, stride) + wsel];
-				const uint32_t nib = (rw >> (28u - xoff)) & 0xFu;
-				out |= nibble_mask(nib) >> (2u * (dy & 1u) + 4u * dz + 16u * (dy >> 1));
+				*reinterpret_cast<uint4*>(d) = o;
+			} else {
+				xor_out(d, 0, o.x, overwrite);
+				xor_out(d, 1, o.y, overwrite);
+				xor_out(d, 2, o.z, overwrite);
+				xor_out(d, 3, o.w, overwrite);
 			}
-		xor_out(J.table, (blk << 7) + m, out, (J.flags & JOB_TABLE_OVERWRITE) != 0);
+		}
 	}
 }
 
@@ -726,14 +688,14 @@ __global__ void __launch_bounds__(256) solid_morton_small(const __grid_constant_
 	xor_out(J.table, m, out, (J.flags & JOB_TABLE_OVERWRITE) != 0);
 }
 
-// Morton jobs with g < 32: clear the resolved flip table, one thread per resolve unit (the larger
-// grids' bricks clear their own words).
+// Morton jobs with g < 32: clear the resolved flip table, one thread per resolve unit
+// (solid_morton_cols clears its own words).
 __global__ void __launch_bounds__(256) solid_zero(const __grid_constant__ LaunchDesc L) {
 	const uint32_t unit_id = blockIdx.x * blockDim.x + threadIdx.x;
 	if (unit_id >= L.n_units) return;
 	const uint32_t j = job_search(L, unit_id, [](const JobDesc& d) { return (uint64_t)d.unit_begin; });
 	const JobDesc& J = job_at(L, j);
-	if (!(J.flags & JOB_MORTON) || J.grid[0] >= 32) return;
+	if (!(J.flags & JOB_MORTON)) return;
 	const uint64_t gx = J.grid[0];
 	const uint64_t rows = (uint64_t)J.grid[1] * J.grid[2];
 	uint64_t a = gx, bb = 32;
@@ -779,22 +741,9 @@ static cudaError_t launch_solid_t(const LaunchDesc& L, const Tune& tune, int col
 			if ((e = launch_k(solid_resolve, (L.n_units + 255) / 256, 256, 0, s, L)) != cudaSuccess) return e;
 			if (prof) (*prof)("solid_resolve", s);
 		}
-		if (L.n_mslabs) {
-			static int attr_set[64] = {};
-			int dev = 0;
-			cudaGetDevice(&dev);
-			if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-				if ((e = cudaFuncSetAttribute(solid_morton_slab, cudaFuncAttributeMaxDynamicSharedMemorySize,
-				                              (256 * (32 + 1) + kSlabSkewWords) * 4)) != cudaSuccess)
-					return e;
-				attr_set[dev] = 1;
-			}
-			if ((e = launch_k(solid_morton_slab, (unsigned)L.n_mslabs, 256, L.slab_smem, s, L)) != cudaSuccess) return e;
-			if (prof) (*prof)("solid_morton_slab", s);
-		}
-		if (L.n_mbricks) {
-			if ((e = launch_k(solid_morton_brick, (unsigned)L.n_mbricks, 256, 0, s, L)) != cudaSuccess) return e;
-			if (prof) (*prof)("solid_morton", s);
+		if (L.n_mwarps) {
+			if ((e = launch_k(solid_morton_cols, (unsigned)((L.n_mwarps * 32 + kMortonThreads - 1) / kMortonThreads), kMortonThreads, 0, s, L)) != cudaSuccess) return e;
+			if (prof) (*prof)("solid_morton_cols", s);
 		}
 		if (L.n_mwords) {
 			if ((e = launch_k(solid_morton_small, (unsigned)((L.n_mwords + 255) / 256), 256, 0, s, L)) != cudaSuccess)
