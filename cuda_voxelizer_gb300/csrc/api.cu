@@ -318,7 +318,9 @@ void finish_group(Group& g, bool solid) {
 		if (solid) {
 			j.unit_begin = unit;
 			const uint64_t mwarps = (j.flags & JOB_MORTON) ? morton_warps(j.grid[0]) : 0;
-			if (!mwarps) unit += (uint32_t)solid_units(j.grid).units;  // solid_morton_cols resolves its rows itself
+			const SolidUnits su = solid_units(j.grid);
+			j.unit_words = su.unit_words;
+			if (!mwarps) unit += (uint32_t)su.units;  // solid_morton_cols resolves its rows itself
 			j.mword_begin = mw;
 			j.mwarp_begin = mc;
 			mc += mwarps;

@@ -98,7 +98,7 @@ struct JobDesc {
 	uint64_t mword_begin;  // solid Morton, g < 32: first Morton word in the launch's word space
 	uint64_t mwarp_begin;  // solid Morton, g >= 32: first warp of solid_morton_cols in the launch
 	uint32_t brick_begin;  // JOB_BRICKS: first 32^3 brick of this job in the launch's brick space
-	uint32_t pad;
+	uint32_t unit_words;   // solid: table words per resolve unit
 };
 
 // Work-queue records written by the classify kernels and consumed by the cooperative kernels.

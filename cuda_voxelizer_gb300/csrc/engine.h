@@ -93,11 +93,15 @@ int solid_cols_blocks_per_sm();
 // (g / 4)^2 row groups, 32 / min(8, g / 32) of them per warp.
 inline uint64_t morton_warps(uint64_t g) { return g < 32 ? 0 : (g / 4) * (g / 4) * (g < 256 ? g / 32 : 8) / 32; }
 
-// Resolve-unit bookkeeping of a solid job: rows per unit and units per job.
+// Resolve units of a solid job: words per unit, units per job.  A unit begins with a row on a word
+// that is a multiple of four, so that a warp can resolve it by itself with 16-byte accesses: a
+// multiple of the shortest such run of rows (gx / gcd(gx, 32) words, times 1, 2 or 4).  The longer
+// the unit, the less it spends on its set-up and the fewer warps there are: 512 words in a table of
+// 2^23 words or more (1024^3: 67 us; 72 us with 256, 84 us with 128), 256 in one of 2^20 or more
+// (512^3: 12 us; 14 us with 128 or 512), else 128, one step of a warp.
 struct SolidUnits {
-	uint64_t rows_per_unit;
+	uint32_t unit_words;
 	uint64_t units;
-	bool aligned;   // gx % 32 == 0: rows start on word boundaries
 };
 SolidUnits solid_units(const uint32_t grid[3]);
 

@@ -202,6 +202,7 @@ extern "C" cvx_status cvx_voxelize_solid_noalloc(const cvx_voxinfo* info, const 
 	}
 	job.flags = (morton ? JOB_MORTON : 0u) | JOB_SOLID | (needs_plain_loads(d_triangles) ? JOB_PLAIN_LOADS : 0u);
 	const SolidUnits su = solid_units(job.grid);
+	job.unit_words = su.unit_words;
 
 	LaunchDesc L{};
 	L.n_jobs = 1;

@@ -14,13 +14,15 @@
 //                       columns of triangles with at most `small_cols` columns are dealt over the
 //                       CTA, the other triangles queued.
 //   solid_cols          persistent; each warp takes items of up to kColsPerItem columns.
-//   solid_resolve       linear jobs: one thread per row run (whole rows; 16-byte words where rows
-//                       are aligned): prefix XOR along x, XORed into the linear table (every word
-//                       stored, for JOB_TABLE_OVERWRITE jobs), flip table cleared.
+//   solid_resolve       linear jobs: a warp per run of whole rows, 128 words at a time: prefix XOR
+//                       along x, XORed into the linear table (every word stored, for
+//                       JOB_TABLE_OVERWRITE jobs), flip table cleared.
 //   solid_morton_cols   Morton jobs with g >= 32: a warp resolves row groups of 4 x 4 rows along x and
 //                       converts them to Morton words in registers.
 //   solid_morton_small  Morton jobs with g < 32 (one word at a time), then solid_zero clears the
 //                       flip table.
+#include <algorithm>
+
 #include "engine.h"
 #include "morton_block.cuh"
 
@@ -473,15 +475,6 @@ __device__ __forceinline__ uint32_t prefix_xor_msb(uint32_t t) {
 	return t;
 }
 
-// Resolve one word: toggles t (MSB first) plus the parity carried in from the row's earlier words.
-__device__ __forceinline__ uint32_t resolve_word(uint32_t t, uint32_t& carry) {
-	const uint32_t res = prefix_xor_msb(t) ^ (carry ? 0xFFFFFFFFu : 0u);
-	carry = res & 1u;  // the row's parity after this word's last bit
-	return res;
-}
-
-// Linear jobs: table ^= resolved, toggles cleared.  Morton jobs (g < 32): toggles replaced by the
-// resolved bits for solid_morton_small to gather.
 // XOR a resolved word into the table (the reference's semantics: the caller's table is XORed), or
 // store it, zero or not, when the engine owns the table's content (JOB_TABLE_OVERWRITE).
 __device__ __forceinline__ void xor_out(uint32_t* dest, uint64_t w, uint32_t v, bool overwrite) {
@@ -489,90 +482,113 @@ __device__ __forceinline__ void xor_out(uint32_t* dest, uint64_t w, uint32_t v, 
 	else if (v) dest[w] ^= v;
 }
 
-__device__ __forceinline__ void resolve_store(uint32_t* flips, uint32_t* dest, uint64_t w, uint32_t t, uint32_t res,
-                                              bool morton, bool overwrite) {
-	if (morton) {
-		if (res != t) flips[w] = res;
-	} else {
-		xor_out(dest, w, res, overwrite);
-		if (t) flips[w] = 0u;
-	}
-}
-
-// One thread per resolve unit.  gx a multiple of 32: a unit is one row (whole words; 16-byte
-// loads when the row and both tables are 16-byte aligned).  Other gx: the shortest run of rows
-// that starts and ends on word boundaries, walked bit by bit (odd grid sizes only).
-__global__ void __launch_bounds__(256) solid_resolve(const __grid_constant__ LaunchDesc L) {
-	const uint32_t unit_id = blockIdx.x * blockDim.x + threadIdx.x;
+// Linear jobs: table ^= resolved bits, toggles cleared.  Morton jobs (g < 32): toggles replaced by
+// the resolved bits for solid_morton_small to gather.
+//
+// One warp per unit of unit_words words, which begins with a row; the warp takes 128 consecutive
+// words at a time, four per lane in one access.  A word's bits are the prefix XOR of its toggles,
+// started again at every row start inside it; the bits before its first row start also take the
+// parity carried in.  So a lane needs two bits of every lane before it -- its last bit, and whether a
+// row starts in it -- and two ballots give both.  The same code serves rows that begin on words and
+// rows that begin inside them.  Bound by memory: the flip table is read, the table read and written.
+// Times here and of one thread per run of rows, which walked rows that begin inside words bit by bit:
+// 100^3 6 / 37 us, 500^3 16 / 188 us, 512^3 12 / 12 us, 1024^3 66 / 82 us.
+__global__ void __launch_bounds__(256, 6) solid_resolve(const __grid_constant__ LaunchDesc L) {
+	const uint32_t unit_id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	if (unit_id >= L.n_units) return;
+	const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
 	const uint32_t j = job_search(L, unit_id, [](const JobDesc& d) { return (uint64_t)d.unit_begin; });
 	const JobDesc& J = job_at(L, j);
-	const uint64_t gx = J.grid[0];
-	const uint64_t rows = (uint64_t)J.grid[1] * J.grid[2];
+	const uint32_t gx = J.grid[0];
+	const uint64_t bits = (uint64_t)gx * J.grid[1] * J.grid[2];
 	const bool morton = (J.flags & JOB_MORTON) != 0;
-	const bool overwrite = (J.flags & JOB_TABLE_OVERWRITE) != 0 && !morton;  // Morton words: written below
+	const bool overwrite = (J.flags & JOB_TABLE_OVERWRITE) != 0 || morton;
 	uint32_t* flips = J.flips;
-	uint32_t* dest = J.table;
-	const uint64_t u = unit_id - J.unit_begin;
-	if (gx % 32 == 0) {
-		const uint32_t wpr = (uint32_t)(gx >> 5);
-		const uint64_t w0 = u * wpr;
-		uint32_t carry = 0;
-		const bool vec = (wpr & 3u) == 0 && ((reinterpret_cast<uintptr_t>(flips + w0) | reinterpret_cast<uintptr_t>(dest + w0)) & 15u) == 0;
-		if (vec) {
-			for (uint32_t i = 0; i < wpr; i += 4) {
-				const uint4 t = *reinterpret_cast<const uint4*>(flips + w0 + i);
-				if ((t.x | t.y | t.z | t.w) == 0u && carry == 0u) {  // outside the solid
-					if (overwrite) *reinterpret_cast<uint4*>(dest + w0 + i) = make_uint4(0u, 0u, 0u, 0u);
-					continue;
+	uint32_t* dest = morton ? flips : J.table;
+	const bool vec = ((reinterpret_cast<uintptr_t>(flips) | reinterpret_cast<uintptr_t>(dest)) & 15u) == 0;
+	const uint64_t w0 = (uint64_t)(unit_id - J.unit_begin) * J.unit_words;
+	const uint64_t w1 = umin64((bits + 31) >> 5, w0 + J.unit_words);
+	const bool quad = gx % 128u == 0;
+	const uint32_t step = 4096u % gx;         // bits of a warp's words, past whole rows
+	uint32_t pos = (lane * 128u) % gx;        // position in its row of the lane's first bit
+	uint32_t carry = 0;                       // parity of the row before the warp's words
+	auto load = [&](uint64_t w) {
+		if (vec && w + 4 <= w1) return *reinterpret_cast<const uint4*>(flips + w);
+		return make_uint4(w < w1 ? flips[w] : 0u, w + 1 < w1 ? flips[w + 1] : 0u, w + 2 < w1 ? flips[w + 2] : 0u,
+		                  w + 3 < w1 ? flips[w + 3] : 0u);
+	};
+	uint4 next = load(w0 + lane * 4u);
+	for (uint64_t wc = w0; wc < w1; wc += 128) {
+		const uint64_t w = wc + lane * 4u;
+		const uint4 t4 = next;
+		if (wc + 128 < w1) next = load(w + 128);
+		const uint32_t t[4] = {t4.x, t4.y, t4.z, t4.w};
+		uint32_t r[4] = {0u, 0u, 0u, 0u};
+		const bool toggles = (t[0] | t[1] | t[2] | t[3]) != 0u;
+		uint32_t p = pos;
+		pos += step;
+		if (pos >= gx) pos -= gx;
+		if (carry || __any_sync(FULL, toggles)) {
+			uint32_t in[4];       // the bits that the parity carried into the lane reaches
+			uint32_t last = 0;    // the lane's last bit, for an even parity carried in
+			bool starts = false;  // a row starts in the lane's words
+			if (quad) {           // rows of whole 16-byte groups: a row starts with the lane's words or not at all
+				starts = p == 0u;
+#pragma unroll
+				for (int k = 0; k < 4; k++) {
+					r[k] = prefix_xor_msb(t[k]) ^ (0u - last);
+					last = r[k] & 1u;
+					in[k] = starts ? 0u : 0xFFFFFFFFu;
 				}
-				const uint32_t r0 = resolve_word(t.x, carry), r1 = resolve_word(t.y, carry);
-				const uint32_t r2 = resolve_word(t.z, carry), r3 = resolve_word(t.w, carry);
-				if (morton) {
-					*reinterpret_cast<uint4*>(flips + w0 + i) = make_uint4(r0, r1, r2, r3);
-				} else if (overwrite) {
-					*reinterpret_cast<uint4*>(dest + w0 + i) = make_uint4(r0, r1, r2, r3);
-					if (t.x | t.y | t.z | t.w) *reinterpret_cast<uint4*>(flips + w0 + i) = make_uint4(0u, 0u, 0u, 0u);
-				} else {
-					uint4 d = *reinterpret_cast<const uint4*>(dest + w0 + i);
-					d.x ^= r0; d.y ^= r1; d.z ^= r2; d.w ^= r3;
-					*reinterpret_cast<uint4*>(dest + w0 + i) = d;
-					if (t.x | t.y | t.z | t.w) *reinterpret_cast<uint4*>(flips + w0 + i) = make_uint4(0u, 0u, 0u, 0u);
+			} else {
+#pragma unroll
+				for (int k = 0; k < 4; k++) {
+					r[k] = prefix_xor_msb(t[k]);
+					uint32_t m = 0xFFFFFFFFu;  // the bits before the word's first row start
+					const uint32_t o0 = p ? gx - p : 0u;
+					if (o0 < 32u) {
+						m = ~(0xFFFFFFFFu >> o0);
+						for (uint32_t o = o0; o < 32u; o += gx)
+							if (o && ((r[k] >> (32u - o)) & 1u)) r[k] ^= 0xFFFFFFFFu >> o;
+					}
+					r[k] ^= last ? m : 0u;
+					last = r[k] & 1u;
+					in[k] = starts ? 0u : m;
+					starts = starts || o0 < 32u;
+					p += 32u;
+					while (p >= gx) p -= gx;
 				}
 			}
-		} else {
-			for (uint32_t i = 0; i < wpr; i++) {
-				const uint32_t t = flips[w0 + i];
-				if (t == 0u && carry == 0u) {
-					if (overwrite) dest[w0 + i] = 0u;
-					continue;
-				}
-				resolve_store(flips, dest, w0 + i, t, resolve_word(t, carry), morton, overwrite);
+			const uint32_t lasts = __ballot_sync(FULL, last != 0u), rows = __ballot_sync(FULL, starts);
+			// parity at the end of the lanes in `from`: their last bits, back to the last row start
+			auto parity = [&](uint32_t from) {
+				const uint32_t s = rows & from;
+				return s ? __popc(lasts & from & (0xFFFFFFFFu << (31 - __clz(s)))) & 1u : (__popc(lasts & from) & 1u) ^ carry;
+			};
+			const uint32_t c = parity(below);
+			carry = parity(FULL);
+			if (c) {
+#pragma unroll
+				for (int k = 0; k < 4; k++) r[k] ^= in[k];
 			}
 		}
-	} else {
-		const uint64_t g = gx;
-		uint64_t a = g, bb = 32;
-		while (bb) { const uint64_t r = a % bb; a = bb; bb = r; }
-		const uint64_t p = 32 / a;  // rows per unit: lcm(gx, 32) / gx
-		const uint64_t r0 = u * p, r1 = umin64(rows, r0 + p);
-		const uint64_t b0 = r0 * g, b1 = r1 * g;
-		uint32_t carry = 0;
-		uint64_t next_row = b0;  // bit index of the next row start
-		for (uint64_t w = b0 >> 5; (w << 5) < b1; w++) {
-			const uint32_t t = flips[w];
-			uint32_t res = 0;
-			for (uint32_t k = 0; k < 32; k++) {
-				const uint64_t bit = (w << 5) + k;
-				if (bit >= b1) break;
-				if (bit == next_row) {
-					carry = 0;
-					next_row += g;
+		const uint32_t any = r[0] | r[1] | r[2] | r[3];
+		if (vec && w + 4 <= w1) {
+			if (overwrite || any) {
+				if (!overwrite) {
+					const uint4 d = *reinterpret_cast<const uint4*>(dest + w);
+					r[0] ^= d.x; r[1] ^= d.y; r[2] ^= d.z; r[3] ^= d.w;
 				}
-				carry ^= (t >> (31 - k)) & 1u;
-				res |= carry << (31 - k);
+				*reinterpret_cast<uint4*>(dest + w) = make_uint4(r[0], r[1], r[2], r[3]);
 			}
-			resolve_store(flips, dest, w, t, res, morton, overwrite);
+			if (toggles && !morton) *reinterpret_cast<uint4*>(flips + w) = make_uint4(0u, 0u, 0u, 0u);
+		} else {
+#pragma unroll
+			for (int k = 0; k < 4; k++)
+				if (w + k < w1) {
+					xor_out(dest, w + k, r[k], overwrite);
+					if (t[k] && !morton) flips[w + k] = 0u;
+				}
 		}
 	}
 }
@@ -688,39 +704,31 @@ __global__ void __launch_bounds__(256) solid_morton_small(const __grid_constant_
 	xor_out(J.table, m, out, (J.flags & JOB_TABLE_OVERWRITE) != 0);
 }
 
-// Morton jobs with g < 32: clear the resolved flip table, one thread per resolve unit
+// Morton jobs with g < 32: clear the resolved flip table, one warp per resolve unit
 // (solid_morton_cols clears its own words).
 __global__ void __launch_bounds__(256) solid_zero(const __grid_constant__ LaunchDesc L) {
-	const uint32_t unit_id = blockIdx.x * blockDim.x + threadIdx.x;
+	const uint32_t unit_id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	if (unit_id >= L.n_units) return;
 	const uint32_t j = job_search(L, unit_id, [](const JobDesc& d) { return (uint64_t)d.unit_begin; });
 	const JobDesc& J = job_at(L, j);
 	if (!(J.flags & JOB_MORTON)) return;
-	const uint64_t gx = J.grid[0];
-	const uint64_t rows = (uint64_t)J.grid[1] * J.grid[2];
-	uint64_t a = gx, bb = 32;
-	while (bb) { const uint64_t r = a % bb; a = bb; bb = r; }
-	const uint64_t p = (gx % 32 == 0) ? 1 : 32 / a;
-	const uint64_t u = unit_id - J.unit_begin;
-	const uint64_t r0 = u * p, r1 = umin64(rows, r0 + p);
-	for (uint64_t w = (r0 * gx) >> 5; w < ((r1 * gx + 31) >> 5); w++) J.flips[w] = 0u;
+	const uint64_t words = ((uint64_t)J.grid[0] * J.grid[1] * J.grid[2] + 31) >> 5;
+	const uint64_t w0 = (uint64_t)(unit_id - J.unit_begin) * J.unit_words, w1 = umin64(words, w0 + J.unit_words);
+	for (uint64_t w = w0 + (threadIdx.x & 31u); w < w1; w += 32) J.flips[w] = 0u;
 }
 
 }  // namespace
 
 SolidUnits solid_units(const uint32_t grid[3]) {
-	const uint64_t gx = grid[0];
-	const uint64_t rows = (uint64_t)grid[1] * grid[2];
+	const uint64_t words = ((uint64_t)grid[0] * grid[1] * grid[2] + 31) / 32;
+	uint32_t a = grid[0], b = 32;
+	while (b) { const uint32_t r = a % b; a = b; b = r; }
+	uint32_t run = grid[0] / a;  // words of the shortest run of rows that begins and ends on words
+	run *= run % 4 == 0 ? 1 : (run % 2 == 0 ? 2 : 4);
+	const uint32_t target = words >= (1u << 23) ? 512 : (words >= (1u << 20) ? 256 : 128);
 	SolidUnits s;
-	s.aligned = gx % 32 == 0;
-	if (s.aligned) {
-		s.rows_per_unit = 1;  // one row per resolve thread
-	} else {
-		uint64_t a = gx, b = 32;
-		while (b) { uint64_t r = a % b; a = b; b = r; }
-		s.rows_per_unit = 32 / a;
-	}
-	s.units = (rows + s.rows_per_unit - 1) / s.rows_per_unit;
+	s.unit_words = run * std::max(1u, target / run);
+	s.units = (words + s.unit_words - 1) / s.unit_words;
 	return s;
 }
 
@@ -738,7 +746,7 @@ static cudaError_t launch_solid_t(const LaunchDesc& L, const Tune& tune, int col
 	}
 	if (phases & kSolidResolve) {
 		if (L.n_units) {
-			if ((e = launch_k(solid_resolve, (L.n_units + 255) / 256, 256, 0, s, L)) != cudaSuccess) return e;
+			if ((e = launch_k(solid_resolve, (L.n_units + 7) / 8, 256, 0, s, L)) != cudaSuccess) return e;
 			if (prof) (*prof)("solid_resolve", s);
 		}
 		if (L.n_mwarps) {
@@ -748,7 +756,7 @@ static cudaError_t launch_solid_t(const LaunchDesc& L, const Tune& tune, int col
 		if (L.n_mwords) {
 			if ((e = launch_k(solid_morton_small, (unsigned)((L.n_mwords + 255) / 256), 256, 0, s, L)) != cudaSuccess)
 				return e;
-			if ((e = launch_k(solid_zero, (L.n_units + 255) / 256, 256, 0, s, L)) != cudaSuccess) return e;
+			if ((e = launch_k(solid_zero, (L.n_units + 7) / 8, 256, 0, s, L)) != cudaSuccess) return e;
 			if (prof) (*prof)("solid_morton_small", s);
 		}
 	}

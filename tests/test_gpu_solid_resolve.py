@@ -108,3 +108,16 @@ def test_morton_2048_beyond_one_kilovoxel_axis():
             word = int(lin[bit >> 5].item()) & 0xFFFFFFFF
             inside = sum(bool(np.all(p >= a) and np.all(p < b)) for a, b in boxes)
             assert (word >> (31 - (bit & 31))) & 1 == inside & 1
+
+
+@pytest.mark.parametrize("plan", [False, True])
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("grid", [
+    (1, 40, 30), (3, 33, 65), (7, 50, 41), (31, 64, 64),        # several rows per word
+    (32, 40, 24), (64, 96, 80), (96, 20, 50), (160, 33, 9),     # rows on word boundaries
+    (33, 64, 64), (100, 100, 100), (250, 31, 77), (500, 40, 41),  # rows that begin inside words
+    (4096, 9, 7), (5000, 5, 6), (4100, 7, 5),                   # rows longer than a warp's words
+    (500, 300, 240),                                            # a table with long units
+])
+def test_linear(grid, offset, plan):
+    _run(grid, False, offset, plan, sum(grid) + offset)
