@@ -15,7 +15,9 @@ constexpr uint32_t kColsPerItem = 256; // solid columns per work item
 constexpr uint32_t kSmallRows = 16;    // surface: rows of a small triangle (every voxel tested)
 constexpr uint32_t kLocalRows = 64;    // surface: rows of a local triangle (row intervals), classify kernel
 constexpr uint32_t kMaskRowVoxels = 16; // surface: local rows up to this long test every voxel (the pass mask holds 16)
-constexpr uint32_t kSmallCols = 16;    // solid: columns of a triangle handled in the classify kernel
+constexpr uint32_t kSmallCols = 16;    // solid: largest small_cols
+constexpr uint32_t kColsPerSmall = 8;  // solid: columns a triangle may have in the classify kernel, per small_cols
+constexpr uint32_t kWarpCols = 448;    // solid: columns of a classify warp that are no longer few, in a small launch
 
 // Device-side check codes written to Counters::error.
 enum : unsigned { kErrBulkTimeout = 1u, kErrQueueOverflow = 2u };
@@ -31,7 +33,7 @@ constexpr uint32_t kMaxBrickPairs = 16;
 
 struct Tune {
 	uint32_t small_vox = 64;    // surface: bbox voxels at or below which a triangle stays in its thread
-	uint32_t small_cols = kSmallCols;  // solid: columns at or below which a triangle stays in the classify kernel
+	uint32_t small_cols = kSmallCols;  // solid: a triangle of up to kColsPerSmall times as many columns stays in the classify kernel
 	// pairs per triangle the brick rasterizer may use; 0 (the default: on the 1024^3 stress soup the
 	// brick path measured about 25% slower than the row path) rasterizes every larger triangle by rows
 	uint32_t brick_pairs = 0;

@@ -10,9 +10,8 @@
 // any set of [0, xmax] ranges is exactly what this produces.
 //
 // Kernels, in launch order:
-//   solid_classify      one CTA per kTile-triangle tile (TMA bulk staging as in surface.cu); the
-//                       columns of triangles with at most `small_cols` columns are dealt over the
-//                       CTA, the other triangles queued.
+//   solid_classify      a warp per 32 triangles (staged by a bulk copy); the columns of the triangles
+//                       with few columns are dealt over the warp, the other triangles queued.
 //   solid_cols          persistent; each warp takes items of up to kColsPerItem columns.
 //   solid_resolve       linear jobs: a warp per run of whole rows, 128 words at a time: prefix XOR
 //                       along x, XORed into the linear table (every word stored, for
@@ -200,20 +199,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
 	return false;
 }
 
-// Stage `cnt` triangles (9 floats each) from global memory into shared memory.  A full, aligned
-// tile of plain device memory goes through one bulk copy completing on an mbarrier; anything else
-// (a partial or unaligned tile, managed or host memory: `plain`) is loaded cooperatively.
-// Returns false (in every thread) if the bulk copy did not complete within the bounded wait: the
-// error word is set, the CTA waits once more (again bounded) for the copy still in flight, and the
-// caller skips the tile without touching the shared memory the copy may still write.
-__device__ __forceinline__ bool stage_tile(const LaunchDesc& L, const float* src, uint32_t cnt, float* s_tri,
+// Stage a warp's `cnt` triangles (9 floats each) from global memory into shared memory.  32 aligned
+// triangles of plain device memory go through one bulk copy completing on the warp's own mbarrier;
+// anything else (a partial or unaligned group, managed or host memory: `plain`) is loaded by the
+// lanes.  Returns false (in every lane) if the bulk copy did not complete within the bounded wait: the
+// error word is set, the warp waits once more (again bounded) for the copy still in flight, and the
+// caller skips the triangles without touching the shared memory the copy may still write.
+__device__ __forceinline__ bool stage_warp(const LaunchDesc& L, const float* src, uint32_t cnt, float* s_tri,
                                            uint64_t* s_bar, bool plain) {
+	const uint32_t lane = threadIdx.x & 31u;
 	const uint32_t bytes = cnt * 36u;
-	const bool bulk = cnt == kTile && ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) && !plain;
+	const bool bulk = cnt == 32u && ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) && !plain;
 	if (bulk) {
 		const uint32_t bar = (uint32_t)__cvta_generic_to_shared(s_bar);
 		const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_tri);
-		if (threadIdx.x == 0) {
+		if (lane == 0) {
 			asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
 			asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 			asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -221,66 +221,52 @@ __device__ __forceinline__ bool stage_tile(const LaunchDesc& L, const float* src
 			             "l"(src), "r"(bytes), "r"(bar)
 			             : "memory");
 		}
-		__syncthreads();  // barrier initialised before anyone waits on it
+		__syncwarp();  // barrier initialised before anyone waits on it
 		const bool late = !mbar_wait(bar, 0);
-		if (__syncthreads_or(late)) {
-			if (threadIdx.x == 0) set_error(L, kErrBulkTimeout);
+		if (__any_sync(FULL, late)) {
+			if (lane == 0) set_error(L, kErrBulkTimeout);
 			mbar_wait(bar, 0);
 			return false;
 		}
 		return true;
 	}
-	for (uint32_t i = threadIdx.x; i < cnt * 9u; i += blockDim.x) s_tri[i] = src[i];
-	__syncthreads();
+	for (uint32_t i = lane; i < cnt * 9u; i += 32) s_tri[i] = src[i];
+	__syncwarp();
 	return true;
 }
 
-// A small triangle's solid setup parked in shared memory between the classify phases.  15 words
+// A small triangle's solid setup parked in shared memory between the classify phases.  16 words
 // padded to 20: records stay 16-byte aligned for vector access, and the 8 lanes of a quarter warp
 // touching 8 records start on banks 0, 20, 8, 28, 16, 4, 24, 12 -- no conflicts (at 16 words, 4-way).
 struct __align__(16) SmallSolid {
 	float nx, ny, nz, v0x, v0y, v0z, ax, ay, bx, by, cx, cy;
 	int y0, z0;
-	uint32_t ext;  // (y1 - y0) | (z1 - z0) << 16
-	uint32_t pad[5];
+	uint32_t nzc;    // columns along z
+	uint32_t start;  // columns of the warp's triangles before this one
+	uint32_t pad[4];
 };
 static_assert(sizeof(SmallSolid) == 80, "SmallSolid stride");
 
-__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_warp, uint32_t* total) {
-	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-	uint32_t incl = v;
-#pragma unroll
-	for (int d = 1; d < 32; d <<= 1) {
-		const uint32_t u = __shfl_up_sync(FULL, incl, d);
-		if (lane >= (uint32_t)d) incl += u;
-	}
-	if (lane == 31) s_warp[warp] = incl;
-	__syncthreads();
-	if (warp == 0) {
-		uint32_t w = lane < kTile / 32 ? s_warp[lane] : 0u;
-#pragma unroll
-		for (int d = 1; d < 32; d <<= 1) {
-			const uint32_t u = __shfl_up_sync(FULL, w, d);
-			if (lane >= (uint32_t)d) w += u;
-		}
-		if (lane < kTile / 32) s_warp[lane] = w;
-	}
-	__syncthreads();
-	*total = s_warp[kTile / 32 - 1];
-	return (warp ? s_warp[warp - 1] : 0u) + incl - v;
-}
-
-// Phase 1: one thread per triangle (setup, classify, queue the big ones, park the small ones).
-// Phase 2: the columns of all small triangles of the tile, one (triangle, column) item per thread.
+// Four independent warps per CTA, 32 triangles each; nothing waits on a CTA barrier.  Phase 1: one
+// lane per triangle: setup, then the triangles of up to kColsPerSmall * small_cols columns park it in
+// the warp's shared memory, packed, and the larger ones are queued for solid_cols.  Phase 2: the
+// parked triangles' columns, 32 at a time, one per lane: a lane finds its triangle by counting the
+// triangles that start at or before its column (one warp-wide OR of start bits and a population
+// count), so no list of columns is written.
+// Bound by instructions on large meshes, by latency on small ones.  A triangle that stays costs its
+// columns; one that is queued costs solid_cols a chain of dependent loads and a second setup.  Times
+// of solid_classify + solid_cols, triangles of up to 128 / up to 16 columns staying, in us:
+//   icosphere 8 at 1024^3 77 + 12 / 150 + 81, 6 at 500^3 28 + 13 / 17 + 36 (10,240 and 640 CTAs);
+//   14,400-triangle torus at 512^3 61 + 11 / 12 + 20 (113 CTAs: a few long warps, hence kWarpCols).
+// With item lists dealt over the CTA and 16 columns the same meshes took 150 + 76, 18 + 36, 12 + 21.
 template <class P>
-__global__ void __launch_bounds__(kTile) solid_classify(const __grid_constant__ LaunchDesc L, const uint32_t small_cols) {
+__global__ void __launch_bounds__(kTile, 12) solid_classify(const __grid_constant__ LaunchDesc L, const uint32_t small_cols,
+                                                              const uint32_t warp_cols) {
 	__shared__ __align__(16) union {
-		float tri[kTile * 9];
-		SmallSolid small[kTile];
-	} sm;
-	__shared__ uint32_t s_items[kTile * kSmallCols];  // (triangle | dy << 8 | dz << 16) per column
-	__shared__ uint32_t s_warp[kTile / 32];
-	__shared__ __align__(8) uint64_t s_bar;
+		float tri[32 * 9];
+		SmallSolid small[32];
+	} s_warp[kTile / 32];
+	__shared__ __align__(8) uint64_t s_bar[kTile / 32];
 	const uint32_t tile = blockIdx.x;
 	const uint32_t j = job_of_tile(L, tile);
 	const JobDesc& J = job_at(L, j);
@@ -291,38 +277,35 @@ __global__ void __launch_bounds__(kTile) solid_classify(const __grid_constant__ 
 	const float inv[3] = {J.inv_unit[0], J.inv_unit[1], J.inv_unit[2]};
 	const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
 	uint32_t* flips = J.flips;
-	const uint64_t t0 = (uint64_t)(tile - J.tile_begin) * kTile;
-	const uint32_t cnt = (uint32_t)umin64((uint64_t)kTile, n - t0);
-	if (!stage_tile(L, J.tris + t0 * 9, cnt, sm.tri, &s_bar, (J.flags & JOB_PLAIN_LOADS) != 0)) return;  // tile not staged: error word set
+	const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+	const uint64_t t0 = (uint64_t)(tile - J.tile_begin) * kTile + wid * 32u;
+	if (t0 >= n) return;
+	auto& sm = s_warp[wid];
+	const uint32_t cnt = (uint32_t)umin64(32u, n - t0);
+	if (!stage_warp(L, J.tris + t0 * 9, cnt, sm.tri, &s_bar[wid], (J.flags & JOB_PLAIN_LOADS) != 0)) return;  // error word set
 
-	const uint32_t lane = threadIdx.x & 31u;
-	const bool valid = threadIdx.x < cnt;
+	const bool valid = lane < cnt;
 	float t[9];
 #pragma unroll
-	for (int k = 0; k < 9; k++) t[k] = valid ? sm.tri[threadIdx.x * 9 + k] : 0.0f;
-	__syncthreads();
+	for (int k = 0; k < 9; k++) t[k] = valid ? sm.tri[lane * 9 + k] : 0.0f;
+	__syncwarp();  // the triangles are consumed; the shared memory now holds records
 
+	SolidTri S;
 	bool is_mid = false, is_big = false;
 	uint32_t n_items = 0, n_cols = 0;
+	uint64_t ncols = 0;
 	if (valid) {
-		SolidTri S;
 		solid_setup<P>(t, bmin, unit, inv, grid, S);
-		if (!S.skip && S.y0 <= S.y1 && S.z0 <= S.z1) {
-			const uint64_t ncols = (uint64_t)(S.y1 - S.y0 + 1) * (uint64_t)(S.z1 - S.z0 + 1);
-			if (ncols <= small_cols && ncols <= kSmallCols) {
-				SmallSolid& o = sm.small[threadIdx.x];
-				o.nx = S.nx; o.ny = S.ny; o.nz = S.nz; o.v0x = S.v0x; o.v0y = S.v0y; o.v0z = S.v0z;
-				o.ax = S.ax; o.ay = S.ay; o.bx = S.bx; o.by = S.by; o.cx = S.cx; o.cy = S.cy;
-				o.y0 = S.y0; o.z0 = S.z0;
-				o.ext = (uint32_t)(S.y1 - S.y0) | ((uint32_t)(S.z1 - S.z0) << 16);
-				n_cols = (uint32_t)ncols;
-			} else {
-				const uint64_t it = (ncols + kColsPerItem - 1) / kColsPerItem;
-				n_items = (uint32_t)umin64(it, 0xFFFFFFu);
-				is_mid = n_items == 1;
-				is_big = n_items > 1;
-			}
-		}
+		if (!S.skip && S.y0 <= S.y1 && S.z0 <= S.z1)
+			ncols = (uint64_t)(S.y1 - S.y0 + 1) * (uint64_t)(S.z1 - S.z0 + 1);
+	}
+	if (ncols <= kColsPerSmall * small_cols) n_cols = (uint32_t)ncols;
+	if (__reduce_add_sync(FULL, n_cols) > warp_cols && n_cols > small_cols) n_cols = 0;
+	if (ncols > n_cols) {
+		const uint64_t it = (ncols + kColsPerItem - 1) / kColsPerItem;
+		n_items = (uint32_t)umin64(it, 0xFFFFFFu);
+		is_mid = n_items == 1;
+		is_big = n_items > 1;
 	}
 	const uint32_t lt = (1u << lane) - 1u;
 	const uint32_t mid_ballot = __ballot_sync(FULL, is_mid);
@@ -333,7 +316,7 @@ __global__ void __launch_bounds__(kTile) solid_classify(const __grid_constant__ 
 		base = __shfl_sync(FULL, base, leader);
 		const uint32_t slot = base + __popc(mid_ballot & lt);
 		if (is_mid) {
-			if (slot < L.scr.cap) L.scr.mid[slot] = MidRec{j, (uint32_t)(t0 + threadIdx.x)};
+			if (slot < L.scr.cap) L.scr.mid[slot] = MidRec{j, (uint32_t)(t0 + lane)};
 			else set_error(L, kErrQueueOverflow);
 		}
 	}
@@ -354,32 +337,50 @@ __global__ void __launch_bounds__(kTile) solid_classify(const __grid_constant__ 
 			const uint32_t rec = (uint32_t)(old >> kBigShift) + __popc(big_ballot & lt);
 			const uint64_t first = (old & kBigItemMask) + incl - n_items;
 			if (rec < L.scr.cap && first + n_items <= kBigItemMask)
-				L.scr.big[rec] = BigRec{first, j, (uint32_t)(t0 + threadIdx.x), n_items, 0u};
+				L.scr.big[rec] = BigRec{first, j, (uint32_t)(t0 + lane), n_items, 0u};
 			else
 				set_error(L, kErrQueueOverflow);
 		}
 	}
 
 	// Phase 2: columns of the small triangles (src/voxelize_solid.cu:115-139).
-	uint32_t total_cols = 0;
-	const uint32_t off = block_scan(n_cols, s_warp, &total_cols);
-	if (n_cols) {
-		const uint32_t ext = sm.small[threadIdx.x].ext;
-		const uint32_t nyc = (ext & 0xFFFFu) + 1u, nzc = (ext >> 16) + 1u;
-		uint32_t c = off;
-		for (uint32_t dy = 0; dy < nyc; dy++)
-			for (uint32_t dz = 0; dz < nzc; dz++) s_items[c++] = threadIdx.x | (dy << 8) | (dz << 16);
+	uint32_t incl = n_cols;
+#pragma unroll
+	for (int d = 1; d < 32; d <<= 1) {
+		const uint32_t v = __shfl_up_sync(FULL, incl, d);
+		if (lane >= (uint32_t)d) incl += v;
 	}
-	__syncthreads();
-	for (uint32_t k = threadIdx.x; k < total_cols; k += kTile) {
-		const uint32_t it = s_items[k];
-		const SmallSolid& o = sm.small[it & 0xFFu];
-		SolidTri S;
-		S.nx = o.nx; S.ny = o.ny; S.nz = o.nz; S.v0x = o.v0x; S.v0y = o.v0y; S.v0z = o.v0z;
-		S.ax = o.ax; S.ay = o.ay; S.bx = o.bx; S.by = o.by; S.cx = o.cx; S.cy = o.cy;
-		const int y = o.y0 + (int)((it >> 8) & 0xFFu), z = o.z0 + (int)(it >> 16);
+	const uint32_t total = __shfl_sync(FULL, incl, 31);
+	const uint32_t start = incl - n_cols;
+	const uint32_t parked = __ballot_sync(FULL, n_cols != 0u);
+	if (n_cols) {
+		SmallSolid& o = sm.small[__popc(parked & lt)];
+		o.nx = S.nx; o.ny = S.ny; o.nz = S.nz; o.v0x = S.v0x; o.v0y = S.v0y; o.v0z = S.v0z;
+		o.ax = S.ax; o.ay = S.ay; o.bx = S.bx; o.by = S.by; o.cx = S.cx; o.cy = S.cy;
+		o.y0 = S.y0; o.z0 = S.z0;
+		o.nzc = (uint32_t)(S.z1 - S.z0 + 1);
+		o.start = start;
+	}
+	__syncwarp();
+	uint32_t begun = 0;  // triangles that start before this step's columns
+	for (uint32_t base = 0; base < total; base += 32) {
+		const uint32_t at = start - base;
+		const uint32_t starts = __reduce_or_sync(FULL, n_cols && at < 32u ? 1u << at : 0u);
+		const uint32_t rec = begun + __popc(starts & (0xFFFFFFFFu >> (31u - lane))) - 1u;
+		begun += __popc(starts);
+		const uint32_t k = base + lane;
+		if (k >= total) break;
+		const SmallSolid& o = sm.small[rec];
+		SolidTri T;
+		T.nx = o.nx; T.ny = o.ny; T.nz = o.nz; T.v0x = o.v0x; T.v0y = o.v0y; T.v0z = o.v0z;
+		T.ax = o.ax; T.ay = o.ay; T.bx = o.bx; T.by = o.by; T.cx = o.cx; T.cy = o.cy;
+		// column c = dz + dy * nzc, c and nzc at most kColsPerSmall * kSmallCols = 128: the approximate
+		// quotient is more than 1e-3 away from the next integer and truncates exactly
+		const uint32_t c = k - o.start, nzc = o.nzc;
+		const uint32_t dy = (uint32_t)__fdividef((float)c + 0.5f, (float)nzc);
+		const int y = o.y0 + (int)dy, z = o.z0 + (int)(c - dy * nzc);
 		int xmax;
-		if (column_hit<P>(S, unit, y, z, morton, xmax)) record_hit(flips, grid, morton, y, z, xmax);
+		if (column_hit<P>(T, unit, y, z, morton, xmax)) record_hit(flips, grid, morton, y, z, xmax);
 	}
 }
 
@@ -738,7 +739,12 @@ static cudaError_t launch_solid_t(const LaunchDesc& L, const Tune& tune, int col
 	cudaError_t e = cudaSuccess;
 	if (prof) (*prof)(nullptr, s);
 	if ((phases & kSolidToggles) && L.n_tiles) {
-		solid_classify<P><<<L.n_tiles, kTile, 0, s>>>(L, tune.small_cols);
+		// As many classify CTAs as the persistent column grid has fill the chip: every triangle of up to
+		// kColsPerSmall * small_cols columns stays.  With fewer, the longest warp is the kernel's time, and
+		// a warp with more than kWarpCols columns leaves those above small_cols to solid_cols, which
+		// spreads them over the chip (both sides measured: solid_classify's comment).
+		const uint32_t warp_cols = L.n_tiles >= (uint32_t)cols_grid ? 0xFFFFFFFFu : kWarpCols;
+		solid_classify<P><<<L.n_tiles, kTile, 0, s>>>(L, std::min(tune.small_cols, kSmallCols), warp_cols);
 		if ((e = cudaGetLastError()) != cudaSuccess) return e;
 		if (prof) (*prof)("solid_classify", s);
 		if ((e = launch_k(solid_cols<P>, (unsigned)cols_grid, kRowsThreads, 0, s, L)) != cudaSuccess) return e;

@@ -277,7 +277,7 @@ cvx_status cvx_encode_voxel_list(const cvx_voxinfo* info, const uint32_t* d_tabl
 
 typedef struct cvx_tuning {
 	uint32_t small_vox;   /* surface: triangles with at most this many bbox voxels stay in one thread */
-	uint32_t small_cols;  /* solid: triangles with at most this many columns stay in one thread */
+	uint32_t small_cols;  /* solid: triangles with at most this many columns (in large launches, 8 times as many) stay in the classify kernel; at most 16 */
 	uint32_t brick_pairs; /* surface, grids of 2^29+ voxels: (brick, triangle) pairs per triangle the
 	                       * shared-memory brick rasterizer may use, at most 16; 0 (the default)
 	                       * rasterizes every larger triangle row by row with global atomics instead */

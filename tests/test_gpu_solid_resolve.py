@@ -121,3 +121,22 @@ def test_morton_2048_beyond_one_kilovoxel_axis():
 ])
 def test_linear(grid, offset, plan):
     _run(grid, False, offset, plan, sum(grid) + offset)
+
+
+@pytest.mark.parametrize("n_boxes", [1, 40, 700])  # x faces: a partial warp, a few tiles, a grid that fills the chip
+@pytest.mark.parametrize("extent", [1, 4, 5, 11, 12, 16, 17])  # columns: 1, 16 | 25, 121 | 144, 256 | 289
+def test_columns_per_triangle(n_boxes, extent):
+    """Column counts around each bin's edge (16 and 128 columns in the classify kernel, 256 per queued
+    item), in launches on both sides of the rule on the number of tiles."""
+    g = 96
+    rng = np.random.default_rng(extent)
+    n = n_boxes * (32 if n_boxes == 700 else 1)
+    lo = rng.integers(0, g - extent + 1, (n, 3))
+    size = np.stack([rng.integers(1, g, n), np.full(n, extent), np.full(n, extent)], 1)
+    boxes = [(a, np.minimum(a + s, g)) for a, s in zip(lo, size)]
+    tris = _mesh(boxes, (g, g, g))
+    info = cv.make_info((0, 0, 0), (float(g),) * 3, g, len(tris))
+    table = torch.zeros(cv.table_words(info), dtype=torch.int32, device="cuda")
+    cv.voxelize_solid(info, torch.from_numpy(tris.reshape(-1)).cuda(), table, False)
+    cv.device_status()
+    assert np.array_equal(table.cpu().numpy().view(np.uint32), _want(boxes, (g, g, g), False))
