@@ -20,7 +20,7 @@ LIB = os.path.join(OUT_DIR, "libcvx.so")
 DIAG_LIB = os.path.join(OUT_DIR, "libcvx_diag.so")  # include/cvx_diag.h: measurement helpers, not the ABI
 DIAG_SOURCES = ["microbench.cu"]
 SOURCES = ["surface.cu", "bricks.cu", "solid.cu", "api.cu", "dropin.cpp", "noalloc.cu", "server.cu", "clear.cu", "mesh.cu", "transcode.cu", "encode.cu"]
-HEADERS = ["cvx_device.cuh", "morton_block.cuh", "surface.cuh", "engine.h"]
+HEADERS = ["cvx_device.cuh", "morton_block.cuh", "stage.cuh", "surface.cuh", "engine.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 

@@ -12,9 +12,9 @@ constexpr uint32_t kTile = 128;        // triangles per classify CTA (one tile; 
 constexpr uint32_t kZch = 32;          // z-slices per surface work item (one per lane)
 constexpr uint32_t kRowsThreads = 256; // threads per cooperative CTA
 constexpr uint32_t kColsPerItem = 256; // solid columns per work item
-constexpr uint32_t kSmallRows = 16;    // surface: rows of a small triangle (every voxel tested)
-constexpr uint32_t kLocalRows = 64;    // surface: rows of a local triangle (row intervals), classify kernel
-constexpr uint32_t kMaskRowVoxels = 16; // surface: local rows up to this long test every voxel (the pass mask holds 16)
+constexpr uint32_t kLocalRows = 64;    // surface: rows a triangle may have in the classify kernel
+constexpr uint32_t kWarpRows = 384;    // surface: rows of a classify warp that are no longer few, in a small launch
+constexpr uint32_t kMaskRowVoxels = 16; // surface: and voxels per row, each of them tested (the pass mask holds 16)
 constexpr uint32_t kSmallCols = 16;    // solid: largest small_cols
 constexpr uint32_t kColsPerSmall = 8;  // solid: columns a triangle may have in the classify kernel, per small_cols
 constexpr uint32_t kWarpCols = 448;    // solid: columns of a classify warp that are no longer few, in a small launch

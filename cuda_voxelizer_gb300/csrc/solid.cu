@@ -24,12 +24,12 @@
 
 #include "engine.h"
 #include "morton_block.cuh"
+#include "stage.cuh"
 
 namespace cvx {
 
 namespace {
 
-constexpr unsigned FULL = 0xFFFFFFFFu;
 constexpr double kFloatError = 0.000001;  // src/voxelize_solid.cu:13 (a double literal)
 // For a float f, (double)f < 0.000001 exactly when f <= 0x1.0c6f7ap-20f, the largest float below the
 // double 1e-6 (floats are exact in double, and 0x1.0c6f7ap-20 < 1e-6 < its successor).
@@ -184,57 +184,6 @@ __device__ __forceinline__ void record_hit(uint32_t* flips, const uint32_t* grid
 	}
 }
 
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-	for (uint32_t it = 0; it < (1u << 24); it++) {
-		uint32_t ok;
-		asm volatile(
-		    "{\n\t.reg .pred p;\n\t"
-		    "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-		    "selp.u32 %0, 1, 0, p;\n\t}"
-		    : "=r"(ok)
-		    : "r"(bar), "r"(parity)
-		    : "memory");
-		if (ok) return true;
-	}
-	return false;
-}
-
-// Stage a warp's `cnt` triangles (9 floats each) from global memory into shared memory.  32 aligned
-// triangles of plain device memory go through one bulk copy completing on the warp's own mbarrier;
-// anything else (a partial or unaligned group, managed or host memory: `plain`) is loaded by the
-// lanes.  Returns false (in every lane) if the bulk copy did not complete within the bounded wait: the
-// error word is set, the warp waits once more (again bounded) for the copy still in flight, and the
-// caller skips the triangles without touching the shared memory the copy may still write.
-__device__ __forceinline__ bool stage_warp(const LaunchDesc& L, const float* src, uint32_t cnt, float* s_tri,
-                                           uint64_t* s_bar, bool plain) {
-	const uint32_t lane = threadIdx.x & 31u;
-	const uint32_t bytes = cnt * 36u;
-	const bool bulk = cnt == 32u && ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) && !plain;
-	if (bulk) {
-		const uint32_t bar = (uint32_t)__cvta_generic_to_shared(s_bar);
-		const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_tri);
-		if (lane == 0) {
-			asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-			asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-			asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-			asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-			             "l"(src), "r"(bytes), "r"(bar)
-			             : "memory");
-		}
-		__syncwarp();  // barrier initialised before anyone waits on it
-		const bool late = !mbar_wait(bar, 0);
-		if (__any_sync(FULL, late)) {
-			if (lane == 0) set_error(L, kErrBulkTimeout);
-			mbar_wait(bar, 0);
-			return false;
-		}
-		return true;
-	}
-	for (uint32_t i = lane; i < cnt * 9u; i += 32) s_tri[i] = src[i];
-	__syncwarp();
-	return true;
-}
-
 // A small triangle's solid setup parked in shared memory between the classify phases.  16 words
 // padded to 20: records stay 16-byte aligned for vector access, and the 8 lanes of a quarter warp
 // touching 8 records start on banks 0, 20, 8, 28, 16, 4, 24, 12 -- no conflicts (at 16 words, 4-way).
@@ -261,13 +210,13 @@ static_assert(sizeof(SmallSolid) == 80, "SmallSolid stride");
 // With item lists dealt over the CTA and 16 columns the same meshes took 150 + 76, 18 + 36, 12 + 21.
 template <class P>
 __global__ void __launch_bounds__(kTile, 12) solid_classify(const __grid_constant__ LaunchDesc L, const uint32_t small_cols,
-                                                              const uint32_t warp_cols) {
+                                                              const uint32_t warp_cols, const uint32_t split) {
 	__shared__ __align__(16) union {
 		float tri[32 * 9];
 		SmallSolid small[32];
 	} s_warp[kTile / 32];
 	__shared__ __align__(8) uint64_t s_bar[kTile / 32];
-	const uint32_t tile = blockIdx.x;
+	const uint32_t tile = blockIdx.x >> split;
 	const uint32_t j = job_of_tile(L, tile);
 	const JobDesc& J = job_at(L, j);
 	const uint64_t n = J.n_tri;
@@ -278,10 +227,11 @@ __global__ void __launch_bounds__(kTile, 12) solid_classify(const __grid_constan
 	const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
 	uint32_t* flips = J.flips;
 	const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-	const uint64_t t0 = (uint64_t)(tile - J.tile_begin) * kTile + wid * 32u;
+	const uint32_t part = (blockIdx.x - (tile << split)) * (kTile / 32) + wid;
+	const uint64_t t0 = (uint64_t)(tile - J.tile_begin) * kTile + part * (32u >> split);
 	if (t0 >= n) return;
 	auto& sm = s_warp[wid];
-	const uint32_t cnt = (uint32_t)umin64(32u, n - t0);
+	const uint32_t cnt = (uint32_t)umin64(32u >> split, n - t0);
 	if (!stage_warp(L, J.tris + t0 * 9, cnt, sm.tri, &s_bar[wid], (J.flags & JOB_PLAIN_LOADS) != 0)) return;  // error word set
 
 	const bool valid = lane < cnt;
@@ -744,7 +694,8 @@ static cudaError_t launch_solid_t(const LaunchDesc& L, const Tune& tune, int col
 		// a warp with more than kWarpCols columns leaves those above small_cols to solid_cols, which
 		// spreads them over the chip (both sides measured: solid_classify's comment).
 		const uint32_t warp_cols = L.n_tiles >= (uint32_t)cols_grid ? 0xFFFFFFFFu : kWarpCols;
-		solid_classify<P><<<L.n_tiles, kTile, 0, s>>>(L, std::min(tune.small_cols, kSmallCols), warp_cols);
+		const uint32_t split = classify_split(L.n_tiles, (uint32_t)cols_grid);
+		solid_classify<P><<<L.n_tiles << split, kTile, 0, s>>>(L, std::min(tune.small_cols, kSmallCols), warp_cols, split);
 		if ((e = cudaGetLastError()) != cudaSuccess) return e;
 		if (prof) (*prof)("solid_classify", s);
 		if ((e = launch_k(solid_cols<P>, (unsigned)cols_grid, kRowsThreads, 0, s, L)) != cudaSuccess) return e;

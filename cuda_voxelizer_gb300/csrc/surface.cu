@@ -2,14 +2,12 @@
 //
 // Two kernels per launch sequence, both over a job table so that one mesh and a batch of meshes
 // run through the same code:
-//   surf_classify  one CTA per tile of kTile triangles of one job.  The tile is staged into shared
-//                  memory with one cp.async.bulk (TMA bulk copy) when it is full and 16-byte
-//                  aligned.  Each thread sets up its triangle; triangles whose grid bbox holds at
-//                  most `small_vox` voxels (every voxel tested, like the reference) or at most
-//                  kLocalRows rows (rows of up to kMaskRowVoxels voxels tested voxel by voxel,
-//                  longer rows by row intervals) are finished by the CTA, their rows dealt over
-//                  its threads; the others are queued, one record per triangle, as one item
-//                  ("mid") or as one item per 32 z-slices ("big").
+//   surf_classify  a warp per 32 triangles of one job, staged into shared memory with one
+//                  cp.async.bulk (TMA bulk copy) when aligned.  Each lane sets up its triangle;
+//                  triangles of at most kLocalRows rows of at most kMaskRowVoxels voxels are finished
+//                  by the warp, their rows dealt over its lanes, every voxel tested like in the
+//                  reference; the others are queued, one record per triangle, as one item ("mid")
+//                  or as one item per 32 z-slices ("big").
 //   surf_rows      persistent CTAs of kRowsCtaThreads threads, seven per SM; each warp takes
 //                  work tickets (big items first, then mid triangles), finds the y-interval of every z-slice of the item (one lane per slice),
 //                  flattens the (y, z) rows and gives one row per lane; each lane finds the exact
@@ -17,171 +15,85 @@
 //                  warp for long rows).  Jobs whose indices fit 32 bits (JOB_NARROW) write with
 //                  32-bit index arithmetic.
 #include "engine.h"
+#include "stage.cuh"
 #include "surface.cuh"
 
 namespace cvx {
 
 namespace {
 
-constexpr unsigned FULL = 0xFFFFFFFFu;
-
-// Bounded wait on an mbarrier phase.  Returns false if the phase did not complete in time.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-	for (uint32_t it = 0; it < (1u << 24); it++) {
-		uint32_t ok;
-		asm volatile(
-		    "{\n\t.reg .pred p;\n\t"
-		    "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-		    "selp.u32 %0, 1, 0, p;\n\t}"
-		    : "=r"(ok)
-		    : "r"(bar), "r"(parity)
-		    : "memory");
-		if (ok) return true;
-	}
-	return false;
-}
-
-// Stage `cnt` triangles (9 floats each) from global memory into shared memory.  A full, aligned
-// tile of plain device memory goes through one bulk copy completing on an mbarrier; anything else
-// (a partial or unaligned tile, managed or host memory: `plain`) is loaded cooperatively.
-// Returns false (in every thread) if the bulk copy did not complete within the bounded wait: the
-// error word is set, the CTA waits once more (again bounded) for the copy still in flight, and the
-// caller skips the tile without touching the shared memory the copy may still write.
-__device__ __forceinline__ bool stage_tile(const LaunchDesc& L, const float* src, uint32_t cnt, float* s_tri,
-                                           uint64_t* s_bar, bool plain) {
-	const uint32_t bytes = cnt * 36u;
-	const bool bulk = cnt == kTile && ((reinterpret_cast<uintptr_t>(src) & 15u) == 0) && !plain;
-	if (bulk) {
-		const uint32_t bar = (uint32_t)__cvta_generic_to_shared(s_bar);
-		const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_tri);
-		if (threadIdx.x == 0) {
-			asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-			asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-			asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-			asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-			             "l"(src), "r"(bytes), "r"(bar)
-			             : "memory");
-		}
-		__syncthreads();  // barrier initialised before anyone waits on it
-		const bool late = !mbar_wait(bar, 0);
-		if (__syncthreads_or(late)) {
-			if (threadIdx.x == 0) set_error(L, kErrBulkTimeout);
-			mbar_wait(bar, 0);
-			return false;
-		}
-		return true;
-	}
-	for (uint32_t i = threadIdx.x; i < cnt * 9u; i += blockDim.x) s_tri[i] = src[i];
-	__syncthreads();
-	return true;
-}
-
-// Exclusive prefix sum over the CTA (kTile threads); returns this thread's offset, total in *total.
-__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_warp, uint32_t* total) {
-	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-	uint32_t incl = v;
-#pragma unroll
-	for (int d = 1; d < 32; d <<= 1) {
-		const uint32_t u = __shfl_up_sync(FULL, incl, d);
-		if (lane >= (uint32_t)d) incl += u;
-	}
-	if (lane == 31) s_warp[warp] = incl;
-	__syncthreads();
-	if (warp == 0) {
-		uint32_t w = lane < kTile / 32 ? s_warp[lane] : 0u;
-#pragma unroll
-		for (int d = 1; d < 32; d <<= 1) {
-			const uint32_t u = __shfl_up_sync(FULL, w, d);
-			if (lane >= (uint32_t)d) w += u;
-		}
-		if (lane < kTile / 32) s_warp[lane] = w;  // inclusive warp prefix
-	}
-	__syncthreads();
-	*total = s_warp[kTile / 32 - 1];
-	return (warp ? s_warp[warp - 1] : 0u) + incl - v;
-}
-
-// Phase 1: one thread per triangle: setup, then one of three bins.  Small triangles (a few voxels)
-// and local ones (at most kLocalRows rows, extents below 256) park their setup in shared memory;
-// the rest are queued for surf_rows.  Phase 2: the rows of the tile's small and local triangles
-// are dealt out evenly over the CTA, one (triangle, row) item per thread at a time, so that no
-// thread idles while another walks a larger bounding box.  A small triangle's row tests every
-// voxel like the reference; a local triangle's row is found with row_interval.
-// Registers (48) allow 10 CTAs of 128 threads per SM, shared memory (22.5 KB) 9.
+// Four independent warps per CTA, 32 triangles each (fewer in a launch with few tiles); nothing waits
+// on a CTA barrier.  Phase 1: one lane per triangle: setup, then the triangles of up to kLocalRows
+// rows of up to kMaskRowVoxels voxels park it in the warp's shared memory, packed, and the larger ones
+// are queued for surf_rows (or the brick kernels).  Phase 2: the parked triangles' rows, 32 at a time,
+// one per lane: a lane finds its triangle by counting the triangles that start at or before its row
+// (one warp-wide OR of start bits and a population count), and tests every voxel of its row.
+// Bound by instructions (82% of issue slots busy on the icosphere at 512^3, 50 per triangle).  There
+// 71 us; 90 us with the rows listed in shared memory and dealt over the CTA behind three barriers, the
+// tests combined with short-circuit branches (15% of all instructions) and the edge sums added up
+// before they are compared.  Nine CTAs per SM at 54 registers; ten at 48 are 1% slower.
+// Triangles with longer rows, or more, cost less in surf_rows, which shares one setup over a warp: with
+// up to 256 rows of any length kept here, the soup of 300,000 at 300^3 took 148 + 642 us in the two
+// kernels, 44 + 701 with this rule.
 template <class P>
-__global__ void __launch_bounds__(kTile, 10) surf_classify(const __grid_constant__ LaunchDesc L, const uint32_t small_vox) {
+__global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant__ LaunchDesc L, const uint32_t small_vox,
+                                                             const uint32_t warp_rows, const uint32_t split) {
 	__shared__ __align__(16) union {
-		float tri[kTile * 9];
-		SmallTri small[kTile];
-	} sm;
-	// per row: small triangle | dy << 8 | dz << 12, or local triangle | row << 8
-	__shared__ uint16_t s_items[kTile * kSmallRows];
-	__shared__ uint32_t s_warp[kTile / 32];
-	__shared__ uint32_t s_fit;  // end of the item list: the first local triangle that did not fit
-	__shared__ __align__(8) uint64_t s_bar;
-	const uint32_t tile = blockIdx.x;
+		float tri[32 * 9];
+		SmallTri small[32];
+	} s_warp[kTile / 32];
+	__shared__ __align__(8) uint64_t s_bar[kTile / 32];
+	const uint32_t tile = blockIdx.x >> split;
 	const uint32_t j = job_of_tile(L, tile);
 	const JobDesc& J = job_at(L, j);
-	const float* tris = J.tris;
-	uint32_t* table = J.table;
 	const uint64_t n = J.n_tri;
+	const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+	const uint32_t part = (blockIdx.x - (tile << split)) * (kTile / 32) + wid;
+	const uint64_t t0 = (uint64_t)(tile - J.tile_begin) * kTile + part * (32u >> split);
+	if (t0 >= n) return;
+	uint32_t* table = J.table;
 	const uint32_t jflags = J.flags;
-	const float bmin[3] = {J.bmin[0], J.bmin[1], J.bmin[2]};
 	const float unit[3] = {J.unit[0], J.unit[1], J.unit[2]};
-	const float inv[3] = {J.inv_unit[0], J.inv_unit[1], J.inv_unit[2]};
 	const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
-	const uint64_t t0 = (uint64_t)(tile - J.tile_begin) * kTile;
-	const uint32_t cnt = (uint32_t)umin64((uint64_t)kTile, n - t0);
-	if (!stage_tile(L, tris + t0 * 9, cnt, sm.tri, &s_bar, (jflags & JOB_PLAIN_LOADS) != 0)) return;  // tile not staged: error word set
+	auto& sm = s_warp[wid];
+	const uint32_t cnt = (uint32_t)umin64(32u >> split, n - t0);
+	if (!stage_warp(L, J.tris + t0 * 9, cnt, sm.tri, &s_bar[wid], (jflags & JOB_PLAIN_LOADS) != 0)) return;  // error word set
 
-	const uint32_t lane = threadIdx.x & 31u;
-	const bool valid = threadIdx.x < cnt;
+	const bool valid = lane < cnt;
 	float t[9];
 #pragma unroll
-	for (int k = 0; k < 9; k++) t[k] = valid ? sm.tri[threadIdx.x * 9 + k] : 0.0f;
-	__syncthreads();  // the tile is consumed; its shared memory now holds SmallTri records
+	for (int k = 0; k < 9; k++) t[k] = valid ? sm.tri[lane * 9 + k] : 0.0f;
+	__syncwarp();  // the triangles are consumed; the shared memory now holds records
 
-	bool is_mid = false, is_big = false;
-	uint32_t n_items = 0, n_small = 0, n_local = 0;
+	SurfTri S;
+	uint32_t n_items = 0, n_rows = 0;
+	bool few = false;
 	if (valid) {
-		SurfTri S;
+		const float bmin[3] = {J.bmin[0], J.bmin[1], J.bmin[2]};
+		const float inv[3] = {J.inv_unit[0], J.inv_unit[1], J.inv_unit[2]};
 		surf_setup<P>(t, bmin, unit, inv, grid, S);
 		const uint32_t ex = (uint32_t)(S.bx1 - S.bx0), ey = (uint32_t)(S.by1 - S.by0), ez = (uint32_t)(S.bz1 - S.bz0);
 		const uint64_t rows = (uint64_t)(ey + 1) * (uint64_t)(ez + 1);
-		const uint64_t nvox = (uint64_t)(ex + 1) * rows;
-		if (nvox <= small_vox && nvox <= 255 && rows <= kSmallRows && ey < 16 && ez < 16) {
-			pack_small(S, sm.small[threadIdx.x]);
-			n_small = (uint32_t)rows;
-		} else {
-			n_items = (ez + kZch) / kZch;
-			if (rows <= kLocalRows && ex < 256 && ey < 256 && ez < 256) {
-				pack_small(S, sm.small[threadIdx.x]);
-				n_local = (uint32_t)rows;
-			}
-		}
+		few = (uint64_t)(ex + 1) * rows <= small_vox;
+		n_items = (ez + kZch) / kZch;
+		if (ex < kMaskRowVoxels && rows <= kLocalRows && !plane_underflows(S)) n_rows = (uint32_t)rows;
 	}
-	// One item list for the tile: the rows of the small triangles, then those of the local ones.
-	// A local triangle whose rows no longer fit is queued like the larger ones.
-	if (threadIdx.x == 0) s_fit = 0xFFFFFFFFu;  // ordered before the atomics by the scan's barriers
-	uint32_t totals = 0;
-	const uint32_t offs = block_scan(n_small | (n_local << 16), s_warp, &totals);
-	const uint32_t total_small = totals & 0xFFFFu;
-	const uint32_t loff = total_small + (offs >> 16);
-	if (n_local && loff + n_local > kTile * kSmallRows) {
-		atomicMin(&s_fit, loff);
-		n_local = 0;
+	if (__reduce_add_sync(FULL, n_rows) > warp_rows && !few) n_rows = 0;
+	uint32_t incl = n_rows;
+#pragma unroll
+	for (int d = 1; d < 32; d <<= 1) {
+		const uint32_t v = __shfl_up_sync(FULL, incl, d);
+		if (lane >= (uint32_t)d) incl += v;
 	}
-	bool is_brick = false;
-	if (n_items && !n_local) {
-		if (jflags & JOB_BRICKS) {
-			is_brick = true;  // rasterized in shared-memory bricks (bricks.cu)
-		} else {
-			is_mid = n_items == 1;
-			is_big = n_items > 1;
-		}
-	}
-	// Queue the other triangles: warp-aggregated appends.
+	const uint32_t total_rows = __shfl_sync(FULL, incl, 31);
+	const uint32_t start = incl - n_rows;
 	const uint32_t lt = (1u << lane) - 1u;
+	const uint32_t parked = __ballot_sync(FULL, n_rows != 0u);
+	if (n_rows) pack_small(S, start, sm.small[__popc(parked & lt)]);
+	const bool queued = n_items && !n_rows;
+	const bool is_brick = queued && (jflags & JOB_BRICKS);  // rasterized in shared-memory bricks (bricks.cu)
+	const bool is_mid = queued && !is_brick && n_items == 1, is_big = queued && !is_brick && n_items > 1;
+	// Queue the other triangles: warp-aggregated appends.
 	const uint32_t brick_ballot = __ballot_sync(FULL, is_brick);
 	if (brick_ballot) {
 		uint32_t base = 0;
@@ -190,7 +102,7 @@ __global__ void __launch_bounds__(kTile, 10) surf_classify(const __grid_constant
 		base = __shfl_sync(FULL, base, leader);
 		const uint32_t slot = base + __popc(brick_ballot & lt);
 		if (is_brick) {
-			if (slot < L.scr.cap) L.scr.bq[slot] = MidRec{j, (uint32_t)(t0 + threadIdx.x)};
+			if (slot < L.scr.cap) L.scr.bq[slot] = MidRec{j, (uint32_t)(t0 + lane)};
 			else set_error(L, kErrQueueOverflow);
 		}
 	}
@@ -202,7 +114,7 @@ __global__ void __launch_bounds__(kTile, 10) surf_classify(const __grid_constant
 		base = __shfl_sync(FULL, base, leader);
 		const uint32_t slot = base + __popc(mid_ballot & lt);
 		if (is_mid) {
-			if (slot < L.scr.cap) L.scr.mid[slot] = MidRec{j, (uint32_t)(t0 + threadIdx.x)};
+			if (slot < L.scr.cap) L.scr.mid[slot] = MidRec{j, (uint32_t)(t0 + lane)};
 			else set_error(L, kErrQueueOverflow);
 		}
 	}
@@ -223,59 +135,36 @@ __global__ void __launch_bounds__(kTile, 10) surf_classify(const __grid_constant
 			const uint32_t rec = (uint32_t)(old >> kBigShift) + __popc(big_ballot & lt);
 			const uint64_t first = (old & kBigItemMask) + incl - n_items;
 			if (rec < L.scr.cap && first + n_items <= kBigItemMask)
-				L.scr.big[rec] = BigRec{first, j, (uint32_t)(t0 + threadIdx.x), n_items, 0u};
+				L.scr.big[rec] = BigRec{first, j, (uint32_t)(t0 + lane), n_items, 0u};
 			else
 				set_error(L, kErrQueueOverflow);
 		}
 	}
 
-	// Phase 2: the rows of the tile's small and local triangles, dealt evenly over the CTA.
-	if (n_small) {
-		const SmallTri& o = sm.small[threadIdx.x];
-		const uint32_t ny = ((o.ext >> 8) & 0xFFu) + 1u, nz = ((o.ext >> 16) & 0xFFu) + 1u;
-		uint32_t c = offs & 0xFFFFu;
-		for (uint32_t dz = 0; dz < nz; dz++)
-			for (uint32_t dy = 0; dy < ny; dy++) s_items[c++] = (uint16_t)(threadIdx.x | (dy << 8) | (dz << 12));
-	}
-	for (uint32_t r = 0; r < n_local; r++) s_items[loff + r] = (uint16_t)(threadIdx.x | (r << 8));
-	__syncthreads();
-	const uint32_t total_items = min(total_small + (totals >> 16), s_fit);
-	for (uint32_t k = threadIdx.x; k < total_items; k += kTile) {
-		const uint32_t it = s_items[k];
-		SurfTri S;
-		unpack_small(sm.small[it & 0xFFu], S);
-		const bool small = k < total_small;
-		int y, z;
-		if (small) {
-			y = S.by0 + (int)((it >> 8) & 0xFu);
-			z = S.bz0 + (int)(it >> 12);
-		} else {
-			// row r of a local triangle: r = dy + dz * ny with r < kLocalRows and ny < 256, so the
-			// approximate quotient is more than 1e-3 away from the next integer and truncates exactly
-			const uint32_t r = it >> 8, ny = (uint32_t)(S.by1 - S.by0) + 1u;
-			const uint32_t dz = (uint32_t)__fdividef((float)r + 0.5f, (float)ny);
-			y = S.by0 + (int)(r - dz * ny);
-			z = S.bz0 + (int)dz;
-		}
+	// Phase 2: the rows of the parked triangles.
+	__syncwarp();
+	uint32_t begun = 0;  // triangles that start before this step's rows
+	for (uint32_t base = 0; base < total_rows; base += 32) {
+		const uint32_t at = start - base;
+		const uint32_t starts = __reduce_or_sync(FULL, n_rows && at < 32u ? 1u << at : 0u);
+		const uint32_t rec = begun + __popc(starts & (0xFFFFFFFFu >> (31u - lane))) - 1u;
+		begun += __popc(starts);
+		const uint32_t k = base + lane;
+		if (k >= total_rows) break;
+		const SmallTri& o = sm.small[rec];
+		const float4 box = o.q[0];
+		const uint32_t bx = __float_as_uint(box.x), by = __float_as_uint(box.y), bz = __float_as_uint(box.z);
+		// row r = dy + dz * ny of the triangle, r and ny at most kLocalRows: the approximate quotient is more than
+		// 1e-3 away from the next integer and truncates exactly
+		const uint32_t r = k - __float_as_uint(box.w), ny = (by >> 24) + 1u;
+		const uint32_t dz = (uint32_t)__fdividef((float)r + 0.5f, (float)ny);
+		const int y = (int)((by & 0xFFFFFFu) + r - dz * ny), z = (int)((bz & 0xFFFFFFu) + dz);
 		const float py = __fmul_rn(__int2float_rn(y), unit[1]);
 		const float pz = __fmul_rn(__int2float_rn(z), unit[2]);
-		if (yz_fail_bits<P>(S, py, pz)) continue;
-		RowK K;
-		row_consts<P>(S, py, pz, K);
-		// Rows of at most kMaskRowVoxels voxels test every voxel (a local triangle's short rows too):
-		// cheaper than setting up the crossing estimates of an exact interval search.
-		if (small || S.bx1 - S.bx0 < (int)kMaskRowVoxels) {
-			// src/voxelize.cu:136-183: every voxel of the row (at most 16), as a pass mask
-			uint32_t pm = 0;
-			for (int i = 0; i <= S.bx1 - S.bx0; i++) pm |= (uint32_t)voxel_pass<P>(S, K, unit[0], S.bx0 + i) << i;
-			if (pm) write_row_mask(table, (jflags & JOB_MORTON) != 0, (jflags & JOB_NARROW) != 0, grid, y, z, S.bx0, pm);
-		} else {
-			RowDirs D;
-			row_dirs(S, unit[0], D);
-			int xl, xh;
-			if (row_interval<P>(S, D, K, unit[0], xl, xh))
-				write_row(table, (jflags & JOB_MORTON) != 0, (jflags & JOB_NARROW) != 0, grid, y, z, xl, xh);
-		}
+		if (!row_in_yz<P>(o, py, pz)) continue;
+		const int x0 = (int)(bx & 0xFFFFFFu);
+		const uint32_t pm = row_mask<P>(o, unit[0], py, pz, x0, (bx >> 24) + 1u);
+		if (pm) write_row_mask(table, (jflags & JOB_MORTON) != 0, (jflags & JOB_NARROW) != 0, grid, y, z, x0, pm);
 	}
 }
 
@@ -416,7 +305,11 @@ static cudaError_t launch_surface_t(const LaunchDesc& L, const Tune& tune, int r
                                     cudaStream_t s, const Prof* prof) {
 	if (L.n_tiles == 0) return cudaSuccess;
 	if (prof) (*prof)(nullptr, s);
-	surf_classify<P><<<L.n_tiles, kTile, 0, s>>>(L, tune.small_vox);
+	// With fewer CTAs than fill the chip the longest warp is the kernel's time: a warp with more than
+	// kWarpRows rows leaves the triangles above small_vox voxels to surf_rows.
+	const uint32_t warp_rows = L.n_tiles >= (uint32_t)rows_grid ? 0xFFFFFFFFu : kWarpRows;
+	const uint32_t split = classify_split(L.n_tiles, (uint32_t)rows_grid);
+	surf_classify<P><<<L.n_tiles << split, kTile, 0, s>>>(L, tune.small_vox, warp_rows, split);
 	cudaError_t e = cudaGetLastError();
 	if (e != cudaSuccess) return e;
 	if (prof) (*prof)("surf_classify", s);

@@ -35,6 +35,22 @@ __device__ __forceinline__ float setup_dot(float ax, float vx, float ay, float v
 	else return mul_add<P>(ax, vx, ay, vy);
 }
 
+// One axis of the grid bbox: b0 = clamp(int(lo / u), 0, g - 1), b1 likewise from hi, from quotients
+// with the reciprocal inv ~ 1 / u.  fl(a * inv) is within 2 ulp of fl(a / u), so within
+// room = 4 * 2^-23 * g for a quotient up to g; clamped to [1/4, g - 1/4] first, which leaves the
+// clamped integer as it is (a quotient below 1/4 gives 0, one above g - 1/4 gives g - 1, and so do a
+// NaN, which fmaxf replaces, and the infinities).  Adding 2^23 rounds it to the nearest integer.
+// `near` becomes at most 0 if a quotient is within room of an integer: the caller divides then.
+__device__ __forceinline__ void bbox_axis(float lo, float hi, float inv, uint32_t g, int& b0, int& b1, float& near) {
+	const float top = (float)g - 0.25f, room = 0x1p-21f * (float)g;
+	const float q0 = fminf(fmaxf(__fmul_rn(lo, inv), 0.25f), top), q1 = fminf(fmaxf(__fmul_rn(hi, inv), 0.25f), top);
+	const float m0 = __fadd_rn(q0, 8388608.0f), m1 = __fadd_rn(q1, 8388608.0f);
+	const float d0 = __fsub_rn(q0, __fsub_rn(m0, 8388608.0f)), d1 = __fsub_rn(q1, __fsub_rn(m1, 8388608.0f));
+	b0 = (__float_as_int(m0) & 0x7FFFFF) - (d0 < 0.0f ? 1 : 0);
+	b1 = (__float_as_int(m1) & 0x7FFFFF) - (d1 < 0.0f ? 1 : 0);
+	near = fminf(near, fminf(fabsf(d0), fabsf(d1)) - room);
+}
+
 // Triangle setup, src/voxelize.cu:71-133.  `t` holds v0.xyz, v1.xyz, v2.xyz in world space.
 template <class P>
 __device__ __forceinline__ void surf_setup(const float* t, const float* bmin, const float* unit, const float* inv,
@@ -54,14 +70,21 @@ __device__ __forceinline__ void surf_setup(const float* t, const float* bmin, co
 	S.ny = __fmul_rn(cy, rlen);
 	S.nz = __fmul_rn(cz, rlen);
 
-	// grid bbox: clamp(int(min(v) / unit), 0, g - 1)  (:83-87)
-	const int gmx = (int)grid[0] - 1, gmy = (int)grid[1] - 1, gmz = (int)grid[2] - 1;
-	S.bx0 = min(max(div_trunc(fminf(v0x, fminf(v1x, v2x)), unit[0], inv[0]), 0), gmx);
-	S.by0 = min(max(div_trunc(fminf(v0y, fminf(v1y, v2y)), unit[1], inv[1]), 0), gmy);
-	S.bz0 = min(max(div_trunc(fminf(v0z, fminf(v1z, v2z)), unit[2], inv[2]), 0), gmz);
-	S.bx1 = min(max(div_trunc(fmaxf(v0x, fmaxf(v1x, v2x)), unit[0], inv[0]), 0), gmx);
-	S.by1 = min(max(div_trunc(fmaxf(v0y, fmaxf(v1y, v2y)), unit[1], inv[1]), 0), gmy);
-	S.bz1 = min(max(div_trunc(fmaxf(v0z, fmaxf(v1z, v2z)), unit[2], inv[2]), 0), gmz);
+	// grid bbox: clamp(int(min(v) / unit), 0, g - 1)  (:83-87).  Reciprocal quotients decide it unless
+	// one is within their error of an integer; then all six divide.
+	float near = 1.0f;
+	bbox_axis(fminf(v0x, fminf(v1x, v2x)), fmaxf(v0x, fmaxf(v1x, v2x)), inv[0], grid[0], S.bx0, S.bx1, near);
+	bbox_axis(fminf(v0y, fminf(v1y, v2y)), fmaxf(v0y, fmaxf(v1y, v2y)), inv[1], grid[1], S.by0, S.by1, near);
+	bbox_axis(fminf(v0z, fminf(v1z, v2z)), fmaxf(v0z, fmaxf(v1z, v2z)), inv[2], grid[2], S.bz0, S.bz1, near);
+	if (!(near > 0.0f)) {
+		const int gmx = (int)grid[0] - 1, gmy = (int)grid[1] - 1, gmz = (int)grid[2] - 1;
+		S.bx0 = min(max(__float2int_rz(__fdiv_rn(fminf(v0x, fminf(v1x, v2x)), unit[0])), 0), gmx);
+		S.by0 = min(max(__float2int_rz(__fdiv_rn(fminf(v0y, fminf(v1y, v2y)), unit[1])), 0), gmy);
+		S.bz0 = min(max(__float2int_rz(__fdiv_rn(fminf(v0z, fminf(v1z, v2z)), unit[2])), 0), gmz);
+		S.bx1 = min(max(__float2int_rz(__fdiv_rn(fmaxf(v0x, fmaxf(v1x, v2x)), unit[0])), 0), gmx);
+		S.by1 = min(max(__float2int_rz(__fdiv_rn(fmaxf(v0y, fmaxf(v1y, v2y)), unit[1])), 0), gmy);
+		S.bz1 = min(max(__float2int_rz(__fdiv_rn(fmaxf(v0z, fmaxf(v1z, v2z)), unit[2])), 0), gmz);
+	}
 
 	// plane test: critical point c and d1, d2  (:90-95)
 	const float cxp = S.nx > 0.0f ? unit[0] : 0.0f;
@@ -153,67 +176,83 @@ __device__ __forceinline__ uint32_t fail_bits(const SurfTri& S, const RowK& K, f
 	return f;
 }
 
-// All x-dependent tests at once, as one pass/fail (the small-triangle path needs no more).
-template <class P>
-__device__ __forceinline__ bool voxel_pass(const SurfTri& S, const RowK& K, float ux, int x) {
-	const float px = __fmul_rn(__int2float_rn(x), ux);
-	float s;
-	if constexpr (P::plane == 1) s = __fmaf_rn(S.nz, K.pz, __fmaf_rn(S.nx, px, K.kpl));
-	else if constexpr (P::plane == 2) s = __fadd_rn(__fmaf_rn(S.nx, px, K.kpl), K.kpl2);
-	else if constexpr (P::plane == 3) s = __fmaf_rn(S.nz, K.pz, __fmaf_rn(S.ny, K.py, __fmul_rn(S.nx, px)));
-	else s = __fadd_rn(__fadd_rn(__fmul_rn(S.nx, px), K.kpl), K.kpl2);
-	bool ok = !(__fmul_rn(__fadd_rn(s, S.d1), __fadd_rn(s, S.d2)) > 0.0f);
-#pragma unroll
-	for (int i = 0; i < 3; i++) {
-		float v;
-		if constexpr (P::edge_xy == 1) v = __fmaf_rn(S.exy[i][0], px, K.kxy[i]);
-		else v = mul_add<P::edge_xy>(S.exy[i][0], px, S.exy[i][1], K.py);
-		ok = ok && !(__fadd_rn(v, S.dxy[i]) < 0.0f);
-	}
-#pragma unroll
-	for (int i = 0; i < 3; i++) {
-		float v;
-		if constexpr (P::edge_zx == 2) v = __fmaf_rn(S.ezx[i][1], px, K.kzx[i]);
-		else v = mul_add<P::edge_zx>(S.ezx[i][0], K.pz, S.ezx[i][1], px);
-		ok = ok && !(__fadd_rn(v, S.dzx[i]) < 0.0f);
-	}
-	return ok;
+// The plane test as two comparisons.  The test fails iff fl(fl(s + d1) * fl(s + d2)) > 0, i.e. both
+// sums are positive or both negative: iff s > hi = max(-d1, -d2) or s < lo = min(-d1, -d2) -- unless
+// the product underflows.  It cannot when |d1|, |d2| >= 2^-49: for |s| < 2^-50 both sums are at least
+// 2^-50; otherwise all operands are multiples of 2^-73, so each nonzero sum is at least that and the
+// product at least 2^-146.  plane_underflows() marks a triangle with a smaller d1 or d2.  A NaN in d1
+// or d2 makes the product NaN (never a failure): lo and hi are then both NaN.
+__device__ __forceinline__ bool plane_underflows(const SurfTri& S) {
+	return (fabsf(S.d1) < 0x1p-49f) | (fabsf(S.d2) < 0x1p-49f);
+}
+__device__ __forceinline__ void plane_bounds(const SurfTri& S, float& lo, float& hi) {
+	const bool nan = (S.d1 != S.d1) | (S.d2 != S.d2);
+	lo = nan ? __int_as_float(0x7FFFFFFF) : fminf(-S.d1, -S.d2);
+	hi = nan ? __int_as_float(0x7FFFFFFF) : fmaxf(-S.d1, -S.d2);
 }
 
-// A small triangle's setup parked in shared memory between the two phases of the classify kernel
-// (36 words): SurfTri without the bbox maxima, which are packed as extents (each below 256).
+// A small triangle's setup (rows of at most kMaskRowVoxels voxels, plane_underflows() false) parked
+// in shared memory between the two phases of the classify kernel, with the tests in the form that
+// takes the fewest instructions per voxel: the plane test as above, and an edge test, which fails iff
+// fl(v + d) < 0, as v < -d.  (Rounding keeps the sign of a sum: the sum of two floats is a multiple of
+// the smallest subnormal, so it never rounds to zero; a NaN or an inf - inf fails neither form.)
+// The record is read as nine 16-byte vectors, those of the YZ tests first; its stride of 36 words
+// starts the 8 lanes of a quarter warp reading 8 records on banks 0, 4, .. 28.  (Pairing the edge
+// tests in packed f32x2 operations was measured: 3% slower.)
 struct SmallTri {
-	float v[32];           // nx ny nz d1 d2, exy[3][2], eyz[3][2], ezx[3][2], dxy[3], dyz[3], dzx[3]
-	int bx0, by0, bz0;
-	uint32_t ext;          // (bx1-bx0) | (by1-by0) << 8 | (bz1-bz0) << 16
+	float4 q[9];
 };
 
-__device__ __forceinline__ void pack_small(const SurfTri& S, SmallTri& o) {
-	o.v[0] = S.nx; o.v[1] = S.ny; o.v[2] = S.nz; o.v[3] = S.d1; o.v[4] = S.d2;
-#pragma unroll
-	for (int i = 0; i < 3; i++) {
-		o.v[5 + 2 * i] = S.exy[i][0]; o.v[6 + 2 * i] = S.exy[i][1];
-		o.v[11 + 2 * i] = S.eyz[i][0]; o.v[12 + 2 * i] = S.eyz[i][1];
-		o.v[17 + 2 * i] = S.ezx[i][0]; o.v[18 + 2 * i] = S.ezx[i][1];
-		o.v[23 + i] = S.dxy[i]; o.v[26 + i] = S.dyz[i]; o.v[29 + i] = S.dzx[i];
-	}
-	o.bx0 = S.bx0; o.by0 = S.by0; o.bz0 = S.bz0;
-	o.ext = (uint32_t)(S.bx1 - S.bx0) | ((uint32_t)(S.by1 - S.by0) << 8) | ((uint32_t)(S.bz1 - S.bz0) << 16);
+// start: rows of the warp's parked triangles before this one.
+__device__ __forceinline__ void pack_small(const SurfTri& S, uint32_t start, SmallTri& o) {
+	float lo, hi;
+	plane_bounds(S, lo, hi);
+	// bbox minimum in 24 bits (an axis has at most 2^22 voxels), extent - 1 in the other 8
+	o.q[0] = make_float4(__int_as_float(S.bx0 | (S.bx1 - S.bx0) << 24), __int_as_float(S.by0 | (S.by1 - S.by0) << 24),
+	                     __int_as_float(S.bz0 | (S.bz1 - S.bz0) << 24), __uint_as_float(start));
+	o.q[1] = make_float4(S.eyz[0][0], S.eyz[1][0], S.eyz[0][1], S.eyz[1][1]);
+	o.q[2] = make_float4(S.eyz[2][0], S.eyz[2][1], -S.dyz[0], -S.dyz[1]);
+	o.q[3] = make_float4(-S.dyz[2], S.nx, S.ny, S.nz);
+	o.q[4] = make_float4(S.exy[2][1], S.ezx[0][0], lo, hi);
+	o.q[5] = make_float4(S.exy[0][0], S.exy[1][0], S.exy[0][1], S.exy[1][1]);
+	o.q[6] = make_float4(S.exy[2][0], S.ezx[0][1], S.ezx[1][1], S.ezx[2][1]);
+	o.q[7] = make_float4(S.ezx[1][0], S.ezx[2][0], -S.dxy[0], -S.dxy[1]);
+	o.q[8] = make_float4(-S.dxy[2], -S.dzx[0], -S.dzx[1], -S.dzx[2]);
 }
 
-__device__ __forceinline__ void unpack_small(const SmallTri& o, SurfTri& S) {
-	S.nx = o.v[0]; S.ny = o.v[1]; S.nz = o.v[2]; S.d1 = o.v[3]; S.d2 = o.v[4];
-#pragma unroll
-	for (int i = 0; i < 3; i++) {
-		S.exy[i][0] = o.v[5 + 2 * i]; S.exy[i][1] = o.v[6 + 2 * i];
-		S.eyz[i][0] = o.v[11 + 2 * i]; S.eyz[i][1] = o.v[12 + 2 * i];
-		S.ezx[i][0] = o.v[17 + 2 * i]; S.ezx[i][1] = o.v[18 + 2 * i];
-		S.dxy[i] = o.v[23 + i]; S.dyz[i] = o.v[26 + i]; S.dzx[i] = o.v[29 + i];
-	}
-	S.bx0 = o.bx0; S.by0 = o.by0; S.bz0 = o.bz0;
-	S.bx1 = o.bx0 + (int)(o.ext & 0xFFu);
-	S.by1 = o.by0 + (int)((o.ext >> 8) & 0xFFu);
-	S.bz1 = o.bz0 + (int)((o.ext >> 16) & 0xFFu);
+// YZ tests of a parked triangle's row.
+template <class P>
+__device__ __forceinline__ bool row_in_yz(const SmallTri& o, float py, float pz) {
+	const float4 a = o.q[1], b = o.q[2];
+	return !(mul_add<P::edge_yz>(a.x, py, a.z, pz) < b.z) & !(mul_add<P::edge_yz>(a.y, py, a.w, pz) < b.w) &
+	       !(mul_add<P::edge_yz>(b.x, py, b.y, pz) < o.q[3].x);
+}
+
+// Pass mask of the n <= kMaskRowVoxels voxels x0, x0 + 1, ... of row (py, pz): bit i set = voxel
+// x0 + i passes every x-dependent test (src/voxelize.cu:136-183).  The tests are combined without
+// branches: a lane that left early would wait for the others anyway.
+template <class P>
+__device__ __forceinline__ uint32_t row_mask(const SmallTri& o, float ux, float py, float pz, int x0, uint32_t n) {
+	static_assert(P::plane == 2 && P::edge_xy == 1 && P::edge_zx == 2,
+	              "the row mask follows the pinned fused-multiply-add pattern");
+	const float4 a = o.q[3], b = o.q[4], c = o.q[5], d = o.q[6], e = o.q[7], f = o.q[8];
+	const float kpl = __fmul_rn(a.z, py), kpl2 = __fmul_rn(a.w, pz);
+	const float kxy0 = __fmul_rn(c.z, py), kxy1 = __fmul_rn(c.w, py), kxy2 = __fmul_rn(b.x, py);
+	const float kzx0 = __fmul_rn(b.y, pz), kzx1 = __fmul_rn(e.x, pz), kzx2 = __fmul_rn(e.y, pz);
+	uint32_t pm = 0, bit = 1u;
+	float x = (float)x0;  // exact, as x0 + 1, ... are
+	const uint32_t end = 1u << n;
+	do {
+		const float px = __fmul_rn(x, ux);
+		const float s = __fadd_rn(__fmaf_rn(a.y, px, kpl), kpl2);
+		const bool fail = (s > b.w) | (s < b.z) | (__fmaf_rn(c.x, px, kxy0) < e.z) | (__fmaf_rn(c.y, px, kxy1) < e.w) |
+		                  (__fmaf_rn(d.x, px, kxy2) < f.x) | (__fmaf_rn(d.y, px, kzx0) < f.y) |
+		                  (__fmaf_rn(d.z, px, kzx1) < f.z) | (__fmaf_rn(d.w, px, kzx2) < f.w);
+		pm |= fail ? 0u : bit;
+		bit += bit;
+		x += 1.0f;
+	} while (bit != end);
+	return pm;
 }
 
 // YZ edge tests for row (y, z): independent of x.  Bit i set = YZ edge i fails.

@@ -1,0 +1,105 @@
+"""The surface classify kernel's bins and launch shapes, against the CPU oracle's GPU-arithmetic mode.
+
+Each mesh is made of triangles whose grid boxes sit on both sides of a bin's edge (voxels per row,
+rows per triangle, extents), in numbers on both sides of the rules on the number of tiles, and in
+groups that are ragged or not 16-byte aligned.  The tables must be equal, bit for bit.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import oracle  # noqa: E402
+from cuda_voxelizer_gb300 import api as cv  # noqa: E402
+from oracle import build as oracle_build  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+GUARD = 64
+
+
+@pytest.fixture(scope="module")
+def rsqrt():
+    """The device's own rsqrtf, which the oracle needs for the normals."""
+    L = ctypes.CDLL(oracle_build.build_gpu_runner())
+    L.refgpu_rsqrt.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p]
+
+    def f(x):
+        a = torch.from_numpy(x).cuda()
+        b = torch.empty_like(a)
+        assert L.refgpu_rsqrt(a.data_ptr(), b.data_ptr(), a.numel(), torch.cuda.current_stream().cuda_stream) == 0
+        return np.ascontiguousarray(b.cpu().numpy())
+
+    return f
+
+
+def _triangles(seed, n, ext, g):
+    """n random triangles, each spanning about ext[k] voxels along axis k of a unit grid of g voxels."""
+    rng = np.random.default_rng(seed)
+    ext = np.minimum(np.asarray(ext, dtype=np.float64), g - 1.0)
+    t = rng.random((n, 3, 3))
+    t = (t - t.min(1, keepdims=True)) / (t.max(1, keepdims=True) - t.min(1, keepdims=True))
+    lo = rng.uniform(0.3, g - ext - 0.3, (n, 3))
+    return (lo[:, None, :] + t * ext).reshape(n, 9).astype(np.float32)
+
+
+def _check(rsqrt, tris, g, morton, offset=0):
+    info = cv.make_info((0, 0, 0), (float(g),) * 3, g, len(tris))
+    buf = torch.zeros(tris.size + 4, dtype=torch.float32, device="cuda")
+    d = buf[offset:offset + tris.size]
+    d.copy_(torch.from_numpy(tris.reshape(-1)))
+    table = torch.zeros(cv.table_words(info) + GUARD, dtype=torch.int32, device="cuda")
+    cv.voxelize(info, d, table, morton)
+    cv.device_status()
+    inv = rsqrt(oracle.len2(bytes(info), tris, oracle.gpu_mode(morton)))
+    want = oracle.voxelize(bytes(info), tris, morton, mode=oracle.gpu_mode(morton, inv_len=inv))
+    got = table.cpu().numpy().view(np.uint32)
+    assert not got[len(want):].any()
+    bad = np.nonzero(got[:len(want)] != want)[0]
+    assert bad.size == 0, f"{bad.size} words differ, first {bad[:5]}"
+
+
+@pytest.mark.parametrize("morton", [False, True])
+@pytest.mark.parametrize("ext", [
+    (0.4, 0.4, 0.4), (2.5, 2.5, 2.5), (15, 3, 3), (16, 3, 3), (17, 3, 3),   # rows of up to and above 16 voxels
+    (40, 0.3, 0.3), (63, 0.2, 0.2),                                          # few voxels, all in one or two rows
+    (3, 14, 14), (3, 16, 16), (3, 20, 20),                                   # rows around 256
+    (2, 254, 0.3), (2, 256, 0.3), (2, 0.3, 256), (255, 2, 2), (257, 2, 2),   # extents around 256
+    (60, 60, 31), (60, 60, 33),                                              # around one queue item per triangle
+])
+def test_bins(rsqrt, ext, morton):
+    _check(rsqrt, _triangles(7, 301, ext, 512), 512, morton)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 31, 33, 127, 129, 8500, 17100, 34100, 68200, 136300])
+def test_launch_shapes(rsqrt, n):
+    """Ragged groups, and triangles per warp of 4, 8, 16 and 32 (136,192 triangles are 1,064 tiles)."""
+    _check(rsqrt, _triangles(n, n, (4, 4, 4), 128), 128, False)
+
+
+@pytest.mark.parametrize("n", [130, 140_001])
+@pytest.mark.parametrize("offset", [1, 2])  # floats past a 16-byte boundary: no bulk copy
+def test_unaligned_triangles(rsqrt, n, offset):
+    _check(rsqrt, _triangles(n, n, (3, 3, 3), 128), 128, True, offset)
+
+
+@pytest.mark.parametrize("n", [200, 140_000])
+def test_mixed_sizes(rsqrt, n):
+    """Warps that hold a few large triangles among small ones, and more rows than a small launch keeps."""
+    t = _triangles(1, n, (2, 2, 2), 256)
+    t[::37] = _triangles(2, len(t[::37]), (9, 15, 15), 256)
+    t[::411] = _triangles(3, len(t[::411]), (90, 90, 90), 256)
+    _check(rsqrt, t, 256, False)
+
+
+def test_grid_aligned_triangles(rsqrt):
+    """Vertices on voxel corners: plane offsets that are exactly zero, and degenerate triangles."""
+    rng = np.random.default_rng(11)
+    lo = rng.integers(1, 50, (4000, 1, 3))
+    t = (lo + rng.integers(0, 6, (4000, 3, 3))).astype(np.float32)
+    t[::3, :, 0] = t[::3, :1, 0]  # in a plane of constant x, y or z
+    t[1::3, :, 1] = t[1::3, :1, 1]
+    t[2::3, :, 2] = t[2::3, :1, 2]
+    _check(rsqrt, t.reshape(-1, 9), 64, False)
