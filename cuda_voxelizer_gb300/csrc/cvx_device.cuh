@@ -90,7 +90,7 @@ struct JobDesc {
 	uint64_t n_tri;
 	float bmin[3];
 	float unit[3];
-	float inv_unit[3];     // 1.0f / unit, correctly rounded (host); only used for the exactly checked div_trunc
+	float inv_unit[3];     // 1.0f / unit, correctly rounded (host); only used for exactly checked quotients
 	uint32_t grid[3];
 	uint32_t flags;        // JOB_MORTON | JOB_SOLID | JOB_NARROW | JOB_TABLE_OVERWRITE | ...
 	uint32_t tile_begin;   // first triangle tile of this job in the launch's tile space
@@ -271,20 +271,6 @@ __device__ __forceinline__ uint32_t compact3(uint64_t v) {
 __device__ __forceinline__ uint32_t nibble_mask(uint32_t nib) {
 	// dx = 0, 1 (nibble bits 3, 2) -> offsets 0, 1 (bits 31, 30); dx = 2, 3 (bits 1, 0) -> offsets 8, 9
 	return ((nib & 0xCu) << 28) | ((nib & 0x3u) << 22);
-}
-
-
-// (int)__fdiv_rn(a, u) (truncation of the correctly rounded quotient, as float3_to_int3 of
-// `a / unit` in the reference, src/util.h:20-22), computed with the per-axis reciprocal inv ~ 1/u.
-// fl(a * inv) is within 2 ulp of fl(a / u); truncation can only differ when the quotient is within
-// that distance of an integer, and there the exact division decides.
-__device__ __forceinline__ int div_trunc(float a, float u, float inv) {
-	const float q = __fmul_rn(a, inv);
-	const float t = truncf(q);
-	const float room = 4.0f * __fmul_rn(fabsf(q), 1.1920929e-07f) + 1.0e-30f;  // 4 ulp-ish, never 0
-	if (fabsf(q) < 8388608.0f && q - t > room && (t + 1.0f) - q > room && fabsf(q) > room)
-		return (int)t;
-	return __float2int_rz(__fdiv_rn(a, u));
 }
 
 // Bit layout (src/voxelize.cu:50-55): word = idx / 32, bit = 31 - idx % 32 (MSB first).

@@ -46,7 +46,7 @@ __device__ __forceinline__ float ceil_half(float q) {
 	return fabsf(q) < 4194304.0f ? ceilf(__fsub_rn(q, 0.5f)) : (float)ceil((double)q - 0.5);
 }
 // floor_half / ceil_half of fl(a / u), using the reciprocal shortcut when the approximate
-// quotient is clearly away from the decision boundary (the half-integers), as div_trunc does.
+// quotient is clearly away from the decision boundary (the half-integers).
 __device__ __forceinline__ float div_floor_half(float a, float u, float inv) {
 	const float q = __fmul_rn(a, inv);
 	const float h = __fsub_rn(q, 0.5f);

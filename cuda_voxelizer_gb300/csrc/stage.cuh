@@ -58,6 +58,37 @@ __device__ __forceinline__ bool stage_warp(const LaunchDesc& L, const float* src
 	return true;
 }
 
+// The queued item of ticket `tk` of a persistent kernel: big items (n_big records, n_big_items items)
+// first, then the mid triangles.  Every lane calls it with the same ticket and gets the same answer;
+// false for a malformed record (only possible after a queue overflow).  The big record is found by a
+// search with 32 probes per round: three dependent loads for 32,768 records instead of fifteen.
+__device__ __forceinline__ bool queue_item(const LaunchDesc& L, unsigned long long tk, uint32_t n_big,
+                                           uint64_t n_big_items, uint32_t lane, uint32_t& job, uint32_t& tri,
+                                           uint32_t& chunk) {
+	chunk = 0;
+	if (tk < n_big_items) {
+		if (n_big == 0) return false;
+		uint32_t first = 0, n = n_big;  // the last record with item_begin <= tk is among n from `first`
+		while (n > 1) {
+			const uint32_t step = (n + 31u) >> 5, at = lane * step;
+			const bool le = at < n && (at == 0u || L.scr.big[first + at].item_begin <= tk);
+			const uint32_t last = 31u - __clz(__ballot_sync(FULL, le));
+			first += last * step;
+			n = min(step, n - last * step);
+		}
+		const BigRec r = L.scr.big[first];
+		job = r.job;
+		tri = r.tri;
+		chunk = (uint32_t)(tk - r.item_begin);
+		if (tk < r.item_begin || chunk >= r.n_items) return false;
+	} else {
+		const MidRec r = L.scr.mid[tk - n_big_items];
+		job = r.job;
+		tri = r.tri;
+	}
+	return job < L.n_jobs && tri < job_at(L, job).n_tri;
+}
+
 // Triangles of a classify warp: 32, or in a launch with few tiles 32 >> split, so that its warps are
 // spread over the chip and none has many rows or columns to walk.  Splits up to kMaxSplit; a split of
 // s launches 2^s CTAs per tile.  (9,216-triangle torus: surf_classify 64^3 11.7 -> 9.5 us, 128^3 16 ->

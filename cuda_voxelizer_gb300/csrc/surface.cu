@@ -8,12 +8,12 @@
 //                  by the warp, their rows dealt over its lanes, every voxel tested like in the
 //                  reference; the others are queued, one record per triangle, as one item ("mid")
 //                  or as one item per 32 z-slices ("big").
-//   surf_rows      persistent CTAs of kRowsCtaThreads threads, seven per SM; each warp takes
-//                  work tickets (big items first, then mid triangles), finds the y-interval of every z-slice of the item (one lane per slice),
-//                  flattens the (y, z) rows and gives one row per lane; each lane finds the exact
-//                  x-interval of its row and ORs it into the table one word at a time (the whole
-//                  warp for long rows).  Jobs whose indices fit 32 bits (JOB_NARROW) write with
-//                  32-bit index arithmetic.
+//   surf_rows      persistent CTAs; each warp takes work tickets (big items first, then mid
+//                  triangles), finds the bounds that the tests of the three projections put on the
+//                  item's slices and rows, one test per slice or row instead of one per voxel row,
+//                  narrows every row to its exact x-interval with the plane test and ORs it into the
+//                  table one word at a time (the whole warp for long rows).  Jobs whose indices fit
+//                  32 bits (JOB_NARROW) write with 32-bit index arithmetic.
 #include "engine.h"
 #include "stage.cuh"
 #include "surface.cuh"
@@ -168,13 +168,34 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 	}
 }
 
-// 128-thread CTAs at 72 registers: seven per SM (28 warps) instead of three 256-thread CTAs at 80
-// registers (24 warps); measured 1% faster on the 256-mesh mix and the 1024^3 soup.
+// Persistent CTAs of four warps; a warp takes one item (a triangle, or 32 z-slices of a larger one) at
+// a time.  Lane = slice: the YZ tests' interval of y and the ZX tests' bounds on x.  Lane = y: the XY
+// tests' bounds on x, into a table of the warp in shared memory (kRowsWindow values of y at a time).
+// Then the item's rows, 32 at a time, one per lane: the row's slice is found by counting the slices that
+// start at or before it, its bounds on x are read from both tables, the plane test narrows them to
+// the row's exact interval, and the interval is ORed into the table.
+// Bound by the L2's scattered atomics on large tables, by instructions and, with few items, by the
+// latency of one item elsewhere.  The soup of 2 M triangles at 1024^3: 27.2 ms for 3.36 G word updates
+// (124 G/s); 39.8 ms with all eight x-dependent tests evaluated per row (41 G warp instructions).  The
+// soup of 300,000 at 300^3 402 us / 701 us.  Six CTAs per SM at 80 registers; seven or eight spill and
+// are no faster.  Reading a word before the atomic, to skip it where its bits are set, cost as many L2
+// requests as it saved: 27.4 - 28.2 ms, and 30% to 90% more where the table fits the L2.
 constexpr uint32_t kRowsCtaThreads = 128;
+constexpr int kRowsWindow = 128;
+
+struct RowsWarp {
+	float4 xy[kRowsWindow];  // per y of the window: bounds of x from the XY tests, ny * py
+	float4 slice[32];        // per slice with rows in the window: start - first y, z, bounds of x from the ZX tests
+	float kz[32];            // and its nz * pz
+};
 
 template <class P>
-__global__ void __launch_bounds__(kRowsCtaThreads, 7) surf_rows(const __grid_constant__ LaunchDesc L) {
+__global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_constant__ LaunchDesc L) {
+	static_assert(P::plane == 2 && P::edge_xy == 1 && P::edge_yz == 1 && P::edge_zx == 2,
+	              "the one-test bounds follow the pinned fused-multiply-add pattern");
+	__shared__ RowsWarp s_warp[kRowsCtaThreads / 32];
 	const uint32_t lane = threadIdx.x & 31u;
+	RowsWarp& W = s_warp[threadIdx.x >> 5];
 	Counters* C = L.scr.ctr;
 	// One thread per CTA reads the queue counters (thousands of warps reading one line would
 	// serialise on its L2 slice), the CTA shares them through shared memory.
@@ -197,32 +218,8 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 7) surf_rows(const __grid_con
 	for (;;) {
 		unsigned long long tk = 0;
 		if (!wt.take(&C->ticket, total, lane, tk)) break;
-		uint32_t job = 0, tri = 0, chunk = 0, ok = 0;
-		if (lane == 0) {
-			if (tk < n_big_items) {
-				if (n_big > 0) {
-					uint32_t lo = 0, hi = n_big - 1;
-					while (lo < hi) {
-						const uint32_t m = (lo + hi + 1) >> 1;
-						if (L.scr.big[m].item_begin <= tk) lo = m; else hi = m - 1;
-					}
-					const BigRec r = L.scr.big[lo];
-					job = r.job; tri = r.tri; chunk = (uint32_t)(tk - r.item_begin);
-					ok = tk >= r.item_begin && chunk < r.n_items;
-				}
-			} else {
-				const MidRec r = L.scr.mid[tk - n_big_items];
-				job = r.job; tri = r.tri;
-				ok = 1;
-			}
-			// never follow a malformed record (only possible after a queue overflow)
-			if (ok && (job >= L.n_jobs || tri >= job_at(L, job).n_tri)) ok = 0;
-		}
-		ok = __shfl_sync(FULL, ok, 0);
-		if (!ok) continue;
-		job = __shfl_sync(FULL, job, 0);
-		tri = __shfl_sync(FULL, tri, 0);
-		chunk = __shfl_sync(FULL, chunk, 0);
+		uint32_t job, tri, chunk = 0;
+		if (!queue_item(L, tk, n_big, n_big_items, lane, job, tri, chunk)) continue;
 		const JobDesc& J = job_at(L, job);
 		const float unit[3] = {J.unit[0], J.unit[1], J.unit[2]};
 		const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
@@ -235,63 +232,95 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 7) surf_rows(const __grid_con
 		for (int k = 0; k < 9; k++) t[k] = __shfl_sync(FULL, tv, k);
 		SurfTri S;
 		surf_setup<P>(t, J.bmin, unit, J.inv_unit, grid, S);
-		RowDirs D;
-		row_dirs(S, unit[0], D);
+		const bool product = plane_underflows(S);
+		float lo, hi;
+		plane_bounds(S, lo, hi);
+		const float plane_m = fmaxf(fabsf(lo), fabsf(hi)), plane_inv = __fdividef(-1.0f, S.nx * unit[0]);
+		const float bx0 = (float)S.bx0, bx1 = (float)S.bx1;
 
-		// y-interval of this lane's z-slice
-		const int z0 = S.bz0 + (int)(chunk * kZch);
-		const int zl = z0 + (int)lane;
-		int ya = 0, yb = -1;
-		if (zl <= S.bz1) {
-			const float pz = __fmul_rn(__int2float_rn(zl), unit[2]);
-			if (!y_interval<P>(S, unit[1], pz, ya, yb)) { ya = 0; yb = -1; }
-		}
-		const int cnt = yb - ya + 1;
-		int incl = cnt;
+		// this lane's z-slice
+		const int z = S.bz0 + (int)(chunk * kZch + lane);
+		float fy0 = (float)S.by0, fy1 = (float)S.by1, zx0 = bx0, zx1 = bx1, kz;
+		{
+			const float pz = __fmul_rn(__int2float_rn(z), unit[2]);
+			kz = __fmul_rn(S.nz, pz);
+			const float b0 = fy0, b1 = fy1;
 #pragma unroll
-		for (int d = 1; d < 32; d <<= 1) {
-			const int v = __shfl_up_sync(FULL, incl, d);
-			if (lane >= (uint32_t)d) incl += v;
-		}
-		const int R = __shfl_sync(FULL, incl, 31);
-		for (int base = 0; base < R; base += 32) {
-			const int k = base + (int)lane;
-			// slice s = first lane whose inclusive count exceeds k
-			int s = 0;
-#pragma unroll
-			for (int step = 16; step >= 1; step >>= 1) {
-				const int v = __shfl_sync(FULL, incl, s + step - 1);
-				if (v <= k) s += step;
+			for (int i = 0; i < 3; i++) {
+				clip_test(S.eyz[i][0], __fmul_rn(S.eyz[i][1], pz), S.dyz[i], unit[1], b0, b1, fy0, fy1);
+				clip_test(S.ezx[i][1], __fmul_rn(S.ezx[i][0], pz), S.dzx[i], unit[0], bx0, bx1, zx0, zx1);
 			}
-			s = min(s, 31);
-			const int incl_s = __shfl_sync(FULL, incl, s);
-			const int cnt_s = __shfl_sync(FULL, cnt, s);
-			const int ya_s = __shfl_sync(FULL, ya, s);
-			int y = 0, z = 0, xl = 0, xh = -1;
-			if (k < R) {
-				y = ya_s + (k - (incl_s - cnt_s));
-				z = z0 + s;
+		}
+		const bool rows = z <= S.bz1 && fy0 <= fy1 && zx0 <= zx1;
+		const int ya = rows ? (int)fy0 : 0x7FFFFFFF, yb = rows ? (int)fy1 : -1;
+		const int y_begin = __reduce_min_sync(FULL, ya), y_last = __reduce_max_sync(FULL, yb);
+		for (int yw = y_begin; yw <= y_last; yw += kRowsWindow) {
+			const int yw1 = min(yw + kRowsWindow - 1, y_last);
+			for (int y = yw + (int)lane; y <= yw1; y += 32) {
 				const float py = __fmul_rn(__int2float_rn(y), unit[1]);
-				const float pz = __fmul_rn(__int2float_rn(z), unit[2]);
-				RowK K;
-				row_consts<P>(S, py, pz, K);
-				if (!row_interval_fast<P>(S, D, K, unit[0], S.bx0, S.bx1, xl, xh)) xh = -1;
+				float x0 = bx0, x1 = bx1;
+#pragma unroll
+				for (int i = 0; i < 3; i++)
+					clip_test(S.exy[i][0], __fmul_rn(S.exy[i][1], py), S.dxy[i], unit[0], bx0, bx1, x0, x1);
+				W.xy[y - yw] = make_float4(x0, x1, __fmul_rn(S.ny, py), 0.0f);
 			}
-			// Short rows are written by their own lane.  Long rows are written by the whole warp, one
-			// row at a time with the lanes on consecutive words (linear) or x groups (Morton): a
-			// scattered atomic costs an L2 transaction of its own, a warp's atomics on one row
-			// share a few lines.
-			const bool has = xh >= xl;
-			const bool wide = has && (morton ? (xh >> 2) - (xl >> 2) >= 4 : (xh >> 5) - (xl >> 5) >= 2);
-			if (has && !wide) write_row(table, morton, narrow, grid, y, z, xl, xh);
-			uint32_t todo = __ballot_sync(FULL, wide);
-			while (todo) {
-				const int src = __ffs(todo) - 1;
-				todo &= todo - 1u;
-				const int ry = __shfl_sync(FULL, y, src), rz = __shfl_sync(FULL, z, src);
-				const int rl = __shfl_sync(FULL, xl, src), rh = __shfl_sync(FULL, xh, src);
-				write_row_warp(table, morton, narrow, grid, ry, rz, rl, rh, lane);
+			const int first = max(ya, yw);
+			const uint32_t cnt = rows ? (uint32_t)max(min(yb, yw1) - first + 1, 0) : 0u;
+			uint32_t incl = cnt;
+#pragma unroll
+			for (int d = 1; d < 32; d <<= 1) {
+				const uint32_t v = __shfl_up_sync(FULL, incl, d);
+				if (lane >= (uint32_t)d) incl += v;
 			}
+			const uint32_t R = __shfl_sync(FULL, incl, 31), start = incl - cnt;
+			const uint32_t slot = __popc(__ballot_sync(FULL, cnt != 0u) & ((1u << lane) - 1u));
+			if (cnt) {
+				W.slice[slot] = make_float4(__int_as_float((int)start - first), __int_as_float(z), zx0, zx1);
+				W.kz[slot] = kz;
+			}
+			__syncwarp();
+			uint32_t begun = 0;  // slices that start before this step's rows
+			for (uint32_t base = 0; base < R; base += 32) {
+				const uint32_t at = start - base;
+				const uint32_t starts = __reduce_or_sync(FULL, cnt && at < 32u ? 1u << at : 0u);
+				const uint32_t rec = begun + __popc(starts & (0xFFFFFFFFu >> (31u - lane))) - 1u;
+				begun += __popc(starts);
+				const uint32_t k = base + lane;
+				int y = 0, rz = 0, xl = 0, xh = -1;
+				if (k < R) {
+					const float4 q = W.slice[rec];
+					y = (int)k - __float_as_int(q.x);
+					rz = __float_as_int(q.y);
+					const float4 e = W.xy[y - yw];
+					float x0 = fmaxf(q.z, e.x), x1 = fminf(q.w, e.y);
+					if (!product) {
+						clip_plane(S.nx, e.z, W.kz[rec], lo, hi, plane_m, plane_inv, unit[0], bx0, bx1, x0, x1);
+						if (x0 <= x1) { xl = (int)x0; xh = (int)x1; }
+					} else {  // a plane offset so small that the test's product may underflow: all tests together
+						RowK K;
+						row_consts<P>(S, __fmul_rn(__int2float_rn(y), unit[1]), __fmul_rn(__int2float_rn(rz), unit[2]), K);
+						RowDirs D;
+						row_dirs(S, unit[0], D);
+						if (!row_interval<P>(S, D, K, unit[0], xl, xh)) xh = -1;
+					}
+				}
+				// Short rows are written by their own lane.  Long rows are written by the whole warp, one
+				// row at a time with the lanes on consecutive words (linear) or x groups (Morton): a
+				// scattered atomic costs an L2 transaction of its own, a warp's atomics on one row
+				// share a few lines.
+				const bool has = xh >= xl;
+				const bool wide = has && (morton ? (xh >> 2) - (xl >> 2) >= 4 : (xh >> 5) - (xl >> 5) >= 2);
+				if (has && !wide) write_row(table, morton, narrow, grid, y, rz, xl, xh);
+				uint32_t todo = __ballot_sync(FULL, wide);
+				while (todo) {
+					const int src = __ffs(todo) - 1;
+					todo &= todo - 1u;
+					const int wy = __shfl_sync(FULL, y, src), wz = __shfl_sync(FULL, rz, src);
+					const int wl = __shfl_sync(FULL, xl, src), wh = __shfl_sync(FULL, xh, src);
+					write_row_warp(table, morton, narrow, grid, wy, wz, wl, wh, lane);
+				}
+			}
+			__syncwarp();  // the tables are rewritten for the next window or item
 		}
 	}
 }

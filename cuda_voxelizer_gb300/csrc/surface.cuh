@@ -445,6 +445,95 @@ __device__ __forceinline__ int row_interval_cert(const SurfTri& S, const RowDirs
 	return 1;
 }
 
+// One test at a time, for the rasterization of a whole triangle (surf_rows).  Every edge test has the
+// form "fails iff fma(a, fl(x * u), k) < -d" in one grid coordinate x, with a triangle constant a and
+// a k that is fixed along x: a YZ test in y and a ZX test in x are fixed by the slice, an XY test in x
+// by the row's y alone.  So the bounds that the ZX tests put on x are found once per slice, those of
+// the XY tests once per y, and a row is left with its plane test.
+//
+// As in row_interval_cert, the test agrees with its real counterpart, whose root is estimated as xe,
+// at every integer further than B from xe; with B < 1/4 only the integer nearest to xe is left, and
+// that one is evaluated.  (B < 1/4 implies |xe| < 2^18, so adding 1.5 * 2^23 rounds to that integer.)
+
+// First integer of [b0, b1 + 1) at which the test stops failing (a > 0) or starts to (a < 0); b1 + 1 if
+// there is none: the test is monotone in x.  For the estimates that are not good enough.
+static __device__ __noinline__ float test_change(float a, float k, float nd, float u, float b0, float b1) {
+	int l = (int)b0, r = (int)b1 + 1;
+	while (l < r) {
+		const int m = l + ((r - l) >> 1);
+		const bool fails = __fmaf_rn(a, __fmul_rn(__int2float_rn(m), u), k) < nd;
+		if (fails == (a < 0.0f)) r = m; else l = m + 1;
+	}
+	return __int2float_rn(l);
+}
+
+// Intersect [lo, hi] with the integers of [b0, b1] at which the test passes.  `a` is the same in every
+// lane of the warp.
+__device__ __forceinline__ void clip_test(float a, float k, float d, float u, float b0, float b1, float& lo, float& hi) {
+	if (a > 0.0f || a < 0.0f) {
+		const float inv = __fdividef(-1.0f, a * u);
+		const float xe = __fmul_rn(__fadd_rn(k, d), inv);
+		const float B = 0x1p-20f * fmaf(fabsf(k) + fabsf(d), fabsf(inv), fabsf(xe) + 1.0f);
+		float n = __fsub_rn(__fadd_rn(xe, 12582912.0f), 12582912.0f);
+		const bool fails = __fmaf_rn(a, __fmul_rn(n, u), k) < -d;
+		const bool good = (B < 0.25f) & (inv != 0.0f);  // false for NaN too
+		if (a > 0.0f) {
+			n = fails ? n + 1.0f : n;
+			if (!good) n = test_change(a, k, -d, u, b0, b1);
+			lo = fmaxf(lo, n);
+		} else {
+			n = fails ? n - 1.0f : n;
+			if (!good) n = test_change(a, k, -d, u, b0, b1) - 1.0f;
+			hi = fminf(hi, n);
+		}
+	} else if (a == 0.0f && k < -d) {
+		hi = lo - 1.0f;  // the test does not depend on x, and fails
+	}
+}
+
+// The plane test of a row, "fails iff s < lo or s > hi" with s(x) = fl(fl(fma(nx, fl(x * u), kpl)) + kpl2)
+// (plane_bounds; not for plane_underflows() triangles), monotone in x with the sign of nx.
+static __device__ __noinline__ float plane_change(float nx, float kpl, float kpl2, float bound, bool below, float u,
+                                                  float b0, float b1) {
+	// below: the side s < bound, else s > bound.  That side fails on a prefix of x iff (nx > 0) == below.
+	const bool prefix = (nx > 0.0f) == below;
+	int l = (int)b0, r = (int)b1 + 1;
+	while (l < r) {
+		const int m = l + ((r - l) >> 1);
+		const float s = __fadd_rn(__fmaf_rn(nx, __fmul_rn(__int2float_rn(m), u), kpl), kpl2);
+		const bool fails = below ? s < bound : s > bound;
+		if (fails != prefix) r = m; else l = m + 1;
+	}
+	return __int2float_rn(l);
+}
+
+// Intersect [x0, x1] with the integers of [b0, b1] at which the row passes the plane test; inv is
+// __fdividef(-1, nx * u), m the bound on its operands max(|lo|, |hi|).
+__device__ __forceinline__ void clip_plane(float nx, float kpl, float kpl2, float lo, float hi, float m, float inv,
+                                           float u, float b0, float b1, float& x0, float& x1) {
+	if (nx > 0.0f || nx < 0.0f) {
+		const float first = nx > 0.0f ? lo : hi, last = nx > 0.0f ? hi : lo;  // bounds of the lower and upper end
+		const float kp = __fadd_rn(kpl, kpl2);
+		const float e0 = __fmul_rn(__fsub_rn(kp, first), inv), e1 = __fmul_rn(__fsub_rn(kp, last), inv);
+		const float B = 0x1p-20f * fmaf(fabsf(kpl) + fabsf(kpl2) + m, fabsf(inv), fmaxf(fabsf(e0), fabsf(e1)) + 1.0f);
+		float n0 = __fsub_rn(__fadd_rn(e0, 12582912.0f), 12582912.0f), n1 = __fsub_rn(__fadd_rn(e1, 12582912.0f), 12582912.0f);
+		const float s0 = __fadd_rn(__fmaf_rn(nx, __fmul_rn(n0, u), kpl), kpl2);
+		const float s1 = __fadd_rn(__fmaf_rn(nx, __fmul_rn(n1, u), kpl), kpl2);
+		const bool f0 = nx > 0.0f ? s0 < first : s0 > first, f1 = nx > 0.0f ? s1 > last : s1 < last;
+		n0 = f0 ? n0 + 1.0f : n0;
+		n1 = f1 ? n1 - 1.0f : n1;
+		if (!((B < 0.25f) & (inv != 0.0f))) {
+			n0 = plane_change(nx, kpl, kpl2, first, nx > 0.0f, u, b0, b1);
+			n1 = plane_change(nx, kpl, kpl2, last, nx < 0.0f, u, b0, b1) - 1.0f;
+		}
+		x0 = fmaxf(x0, n0);
+		x1 = fminf(x1, n1);
+	} else if (nx == 0.0f) {
+		const float s = __fadd_rn(__fmaf_rn(nx, __fmul_rn(b0, u), kpl), kpl2);
+		if ((s < lo) | (s > hi)) x1 = x0 - 1.0f;
+	}
+}
+
 // Exact x-interval of a row within [bx0, bx1]: the certified computation, or the walk where that
 // declines.
 template <class P>
@@ -491,11 +580,6 @@ __device__ __forceinline__ bool y_interval_in(const SurfTri& S, float uy, float 
 	}
 	yb = f;
 	return true;
-}
-
-template <class P>
-__device__ __forceinline__ bool y_interval(const SurfTri& S, float uy, float pz, int& ya, int& yb) {
-	return y_interval_in<P>(S, uy, pz, S.by0, S.by1, ya, yb);
 }
 
 // The writers below come in two code types C: uint64_t in general, uint32_t for JOB_NARROW jobs

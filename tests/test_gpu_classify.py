@@ -75,7 +75,7 @@ def test_bins(rsqrt, ext, morton):
 
 @pytest.mark.parametrize("n", [1, 3, 4, 5, 31, 33, 127, 129, 8500, 17100, 34100, 68200, 136300])
 def test_launch_shapes(rsqrt, n):
-    """Ragged groups, and triangles per warp of 4, 8, 16 and 32 (136,192 triangles are 1,064 tiles)."""
+    """Ragged groups, and triangles per warp of 4, 8, 16 and 32 (the last from about 900 tiles of 128 on)."""
     _check(rsqrt, _triangles(n, n, (4, 4, 4), 128), 128, False)
 
 
@@ -103,3 +103,23 @@ def test_grid_aligned_triangles(rsqrt):
     t[1::3, :, 1] = t[1::3, :1, 1]
     t[2::3, :, 2] = t[2::3, :1, 2]
     _check(rsqrt, t.reshape(-1, 9), 64, False)
+
+
+@pytest.mark.parametrize("morton", [False, True])
+@pytest.mark.parametrize("ext", [
+    (100, 120, 31), (100, 120, 33), (100, 129, 70), (20, 300, 40), (1, 200, 200),  # windows of 128 y, items of 32 z
+    (300, 200, 1), (300, 1, 200), (400, 0.5, 0.5), (0.2, 300, 300),                # one row of y or z, thin in x
+])
+def test_large_triangles(rsqrt, ext, morton):
+    _check(rsqrt, _triangles(5, 60, ext, 512), 512, morton)
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("tilt", [0.0, 1e-6, 1e-4, 1e-2])
+def test_large_triangles_nearly_parallel_to_an_axis(rsqrt, axis, tilt):
+    """Edges and planes whose tests hardly depend on a coordinate: estimates that are not good enough."""
+    rng = np.random.default_rng(axis)
+    t = _triangles(9, 80, (200, 200, 200), 256).reshape(-1, 3, 3)
+    t[:40, :, axis] = t[:40, :1, axis] + tilt * rng.uniform(-1, 1, (40, 3))        # the plane
+    t[40:, 1, axis] = t[40:, 0, axis] + tilt * rng.uniform(-1, 1, 40)              # one edge
+    _check(rsqrt, t.reshape(-1, 9).astype(np.float32), 256, False)
