@@ -99,6 +99,9 @@ SIGNATURES = {
     "cvx_transcode": (c_status, [vp, vp, u32, ctypes.c_int, vp]),
     "cvx_encode_binvox": (c_status, [ctypes.POINTER(CvxVoxinfo), vp, vp, u64, ctypes.POINTER(u64), vp]),
     "cvx_encode_voxel_list": (c_status, [ctypes.POINTER(CvxVoxinfo), vp, vp, u64, ctypes.POINTER(u64), vp]),
+    "cvx_encode_workspace_size": (u64, [ctypes.POINTER(CvxVoxinfo)]),
+    "cvx_encode_binvox_ws": (c_status, [ctypes.POINTER(CvxVoxinfo), vp, vp, u64, vp, u64, ctypes.POINTER(u64), vp]),
+    "cvx_encode_voxel_list_ws": (c_status, [ctypes.POINTER(CvxVoxinfo), vp, vp, u64, vp, u64, ctypes.POINTER(u64), vp]),
     "cvx_get_tuning": (c_status, [ctypes.c_int, ctypes.POINTER(CvxTuning)]),
     "cvx_set_tuning": (c_status, [ctypes.c_int, ctypes.POINTER(CvxTuning)]),
     "cvx_profile_enable": (c_status, [ctypes.c_int]),

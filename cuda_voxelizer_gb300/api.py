@@ -536,16 +536,52 @@ def transcode(table, gridsize: int, to_morton: bool, stream=None):
     return out
 
 
+def _encode_scratch(info: VoxInfo, table, stream):
+    """Scratch of the encoders, allocated on the stream that uses it."""
+    import contextlib
+
+    import torch
+    on = contextlib.nullcontext()
+    if stream is not None:
+        on = torch.cuda.stream(torch.cuda.ExternalStream(stream) if isinstance(stream, int) else stream)
+    with on:
+        return torch.empty(int(lib.cvx_encode_workspace_size(ctypes.byref(info))), dtype=torch.uint8, device=table.device)
+
+
+_bytes_new = ctypes.pythonapi.PyBytes_FromStringAndSize
+_bytes_new.argtypes, _bytes_new.restype = [ctypes.c_void_p, ctypes.c_ssize_t], ctypes.py_object
+_bytes_data = ctypes.pythonapi.PyBytes_AsString
+_bytes_data.argtypes, _bytes_data.restype = [ctypes.py_object], ctypes.c_void_p
+
+
+def _to_bytes(t) -> bytes:
+    """A uint8 CUDA tensor as bytes: copied straight into the new object (the C API's way of filling
+    one), where .cpu().numpy().tobytes() copies a second time into memory that faults in page by page."""
+    import torch
+    n = t.numel()
+    if n == 0:
+        return b""
+    out = _bytes_new(None, n)
+    torch.frombuffer((ctypes.c_char * n).from_address(_bytes_data(out)), dtype=torch.uint8).copy_(t)
+    return out
+
+
 def encode_binvox(info: VoxInfo, table, stream=None) -> bytes:
     """binvox run-length payload of a linear-order device table (the bytes after the header)."""
     import torch
+    ws = _encode_scratch(info, table, stream)
     n = ctypes.c_uint64()
-    check(lib.cvx_encode_binvox(ctypes.byref(info), _ptr(table), None, 0, ctypes.byref(n), _stream(stream)),
-          "cvx_encode_binvox")
-    out = torch.empty(max(1, n.value), dtype=torch.uint8, device=table.device)
-    check(lib.cvx_encode_binvox(ctypes.byref(info), _ptr(table), _ptr(out), n.value, ctypes.byref(n),
-                                _stream(stream)), "cvx_encode_binvox")
-    return out[:n.value].cpu().numpy().tobytes()
+    # Closed meshes need about 2 bytes per 255 voxels and a few per line along y: a fifth to a third of
+    # the table.  A payload that does not fit is encoded again, into a buffer of its size.
+    capacity = max(4 * table_words(info), 1 << 16)
+    while True:
+        out = torch.empty(capacity, dtype=torch.uint8, device=table.device)
+        st = lib.cvx_encode_binvox_ws(ctypes.byref(info), _ptr(table), _ptr(ws), ws.numel(), _ptr(out), capacity,
+                                      ctypes.byref(n), _stream(stream))
+        if n.value <= capacity:
+            check(st, "cvx_encode_binvox_ws")
+            return _to_bytes(out[:n.value])
+        capacity = n.value
 
 
 def binvox_header(info: VoxInfo) -> bytes:
@@ -564,10 +600,11 @@ def binvox_header(info: VoxInfo) -> bytes:
 def encode_voxel_list(info: VoxInfo, table, stream=None):
     """The (x, gz - z, y) int32 triples write_vox hands to its MagicaVoxel writer, in its order."""
     import torch
+    ws = _encode_scratch(info, table, stream)
     n = ctypes.c_uint64()
-    check(lib.cvx_encode_voxel_list(ctypes.byref(info), _ptr(table), None, 0, ctypes.byref(n), _stream(stream)),
-          "cvx_encode_voxel_list")
+    check(lib.cvx_encode_voxel_list_ws(ctypes.byref(info), _ptr(table), _ptr(ws), ws.numel(), None, 0, ctypes.byref(n),
+                                       _stream(stream)), "cvx_encode_voxel_list_ws")
     out = torch.empty((max(1, n.value), 3), dtype=torch.int32, device=table.device)
-    check(lib.cvx_encode_voxel_list(ctypes.byref(info), _ptr(table), _ptr(out), n.value, ctypes.byref(n),
-                                    _stream(stream)), "cvx_encode_voxel_list")
+    check(lib.cvx_encode_voxel_list_ws(ctypes.byref(info), _ptr(table), _ptr(ws), ws.numel(), _ptr(out), n.value,
+                                       ctypes.byref(n), _stream(stream)), "cvx_encode_voxel_list_ws")
     return out[:n.value]

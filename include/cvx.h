@@ -267,11 +267,20 @@ cvx_status cvx_transcode(const uint32_t* d_src, uint32_t* d_dst, uint32_t gridsi
  * temporary device memory. */
 cvx_status cvx_encode_binvox(const cvx_voxinfo* info, const uint32_t* d_table, uint8_t* d_out, uint64_t out_capacity,
                              uint64_t* out_bytes, cvx_stream_t stream);
+/* The same with caller-owned scratch: d_ws of cvx_encode_workspace_size(info) bytes, 256-byte aligned
+ * (one size serves both encoders; 0 for an empty grid).  Nothing is written to d_out when it is too
+ * small. */
+uint64_t cvx_encode_workspace_size(const cvx_voxinfo* info);
+cvx_status cvx_encode_binvox_ws(const cvx_voxinfo* info, const uint32_t* d_table, void* d_ws, uint64_t ws_bytes,
+                                uint8_t* d_out, uint64_t out_capacity, uint64_t* out_bytes, cvx_stream_t stream);
 /* The voxels write_vox hands to VoxWriter::AddVoxel (src/util_io.cpp:264-280), in its order, as
  * int32 triples (x, gz - z, y) into d_xyz (3 * capacity int32).  Needs gridsize y == z.
  * *out_count receives the number of set voxels; d_xyz == NULL computes only that.  Synchronizes. */
 cvx_status cvx_encode_voxel_list(const cvx_voxinfo* info, const uint32_t* d_table, int32_t* d_xyz, uint64_t capacity,
                                  uint64_t* out_count, cvx_stream_t stream);
+/* The same with caller-owned scratch (cvx_encode_workspace_size). */
+cvx_status cvx_encode_voxel_list_ws(const cvx_voxinfo* info, const uint32_t* d_table, void* d_ws, uint64_t ws_bytes,
+                                    int32_t* d_xyz, uint64_t capacity, uint64_t* out_count, cvx_stream_t stream);
 
 /* ---- tuning ---------------------------------------------------------------------------------- */
 

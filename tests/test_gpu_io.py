@@ -146,3 +146,60 @@ def test_gather_soup_matches_indexing_and_flags_bad_faces():
     soup, bad = cv.gather_soup(torch.from_numpy(verts).cuda(), torch.from_numpy(faces).cuda())
     s = soup.cpu().numpy().reshape(-1, 9)
     assert bad == 2 and np.isnan(s[[3, 77]]).all() and not np.isnan(np.delete(s, [3, 77], axis=0)).any()
+
+
+def _pattern(grid, kind, seed):
+    """A linear-order table: bits of the given density, or boxes, whose runs are long."""
+    rng = np.random.default_rng(seed)
+    v = np.zeros((grid[2], grid[1], grid[0]), dtype=np.uint8)
+    if kind == "boxes":
+        for _ in range(4):
+            a, b = (np.sort(rng.integers(0, np.array(grid) + 1, (2, 3)), axis=0))
+            v[a[2]:b[2], a[1]:b[1], a[0]:b[0]] ^= 1
+    elif kind == "full":
+        v[:] = 1
+    elif kind != "empty":
+        v[:] = rng.random(v.shape) < float(kind)
+    bits = np.concatenate([v.reshape(-1), np.zeros(-v.size % 32, np.uint8)])
+    return np.packbits(bits).view(np.uint32).byteswap()
+
+
+ENCODE_GRIDS = [(1, 1, 1), (2, 3, 5), (5, 16, 16), (40, 17, 17), (33, 31, 31), (32, 32, 32), (31, 33, 33), (64, 64, 64),
+                (100, 100, 100), (7, 255, 255), (9, 256, 256), (130, 96, 96), (300, 65, 65), (3, 500, 500),
+                (40, 1, 700), (40, 16, 300), (64, 64, 20), (50, 290, 31)]
+
+
+@pytest.mark.parametrize("kind", ["empty", "full", "boxes", "0.5", "0.01"])
+@pytest.mark.parametrize("grid", ENCODE_GRIDS)
+def test_encoders_on_any_grid(grid, kind):
+    """Stream rows that end inside, on and before words, dense streams (gy <= 16), one tile and many."""
+    table = _pattern(grid, kind, sum(grid))
+    info = cv.make_info((0, 0, 0), [float(g) for g in grid], grid, 0)
+    d = _dev(table)
+    assert cv.encode_binvox(info, d) == oracle.binvox_payload(bytes(info), table)
+    if grid[1] == grid[2]:
+        got = cv.encode_voxel_list(info, d).cpu().numpy()
+        assert np.array_equal(got, oracle.vox_list(bytes(info), table)[:got.shape[0]])
+        assert got.shape[0] == int(np.unpackbits(table.view(np.uint8)).sum())
+
+
+def test_encoders_refuse_small_buffers_and_write_nothing():
+    import ctypes
+    grid = (40, 33, 33)
+    table = _pattern(grid, "0.5", 1)
+    info = cv.make_info((0, 0, 0), [float(g) for g in grid], grid, 0)
+    d = _dev(table)
+    payload = oracle.binvox_payload(bytes(info), table)
+    n_vox = int(np.unpackbits(table.view(np.uint8)).sum())
+    s = torch.cuda.current_stream().cuda_stream
+    n = ctypes.c_uint64()
+    for f, size, dtype, unit in ((cv.lib.cvx_encode_binvox, len(payload), torch.uint8, 1),
+                                 (cv.lib.cvx_encode_voxel_list, n_vox, torch.int32, 3)):
+        out = torch.full((size * unit + 8,), 77, dtype=dtype, device="cuda")
+        assert f(ctypes.byref(info), d.data_ptr(), out.data_ptr(), size - 1, ctypes.byref(n), s) == 1
+        assert n.value == size and bool((out == 77).all())
+        assert f(ctypes.byref(info), d.data_ptr(), out.data_ptr(), size, ctypes.byref(n), s) == 0
+        assert n.value == size and bool((out[size * unit:] == 77).all())
+        ws = torch.empty(256, dtype=torch.uint8, device="cuda")
+        g = cv.lib.cvx_encode_binvox_ws if unit == 1 else cv.lib.cvx_encode_voxel_list_ws
+        assert g(ctypes.byref(info), d.data_ptr(), ws.data_ptr(), 256, out.data_ptr(), size, ctypes.byref(n), s) == 1
