@@ -95,6 +95,8 @@ SIGNATURES = {
     "cvx_server_destroy": (c_status, [vp]),
     "cvx_mesh_bbox_device": (c_status, [vp, u64, vp, vp, vp]),
     "cvx_voxinfo_from_device": (c_status, [vp, u64, vp, ctypes.POINTER(CvxVoxinfo), vp]),
+    "cvx_mesh_bbox_device_ws": (c_status, [vp, u64, vp, u64, vp, vp, vp]),
+    "cvx_voxinfo_from_device_ws": (c_status, [vp, u64, vp, vp, u64, ctypes.POINTER(CvxVoxinfo), vp]),
     "cvx_gather_soup": (c_status, [vp, u64, vp, u64, vp, vp, vp]),
     "cvx_transcode": (c_status, [vp, vp, u32, ctypes.c_int, vp]),
     "cvx_encode_binvox": (c_status, [ctypes.POINTER(CvxVoxinfo), vp, vp, u64, ctypes.POINTER(u64), vp]),

@@ -495,12 +495,29 @@ class Server:
 
 # ---- mesh ingest, layouts and output encoders on the GPU ------------------------------------------
 
+_BBOX_WORKSPACE = 256  # CVX_BBOX_WORKSPACE
+
+
+def _scratch(nbytes: int, device, stream):
+    """Temporary device memory from torch's allocator, allocated on the stream that uses it."""
+    import contextlib
+
+    import torch
+    on = contextlib.nullcontext()
+    if stream is not None:
+        on = torch.cuda.stream(torch.cuda.ExternalStream(stream) if isinstance(stream, int) else stream)
+    with on:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+
+
 def mesh_bbox_device(triangles, stream=None):
     """Vertex bounding box of a device triangle soup (CUDA tensor); host float32 arrays."""
     n = triangles.numel() // 9
     lo = (ctypes.c_float * 3)()
     hi = (ctypes.c_float * 3)()
-    check(lib.cvx_mesh_bbox_device(_ptr(triangles), n, lo, hi, _stream(stream)), "cvx_mesh_bbox_device")
+    ws = _scratch(_BBOX_WORKSPACE, triangles.device, stream)
+    check(lib.cvx_mesh_bbox_device_ws(_ptr(triangles), n, _ptr(ws), _BBOX_WORKSPACE, lo, hi, _stream(stream)),
+          "cvx_mesh_bbox_device_ws")
     return np.array(lo[:], dtype=np.float32), np.array(hi[:], dtype=np.float32)
 
 
@@ -510,8 +527,9 @@ def voxinfo_from_device(triangles, gridsize, stream=None) -> VoxInfo:
         gridsize = (gridsize, gridsize, gridsize)
     g = (ctypes.c_uint32 * 3)(*[int(x) for x in gridsize])
     info = VoxInfo()
-    check(lib.cvx_voxinfo_from_device(_ptr(triangles), triangles.numel() // 9, g, ctypes.byref(info),
-                                      _stream(stream)), "cvx_voxinfo_from_device")
+    ws = _scratch(_BBOX_WORKSPACE, triangles.device, stream)
+    check(lib.cvx_voxinfo_from_device_ws(_ptr(triangles), triangles.numel() // 9, g, _ptr(ws), _BBOX_WORKSPACE,
+                                         ctypes.byref(info), _stream(stream)), "cvx_voxinfo_from_device_ws")
     return info
 
 
@@ -537,15 +555,7 @@ def transcode(table, gridsize: int, to_morton: bool, stream=None):
 
 
 def _encode_scratch(info: VoxInfo, table, stream):
-    """Scratch of the encoders, allocated on the stream that uses it."""
-    import contextlib
-
-    import torch
-    on = contextlib.nullcontext()
-    if stream is not None:
-        on = torch.cuda.stream(torch.cuda.ExternalStream(stream) if isinstance(stream, int) else stream)
-    with on:
-        return torch.empty(int(lib.cvx_encode_workspace_size(ctypes.byref(info))), dtype=torch.uint8, device=table.device)
+    return _scratch(int(lib.cvx_encode_workspace_size(ctypes.byref(info))), table.device, stream)
 
 
 _bytes_new = ctypes.pythonapi.PyBytes_FromStringAndSize

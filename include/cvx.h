@@ -247,6 +247,12 @@ cvx_status cvx_mesh_bbox_device(const float* d_triangles, uint64_t n_triangles, 
 /* main()'s setup from a device soup: bounding box, createMeshBBCube, voxinfo (synchronizes). */
 cvx_status cvx_voxinfo_from_device(const float* d_triangles, uint64_t n_triangles, const uint32_t gridsize[3],
                                    cvx_voxinfo* out, cvx_stream_t stream);
+/* The same two with caller-owned scratch: CVX_BBOX_WORKSPACE bytes, 16-byte aligned. */
+#define CVX_BBOX_WORKSPACE 256
+cvx_status cvx_mesh_bbox_device_ws(const float* d_triangles, uint64_t n_triangles, void* d_ws, uint64_t ws_bytes,
+                                   float out_min[3], float out_max[3], cvx_stream_t stream);
+cvx_status cvx_voxinfo_from_device_ws(const float* d_triangles, uint64_t n_triangles, const uint32_t gridsize[3],
+                                      void* d_ws, uint64_t ws_bytes, cvx_voxinfo* out, cvx_stream_t stream);
 /* Indexed mesh -> soup: face f's vertices d_vertices[3*d_faces[3f+k] ..] become floats 9f..9f+8
  * of d_soup (the loop of meshToGPU_managed, src/main.cpp:68-77).  A face with an index >=
  * n_vertices is written as NaNs and counted into *d_bad_faces (device counter, may be NULL);

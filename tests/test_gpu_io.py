@@ -203,3 +203,25 @@ def test_encoders_refuse_small_buffers_and_write_nothing():
         ws = torch.empty(256, dtype=torch.uint8, device="cuda")
         g = cv.lib.cvx_encode_binvox_ws if unit == 1 else cv.lib.cvx_encode_voxel_list_ws
         assert g(ctypes.byref(info), d.data_ptr(), ws.data_ptr(), 256, out.data_ptr(), size, ctypes.byref(n), s) == 1
+
+
+@pytest.mark.parametrize("offset", [0, 1])  # 1: a soup that is not 16-byte aligned
+@pytest.mark.parametrize("n", [1, 2, 3, 255, 256, 257, 70_001])
+def test_bbox_and_gather_at_odd_sizes(n, offset):
+    rng = np.random.default_rng(n)
+    verts = rng.normal(size=(n + 2, 3)).astype(np.float32)
+    verts[rng.integers(0, n + 2)] *= 100  # an extreme corner anywhere, the ragged end included
+    faces = rng.integers(0, n + 2, size=(n, 3)).astype(np.int32)
+    faces[-1] = [n + 1, 0, n]
+    buf = torch.zeros(9 * n + 8, dtype=torch.float32, device="cuda")
+    soup = buf[offset:offset + 9 * n]
+    bad = torch.zeros(1, dtype=torch.int64, device="cuda")
+    v, f = torch.from_numpy(verts).cuda(), torch.from_numpy(faces).cuda()
+    s = torch.cuda.current_stream().cuda_stream
+    assert cv.lib.cvx_gather_soup(v.data_ptr(), n + 2, f.data_ptr(), n, soup.data_ptr(), bad.data_ptr(), s) == 0
+    host = buf.cpu().numpy()
+    want = verts[faces].reshape(-1)
+    assert int(bad.item()) == 0 and np.array_equal(host[offset:offset + 9 * n], want)
+    assert not host[:offset].any() and not host[offset + 9 * n:].any()
+    lo, hi = cv.mesh_bbox_device(soup)
+    assert np.array_equal(lo, want.reshape(-1, 3).min(0)) and np.array_equal(hi, want.reshape(-1, 3).max(0))
