@@ -87,10 +87,27 @@ def _ptr(x) -> int:
     raise TypeError(f"cannot take a device pointer of {type(x)}")
 
 
+_current_stream = None
+
+
+def _bind_current_stream():
+    """A function returning the raw handle of torch's current stream.  torch's own raw accessor takes
+    0.3 us where torch.cuda.current_stream().cuda_stream builds a stream object and takes 3 us, a tenth
+    of a small voxelization call."""
+    global _current_stream
+    import torch
+    torch.cuda.current_device()  # initializes torch's CUDA state
+    raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    if raw is None or device is None:
+        _current_stream = lambda: int(torch.cuda.current_stream().cuda_stream)  # noqa: E731
+    else:
+        _current_stream = lambda: raw(device())  # noqa: E731
+    return _current_stream
+
+
 def _stream(stream) -> int:
     if stream is None:
-        import torch
-        return int(torch.cuda.current_stream().cuda_stream)
+        return (_current_stream or _bind_current_stream())()
     if isinstance(stream, int):
         return stream
     return int(stream.cuda_stream)

@@ -392,6 +392,7 @@ struct Runner {
 	size_t jobs_off;
 	uint32_t bricks = 0;   // brick capacity of the record area (largest group's bricks)
 	bool timed = true;     // per-kernel events for cvx_profile_collect (callers on this thread only)
+	bool fresh = true;     // the counters are zero: the caller cleared the area before run()
 	const Prof* p() const { return timed ? prof() : nullptr; }
 
 	cvx_status prepare(Group& g, LaunchDesc& L) {
@@ -420,12 +421,18 @@ struct Runner {
 		return CVX_OK;
 	}
 
+	cvx_status reset_counters() {
+		if (!fresh) CVX_CUDA(cudaMemsetAsync(rec, 0, kCountersResetBytes, s));
+		fresh = false;
+		return CVX_OK;
+	}
+
 	cvx_status run(const std::vector<JobDesc>& surf, const std::vector<JobDesc>& solid) {
 		for (Group& g : make_groups(surf, false)) {
 			LaunchDesc L;
 			cvx_status st = prepare(g, L);
 			if (st != CVX_OK) return st;
-			CVX_CUDA(cudaMemsetAsync(rec, 0, kCountersResetBytes, s));
+			if ((st = reset_counters()) != CVX_OK) return st;
 			CVX_CUDA(launch_surface(L, dev.tune, dev.rows_grid, dev.raster_grid, s, p()));
 		}
 		if (!solid.empty()) {
@@ -433,7 +440,7 @@ struct Runner {
 				LaunchDesc L;
 				cvx_status st = prepare(g, L);
 				if (st != CVX_OK) return st;
-				CVX_CUDA(cudaMemsetAsync(rec, 0, kCountersResetBytes, s));
+				if ((st = reset_counters()) != CVX_OK) return st;
 				CVX_CUDA(launch_solid(L, dev.tune, dev.cols_grid, s, kSolidToggles, p()));
 			}
 			Group r = resolve_group(solid);
@@ -816,9 +823,10 @@ struct cvx_plan {
 constexpr int kPlanSurfaceLanes = 2;
 
 // One group's launches on a capturing stream, as Runner::run issues them but with the group's job
-// array (when it has more than one job) already resident at `jobs_dev`.
-static cudaError_t capture_group(const Group& g, bool solid, bool resolve, void* rec, uint64_t cap, uint32_t bricks,
-                                 JobDesc* jobs_dev, const DevState& dev, cudaStream_t s) {
+// array (when it has more than one job) already resident at `jobs_dev`.  `fresh`: the counters were
+// cleared just before.
+static cudaError_t capture_group(const Group& g, bool solid, bool resolve, bool fresh, void* rec, uint64_t cap,
+                                 uint32_t bricks, JobDesc* jobs_dev, const DevState& dev, cudaStream_t s) {
 	if (g.bricks > bricks) return cudaErrorInvalidValue;
 	LaunchDesc L;
 	std::memset(&L, 0, sizeof(L));
@@ -834,7 +842,7 @@ static cudaError_t capture_group(const Group& g, bool solid, bool resolve, void*
 	else
 		L.jobs = jobs_dev;
 	if (resolve) return launch_solid(L, dev.tune, dev.cols_grid, s, kSolidResolve, nullptr);
-	const cudaError_t e = cudaMemsetAsync(rec, 0, kCountersResetBytes, s);
+	const cudaError_t e = fresh ? cudaSuccess : cudaMemsetAsync(rec, 0, kCountersResetBytes, s);
 	if (e != cudaSuccess) return e;
 	return solid ? launch_solid(L, dev.tune, dev.cols_grid, s, kSolidToggles, nullptr)
 	             : launch_surface(L, dev.tune, dev.rows_grid, dev.raster_grid, s, nullptr);
@@ -1036,7 +1044,7 @@ cvx_status cvx_plan_create(const cvx_job* jobs, uint32_t n_jobs, uint32_t flags,
 		for (size_t gi = 0; gi < l.groups.size() && cst == CVX_OK; gi++) {
 			const Group& g = l.groups[gi];
 			const bool resolve = l.solid && gi + 1 == l.groups.size();
-			const cudaError_t e = capture_group(g, l.solid, resolve, rec, l.cap, l.bricks, p->job_area + used, dev, l.stream);
+			const cudaError_t e = capture_group(g, l.solid, resolve, gi == 0, rec, l.cap, l.bricks, p->job_area + used, dev, l.stream);
 			if (g.jobs.size() > 1) used += g.jobs.size();
 			if (e != cudaSuccess) cst = cuda_fail(e, "capture launch");
 		}
@@ -1349,6 +1357,7 @@ cvx_status cvx_plan_create_host(const cvx_host_job* jobs, uint32_t n_jobs, uint3
 	for (uint32_t i = 0; i < n_jobs; i++)
 		if (!overwrites(i)) ck(cudaMemsetAsync(jobs[i].d_table, 0, words_of(jobs[i].info) * 4, cs), "capture clear");
 	ck(cudaMemsetAsync(rec, 0, rec_layout(cap, 0, bricks).big, cs), "capture clear");
+	bool fresh = true;
 	for (const HostStep& st : steps) {
 		if (cst != CVX_OK) break;
 		switch (st.kind) {
@@ -1357,8 +1366,9 @@ cvx_status cvx_plan_create_host(const cvx_host_job* jobs, uint32_t n_jobs, uint3
 			break;
 		case HostStep::kLaunch:
 		case HostStep::kResolve:
-			ck(capture_group(st.g, st.solid, st.kind == HostStep::kResolve, rec, cap, bricks, p->job_area + st.slot, dev, cs),
+			ck(capture_group(st.g, st.solid, st.kind == HostStep::kResolve, fresh, rec, cap, bricks, p->job_area + st.slot, dev, cs),
 			   "capture launch");
+			fresh = false;
 			break;
 		case HostStep::kFinal: {
 			const cvx_host_job& J = jobs[st.job];

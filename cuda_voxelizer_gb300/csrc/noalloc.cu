@@ -217,7 +217,7 @@ extern "C" cvx_status cvx_voxelize_solid_noalloc(const cvx_voxinfo* info, const 
 		L.single.tris = d_triangles + off * 9;
 		L.single.n_tri = n;
 		L.n_tiles = (uint32_t)((n + kTile - 1) / kTile);
-		if ((st = cuda_status(cudaMemsetAsync(scr, 0, kCountersResetBytes, s), "cudaMemsetAsync(counters)")) != CVX_OK)
+		if (off && (st = cuda_status(cudaMemsetAsync(scr, 0, kCountersResetBytes, s), "cudaMemsetAsync(counters)")) != CVX_OK)
 			return st;
 		if ((st = cuda_status(launch_solid(L, tune, cols_grid, s, kSolidToggles, nullptr), "solid toggles")) != CVX_OK)
 			return st;
