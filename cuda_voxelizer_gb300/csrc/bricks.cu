@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kBinThreads) brick_bin(const __grid_constant__
 	__syncthreads();
 	const uint32_t n = min(s_n, L.scr.cap);
 	if ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) >= n) return;
-	WarpTickets wt(n, gridDim.x * (blockDim.x >> 5));
+	WarpTickets wt(n, blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), gridDim.x * (blockDim.x >> 5));
 	for (;;) {
 		unsigned long long tk = 0;
 		if (!wt.take(&C->bticket, n, lane, tk)) break;
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(kBinThreads) brick_fill(const __grid_constant_
 	__syncthreads();
 	const uint32_t n = min(s_n, L.scr.cap);
 	if ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) >= n) return;
-	WarpTickets wt(n, gridDim.x * (blockDim.x >> 5));
+	WarpTickets wt(n, blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), gridDim.x * (blockDim.x >> 5));
 	for (;;) {
 		unsigned long long tk = 0;
 		if (!wt.take(&C->fticket, n, lane, tk)) break;
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kRowsThreads, 3) brick_raster(const __grid_con
 	Counters* C = L.scr.ctr;
 	const uint32_t units = *reinterpret_cast<volatile unsigned*>(&C->units);
 	if ((uint64_t)blockIdx.x * kRasterWarps + warp >= units) return;
-	WarpTickets wt(units, gridDim.x * kRasterWarps);
+	WarpTickets wt(units, blockIdx.x * kRasterWarps + warp, gridDim.x * kRasterWarps);
 	for (;;) {
 		unsigned long long tk = 0;
 		if (!wt.take(&C->rticket, units, lane, tk)) break;

@@ -353,36 +353,12 @@ __global__ void __launch_bounds__(kRowsThreads) solid_cols(const __grid_constant
 	// Warps beyond the number of queued items have nothing to claim: they leave without touching
 	// the ticket counter (all of them do when only small triangles were queued).
 	if ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) >= total) return;
-	WarpTickets wt(total, gridDim.x * (blockDim.x >> 5));
+	WarpTickets wt(total, blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), gridDim.x * (blockDim.x >> 5));
 	for (;;) {
 		unsigned long long tk = 0;
 		if (!wt.take(&C->ticket, total, lane, tk)) break;
-		uint32_t job = 0, tri = 0, chunk = 0, ok = 0;
-		if (lane == 0) {
-			if (tk < n_big_items) {
-				if (n_big > 0) {
-					uint32_t lo = 0, hi = n_big - 1;
-					while (lo < hi) {
-						const uint32_t m = (lo + hi + 1) >> 1;
-						if (L.scr.big[m].item_begin <= tk) lo = m; else hi = m - 1;
-					}
-					const BigRec r = L.scr.big[lo];
-					job = r.job; tri = r.tri; chunk = (uint32_t)(tk - r.item_begin);
-					ok = tk >= r.item_begin && chunk < r.n_items;
-				}
-			} else {
-				const MidRec r = L.scr.mid[tk - n_big_items];
-				job = r.job; tri = r.tri;
-				ok = 1;
-			}
-			// never follow a malformed record (only possible after a queue overflow)
-			if (ok && (job >= L.n_jobs || tri >= job_at(L, job).n_tri)) ok = 0;
-		}
-		ok = __shfl_sync(FULL, ok, 0);
-		if (!ok) continue;
-		job = __shfl_sync(FULL, job, 0);
-		tri = __shfl_sync(FULL, tri, 0);
-		chunk = __shfl_sync(FULL, chunk, 0);
+		uint32_t job, tri, chunk;
+		if (!queue_item(L, tk, n_big, n_big_items, lane, job, tri, chunk)) continue;
 		const JobDesc& J = job_at(L, job);
 		const float unit[3] = {J.unit[0], J.unit[1], J.unit[2]};
 		const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
@@ -448,7 +424,7 @@ __global__ void __launch_bounds__(256, 6) solid_resolve(const __grid_constant__ 
 	const uint32_t unit_id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	if (unit_id >= L.n_units) return;
 	const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-	const uint32_t j = job_search(L, unit_id, [](const JobDesc& d) { return (uint64_t)d.unit_begin; });
+	const uint32_t j = warp_job(L, unit_id, [](const JobDesc& d) { return (uint64_t)d.unit_begin; });
 	const JobDesc& J = job_at(L, j);
 	const uint32_t gx = J.grid[0];
 	const uint64_t bits = (uint64_t)gx * J.grid[1] * J.grid[2];
@@ -561,7 +537,7 @@ __global__ void __launch_bounds__(kMortonThreads, 7) solid_morton_cols(const __g
 	const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	if (warp >= L.n_mwarps) return;
 	const uint32_t lane = threadIdx.x & 31u;
-	const uint32_t j = job_search(L, warp, [](const JobDesc& d) { return d.mwarp_begin; });
+	const uint32_t j = warp_job(L, warp, [](const JobDesc& d) { return d.mwarp_begin; });
 	const JobDesc& J = job_at(L, j);
 	const uint32_t lg = 31u - __clz(J.grid[0]);
 	const MortonCols m = morton_cols(lg);
@@ -660,7 +636,7 @@ __global__ void __launch_bounds__(256) solid_morton_small(const __grid_constant_
 __global__ void __launch_bounds__(256) solid_zero(const __grid_constant__ LaunchDesc L) {
 	const uint32_t unit_id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	if (unit_id >= L.n_units) return;
-	const uint32_t j = job_search(L, unit_id, [](const JobDesc& d) { return (uint64_t)d.unit_begin; });
+	const uint32_t j = warp_job(L, unit_id, [](const JobDesc& d) { return (uint64_t)d.unit_begin; });
 	const JobDesc& J = job_at(L, j);
 	if (!(J.flags & JOB_MORTON)) return;
 	const uint64_t words = ((uint64_t)J.grid[0] * J.grid[1] * J.grid[2] + 31) >> 5;

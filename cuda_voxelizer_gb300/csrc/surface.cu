@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 	// Warps beyond the number of queued items have nothing to claim: they leave without touching
 	// the ticket counter (all of them do when only small triangles were queued).
 	if ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) >= total) return;
-	WarpTickets wt(total, gridDim.x * (blockDim.x >> 5));
+	WarpTickets wt(total, blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), gridDim.x * (blockDim.x >> 5));
 	for (;;) {
 		unsigned long long tk = 0;
 		if (!wt.take(&C->ticket, total, lane, tk)) break;
