@@ -105,19 +105,20 @@ const Prof* prof() { return g_profile ? &g_prof : nullptr; }
 
 // ---- scratch ------------------------------------------------------------------------------------
 
-// Record area of a launch sequence: counters, per-brick pair counts (for up to `bricks` bricks per
+// Record area of a launch sequence: ticket counters and counters, per-brick pair counts (for up to `bricks` bricks per
 // launch; none without JOB_BRICKS jobs), the queues (cap triangles), the other brick arrays, then
 // `n_jobs` uploaded job descriptors.  [0, big) must be zero before the first launch sequence on the
 // area (the counts are zero again after every sequence).  Pairs: about 27 per queued triangle on the
 // 1024^3 stress soup; triangles whose pairs do not fit are rasterized by surf_rows instead.
 struct RecLayout {
-	size_t ctr, bcnt, big, mid, bq, tri, boff, bcur, ubeg, psorted, jobs, end;
+	size_t tickets, ctr, bcnt, big, mid, bq, tri, boff, bcur, ubeg, psorted, jobs, end;
 	uint64_t pair_cap;
 };
 RecLayout rec_layout(uint64_t cap, uint64_t n_jobs, uint32_t bricks = 0) {
 	RecLayout l;
-	l.ctr = 0;
-	l.bcnt = align_up(sizeof(Counters));
+	l.tickets = 0;
+	l.ctr = align_up(kTicketBytes);
+	l.bcnt = align_up(l.ctr + sizeof(Counters));
 	l.big = align_up(l.bcnt + (uint64_t)bricks * 4);
 	l.mid = align_up(l.big + cap * sizeof(BigRec));
 	l.bq = align_up(l.mid + cap * sizeof(MidRec));
@@ -137,6 +138,7 @@ RecLayout rec_layout(uint64_t cap, uint64_t n_jobs, uint32_t bricks = 0) {
 // tuning may use less of the pair area (brick_pairs per triangle; 0 sends every triangle to surf_rows).
 void bind_scratch(LaunchDesc& L, char* rec, uint64_t cap, uint32_t bricks, const Tune& tune) {
 	const RecLayout l = rec_layout(cap, 0, bricks);
+	L.scr.tickets = reinterpret_cast<unsigned long long*>(rec + l.tickets);
 	L.scr.ctr = reinterpret_cast<Counters*>(rec + l.ctr);
 	L.scr.big = reinterpret_cast<BigRec*>(rec + l.big);
 	L.scr.mid = reinterpret_cast<MidRec*>(rec + l.mid);
@@ -152,6 +154,9 @@ void bind_scratch(LaunchDesc& L, char* rec, uint64_t cap, uint32_t bricks, const
 	L.scr.unit_begin = reinterpret_cast<uint32_t*>(rec + l.ubeg);
 	L.scr.pair_sorted = reinterpret_cast<uint32_t*>(rec + l.psorted);
 }
+
+// What is cleared between the launch sequences on an area: everything up to the error word.
+size_t reset_bytes() { return rec_layout(0, 0).ctr + kCountersResetBytes; }
 
 struct StreamScratch {
 	void* rec = nullptr;
@@ -422,7 +427,7 @@ struct Runner {
 	}
 
 	cvx_status reset_counters() {
-		if (!fresh) CVX_CUDA(cudaMemsetAsync(rec, 0, kCountersResetBytes, s));
+		if (!fresh) CVX_CUDA(cudaMemsetAsync(rec, 0, reset_bytes(), s));
 		fresh = false;
 		return CVX_OK;
 	}
@@ -760,7 +765,7 @@ cvx_status cvx_device_status(cvx_stream_t stream) {
 	}
 	if (rec) {
 		Counters c;
-		CVX_CUDA(cudaMemcpy(&c, rec, sizeof(c), cudaMemcpyDeviceToHost));
+		CVX_CUDA(cudaMemcpy(&c, static_cast<char*>(rec) + rec_layout(0, 0).ctr, sizeof(c), cudaMemcpyDeviceToHost));
 		if (c.error) return fail(CVX_ERR_DEVICE_CHECK, "device check failed (code %u)", c.error);
 	}
 	// the last cvx_voxelize_solid_noalloc call on this device keeps its counters in the library's
@@ -842,7 +847,7 @@ static cudaError_t capture_group(const Group& g, bool solid, bool resolve, bool 
 	else
 		L.jobs = jobs_dev;
 	if (resolve) return launch_solid(L, dev.tune, dev.cols_grid, s, kSolidResolve, nullptr);
-	const cudaError_t e = fresh ? cudaSuccess : cudaMemsetAsync(rec, 0, kCountersResetBytes, s);
+	const cudaError_t e = fresh ? cudaSuccess : cudaMemsetAsync(rec, 0, reset_bytes(), s);
 	if (e != cudaSuccess) return e;
 	return solid ? launch_solid(L, dev.tune, dev.cols_grid, s, kSolidToggles, nullptr)
 	             : launch_surface(L, dev.tune, dev.rows_grid, dev.raster_grid, s, nullptr);

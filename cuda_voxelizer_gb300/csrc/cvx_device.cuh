@@ -119,7 +119,6 @@ constexpr int kBigShift = 40;
 constexpr unsigned long long kBigItemMask = (1ull << kBigShift) - 1ull;
 struct Counters {
 	unsigned long long big;
-	unsigned long long ticket;   // next work ticket of the cooperative kernel
 	unsigned long long pairs;    // (brick, triangle) pairs reserved by brick_bin
 	unsigned long long bticket;  // next triangle of the brick queue for brick_bin
 	unsigned long long fticket;  // next triangle of the brick queue for brick_fill
@@ -133,12 +132,10 @@ struct Counters {
 // Everything before `error` is reset before every launch sequence; `error` persists until read.
 constexpr size_t kCountersResetBytes = offsetof(Counters, error);
 
-// Work tickets of the cooperative kernels, claimed by a warp K at a time: one atomic on the shared
-// counter per K items instead of per item (a single hot address serialises in its L2 slice when
-// hundreds of thousands of small items are queued).  K grows with the items per warp, up to 16,
-// so the tail left when the counter runs out stays short.  A warp's first K tickets are its own by its
-// number (`warp` of n_warps): with fewer items than warps nothing waits for the counter (the 512^3
-// icosphere's 1,500 queued triangles: surf_rows 12.9 us -> 10.9 us).
+// Work tickets of the brick kernels, claimed by a warp K at a time: one atomic on the shared counter
+// per K items instead of per item.  K grows with the items per warp, up to 16, so the tail left when
+// the counter runs out stays short.  A warp's first K tickets are its own by its number (`warp` of
+// n_warps): with fewer items than warps nothing waits for the counter.
 struct WarpTickets {
 	unsigned long long next, end;
 	uint32_t K;
@@ -166,6 +163,49 @@ struct WarpTickets {
 	}
 };
 
+// Work tickets of surf_rows.  A counter at one address hands out about 0.4 tickets per ns -- 60,000
+// items of a few hundred ns each took 150 us whatever the warps did -- so the tickets are dealt over
+// kTicketQueues counters on cache lines of their own, queue q holding the tickets q, q + kTicketQueues,
+// ...: a warp claims from its own queue, K at a time as above, its first K without an atomic, and when
+// that is empty from any other that is not (one load by the warp shows which are).
+constexpr uint32_t kTicketQueues = 32;        // one per lane
+constexpr uint32_t kTicketStride = 16;        // 128 bytes
+constexpr size_t kTicketBytes = kTicketQueues * kTicketStride * sizeof(unsigned long long);
+struct SpreadTickets {
+	unsigned long long next, end;   // claimed positions of queue q not yet taken
+	uint32_t q, K, warp0, n_warps;  // warp0: the warp's own queue
+	__device__ SpreadTickets(uint64_t total, uint32_t warp, uint32_t n_warps_) : n_warps(n_warps_) {
+		const uint64_t per = total / ((uint64_t)n_warps * 8u);
+		K = (uint32_t)(per < 1 ? 1 : (per > 16 ? 16 : per));
+		warp0 = q = warp % kTicketQueues;
+		next = (unsigned long long)(warp / kTicketQueues) * K;
+		end = next + K;
+	}
+	// Positions of queue i that belong to warps by their number.
+	__device__ __forceinline__ unsigned long long own(uint32_t i) const {
+		return (unsigned long long)((n_warps + kTicketQueues - 1u - i) / kTicketQueues) * K;
+	}
+	// Next ticket of this warp (the same in every lane); false once every ticket is claimed.
+	__device__ __forceinline__ bool take(unsigned long long* ctr, uint64_t total, uint32_t lane,
+	                                     unsigned long long& tk) {
+		while (next >= end || next * kTicketQueues + q >= total) {
+			if ((unsigned long long)n_warps * K >= total) return false;  // every ticket is some warp's own
+			if (next * kTicketQueues + q >= total) {  // the queue is empty: the nearest one that is not
+				const unsigned long long c = *reinterpret_cast<volatile unsigned long long*>(ctr + lane * kTicketStride);
+				const uint32_t left = __ballot_sync(0xFFFFFFFFu, (own(lane) + c) * kTicketQueues + lane < total);
+				if (!left) return false;
+				q = (warp0 + __ffs(__funnelshift_r(left, left, warp0)) - 1u) % kTicketQueues;
+			}
+			unsigned long long b = 0;
+			if (lane == 0) b = atomicAdd(ctr + q * kTicketStride, (unsigned long long)K);
+			next = own(q) + __shfl_sync(0xFFFFFFFFu, b, 0);
+			end = next + K;
+		}
+		tk = next++ * kTicketQueues + q;
+		return true;
+	}
+};
+
 // Brick rasterization (JOB_BRICKS jobs, bricks.cu): the queued triangles of those jobs are binned to
 // the 32^3 bricks of their tables that their planes cross, the (brick, triangle) pairs are grouped
 // by brick with a counting sort, and each warp rasterizes a brick's pairs into a brick of its own in
@@ -186,6 +226,7 @@ static_assert(sizeof(BrickTri) == 176, "BrickTri is eleven 16-byte vectors");
 
 struct Scratch {
 	Counters* ctr;
+	unsigned long long* tickets;  // kTicketBytes: the ticket counters of surf_rows, zero before a launch sequence
 	BigRec* big;
 	MidRec* mid;
 	uint32_t cap;          // capacity of big[], mid[], bq[] and tri[] (>= triangles in the launch)

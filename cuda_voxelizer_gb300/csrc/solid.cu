@@ -12,7 +12,7 @@
 // Kernels, in launch order:
 //   solid_classify      a warp per 32 triangles (staged by a bulk copy); the columns of the triangles
 //                       with few columns are dealt over the warp, the other triangles queued.
-//   solid_cols          persistent; each warp takes items of up to kColsPerItem columns.
+//   solid_cols          persistent; each warp takes items of up to kColsPerItem columns in turn.
 //   solid_resolve       linear jobs: a warp per run of whole rows, 128 words at a time: prefix XOR
 //                       along x, XORed into the linear table (every word stored, for
 //                       JOB_TABLE_OVERWRITE jobs), flip table cleared.
@@ -190,7 +190,7 @@ __device__ __forceinline__ void record_hit(uint32_t* flips, const uint32_t* grid
 struct __align__(16) SmallSolid {
 	float nx, ny, nz, v0x, v0y, v0z, ax, ay, bx, by, cx, cy;
 	int y0, z0;
-	uint32_t nzc;    // columns along z
+	uint32_t nyc;    // columns along y
 	uint32_t start;  // columns of the warp's triangles before this one
 	uint32_t pad[4];
 };
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(kTile, 12) solid_classify(const __grid_constan
 		o.nx = S.nx; o.ny = S.ny; o.nz = S.nz; o.v0x = S.v0x; o.v0y = S.v0y; o.v0z = S.v0z;
 		o.ax = S.ax; o.ay = S.ay; o.bx = S.bx; o.by = S.by; o.cx = S.cx; o.cy = S.cy;
 		o.y0 = S.y0; o.z0 = S.z0;
-		o.nzc = (uint32_t)(S.z1 - S.z0 + 1);
+		o.nyc = (uint32_t)(S.y1 - S.y0 + 1);
 		o.start = start;
 	}
 	__syncwarp();
@@ -324,11 +324,11 @@ __global__ void __launch_bounds__(kTile, 12) solid_classify(const __grid_constan
 		SolidTri T;
 		T.nx = o.nx; T.ny = o.ny; T.nz = o.nz; T.v0x = o.v0x; T.v0y = o.v0y; T.v0z = o.v0z;
 		T.ax = o.ax; T.ay = o.ay; T.bx = o.bx; T.by = o.by; T.cx = o.cx; T.cy = o.cy;
-		// column c = dz + dy * nzc, c and nzc at most kColsPerSmall * kSmallCols = 128: the approximate
+		// column c = dy + dz * nyc, c and nyc at most kColsPerSmall * kSmallCols = 128: the approximate
 		// quotient is more than 1e-3 away from the next integer and truncates exactly
-		const uint32_t c = k - o.start, nzc = o.nzc;
-		const uint32_t dy = (uint32_t)__fdividef((float)c + 0.5f, (float)nzc);
-		const int y = o.y0 + (int)dy, z = o.z0 + (int)(c - dy * nzc);
+		const uint32_t c = k - o.start, nyc = o.nyc;
+		const uint32_t dz = (uint32_t)__fdividef((float)c + 0.5f, (float)nyc);
+		const int y = o.y0 + (int)(c - dz * nyc), z = o.z0 + (int)dz;
 		int xmax;
 		if (column_hit<P>(T, unit, y, z, morton, xmax)) record_hit(flips, grid, morton, y, z, xmax);
 	}
@@ -350,43 +350,44 @@ __global__ void __launch_bounds__(kRowsThreads) solid_cols(const __grid_constant
 	const uint64_t n_big_items = bigc & kBigItemMask;
 	const uint32_t n_mid = min(s_mid, L.scr.cap);
 	const uint64_t total = n_big_items + n_mid;
-	// Warps beyond the number of queued items have nothing to claim: they leave without touching
-	// the ticket counter (all of them do when only small triangles were queued).
-	if ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) >= total) return;
-	WarpTickets wt(total, blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), gridDim.x * (blockDim.x >> 5));
-	for (;;) {
-		unsigned long long tk = 0;
-		if (!wt.take(&C->ticket, total, lane, tk)) break;
+	// Items are of about the same size (at most kColsPerItem columns), so every warp takes its share in
+	// turn, without a counter (the icosphere 5 at 1000^3, 60,000 items: 154 us -> 63 us).
+	const uint32_t n_warps = gridDim.x * (blockDim.x >> 5);
+	for (uint64_t tk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tk < total; tk += n_warps) {
 		uint32_t job, tri, chunk;
 		if (!queue_item(L, tk, n_big, n_big_items, lane, job, tri, chunk)) continue;
 		const JobDesc& J = job_at(L, job);
 		const float unit[3] = {J.unit[0], J.unit[1], J.unit[2]};
 		const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
 		const bool morton = (J.flags & JOB_MORTON) != 0;
+		uint32_t* flips = J.flips;
 		float tv = lane < 9 ? J.tris[(uint64_t)tri * 9 + lane] : 0.0f;
 		float t[9];
 #pragma unroll
 		for (int k = 0; k < 9; k++) t[k] = __shfl_sync(FULL, tv, k);
 		SolidTri S;
 		solid_setup<P>(t, J.bmin, unit, J.inv_unit, grid, S);
-		const uint64_t nzc = (uint64_t)(S.z1 - S.z0 + 1);
-		const uint64_t ncols = (uint64_t)(S.y1 - S.y0 + 1) * nzc;
+		const uint64_t nyc = (uint64_t)(S.y1 - S.y0 + 1);
+		const uint64_t ncols = nyc * (uint64_t)(S.z1 - S.z0 + 1);
 		const uint64_t c0 = (uint64_t)chunk * kColsPerItem;
 		const uint64_t c1 = umin64(ncols, c0 + kColsPerItem);
-		// column c is (y0 + c / nzc, z0 + c % nzc): one division for the lane's first column, then
-		// steps of 32 columns (dy rows and dz slices, carrying z into y)
+		// column c is (y0 + c % nyc, z0 + c / nyc): one division for the lane's first column, then
+		// steps of 32 columns (dz slices and dy rows, carrying y into z)
 		const uint64_t cf = c0 + lane;
-		if (cf < c1) {  // (no lane enters when the range is empty: nzc may be 0 then)
-			int y = S.y0 + (int)(cf / nzc), z = S.z0 + (int)(cf % nzc);
-			const int dy = (int)(32u / nzc), dz = (int)(32u % nzc);
+		if (cf < c1) {  // (no lane enters when the range is empty: nyc may be 0 then)
+			const bool small = (ncols >> 32) == 0;
+			int z = (int)(small ? (uint32_t)cf / (uint32_t)nyc : cf / nyc), y = (int)(cf - (uint64_t)z * nyc);
+			const int dz = (int)(32u / (uint32_t)nyc), dy = 32 - dz * (int)nyc;
+			y += S.y0;
+			z += S.z0;
 			for (uint64_t c = cf; c < c1; c += 32) {
 				int xmax;
-				if (column_hit<P>(S, unit, y, z, morton, xmax)) record_hit(J.flips, grid, morton, y, z, xmax);
-				y += dy;
+				if (column_hit<P>(S, unit, y, z, morton, xmax)) record_hit(flips, grid, morton, y, z, xmax);
 				z += dz;
-				if (z > S.z1) {
-					z -= (int)nzc;
-					y++;
+				y += dy;
+				if (y > S.y1) {
+					y -= (int)nyc;
+					z++;
 				}
 			}
 		}

@@ -211,13 +211,13 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 	const uint64_t n_big_items = bigc & kBigItemMask;
 	const uint32_t n_mid = min(s_mid, L.scr.cap);
 	const uint64_t total = n_big_items + n_mid;
-	// Warps beyond the number of queued items have nothing to claim: they leave without touching
-	// the ticket counter (all of them do when only small triangles were queued).
+	// Warps beyond the number of queued items have nothing to claim (all of them when only small
+	// triangles were queued).
 	if ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) >= total) return;
-	WarpTickets wt(total, blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), gridDim.x * (blockDim.x >> 5));
+	SpreadTickets wt(total, blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), gridDim.x * (blockDim.x >> 5));
 	for (;;) {
 		unsigned long long tk = 0;
-		if (!wt.take(&C->ticket, total, lane, tk)) break;
+		if (!wt.take(L.scr.tickets, total, lane, tk)) break;
 		uint32_t job, tri, chunk = 0;
 		if (!queue_item(L, tk, n_big, n_big_items, lane, job, tri, chunk)) continue;
 		const JobDesc& J = job_at(L, job);
