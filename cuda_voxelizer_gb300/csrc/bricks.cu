@@ -128,7 +128,7 @@ __device__ __forceinline__ void queue_for_rows(const LaunchDesc& L, uint32_t job
 	const uint32_t r = (uint32_t)(old >> kBigShift);
 	const uint64_t first = old & kBigItemMask;
 	if (r < L.scr.cap && first + items <= kBigItemMask)
-		L.scr.big[r] = BigRec{first, job, tri, items, 0u};
+		L.scr.big[r] = BigRec{first, job, tri, items, kZch};
 	else
 		set_error(L, kErrQueueOverflow);
 }

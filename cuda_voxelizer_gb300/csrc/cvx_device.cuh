@@ -104,7 +104,8 @@ struct JobDesc {
 // Work-queue records written by the classify kernels and consumed by the cooperative kernels.
 struct BigRec {            // triangle whose work is split into several items
 	uint64_t item_begin;
-	uint32_t job, tri, n_items, pad;
+	uint32_t job, tri, n_items;
+	uint32_t slices;         // surface: z-slices per item
 };
 struct MidRec {            // triangle handled as a single item
 	uint32_t job, tri;

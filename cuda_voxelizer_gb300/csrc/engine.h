@@ -9,7 +9,8 @@
 namespace cvx {
 
 constexpr uint32_t kTile = 128;        // triangles per classify CTA (one tile; 2.6% faster than 256 on the bench step's plan)
-constexpr uint32_t kZch = 32;          // z-slices per surface work item (one per lane)
+constexpr uint32_t kZch = 32;          // most z-slices of a surface work item (one per lane)
+constexpr uint32_t kMinSlices = 4;     // fewest, of a triangle with many rows in a small launch
 constexpr uint32_t kRowsThreads = 256; // threads per cooperative CTA
 constexpr uint32_t kColsPerItem = 256; // solid columns per work item
 constexpr uint32_t kLocalRows = 64;    // surface: rows a triangle may have in the classify kernel

@@ -354,8 +354,8 @@ __global__ void __launch_bounds__(kRowsThreads) solid_cols(const __grid_constant
 	// turn, without a counter (the icosphere 5 at 1000^3, 60,000 items: 154 us -> 63 us).
 	const uint32_t n_warps = gridDim.x * (blockDim.x >> 5);
 	for (uint64_t tk = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tk < total; tk += n_warps) {
-		uint32_t job, tri, chunk;
-		if (!queue_item(L, tk, n_big, n_big_items, lane, job, tri, chunk)) continue;
+		uint32_t job, tri, chunk, slices;
+		if (!queue_item(L, tk, n_big, n_big_items, lane, job, tri, chunk, slices)) continue;
 		const JobDesc& J = job_at(L, job);
 		const float unit[3] = {J.unit[0], J.unit[1], J.unit[2]};
 		const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};

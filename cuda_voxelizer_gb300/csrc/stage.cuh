@@ -64,8 +64,9 @@ __device__ __forceinline__ bool stage_warp(const LaunchDesc& L, const float* src
 // search with 32 probes per round: three dependent loads for 32,768 records instead of fifteen.
 __device__ __forceinline__ bool queue_item(const LaunchDesc& L, unsigned long long tk, uint32_t n_big,
                                            uint64_t n_big_items, uint32_t lane, uint32_t& job, uint32_t& tri,
-                                           uint32_t& chunk) {
+                                           uint32_t& chunk, uint32_t& slices) {
 	chunk = 0;
+	slices = kZch;
 	if (tk < n_big_items) {
 		if (n_big == 0) return false;
 		uint32_t first = 0, n = n_big;  // the last record with item_begin <= tk is among n from `first`
@@ -79,6 +80,7 @@ __device__ __forceinline__ bool queue_item(const LaunchDesc& L, unsigned long lo
 		const BigRec r = L.scr.big[first];
 		job = r.job;
 		tri = r.tri;
+		slices = r.slices;
 		chunk = (uint32_t)(tk - r.item_begin);
 		if (tk < r.item_begin || chunk >= r.n_items) return false;
 	} else {

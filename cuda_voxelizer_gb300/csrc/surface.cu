@@ -37,7 +37,7 @@ namespace {
 // kernels, 44 + 701 with this rule.
 template <class P>
 __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant__ LaunchDesc L, const uint32_t small_vox,
-                                                             const uint32_t warp_rows, const uint32_t split) {
+                                                             const uint32_t warp_rows, const uint32_t item_rows, const uint32_t split) {
 	__shared__ __align__(16) union {
 		float tri[32 * 9];
 		SmallTri small[32];
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 	__syncwarp();  // the triangles are consumed; the shared memory now holds records
 
 	SurfTri S;
-	uint32_t n_items = 0, n_rows = 0;
+	uint32_t n_items = 0, n_rows = 0, slices = kZch;
 	bool few = false;
 	if (valid) {
 		const float bmin[3] = {J.bmin[0], J.bmin[1], J.bmin[2]};
@@ -75,7 +75,8 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 		const uint32_t ex = (uint32_t)(S.bx1 - S.bx0), ey = (uint32_t)(S.by1 - S.by0), ez = (uint32_t)(S.bz1 - S.bz0);
 		const uint64_t rows = (uint64_t)(ey + 1) * (uint64_t)(ez + 1);
 		few = (uint64_t)(ex + 1) * rows <= small_vox;
-		n_items = (ez + kZch) / kZch;
+		while (slices > kMinSlices && (uint64_t)(ey + 1) * slices > item_rows) slices >>= 1;
+		n_items = ez / slices + 1u;
 		if (ex < kMaskRowVoxels && rows <= kLocalRows && !plane_underflows(S)) n_rows = (uint32_t)rows;
 	}
 	if (__reduce_add_sync(FULL, n_rows) > warp_rows && !few) n_rows = 0;
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 			const uint32_t rec = (uint32_t)(old >> kBigShift) + __popc(big_ballot & lt);
 			const uint64_t first = (old & kBigItemMask) + incl - n_items;
 			if (rec < L.scr.cap && first + n_items <= kBigItemMask)
-				L.scr.big[rec] = BigRec{first, j, (uint32_t)(t0 + lane), n_items, 0u};
+				L.scr.big[rec] = BigRec{first, j, (uint32_t)(t0 + lane), n_items, slices};
 			else
 				set_error(L, kErrQueueOverflow);
 		}
@@ -218,8 +219,8 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 	for (;;) {
 		unsigned long long tk = 0;
 		if (!wt.take(L.scr.tickets, total, lane, tk)) break;
-		uint32_t job, tri, chunk = 0;
-		if (!queue_item(L, tk, n_big, n_big_items, lane, job, tri, chunk)) continue;
+		uint32_t job, tri, chunk, slices;
+		if (!queue_item(L, tk, n_big, n_big_items, lane, job, tri, chunk, slices)) continue;
 		const JobDesc& J = job_at(L, job);
 		const float unit[3] = {J.unit[0], J.unit[1], J.unit[2]};
 		const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
@@ -239,7 +240,7 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 		const float bx0 = (float)S.bx0, bx1 = (float)S.bx1;
 
 		// this lane's z-slice
-		const int z = S.bz0 + (int)(chunk * kZch + lane);
+		const int z = S.bz0 + (int)(chunk * slices + lane);
 		float fy0 = (float)S.by0, fy1 = (float)S.by1, zx0 = bx0, zx1 = bx1, kz;
 		{
 			const float pz = __fmul_rn(__int2float_rn(z), unit[2]);
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 				clip_test(S.ezx[i][1], __fmul_rn(S.ezx[i][0], pz), S.dzx[i], unit[0], bx0, bx1, zx0, zx1);
 			}
 		}
-		const bool rows = z <= S.bz1 && fy0 <= fy1 && zx0 <= zx1;
+		const bool rows = lane < slices && z <= S.bz1 && fy0 <= fy1 && zx0 <= zx1;
 		const int ya = rows ? (int)fy0 : 0x7FFFFFFF, yb = rows ? (int)fy1 : -1;
 		const int y_begin = __reduce_min_sync(FULL, ya), y_last = __reduce_max_sync(FULL, yb);
 		for (int yw = y_begin; yw <= y_last; yw += kRowsWindow) {
@@ -337,8 +338,15 @@ static cudaError_t launch_surface_t(const LaunchDesc& L, const Tune& tune, int r
 	// With fewer CTAs than fill the chip the longest warp is the kernel's time: a warp with more than
 	// kWarpRows rows leaves the triangles above small_vox voxels to surf_rows.
 	const uint32_t warp_rows = L.n_tiles >= (uint32_t)rows_grid ? 0xFFFFFFFFu : kWarpRows;
+	// Rows (of the bounding box) that a queued triangle's items may have: with few triangles there are
+	// fewer items than surf_rows has warps, and one item of a large triangle is its time.  In surf_rows,
+	// with items of up to 1024 rows / 4096 / 32 slices whatever their rows: icosphere 3 at 1000^3 (1,280
+	// triangles) 45 / 55 / 59 us, soups of 5,000 at 400^3 32 / 56 / 61 us, of 30,000 at 600^3 197 / 161 / 179,
+	// of 300,000 at 300^3 488 / 410 / 411 us.
+	const uint64_t triangles = (uint64_t)L.n_tiles * kTile, warps = (uint64_t)rows_grid * (kRowsCtaThreads / 32);
+	const uint32_t item_rows = triangles < 4 * warps ? 1024u : (triangles < 16 * warps ? 4096u : 0xFFFFFFFFu);
 	const uint32_t split = classify_split(L.n_tiles, (uint32_t)rows_grid);
-	surf_classify<P><<<L.n_tiles << split, kTile, 0, s>>>(L, tune.small_vox, warp_rows, split);
+	surf_classify<P><<<L.n_tiles << split, kTile, 0, s>>>(L, tune.small_vox, warp_rows, item_rows, split);
 	cudaError_t e = cudaGetLastError();
 	if (e != cudaSuccess) return e;
 	if (prof) (*prof)("surf_classify", s);
