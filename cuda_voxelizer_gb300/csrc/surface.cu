@@ -175,20 +175,67 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 // Then the item's rows, 32 at a time, one per lane: the row's slice is found by counting the slices that
 // start at or before it, its bounds on x are read from both tables, the plane test narrows them to
 // the row's exact interval, and the interval is ORed into the table.
-// Bound by the L2's scattered atomics on large tables, by instructions and, with few items, by the
-// latency of one item elsewhere.  The soup of 2 M triangles at 1024^3: 27.2 ms for 3.36 G word updates
-// (124 G/s); 39.8 ms with all eight x-dependent tests evaluated per row (41 G warp instructions).  The
-// soup of 300,000 at 300^3 402 us / 701 us.  Six CTAs per SM at 80 registers; seven or eight spill and
-// are no faster.  Reading a word before the atomic, to skip it where its bits are set, cost as many L2
-// requests as it saved: 27.4 - 28.2 ms, and 30% to 90% more where the table fits the L2.
+// Bound by the L2's scattered atomics on large tables (issue slots 53% busy), by instructions and, with
+// few items, by the latency of one item elsewhere.  The soup of 2 M triangles at 1024^3: 26.9 ms for
+// 3.36 G word updates (125 G/s); 39.8 ms with all eight x-dependent tests evaluated per row (41 G warp
+// instructions).  The soup of 300,000 at 300^3 390 us / 697 us.  Six CTAs per SM at 80 registers; five
+// are 2% faster on the first soup and 3% slower on the second, seven spill.  Reading a word before the
+// atomic, to skip it where its bits are set, cost as many L2 requests as it saved (27.4 - 28.2 ms, and
+// 30% to 90% more where the table fits the L2), and walking the items twice or four times, each time for
+// a half or quarter of the table that stays in the L2, was 2% to 7% slower.
 constexpr uint32_t kRowsCtaThreads = 128;
 constexpr int kRowsWindow = 128;
 
 struct RowsWarp {
-	float4 xy[kRowsWindow];  // per y of the window: bounds of x from the XY tests, ny * py
-	float4 slice[32];        // per slice with rows in the window: start - first y, z, bounds of x from the ZX tests
+	float4 xy[kRowsWindow];  // per y of the window: bounds of x from the XY tests, ny * py, its part of the row's place
+	float4 slice[32];        // per slice with rows in the window: start - first y, its part, bounds of x from the ZX tests
 	float kz[32];            // and its nz * pz
 };
+
+// A row's place in a narrow job's table is the sum of a part of its y and a part of its slice: linear
+// index y * gx + z * gx * gy, or the Morton code's y and z bits.  (Other jobs keep y and z.)
+__device__ __forceinline__ uint32_t y_part(const uint32_t* grid, bool morton, bool narrow, int y) {
+	return !narrow ? (uint32_t)y : (morton ? spread3_narrow((uint32_t)y) << 1 : (uint32_t)y * grid[0]);
+}
+__device__ __forceinline__ uint32_t z_part(const uint32_t* grid, bool morton, bool narrow, int z) {
+	return !narrow ? (uint32_t)z : (morton ? spread3_narrow((uint32_t)z) << 2 : (uint32_t)z * grid[1] * grid[0]);
+}
+
+// Writes of one row's interval [xl, xh] in a narrow job: its own lane's, of a few words, and the whole
+// warp's, one row at a time with the lanes on consecutive words (linear) or x groups (Morton) -- a
+// scattered atomic costs an L2 transaction of its own, a warp's atomics on one row share a few lines.
+__device__ __forceinline__ void write_linear(uint32_t* table, uint32_t place, uint32_t xl, uint32_t xh) {
+	const uint32_t lo = place + xl, hi = place + xh, w0 = lo >> 5, w1 = hi >> 5;  // at most three words
+	const uint32_t m0 = 0xFFFFFFFFu >> (lo & 31u), m1 = 0xFFFFFFFFu << (~hi & 31u);
+	atomicOr(table + w0, w0 == w1 ? m0 & m1 : m0);
+	if (w0 != w1) {
+		atomicOr(table + w1, m1);
+		if (w1 - w0 > 1u) atomicOr(table + w0 + 1, 0xFFFFFFFFu);
+	}
+}
+__device__ __forceinline__ void write_linear_warp(uint32_t* table, uint32_t place, uint32_t xl, uint32_t xh, uint32_t lane) {
+	const uint32_t lo = place + xl, hi = place + xh, w0 = lo >> 5, w1 = hi >> 5;
+	for (uint32_t w = w0 + lane; w <= w1; w += 32)
+		atomicOr(table + w, (w == w0 ? 0xFFFFFFFFu >> (lo & 31u) : 0xFFFFFFFFu) & (w == w1 ? 0xFFFFFFFFu << (~hi & 31u) : 0xFFFFFFFFu));
+}
+// Bits of x offsets j0 .. j1 of the 4-voxel group k of a Morton row, at their place in its word.
+__device__ __forceinline__ void write_morton_group(uint32_t* table, uint32_t code, int k, int xl, int xh) {
+	const int j0 = max(xl - (k << 2), 0), j1 = min(xh - (k << 2), 3);
+	const uint32_t n = (0xFu << j0) & (0xFu >> (3 - j1));
+	const uint32_t m = ((n & 1u) << 31) | ((n & 2u) << 29) | ((n & 4u) << 21) | ((n & 8u) << 19);
+	atomicOr(table + (code >> 5), m >> (code & 31u));
+}
+__device__ __forceinline__ void write_morton(uint32_t* table, uint32_t place, int xl, int xh) {
+	uint32_t xd = spread3_narrow((uint32_t)(xl & ~3));
+	for (int k = xl >> 2; k <= (xh >> 2); k++) {
+		write_morton_group(table, xd | place, k, xl, xh);
+		xd = morton_x_add_t<uint32_t>(xd, (uint32_t)kMortonX4);
+	}
+}
+__device__ __forceinline__ void write_morton_warp(uint32_t* table, uint32_t place, int xl, int xh, uint32_t lane) {
+	for (int k = (xl >> 2) + (int)lane; k <= (xh >> 2); k += 32)
+		write_morton_group(table, spread3_narrow((uint32_t)(k << 2)) | place, k, xl, xh);
+}
 
 template <class P>
 __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_constant__ LaunchDesc L) {
@@ -240,7 +287,7 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 		const float bx0 = (float)S.bx0, bx1 = (float)S.bx1;
 
 		// this lane's z-slice
-		const int z = S.bz0 + (int)(chunk * slices + lane);
+		const int z0 = S.bz0 + (int)(chunk * slices), z = z0 + (int)lane;
 		float fy0 = (float)S.by0, fy1 = (float)S.by1, zx0 = bx0, zx1 = bx1, kz;
 		{
 			const float pz = __fmul_rn(__int2float_rn(z), unit[2]);
@@ -263,7 +310,7 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 #pragma unroll
 				for (int i = 0; i < 3; i++)
 					clip_test(S.exy[i][0], __fmul_rn(S.exy[i][1], py), S.dxy[i], unit[0], bx0, bx1, x0, x1);
-				W.xy[y - yw] = make_float4(x0, x1, __fmul_rn(S.ny, py), 0.0f);
+				W.xy[y - yw] = make_float4(x0, x1, __fmul_rn(S.ny, py), __uint_as_float(y_part(grid, morton, narrow, y)));
 			}
 			const int first = max(ya, yw);
 			const uint32_t cnt = rows ? (uint32_t)max(min(yb, yw1) - first + 1, 0) : 0u;
@@ -276,7 +323,8 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 			const uint32_t R = __shfl_sync(FULL, incl, 31), start = incl - cnt;
 			const uint32_t slot = __popc(__ballot_sync(FULL, cnt != 0u) & ((1u << lane) - 1u));
 			if (cnt) {
-				W.slice[slot] = make_float4(__int_as_float((int)start - first), __int_as_float(z), zx0, zx1);
+				W.slice[slot] = make_float4(__int_as_float((int)start - first), __uint_as_float(z_part(grid, morton, narrow, z)),
+				                            zx0, zx1);
 				W.kz[slot] = kz;
 			}
 			__syncwarp();
@@ -287,38 +335,51 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 				const uint32_t rec = begun + __popc(starts & (0xFFFFFFFFu >> (31u - lane))) - 1u;
 				begun += __popc(starts);
 				const uint32_t k = base + lane;
-				int y = 0, rz = 0, xl = 0, xh = -1;
+				uint32_t yp = 0, zp = 0;  // the row's place
+				int xl = 0, xh = -1;
 				if (k < R) {
 					const float4 q = W.slice[rec];
-					y = (int)k - __float_as_int(q.x);
-					rz = __float_as_int(q.y);
+					const int y = (int)k - __float_as_int(q.x);
 					const float4 e = W.xy[y - yw];
+					yp = __float_as_uint(e.w);
+					zp = __float_as_uint(q.y);
 					float x0 = fmaxf(q.z, e.x), x1 = fminf(q.w, e.y);
 					if (!product) {
 						clip_plane(S.nx, e.z, W.kz[rec], lo, hi, plane_m, plane_inv, unit[0], bx0, bx1, x0, x1);
-						if (x0 <= x1) { xl = (int)x0; xh = (int)x1; }
+						if (x0 <= x1) {  // integers of [0, 2^22]: their bits after adding 2^23
+							xl = __float_as_int(__fadd_rn(x0, 8388608.0f)) & 0x7FFFFF;
+							xh = __float_as_int(__fadd_rn(x1, 8388608.0f)) & 0x7FFFFF;
+						}
 					} else {  // a plane offset so small that the test's product may underflow: all tests together
+						int z = z0;
+						for (uint32_t i = 0; i < slices; i++)
+							if (z_part(grid, morton, narrow, z0 + (int)i) == zp) z = z0 + (int)i;
 						RowK K;
-						row_consts<P>(S, __fmul_rn(__int2float_rn(y), unit[1]), __fmul_rn(__int2float_rn(rz), unit[2]), K);
+						row_consts<P>(S, __fmul_rn(__int2float_rn(y), unit[1]), __fmul_rn(__int2float_rn(z), unit[2]), K);
 						RowDirs D;
 						row_dirs(S, unit[0], D);
 						if (!row_interval<P>(S, D, K, unit[0], xl, xh)) xh = -1;
 					}
 				}
-				// Short rows are written by their own lane.  Long rows are written by the whole warp, one
-				// row at a time with the lanes on consecutive words (linear) or x groups (Morton): a
-				// scattered atomic costs an L2 transaction of its own, a warp's atomics on one row
-				// share a few lines.
+				// Short rows are written by their own lane, long ones by the whole warp.
 				const bool has = xh >= xl;
 				const bool wide = has && (morton ? (xh >> 2) - (xl >> 2) >= 4 : (xh >> 5) - (xl >> 5) >= 2);
-				if (has && !wide) write_row(table, morton, narrow, grid, y, rz, xl, xh);
 				uint32_t todo = __ballot_sync(FULL, wide);
+				if (narrow && !morton) {
+					if (has && !wide) write_linear(table, yp + zp, (uint32_t)xl, (uint32_t)xh);
+				} else if (narrow) {
+					if (has && !wide) write_morton(table, yp | zp, xl, xh);
+				} else {
+					if (has && !wide) write_row_t<uint64_t>(table, morton, grid, (int)yp, (int)zp, xl, xh);
+				}
 				while (todo) {
 					const int src = __ffs(todo) - 1;
 					todo &= todo - 1u;
-					const int wy = __shfl_sync(FULL, y, src), wz = __shfl_sync(FULL, rz, src);
+					const uint32_t wy = __shfl_sync(FULL, yp, src), wz = __shfl_sync(FULL, zp, src);
 					const int wl = __shfl_sync(FULL, xl, src), wh = __shfl_sync(FULL, xh, src);
-					write_row_warp(table, morton, narrow, grid, wy, wz, wl, wh, lane);
+					if (narrow && !morton) write_linear_warp(table, wy + wz, (uint32_t)wl, (uint32_t)wh, lane);
+					else if (narrow) write_morton_warp(table, wy | wz, wl, wh, lane);
+					else write_row_warp_t<uint64_t>(table, morton, grid, (int)wy, (int)wz, wl, wh, lane);
 				}
 			}
 			__syncwarp();  // the tables are rewritten for the next window or item

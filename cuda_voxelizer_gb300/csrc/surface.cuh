@@ -632,7 +632,7 @@ __device__ __forceinline__ void write_row_mask_t(uint32_t* table, bool morton, c
 	}
 }
 
-// write_row by a whole warp (every lane calls it with the same row): lane i takes words
+// write_row_t by a whole warp (every lane calls it with the same row): lane i takes words
 // w0 + i, w0 + i + 32, ... of the linear span, or x groups k0 + i, ... of the Morton span.
 template <class C>
 __device__ __forceinline__ void write_row_warp_t(uint32_t* table, bool morton, const uint32_t* grid, int y, int z,
@@ -658,20 +658,9 @@ __device__ __forceinline__ void write_row_warp_t(uint32_t* table, bool morton, c
 	}
 }
 
-__device__ __forceinline__ void write_row(uint32_t* table, bool morton, bool narrow, const uint32_t* grid, int y,
-                                          int z, int xl, int xh) {
-	if (narrow) write_row_t<uint32_t>(table, morton, grid, y, z, xl, xh);
-	else write_row_t<uint64_t>(table, morton, grid, y, z, xl, xh);
-}
 __device__ __forceinline__ void write_row_mask(uint32_t* table, bool morton, bool narrow, const uint32_t* grid, int y,
                                                int z, int x0, uint32_t pm) {
 	if (narrow) write_row_mask_t<uint32_t>(table, morton, grid, y, z, x0, pm);
 	else write_row_mask_t<uint64_t>(table, morton, grid, y, z, x0, pm);
 }
-__device__ __forceinline__ void write_row_warp(uint32_t* table, bool morton, bool narrow, const uint32_t* grid, int y,
-                                               int z, int xl, int xh, uint32_t lane) {
-	if (narrow) write_row_warp_t<uint32_t>(table, morton, grid, y, z, xl, xh, lane);
-	else write_row_warp_t<uint64_t>(table, morton, grid, y, z, xl, xh, lane);
-}
-
 }  // namespace cvx
