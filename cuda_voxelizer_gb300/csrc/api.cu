@@ -105,20 +105,26 @@ const Prof* prof() { return g_profile ? &g_prof : nullptr; }
 
 // ---- scratch ------------------------------------------------------------------------------------
 
-// Record area of a launch sequence: ticket counters and counters, per-brick pair counts (for up to `bricks` bricks per
-// launch; none without JOB_BRICKS jobs), the queues (cap triangles), the other brick arrays, then
-// `n_jobs` uploaded job descriptors.  [0, big) must be zero before the first launch sequence on the
-// area (the counts are zero again after every sequence).  Pairs: about 27 per queued triangle on the
-// 1024^3 stress soup; triangles whose pairs do not fit are rasterized by surf_rows instead.
+// Record area of a launch sequence: kCounterBlocks blocks of ticket counters and counters, per-brick pair
+// counts (for up to `bricks` bricks per launch; none without JOB_BRICKS jobs), the queues (cap
+// triangles), the other brick arrays, then `n_jobs` uploaded job descriptors.  [0, big) must be zero
+// before the first launch sequence on the area (the counts are zero again after every sequence).
+// Pairs: about 27 per queued triangle on the 1024^3 stress soup; triangles whose pairs do not fit are
+// rasterized by surf_rows instead.
+// The per-stream areas use blocks 0 and 1 in turn, each cleared by the sequence before the one that uses
+// it, and block 2 for calls under capture (a graph may be launched any number of times) and for brick
+// jobs; there, and in the other areas, which use block 0, the host clears the counters.
+constexpr uint32_t kCounterBlocks = 3, kCaptureBlock = 2;
 struct RecLayout {
-	size_t tickets, ctr, bcnt, big, mid, bq, tri, boff, bcur, ubeg, psorted, jobs, end;
+	size_t tickets, ctr, block, bcnt, big, mid, bq, tri, boff, bcur, ubeg, psorted, jobs, end;
 	uint64_t pair_cap;
 };
 RecLayout rec_layout(uint64_t cap, uint64_t n_jobs, uint32_t bricks = 0) {
 	RecLayout l;
 	l.tickets = 0;
 	l.ctr = align_up(kTicketBytes);
-	l.bcnt = align_up(l.ctr + sizeof(Counters));
+	l.block = align_up(l.ctr + sizeof(Counters));
+	l.bcnt = kCounterBlocks * l.block;
 	l.big = align_up(l.bcnt + (uint64_t)bricks * 4);
 	l.mid = align_up(l.big + cap * sizeof(BigRec));
 	l.bq = align_up(l.mid + cap * sizeof(MidRec));
@@ -136,10 +142,10 @@ RecLayout rec_layout(uint64_t cap, uint64_t n_jobs, uint32_t bricks = 0) {
 
 // Point a launch descriptor's scratch at a record area laid out by rec_layout(cap, *, bricks); the
 // tuning may use less of the pair area (brick_pairs per triangle; 0 sends every triangle to surf_rows).
-void bind_scratch(LaunchDesc& L, char* rec, uint64_t cap, uint32_t bricks, const Tune& tune) {
+void bind_scratch(LaunchDesc& L, char* rec, uint64_t cap, uint32_t bricks, const Tune& tune, uint32_t block = 0) {
 	const RecLayout l = rec_layout(cap, 0, bricks);
-	L.scr.tickets = reinterpret_cast<unsigned long long*>(rec + l.tickets);
-	L.scr.ctr = reinterpret_cast<Counters*>(rec + l.ctr);
+	L.scr.tickets = reinterpret_cast<unsigned long long*>(rec + block * l.block + l.tickets);
+	L.scr.ctr = reinterpret_cast<Counters*>(rec + block * l.block + l.ctr);
 	L.scr.big = reinterpret_cast<BigRec*>(rec + l.big);
 	L.scr.mid = reinterpret_cast<MidRec*>(rec + l.mid);
 	L.scr.cap = (uint32_t)cap;
@@ -155,12 +161,14 @@ void bind_scratch(LaunchDesc& L, char* rec, uint64_t cap, uint32_t bricks, const
 	L.scr.pair_sorted = reinterpret_cast<uint32_t*>(rec + l.psorted);
 }
 
-// What is cleared between the launch sequences on an area: everything up to the error word.
+// What is cleared of a block between the launch sequences of a call: everything up to the error word.
 size_t reset_bytes() { return rec_layout(0, 0).ctr + kCountersResetBytes; }
 
 struct StreamScratch {
 	void* rec = nullptr;
 	size_t rec_bytes = 0;
+	uint32_t block = 0;         // counter block of the next call
+	bool ready = false;         // it is zero: the last call on the stream went through
 	uint32_t* flips = nullptr;  // zero between launch sequences
 	size_t flip_bytes = 0;
 	JobDesc* staging = nullptr; // pinned host copy of uploaded job arrays
@@ -171,7 +179,10 @@ std::map<std::pair<int, cudaStream_t>, StreamScratch> g_ws;
 
 bool capturing(cudaStream_t s) {
 	cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-	if (cudaStreamIsCapturing(s, &st) != cudaSuccess) return false;
+	if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+		cudaGetLastError();
+		return false;
+	}
 	return st != cudaStreamCaptureStatusNone;
 }
 
@@ -189,6 +200,7 @@ cvx_status ensure_scratch(int dev, cudaStream_t s, size_t rec_bytes, size_t flip
 		if (w.rec) cudaFree(w.rec);
 		w.rec = nullptr;
 		w.rec_bytes = 0;
+		w.ready = false;
 		size_t b = std::max(rec_bytes, (size_t)1 << 20);
 		if (cudaMalloc(&w.rec, b) != cudaSuccess) {
 			cudaGetLastError();
@@ -410,6 +422,8 @@ struct Runner {
 	uint32_t bricks = 0;   // brick capacity of the record area (largest group's bricks)
 	bool timed = true;     // per-kernel events for cvx_profile_collect (callers on this thread only)
 	bool fresh = true;     // the counters are zero: the caller cleared the area before run()
+	uint32_t block = 0;    // counter block in use
+	bool alternate = false;  // the sequences use blocks 0 and 1 in turn, each clearing the other for the next
 	const Prof* p() const { return timed ? prof() : nullptr; }
 
 	cvx_status prepare(Group& g, LaunchDesc& L) {
@@ -421,7 +435,12 @@ struct Runner {
 		L.n_mwarps = g.mwarps;
 		if (g.bricks > bricks) return fail(CVX_ERR_INVALID_VALUE, "brick scratch too small");
 		L.n_bricks = g.bricks;
-		bind_scratch(L, rec, cap, bricks, dev.tune);
+		bind_scratch(L, rec, cap, bricks, dev.tune, block);
+		if (alternate) {  // an earlier sequence of this call may have left an error there: keep it
+			const RecLayout l = rec_layout(0, 0);
+			L.scr.next = reinterpret_cast<uint32_t*>(rec + (block ^ 1u) * l.block);
+			L.scr.next_words = (uint32_t)((reset_bytes() + (fresh ? sizeof(Counters::error) : 0)) / 4);
+		}
 		if (g.jobs.size() == 1) {
 			L.single = g.jobs[0];
 			L.jobs = nullptr;
@@ -438,10 +457,14 @@ struct Runner {
 		return CVX_OK;
 	}
 
+	// Between two sequences: the first finds the counters cleared.
 	cvx_status reset_counters() {
-		if (!fresh) CVX_CUDA(cudaMemsetAsync(rec, 0, reset_bytes(), s));
+		if (!fresh && !alternate) CVX_CUDA(cudaMemsetAsync(rec + block * rec_layout(0, 0).block, 0, reset_bytes(), s));
 		fresh = false;
 		return CVX_OK;
+	}
+	void sequence_done() {
+		if (alternate) block ^= 1u;
 	}
 
 	cvx_status run(const std::vector<JobDesc>& surf, const std::vector<JobDesc>& solid) {
@@ -451,6 +474,7 @@ struct Runner {
 			if (st != CVX_OK) return st;
 			if ((st = reset_counters()) != CVX_OK) return st;
 			CVX_CUDA(launch_surface(L, dev.tune, dev.rows_grid, dev.raster_grid, s, p()));
+			sequence_done();
 		}
 		if (!solid.empty()) {
 			for (Group& g : make_groups(solid, true)) {
@@ -459,6 +483,7 @@ struct Runner {
 				if (st != CVX_OK) return st;
 				if ((st = reset_counters()) != CVX_OK) return st;
 				CVX_CUDA(launch_solid(L, dev.tune, dev.cols_grid, s, kSolidToggles, p()));
+				sequence_done();
 			}
 			Group r = resolve_group(solid);
 			LaunchDesc L;
@@ -526,9 +551,22 @@ cvx_status run_internal(std::vector<JobDesc> surf, std::vector<JobDesc> solid, c
 	r.cap = cap;
 	r.jobs_off = lay.jobs;
 	r.bricks = bricks;
-	CVX_CUDA(cudaMemsetAsync(w->rec, 0, lay.big, s));  // counters and brick counts
+	r.alternate = !bricks && !capturing(s);
+	if (r.alternate) {
+		r.block = w->block;
+		if (!w->ready) CVX_CUDA(cudaMemsetAsync(w->rec, 0, lay.big, s));
+		w->ready = false;  // until the call has gone through
+	} else {
+		r.block = kCaptureBlock;  // the last one, beside the brick counts
+		const size_t at = kCaptureBlock * lay.block;
+		CVX_CUDA(cudaMemsetAsync(static_cast<char*>(w->rec) + at, 0, lay.big - at, s));
+	}
 	st = r.run(surf, solid);
 	if (st != CVX_OK) return st;
+	if (r.alternate) {
+		w->block = r.block;
+		w->ready = true;
+	}
 	if (slots) CVX_CUDA(cudaEventRecord(w->staging_done, s));
 	return CVX_OK;
 }
@@ -776,9 +814,12 @@ cvx_status cvx_device_status(cvx_stream_t stream) {
 		if (it != g_ws.end()) rec = it->second.rec;
 	}
 	if (rec) {
-		Counters c;
-		CVX_CUDA(cudaMemcpy(&c, static_cast<char*>(rec) + rec_layout(0, 0).ctr, sizeof(c), cudaMemcpyDeviceToHost));
-		if (c.error) return fail(CVX_ERR_DEVICE_CHECK, "device check failed (code %u)", c.error);
+		const RecLayout l = rec_layout(0, 0);
+		for (uint32_t i = 0; i < kCounterBlocks; i++) {
+			Counters c;
+			CVX_CUDA(cudaMemcpy(&c, static_cast<char*>(rec) + i * l.block + l.ctr, sizeof(c), cudaMemcpyDeviceToHost));
+			if (c.error) return fail(CVX_ERR_DEVICE_CHECK, "device check failed (code %u)", c.error);
+		}
 	}
 	// the last cvx_voxelize_solid_noalloc call on this device keeps its counters in the library's
 	// fixed scratch array

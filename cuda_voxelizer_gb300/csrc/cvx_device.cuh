@@ -228,6 +228,8 @@ static_assert(sizeof(BrickTri) == 176, "BrickTri is eleven 16-byte vectors");
 struct Scratch {
 	Counters* ctr;
 	unsigned long long* tickets;  // kTicketBytes: the ticket counters of surf_rows, zero before a launch sequence
+	uint32_t* next;        // the counter block of the next launch sequence: the persistent kernel of this one
+	uint32_t next_words;   // zeroes that many words of it (null: the host clears the counters)
 	BigRec* big;
 	MidRec* mid;
 	uint32_t cap;          // capacity of big[], mid[], bq[] and tri[] (>= triangles in the launch)

@@ -338,6 +338,7 @@ template <class P>
 __global__ void __launch_bounds__(kRowsThreads) solid_cols(const __grid_constant__ LaunchDesc L) {
 	const uint32_t lane = threadIdx.x & 31u;
 	Counters* C = L.scr.ctr;
+	clear_next_counters(L);
 	__shared__ unsigned long long s_bigc;  // read once per CTA (see surf_rows)
 	__shared__ unsigned s_mid;
 	if (threadIdx.x == 0) {

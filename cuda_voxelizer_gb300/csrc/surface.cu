@@ -245,6 +245,7 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 	const uint32_t lane = threadIdx.x & 31u;
 	RowsWarp& W = s_warp[threadIdx.x >> 5];
 	Counters* C = L.scr.ctr;
+	clear_next_counters(L);
 	// One thread per CTA reads the queue counters (thousands of warps reading one line would
 	// serialise on its L2 slice), the CTA shares them through shared memory.
 	__shared__ unsigned long long s_bigc;

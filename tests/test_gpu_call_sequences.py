@@ -1,0 +1,97 @@
+"""Calls in any order on one stream: each finds its counters cleared, whoever cleared them.
+
+The meshes have triangles of every size, so that every call queues work: a counter left over from an
+earlier call would show as missing or repeated rows.
+"""
+import random
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from cuda_voxelizer_gb300 import api as cv  # noqa: E402
+from cuda_voxelizer_gb300 import meshgen  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+class _Work:
+    def __init__(self):
+        self.items = []
+        for tris, g in ((meshgen.soup(1, n=3000), 200), (meshgen.icosphere(2, level=3), 256), (meshgen.torus(3), 64)):
+            info = cv.make_voxinfo(tris, g)
+            d = torch.from_numpy(np.ascontiguousarray(tris).reshape(-1)).cuda()
+            for solid in ((False,) if g == 200 else (False, True)):
+                ws = torch.empty(cv.workspace_size(info, solid), dtype=torch.uint8, device="cuda")
+                want = self.table(info)
+                cv.voxelize_ws(info, d, want, ws, solid=solid)  # its own counters, cleared by the host
+                self.items.append((info, d, solid, want))
+
+    @staticmethod
+    def table(info):
+        return torch.zeros(cv.table_words(info), dtype=torch.int32, device="cuda")
+
+    def call(self, k, table):
+        info, d, solid, _ = self.items[k]
+        (cv.voxelize_solid if solid else cv.voxelize)(info, d, table)
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_direct_batched_and_captured_calls_interleaved(seed):
+    rng = random.Random(seed)
+    work = _Work()
+    stream = torch.cuda.Stream()
+    graphs = []
+    with torch.cuda.stream(stream):
+        # the scratch has to exist before a capture, in the size of the largest call that will be made
+        cv.voxelize_batch([cv.Job(info, d, work.table(info), False, solid) for info, d, solid, _ in work.items])
+        torch.cuda.synchronize()
+        for k in rng.sample(range(len(work.items)), 3):
+            table = work.table(work.items[k][0])
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=stream):
+                table.zero_()
+                work.call(k, table)
+            graphs.append((g, k, table))
+        done = []
+        for _ in range(40):
+            what = rng.randrange(3)
+            if what == 0:
+                k = rng.randrange(len(work.items))
+                table = work.table(work.items[k][0])
+                work.call(k, table)
+                done.append((k, table))
+            elif what == 1:  # surface and solid jobs: two launch sequences in one call
+                ks = rng.sample(range(len(work.items)), rng.randint(2, len(work.items)))
+                tables = [work.table(work.items[k][0]) for k in ks]
+                cv.voxelize_batch([cv.Job(work.items[k][0], work.items[k][1], t, False, work.items[k][2])
+                                   for k, t in zip(ks, tables)])
+                done += list(zip(ks, tables))
+            else:
+                g, k, table = rng.choice(graphs)
+                g.replay()
+                done.append((k, table.clone()))
+        cv.device_status(stream)
+    torch.cuda.synchronize()
+    for k, table in done:
+        assert torch.equal(table, work.items[k][3])
+
+
+def test_calls_on_several_streams():
+    work = _Work()
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    done = []
+    for r in range(5):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                k = (r + i) % len(work.items)
+                table = work.table(work.items[k][0])
+                work.call(k, table)
+                done.append((k, table))
+    torch.cuda.synchronize()
+    for s in streams:
+        cv.device_status(s)
+        cv.stream_release(s)
+    for k, table in done:
+        assert torch.equal(table, work.items[k][3])
