@@ -246,7 +246,7 @@ class HostJob:
 
 class HostPlan:
     """cvx_plan_create_host: the whole round trip -- tables zeroed, triangles up in ``n_chunks``
-    pieces (0: the library's default), surface jobs voxelizing each piece as it lands, solid jobs
+    pieces (0: the library's default), surface jobs voxelizing the pieces as they land, solid jobs
     after the last, each table copied down as soon as it is complete -- as one CUDA graph launch.
     Plans share no device state: two plans over their own device buffers and host tables, launched
     on two streams in turn, overlap one round trip's upload with the other's read-back."""
@@ -296,7 +296,7 @@ class HostPipeline:
     """Round trips back to back: ``len(slots)`` host plans, each over its own device buffers and
     host tables (``slots[i]`` is slot i's list of HostJob), launched on their own streams in turn,
     so that one round trip's upload and kernels run while the previous one's tables are still
-    going down.  ``submit()`` launches the next slot and returns its index; that slot's host tables
+    going down; a round trip's upload follows the previous one's (cvx_plan_wait_uploads).  ``submit()`` launches the next slot and returns its index; that slot's host tables
     are complete once ``wait(slot)`` returns.  A slot's next launch rewrites its host tables, so
     read them before the rotation comes back to it (after ``len(slots)`` more submits)."""
 
@@ -330,6 +330,8 @@ class HostPipeline:
 
     def submit(self) -> int:
         i = self._next
+        if len(self._plans) > 1:
+            check(lib.cvx_plan_wait_uploads(self._plans[i - 1]._h, _stream(self._streams[i])), "cvx_plan_wait_uploads")
         self._plans[i].launch(self._streams[i])
         self._done[i].record(self._streams[i])
         self._next = (i + 1) % len(self._plans)

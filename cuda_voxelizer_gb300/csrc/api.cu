@@ -872,6 +872,7 @@ struct cvx_plan {
 	JobDesc* job_area = nullptr;   // the job arrays of every lane's multi-job launches
 	uint32_t* flips = nullptr;
 	ClearRange* clears = nullptr;  // the tables the graph zeroes (CVX_PLAN_CLEAR_TABLES)
+	cudaEvent_t uploaded = nullptr;  // host plans: recorded by the graph when its triangles are up
 };
 
 // A plan runs its jobs in lanes: the surface jobs split into up to kPlanSurfaceLanes groups of
@@ -1128,8 +1129,8 @@ cvx_status cvx_plan_create(const cvx_job* jobs, uint32_t n_jobs, uint32_t flags,
 
 namespace {
 
-constexpr uint32_t kHostPlanDefaultChunks = 2;
 constexpr uint32_t kHostPlanMaxChunks = 64;
+constexpr uint64_t kHostPlanSplit = 1u << 17;  // triangles (4.7 MB: 23 us of upload) from which a mesh goes up in pieces
 
 bool page_locked(const void* p) {
 	cudaPointerAttributes a;
@@ -1165,15 +1166,16 @@ struct HostStep {
 // A host-buffer plan is the round trip of plain calls on host memory -- copy the triangles up,
 // voxelize, copy the tables down -- arranged for a link that is slower than the kernels: the copies
 // bound it, so the plan keeps the link busy.  Meshes go up one after another, each in chunks, on a
-// copy stream; one compute stream runs the surface jobs on each chunk as soon as it lands (exact: a
-// surface table is the OR of its chunks' bits), so they complete with the last chunk; then each
+// copy stream; one compute stream runs the surface jobs on the chunks as they land (exact: a surface
+// table is the OR of its chunks' bits), so they complete with or soon after the last chunk; then each
 // solid table in turn over the whole mesh.  Tables are completed one at a time so that a read-back
-// stream can copy each down while the next is still being computed.
+// stream can copy each down while the next is still being computed.  Icosphere 8 at 512^3, four modes: 636 us a launch, 661 us with every
+// surface job on both halves of the mesh (its copies alone take 577 us); at 256^3 362 / 422 us,
+// icosphere 5 at 512^3 419 / 487 us, the 9,216-triangle torus at 64^3 51 / 88 us.
 cvx_status cvx_plan_create_host(const cvx_host_job* jobs, uint32_t n_jobs, uint32_t n_chunks, cvx_plan** out) {
 	if (!out) return fail(CVX_ERR_INVALID_VALUE, "out is null");
 	*out = nullptr;
 	if (n_jobs && !jobs) return fail(CVX_ERR_INVALID_VALUE, "jobs is null");
-	if (n_chunks == 0) n_chunks = kHostPlanDefaultChunks;
 	if (n_chunks > kHostPlanMaxChunks) return fail(CVX_ERR_INVALID_VALUE, "n_chunks above %u", kHostPlanMaxChunks);
 	for (uint32_t i = 0; i < n_jobs; i++) {
 		const cvx_host_job& J = jobs[i];
@@ -1205,13 +1207,26 @@ cvx_status cvx_plan_create_host(const cvx_host_job* jobs, uint32_t n_jobs, uint3
 			up.h = J.h_triangles;
 			up.d = J.d_triangles;
 			up.n = J.info.n_triangles;
-			up.bounds.resize(n_chunks + 1);
-			for (uint32_t c = 0; c < n_chunks; c++) up.bounds[c] = up.n * c / n_chunks / kTile * kTile;
-			up.bounds[n_chunks] = up.n;
 			u = (int)ups.size();
 			ups.push_back(std::move(up));
 		}
 		up_of[i] = u;
+	}
+	// The chunks.  By default a mesh that uploads in a few microseconds goes up in one piece; a larger one
+	// in a half, three eighths and an eighth.  Its first surface job follows every piece, so that its table
+	// -- the first one to go down -- waits only for the work of the last; the others take the first half when
+	// it lands and the rest after the last piece.
+	for (Upload& up : ups) {
+		if (n_chunks) {
+			for (uint32_t c = 0; c < n_chunks; c++) up.bounds.push_back(up.n * c / n_chunks / kTile * kTile);
+		} else {
+			up.bounds.push_back(0);
+			if (up.n >= kHostPlanSplit) {
+				up.bounds.push_back(up.n / 2 / kTile * kTile);
+				up.bounds.push_back(up.n / 8 * 7 / kTile * kTile);
+			}
+		}
+		up.bounds.push_back(up.n);
 	}
 
 	cvx_plan* p = new cvx_plan();
@@ -1284,9 +1299,13 @@ cvx_status cvx_plan_create_host(const cvx_host_job* jobs, uint32_t n_jobs, uint3
 	};
 	for (uint32_t u = 0; u < (uint32_t)ups.size(); u++) {
 		std::vector<uint32_t> mine;
+		uint32_t first_surface = n_jobs;
 		for (uint32_t i = 0; i < n_jobs; i++)
-			if (up_of[i] == (int)u) mine.push_back(i);
-		for (uint32_t c = 0; c < n_chunks; c++) {
+			if (up_of[i] == (int)u) {
+				mine.push_back(i);
+				if (!jobs[i].solid && first_surface == n_jobs) first_surface = i;
+			}
+		for (uint32_t c = 0; c + 1 < (uint32_t)ups[u].bounds.size(); c++) {
 			const uint64_t b0 = ups[u].bounds[c], b1 = ups[u].bounds[c + 1];
 			if (b1 == b0) continue;
 			HostStep w;
@@ -1298,7 +1317,7 @@ cvx_status cvx_plan_create_host(const cvx_host_job* jobs, uint32_t n_jobs, uint3
 			std::vector<JobDesc> part;
 			if (!last) {
 				for (uint32_t i : mine)
-					if (!jobs[i].solid) part.push_back(job_of(i, b0, b1));
+					if (!jobs[i].solid && (n_chunks || c == 0 || i == first_surface)) part.push_back(job_of(i, b0, b1));
 				add_groups(part, false);
 				continue;
 			}
@@ -1306,7 +1325,7 @@ cvx_status cvx_plan_create_host(const cvx_host_job* jobs, uint32_t n_jobs, uint3
 			// the link starts on the first table after a fraction of the chunk's work.
 			for (uint32_t i : mine)
 				if (!jobs[i].solid) {
-					part.push_back(job_of(i, b0, b1));
+					part.push_back(job_of(i, n_chunks || i == first_surface || c == 0 ? b0 : ups[u].bounds[1], b1));
 					add_groups(part, false);
 					HostStep f;
 					f.kind = HostStep::kFinal;
@@ -1353,7 +1372,8 @@ cvx_status cvx_plan_create_host(const cvx_host_job* jobs, uint32_t n_jobs, uint3
 	// The capture: compute on the origin stream, uploads on cp, read-backs on rb.
 	cudaStream_t cs = nullptr, cp = nullptr, rb = nullptr;
 	cudaEvent_t fork_ev = nullptr, copied = nullptr, read = nullptr;
-	std::vector<std::vector<cudaEvent_t>> landed(ups.size(), std::vector<cudaEvent_t>(n_chunks, nullptr));
+	std::vector<std::vector<cudaEvent_t>> landed;
+	for (const Upload& up : ups) landed.emplace_back(up.bounds.size() - 1, nullptr);
 	std::vector<cudaEvent_t> final_ev(n_jobs, nullptr);
 	cvx_status cst = CVX_OK;
 	auto mk_stream = [&](cudaStream_t* st) {
@@ -1374,6 +1394,7 @@ cvx_status cvx_plan_create_host(const cvx_host_job* jobs, uint32_t n_jobs, uint3
 	mk_event(&fork_ev);
 	mk_event(&copied);
 	mk_event(&read);
+	mk_event(&p->uploaded);
 	for (auto& v : landed)
 		for (cudaEvent_t& e : v) mk_event(&e);
 	for (cudaEvent_t& e : final_ev) mk_event(&e);
@@ -1403,7 +1424,7 @@ cvx_status cvx_plan_create_host(const cvx_host_job* jobs, uint32_t n_jobs, uint3
 	ck(cudaStreamWaitEvent(cp, fork_ev, 0), "capture fork");
 	ck(cudaStreamWaitEvent(rb, fork_ev, 0), "capture fork");
 	for (size_t u = 0; u < ups.size() && cst == CVX_OK; u++)
-		for (uint32_t c = 0; c < n_chunks && cst == CVX_OK; c++) {
+		for (uint32_t c = 0; c + 1 < (uint32_t)ups[u].bounds.size() && cst == CVX_OK; c++) {
 			const uint64_t b0 = ups[u].bounds[c], b1 = ups[u].bounds[c + 1];
 			if (b1 == b0) continue;
 			ck(cudaMemcpyAsync(const_cast<float*>(ups[u].d) + 9 * b0, ups[u].h + 9 * b0, (b1 - b0) * 36,
@@ -1411,6 +1432,7 @@ cvx_status cvx_plan_create_host(const cvx_host_job* jobs, uint32_t n_jobs, uint3
 			   "capture upload");
 			ck(cudaEventRecord(landed[u][c], cp), "capture upload");
 		}
+	ck(cudaEventRecordWithFlags(p->uploaded, cp, cudaEventRecordExternal), "capture upload");
 	ck(cudaEventRecord(copied, cp), "capture upload");
 	for (uint32_t i = 0; i < n_jobs; i++)
 		if (!overwrites(i)) ck(cudaMemsetAsync(jobs[i].d_table, 0, words_of(jobs[i].info) * 4, cs), "capture clear");
@@ -1460,6 +1482,12 @@ cvx_status cvx_plan_launch(cvx_plan* p, cvx_stream_t stream) {
 	return CVX_OK;
 }
 
+cvx_status cvx_plan_wait_uploads(const cvx_plan* p, cvx_stream_t stream) {
+	if (!p) return fail(CVX_ERR_INVALID_VALUE, "plan is null");
+	if (p->uploaded) CVX_CUDA(cudaStreamWaitEvent((cudaStream_t)stream, p->uploaded, 0));
+	return CVX_OK;
+}
+
 cvx_status cvx_plan_kernel_nodes(const cvx_plan* p, uint32_t* n_kernels) {
 	if (!p || !p->graph || !n_kernels) return fail(CVX_ERR_INVALID_VALUE, "plan or output is null");
 	size_t n = 0;
@@ -1484,6 +1512,7 @@ cvx_status cvx_plan_destroy(cvx_plan* p) {
 	if (p->job_area) cudaFree(p->job_area);
 	if (p->flips) cudaFree(p->flips);
 	if (p->clears) cudaFree(p->clears);
+	if (p->uploaded) cudaEventDestroy(p->uploaded);
 	delete p;
 	return CVX_OK;
 }

@@ -153,10 +153,10 @@ cvx_status cvx_plan_destroy(cvx_plan* plan);
 /* Host-buffer plans: the reference's round trip (src/main.cpp:209-222 hands voxelize host-visible
  * triangles and table) as one graph.  Each launch copies every job's triangles from h_triangles into
  * d_triangles, zeroes d_table, voxelizes, and copies d_table into h_table; the tables are
- * bit-identical to plain calls.  Meshes go up in job order, each in n_chunks pieces (0 = 2, at most
- * 64); the surface jobs voxelize each piece as soon as it lands, the solid jobs follow the mesh's
- * last piece, and each table is copied down as soon as it is complete, so the kernels run under
- * the copies and the link stays busy.  Jobs that share
+ * bit-identical to plain calls.  Meshes go up in job order, each in n_chunks pieces (at most 64; 0: one
+ * or three, by the mesh's size); the surface jobs voxelize the pieces as they land, the solid jobs
+ * follow the mesh's last piece, and each table is copied down as soon as it is complete, so the
+ * kernels run under the copies and the link stays busy.  Jobs that share
  * d_triangles must share h_triangles and n_triangles (one upload serves them); different uploads
  * and different tables must not overlap.  Host buffers must be page-locked (cudaHostAlloc or
  * cudaHostRegister).  Launch with cvx_plan_launch; the host tables are complete when the launch's
@@ -174,6 +174,11 @@ typedef struct cvx_host_job {
 	int32_t solid;
 } cvx_host_job;
 cvx_status cvx_plan_create_host(const cvx_host_job* jobs, uint32_t n_jobs, uint32_t n_chunks, cvx_plan** out);
+/* Work queued on `stream` after this call waits until the last launch of a host plan has its triangles
+ * on the device (no wait before the first launch, or for other plans).  Plans launched in turn on
+ * their own streams should wait for each other's uploads: two that upload at the same time also read
+ * back at the same time and leave each direction of the link idle in turn. */
+cvx_status cvx_plan_wait_uploads(const cvx_plan* plan, cvx_stream_t stream);
 
 /* ---- serving: requests admitted by device memory and batched continuously --------------------
  * No counterpart in the reference (src/main.cpp voxelizes one mesh per process).  A server owns
