@@ -1,8 +1,8 @@
 """Autotuner for the engine's tuning knobs (cvx_tuning), with a per-device cache.
 
 The knobs decide where a triangle's work goes; results never depend on them, only the time does:
-``small_vox`` (surface: triangles whose grid bounding box holds at most this many voxels are tested
-voxel by voxel in the classify kernel), ``small_cols`` (solid: triangles with at most this many
+``small_vox`` (surface: triangles of at most this many rows, and 64, of at most 16 voxels are tested
+voxel by voxel in the classify kernel), ``small_cols`` (solid: triangles with at most 8 times this many
 voxel-centre columns stay in the classify kernel) and ``brick_pairs`` (surface, grids of 2^29+
 voxels: (brick, triangle) pairs per triangle the shared-memory brick rasterizer may use; 0 sends
 every larger triangle to the row-by-row path with global atomics).  ``autotune()`` times a fixed set

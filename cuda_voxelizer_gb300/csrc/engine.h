@@ -13,12 +13,10 @@ constexpr uint32_t kZch = 32;          // most z-slices of a surface work item (
 constexpr uint32_t kMinSlices = 4;     // fewest, of a triangle with many rows in a small launch
 constexpr uint32_t kRowsThreads = 256; // threads per cooperative CTA
 constexpr uint32_t kColsPerItem = 256; // solid columns per work item
-constexpr uint32_t kLocalRows = 64;    // surface: rows a triangle may have in the classify kernel
-constexpr uint32_t kWarpRows = 384;    // surface: rows of a classify warp that are no longer few, in a small launch
+constexpr uint32_t kLocalRows = 64;    // surface: most rows of a triangle in the classify kernel
 constexpr uint32_t kMaskRowVoxels = 16; // surface: and voxels per row, each of them tested (the pass mask holds 16)
 constexpr uint32_t kSmallCols = 16;    // solid: largest small_cols
 constexpr uint32_t kColsPerSmall = 8;  // solid: columns a triangle may have in the classify kernel, per small_cols
-constexpr uint32_t kWarpCols = 448;    // solid: columns of a classify warp that are no longer few, in a small launch
 
 // Device-side check codes written to Counters::error.
 enum : unsigned { kErrBulkTimeout = 1u, kErrQueueOverflow = 2u };
@@ -33,7 +31,7 @@ constexpr uint64_t kMaxTriPerLaunch = (1ull << 24) - 1;
 constexpr uint32_t kMaxBrickPairs = 16;
 
 struct Tune {
-	uint32_t small_vox = 64;    // surface: bbox voxels at or below which a triangle stays in its thread
+	uint32_t small_vox = kLocalRows;   // surface: a triangle of up to this many rows stays in the classify kernel (at most kLocalRows)
 	uint32_t small_cols = kSmallCols;  // solid: a triangle of up to kColsPerSmall times as many columns stays in the classify kernel
 	// pairs per triangle the brick rasterizer may use; 0 (the default: on the 1024^3 stress soup the
 	// brick path measured about 25% slower than the row path) rasterizes every larger triangle by rows

@@ -205,12 +205,13 @@ static_assert(sizeof(SmallSolid) == 80, "SmallSolid stride");
 // Bound by instructions on large meshes, by latency on small ones.  A triangle that stays costs its
 // columns; one that is queued costs solid_cols a chain of dependent loads and a second setup.  Times
 // of solid_classify + solid_cols, triangles of up to 128 / up to 16 columns staying, in us:
-//   icosphere 8 at 1024^3 77 + 12 / 150 + 81, 6 at 500^3 28 + 13 / 17 + 36 (10,240 and 640 CTAs);
-//   14,400-triangle torus at 512^3 61 + 11 / 12 + 20 (113 CTAs: a few long warps, hence kWarpCols).
+//   icosphere 8 at 1024^3 77 + 12 / 150 + 81, 6 at 500^3 28 + 13 / 17 + 36 (10,240 and 640 CTAs).
+// In a launch of few CTAs the split (classify_split) spreads the columns; a limit of 448 columns to a
+// warp, with the rest left to solid_cols, gained nothing beside it.
 // With item lists dealt over the CTA and 16 columns the same meshes took 150 + 76, 18 + 36, 12 + 21.
 template <class P>
 __global__ void __launch_bounds__(kTile, 12) solid_classify(const __grid_constant__ LaunchDesc L, const uint32_t small_cols,
-                                                              const uint32_t warp_cols, const uint32_t split) {
+                                                              const uint32_t split) {
 	__shared__ __align__(16) union {
 		float tri[32 * 9];
 		SmallSolid small[32];
@@ -250,7 +251,6 @@ __global__ void __launch_bounds__(kTile, 12) solid_classify(const __grid_constan
 			ncols = (uint64_t)(S.y1 - S.y0 + 1) * (uint64_t)(S.z1 - S.z0 + 1);
 	}
 	if (ncols <= kColsPerSmall * small_cols) n_cols = (uint32_t)ncols;
-	if (__reduce_add_sync(FULL, n_cols) > warp_cols && n_cols > small_cols) n_cols = 0;
 	if (ncols > n_cols) {
 		const uint64_t it = (ncols + kColsPerItem - 1) / kColsPerItem;
 		n_items = (uint32_t)umin64(it, 0xFFFFFFu);
@@ -667,13 +667,9 @@ static cudaError_t launch_solid_t(const LaunchDesc& L, const Tune& tune, int col
 	cudaError_t e = cudaSuccess;
 	if (prof) (*prof)(nullptr, s);
 	if ((phases & kSolidToggles) && L.n_tiles) {
-		// As many classify CTAs as the persistent column grid has fill the chip: every triangle of up to
-		// kColsPerSmall * small_cols columns stays.  With fewer, the longest warp is the kernel's time, and
-		// a warp with more than kWarpCols columns leaves those above small_cols to solid_cols, which
-		// spreads them over the chip (both sides measured: solid_classify's comment).
-		const uint32_t warp_cols = L.n_tiles >= (uint32_t)cols_grid ? 0xFFFFFFFFu : kWarpCols;
+		// fewer classify CTAs than the persistent column grid has do not fill the chip
 		const uint32_t split = classify_split(L.n_tiles, (uint32_t)cols_grid);
-		solid_classify<P><<<L.n_tiles << split, kTile, 0, s>>>(L, std::min(tune.small_cols, kSmallCols), warp_cols, split);
+		solid_classify<P><<<L.n_tiles << split, kTile, 0, s>>>(L, std::min(tune.small_cols, kSmallCols), split);
 		if ((e = cudaGetLastError()) != cudaSuccess) return e;
 		if (prof) (*prof)("solid_classify", s);
 		if ((e = launch_k(solid_cols<P>, (unsigned)cols_grid, kRowsThreads, 0, s, L)) != cudaSuccess) return e;

@@ -23,7 +23,7 @@ namespace cvx {
 namespace {
 
 // Four independent warps per CTA, 32 triangles each (fewer in a launch with few tiles); nothing waits
-// on a CTA barrier.  Phase 1: one lane per triangle: setup, then the triangles of up to kLocalRows
+// on a CTA barrier.  Phase 1: one lane per triangle: setup, then the triangles of up to local_rows
 // rows of up to kMaskRowVoxels voxels park it in the warp's shared memory, packed, and the larger ones
 // are queued for surf_rows (or the brick kernels).  Phase 2: the parked triangles' rows, 32 at a time,
 // one per lane: a lane finds its triangle by counting the triangles that start at or before its row
@@ -34,10 +34,12 @@ namespace {
 // before they are compared.  Nine CTAs per SM at 54 registers; ten at 48 are 1% slower.
 // Triangles with longer rows, or more, cost less in surf_rows, which shares one setup over a warp: with
 // up to 256 rows of any length kept here, the soup of 300,000 at 300^3 took 148 + 642 us in the two
-// kernels, 44 + 701 with this rule.
+// kernels, 44 + 701 with this rule.  A warp keeps all such triangles, also in a launch of few CTAs:
+// leaving those of a warp with more than 384 rows to surf_rows took 31 + 75 us instead of 43 + 37 on
+// icosphere 6 at 700^3 (640 CTAs), 31 + 44 / 35 + 19 at 500^3, and the same on meshes of up to 160 CTAs.
 template <class P>
-__global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant__ LaunchDesc L, const uint32_t small_vox,
-                                                             const uint32_t warp_rows, const uint32_t item_rows, const uint32_t split) {
+__global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant__ LaunchDesc L, const uint32_t local_rows,
+                                                             const uint32_t item_rows, const uint32_t split) {
 	__shared__ __align__(16) union {
 		float tri[32 * 9];
 		SmallTri small[32];
@@ -67,19 +69,16 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 
 	SurfTri S;
 	uint32_t n_items = 0, n_rows = 0, slices = kZch;
-	bool few = false;
 	if (valid) {
 		const float bmin[3] = {J.bmin[0], J.bmin[1], J.bmin[2]};
 		const float inv[3] = {J.inv_unit[0], J.inv_unit[1], J.inv_unit[2]};
 		surf_setup<P>(t, bmin, unit, inv, grid, S);
 		const uint32_t ex = (uint32_t)(S.bx1 - S.bx0), ey = (uint32_t)(S.by1 - S.by0), ez = (uint32_t)(S.bz1 - S.bz0);
 		const uint64_t rows = (uint64_t)(ey + 1) * (uint64_t)(ez + 1);
-		few = (uint64_t)(ex + 1) * rows <= small_vox;
 		while (slices > kMinSlices && (uint64_t)(ey + 1) * slices > item_rows) slices >>= 1;
 		n_items = ez / slices + 1u;
-		if (ex < kMaskRowVoxels && rows <= kLocalRows && !plane_underflows(S)) n_rows = (uint32_t)rows;
+		if (ex < kMaskRowVoxels && rows <= local_rows && !plane_underflows(S)) n_rows = (uint32_t)rows;
 	}
-	if (__reduce_add_sync(FULL, n_rows) > warp_rows && !few) n_rows = 0;
 	uint32_t incl = n_rows;
 #pragma unroll
 	for (int d = 1; d < 32; d <<= 1) {
@@ -397,9 +396,6 @@ static cudaError_t launch_surface_t(const LaunchDesc& L, const Tune& tune, int r
                                     cudaStream_t s, const Prof* prof) {
 	if (L.n_tiles == 0) return cudaSuccess;
 	if (prof) (*prof)(nullptr, s);
-	// With fewer CTAs than fill the chip the longest warp is the kernel's time: a warp with more than
-	// kWarpRows rows leaves the triangles above small_vox voxels to surf_rows.
-	const uint32_t warp_rows = L.n_tiles >= (uint32_t)rows_grid ? 0xFFFFFFFFu : kWarpRows;
 	// Rows (of the bounding box) that a queued triangle's items may have: with few triangles there are
 	// fewer items than surf_rows has warps, and one item of a large triangle is its time.  In surf_rows,
 	// with items of up to 1024 rows / 4096 / 32 slices whatever their rows: icosphere 3 at 1000^3 (1,280
@@ -408,7 +404,7 @@ static cudaError_t launch_surface_t(const LaunchDesc& L, const Tune& tune, int r
 	const uint64_t triangles = (uint64_t)L.n_tiles * kTile, warps = (uint64_t)rows_grid * (kRowsCtaThreads / 32);
 	const uint32_t item_rows = triangles < 4 * warps ? 1024u : (triangles < 16 * warps ? 4096u : 0xFFFFFFFFu);
 	const uint32_t split = classify_split(L.n_tiles, (uint32_t)rows_grid);
-	surf_classify<P><<<L.n_tiles << split, kTile, 0, s>>>(L, tune.small_vox, warp_rows, item_rows, split);
+	surf_classify<P><<<L.n_tiles << split, kTile, 0, s>>>(L, std::min(tune.small_vox, kLocalRows), item_rows, split);
 	cudaError_t e = cudaGetLastError();
 	if (e != cudaSuccess) return e;
 	if (prof) (*prof)("surf_classify", s);

@@ -296,8 +296,8 @@ cvx_status cvx_encode_voxel_list_ws(const cvx_voxinfo* info, const uint32_t* d_t
 /* ---- tuning ---------------------------------------------------------------------------------- */
 
 typedef struct cvx_tuning {
-	uint32_t small_vox;   /* surface: triangles with at most this many bbox voxels stay in one thread */
-	uint32_t small_cols;  /* solid: triangles with at most this many columns (in large launches, 8 times as many) stay in the classify kernel; at most 16 */
+	uint32_t small_vox;   /* surface: triangles with at most this many rows (of at most 16 voxels) stay in the classify kernel; at most 64 */
+	uint32_t small_cols;  /* solid: triangles with at most 8 times this many columns stay in the classify kernel; at most 16 */
 	uint32_t brick_pairs; /* surface, grids of 2^29+ voxels: (brick, triangle) pairs per triangle the
 	                       * shared-memory brick rasterizer may use, at most 16; 0 (the default)
 	                       * rasterizes every larger triangle row by row with global atomics instead */
