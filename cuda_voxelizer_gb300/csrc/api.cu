@@ -306,6 +306,10 @@ JobDesc make_job(const cvx_voxinfo& v, const float* tris, uint32_t* table, int m
 	j.flags = (morton ? JOB_MORTON : 0u) | (solid ? JOB_SOLID : 0u);
 	const uint64_t voxels = (uint64_t)v.gridsize[0] * v.gridsize[1] * v.gridsize[2];
 	if (morton ? v.gridsize[0] <= 1024 : voxels <= (1ull << 32)) j.flags |= JOB_NARROW;
+	// From about 100 triangles per word of the table the atomics on a word wait for each other.  surf_classify
+	// with / without the test of the word: 1,000,000-triangle torus at 64^3 (122 a word) 36 / 70 us, at 33^3
+	// 33 / 209, icosphere 8 at 64^3 (160) 52 / 66; icosphere 9 at 128^3 (80) 152 / 143, 8 at 128^3 (20) 50 / 43.
+	if (!solid && v.n_triangles > 3 * voxels) j.flags |= JOB_DENSE;
 	if (!solid && brick_grid(j.grid) && current_brick_pairs()) j.flags |= JOB_BRICKS;
 	if (v.n_triangles && needs_plain_loads(tris)) j.flags |= JOB_PLAIN_LOADS;
 	return j;
@@ -320,6 +324,7 @@ struct Group {
 	uint32_t tiles = 0, units = 0;
 	uint64_t mwords = 0, mwarps = 0;
 	uint32_t bricks = 0;  // 64^3 bricks of the group's JOB_BRICKS jobs
+	bool dense = false;   // whether one is JOB_DENSE
 };
 
 // Voxel columns of the grid's faces per triangle: how much larger than a voxel a mesh's triangles are.
@@ -338,7 +343,9 @@ void finish_group(Group& g, bool solid) {
 	uint32_t tile = 0, unit = 0, brick = 0;
 	uint64_t mw = 0, mc = 0;
 	g.tris = 0;
+	g.dense = false;
 	for (JobDesc& j : g.jobs) {
+		g.dense |= (j.flags & JOB_DENSE) != 0;
 		j.tile_begin = tile;
 		tile += tiles_of(j.n_tri);
 		g.tris += j.n_tri;
@@ -435,6 +442,7 @@ struct Runner {
 		L.n_mwarps = g.mwarps;
 		if (g.bricks > bricks) return fail(CVX_ERR_INVALID_VALUE, "brick scratch too small");
 		L.n_bricks = g.bricks;
+		L.any_dense = g.dense;
 		bind_scratch(L, rec, cap, bricks, dev.tune, block);
 		if (alternate) {  // an earlier sequence of this call may have left an error there: keep it
 			const RecLayout l = rec_layout(0, 0);
@@ -895,6 +903,7 @@ static cudaError_t capture_group(const Group& g, bool solid, bool resolve, bool 
 	L.n_mwords = g.mwords;
 	L.n_mwarps = g.mwarps;
 	L.n_bricks = g.bricks;
+	L.any_dense = g.dense;
 	bind_scratch(L, static_cast<char*>(rec), cap, bricks, dev.tune);
 	if (g.jobs.size() == 1)
 		L.single = g.jobs[0];

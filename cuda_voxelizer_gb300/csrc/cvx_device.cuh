@@ -78,8 +78,10 @@ __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, fl
 // read them with ordinary loads instead of bulk copies.
 // JOB_BRICKS: a surface job whose queued (larger) triangles are rasterized brick by brick in shared
 // memory (bricks.cu) instead of by per-row global atomics.
+// JOB_DENSE: a surface job with many triangles per word of its table, whose classify kernel looks at a word
+// before it ORs into it.  Set by the host; the words are the same either way.
 enum : uint32_t { JOB_MORTON = 1u, JOB_SOLID = 2u, JOB_NARROW = 4u, JOB_TABLE_OVERWRITE = 8u, JOB_PLAIN_LOADS = 16u,
-                  JOB_BRICKS = 32u };
+                  JOB_BRICKS = 32u, JOB_DENSE = 64u };
 
 // One mesh voxelization.  Plain data, uploaded as an array for batches or passed by value for a
 // single mesh.
@@ -252,6 +254,7 @@ struct LaunchDesc {
 	uint64_t n_mwords;     // Morton words of solid Morton jobs with g < 32
 	uint64_t n_mwarps;     // warps of solid_morton_cols: solid Morton jobs with g >= 32
 	uint32_t n_bricks;     // 32^3 bricks of the launch's JOB_BRICKS jobs
+	uint32_t any_dense;    // whether a job of the launch is JOB_DENSE
 	Scratch scr;
 };
 

@@ -598,11 +598,27 @@ __device__ __forceinline__ void write_row_t(uint32_t* table, bool morton, const 
 	}
 }
 
+// OR `m` into a word of the table.  kDense (JOB_DENSE): not if the word is seen to hold the bits already,
+// and lanes with the same word share one atomic.  Bits of a surface job's table are only ever set, so a stale
+// word in the L1 costs an atomic and never loses a voxel.  On triangles in the order of their place the
+// sharing is what counts (1,000,000-triangle torus at 33^3: 33 us, 91 with the look alone), elsewhere the
+// look (icosphere 9 at 40^3: 155 us, 393 with the sharing alone, 400 with neither).
+template <bool kDense>
+__device__ __forceinline__ void or_word(uint32_t* p, uint32_t m) {
+	if (kDense) {
+		if (!(m & ~__ldca(p))) return;
+		const uint32_t peers = __match_any_sync(__activemask(), (unsigned long long)(uintptr_t)p);
+		m = __reduce_or_sync(peers, m);
+		if ((threadIdx.x & 31u) != __ffs(peers) - 1u) return;
+	}
+	atomicOr(p, m);
+}
+
 // OR the voxels x0 + i of row (y, z) for the set bits i of `pm` (i < 16).  Linear: the run spans at
 // most two words; the bit of voxel idx is 31 - idx % 32, so a word's bits are the bit-reversed mask
 // shifted by the first voxel's offset.  Morton: one word per 4-voxel x-group (offsets {0, 1, 8, 9}
 // from the group's code, as in or_span_morton).
-template <class C>
+template <class C, bool kDense>
 __device__ __forceinline__ void write_row_mask_t(uint32_t* table, bool morton, const uint32_t* grid, int y, int z,
                                                  int x0, uint32_t pm) {
 	if (morton) {
@@ -615,7 +631,7 @@ __device__ __forceinline__ void write_row_mask_t(uint32_t* table, bool morton, c
 			if (n) {
 				const C code = xd | yz;
 				const uint32_t m = ((n & 1u) << 31) | ((n & 2u) << 29) | ((n & 4u) << 21) | ((n & 8u) << 19);
-				atomicOr(table + (code >> 5), m >> (uint32_t)(code & 31u));
+				or_word<kDense>(table + (code >> 5), m >> (uint32_t)(code & 31u));
 			}
 			xd = morton_x_add_t<C>(xd, (C)kMortonX4);
 		}
@@ -624,10 +640,10 @@ __device__ __forceinline__ void write_row_mask_t(uint32_t* table, bool morton, c
 		const C w = idx >> 5;
 		const uint32_t off = (uint32_t)(idx & 31u);
 		const uint32_t m0 = __brev(pm) >> off;
-		if (m0) atomicOr(table + w, m0);
+		if (m0) or_word<kDense>(table + w, m0);
 		if (off) {
 			const uint32_t m1 = __brev(pm >> (32u - off));
-			if (m1) atomicOr(table + w + 1, m1);
+			if (m1) or_word<kDense>(table + w + 1, m1);
 		}
 	}
 }
@@ -658,9 +674,10 @@ __device__ __forceinline__ void write_row_warp_t(uint32_t* table, bool morton, c
 	}
 }
 
+template <bool kDense>
 __device__ __forceinline__ void write_row_mask(uint32_t* table, bool morton, bool narrow, const uint32_t* grid, int y,
                                                int z, int x0, uint32_t pm) {
-	if (narrow) write_row_mask_t<uint32_t>(table, morton, grid, y, z, x0, pm);
-	else write_row_mask_t<uint64_t>(table, morton, grid, y, z, x0, pm);
+	if (narrow) write_row_mask_t<uint32_t, kDense>(table, morton, grid, y, z, x0, pm);
+	else write_row_mask_t<uint64_t, kDense>(table, morton, grid, y, z, x0, pm);
 }
 }  // namespace cvx

@@ -123,3 +123,36 @@ def test_large_triangles_nearly_parallel_to_an_axis(rsqrt, axis, tilt):
     t[:40, :, axis] = t[:40, :1, axis] + tilt * rng.uniform(-1, 1, (40, 3))        # the plane
     t[40:, 1, axis] = t[40:, 0, axis] + tilt * rng.uniform(-1, 1, 40)              # one edge
     _check(rsqrt, t.reshape(-1, 9).astype(np.float32), 256, False)
+
+
+@pytest.mark.parametrize("morton", [False, True])
+@pytest.mark.parametrize("g", [2, 8, 32])
+@pytest.mark.parametrize("extra", [0, 1, 5000])
+def test_many_triangles_per_word(rsqrt, g, morton, extra):
+    """Around three triangles per voxel of the grid, where rows are tested against the table before the atomic."""
+    n = 3 * g ** 3 + extra
+    t = _triangles(g, n, (0.6, 0.6, 0.6) if extra < 5000 else (1.5, 1.5, 1.5), g)
+    if g == 32:
+        t = t[np.lexsort(np.floor(t[:, :3]).T)]  # neighbours in space next to each other
+    _check(rsqrt, t, g, morton)
+
+
+def test_dense_and_sparse_jobs_in_one_plan():
+    """A plan with jobs on both sides of the rule writes the tables of its jobs one by one."""
+    rng = np.random.default_rng(4)
+    metas = [(16, 13_000, False), (64, 900, False), (33, 120_000, False), (16, 12_000, True), (32, 100_000, True)]
+    jobs, alone = [], []
+    for g, n, morton in metas:
+        tris = _triangles(rng.integers(1 << 30), n, (1, 1, 1), g)
+        info = cv.make_info((0, 0, 0), (float(g),) * 3, g, n)
+        d = torch.from_numpy(tris.reshape(-1)).cuda()
+        one, many = (torch.zeros(cv.table_words(info), dtype=torch.int32, device="cuda") for _ in range(2))
+        cv.voxelize(info, d, one, morton)
+        alone.append(one)
+        jobs.append(cv.Job(info, d, many, morton))
+    plan = cv.Plan(jobs, clear_tables=True)
+    for _ in range(2):
+        plan.launch()
+    torch.cuda.synchronize()
+    for one, job in zip(alone, jobs):
+        assert torch.equal(one, job.table)
