@@ -99,7 +99,7 @@ inline uint64_t morton_warps(uint64_t g) { return g < 32 ? 0 : (g / 4) * (g / 4)
 // multiple of the shortest such run of rows (gx / gcd(gx, 32) words, times 1, 2 or 4).  The longer
 // the unit, the less it spends on its set-up and the fewer warps there are: 512 words in a table of
 // 2^23 words or more (1024^3: 67 us; 72 us with 256, 84 us with 128), 256 in one of 2^20 or more
-// (512^3: 12 us; 14 us with 128 or 512), else 128, one step of a warp.
+// (500^3: 16 us), else 128, one step of a warp.  Grids whose rows go to one lane each: 32 rows.
 struct SolidUnits {
 	uint32_t unit_words;
 	uint64_t units;

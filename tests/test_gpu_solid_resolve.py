@@ -123,6 +123,15 @@ def test_linear(grid, offset, plan):
     _run(grid, False, offset, plan, sum(grid) + offset)
 
 
+@pytest.mark.parametrize("plan", [False, True])
+@pytest.mark.parametrize("offset", [0, 1])  # 1: not 16-byte aligned, so not by lane
+@pytest.mark.parametrize("grid", [(128, 7, 5), (128, 32, 32), (256, 31, 33), (384, 13, 5), (512, 64, 40), (640, 11, 3),
+                                  (768, 11, 3), (128, 1, 1), (640, 32, 1)])
+def test_linear_rows_by_lane(grid, offset, plan):
+    """Rows of 16-byte groups, up to the longest one that a lane walks by itself and beyond it."""
+    _run(grid, False, offset, plan, sum(grid) + offset)
+
+
 @pytest.mark.parametrize("n_boxes", [1, 40, 700])  # x faces: a partial warp, a few tiles, a grid that fills the chip
 @pytest.mark.parametrize("extent", [1, 4, 5, 11, 12, 16, 17])  # columns: 1, 16 | 25, 121 | 144, 256 | 289
 def test_columns_per_triangle(n_boxes, extent):
