@@ -22,12 +22,28 @@ namespace cvx {
 
 namespace {
 
+constexpr uint32_t kCollectRows = 384;  // rows of a classify warp from which those that pass the YZ tests are collected
+constexpr uint32_t kQueueRows = 64;     // fewer than 32 rows wait when 32 more are tested
+
+// The place of row r = dy + dz * ny of a parked triangle, r and ny at most kLocalRows: the approximate quotient is
+// more than 1e-3 away from the next integer and truncates exactly.
+__device__ __forceinline__ void row_place(const float4& box, uint32_t r, int& y, int& z) {
+	const uint32_t by = __float_as_uint(box.y), bz = __float_as_uint(box.z), ny = (by >> 24) + 1u;
+	const uint32_t dz = (uint32_t)__fdividef((float)r + 0.5f, (float)ny);
+	y = (int)((by & 0xFFFFFFu) + r - dz * ny);
+	z = (int)((bz & 0xFFFFFFu) + dz);
+}
+
 // Four independent warps per CTA, 32 triangles each (fewer in a launch with few tiles); nothing waits
 // on a CTA barrier.  Phase 1: one lane per triangle: setup, then the triangles of up to local_rows
 // rows of up to kMaskRowVoxels voxels park it in the warp's shared memory, packed, and the larger ones
 // are queued for surf_rows (or the brick kernels).  Phase 2: the parked triangles' rows, 32 at a time,
 // one per lane: a lane finds its triangle by counting the triangles that start at or before its row
 // (one warp-wide OR of start bits and a population count), and tests every voxel of its row.
+// Where the triangles have many rows, about half fail the YZ tests, and a warp tests the voxels of 32
+// rows that passed at a time: the 512^3 meshes of a 256-mesh mix 546 -> 507 us, its 256^3 meshes 356 ->
+// 343.  With few rows most pass: the icosphere at 512^3 (125 rows a warp) takes 77 us that way, and 74 with
+// one loop for both.
 // Bound by instructions (82% of issue slots busy on the icosphere at 512^3, 50 per triangle).  There
 // 71 us; 90 us with the rows listed in shared memory and dealt over the CTA behind three barriers, the
 // tests combined with short-circuit branches (15% of all instructions) and the edge sums added up
@@ -45,6 +61,7 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 		SmallTri small[32];
 	} s_warp[kTile / 32];
 	__shared__ __align__(8) uint64_t s_bar[kTile / 32];
+	__shared__ uint16_t s_queue[kTile / 32][kQueueRows];
 	const uint32_t tile = blockIdx.x >> split;
 	const uint32_t j = job_of_tile(L, tile);
 	const JobDesc& J = job_at(L, j);
@@ -143,32 +160,60 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 
 	// Phase 2: the rows of the parked triangles.
 	__syncwarp();
-	uint32_t begun = 0;  // triangles that start before this step's rows
-	for (uint32_t base = 0; base < total_rows; base += 32) {
-		const uint32_t at = start - base;
-		const uint32_t starts = __reduce_or_sync(FULL, n_rows && at < 32u ? 1u << at : 0u);
-		const uint32_t rec = begun + __popc(starts & (0xFFFFFFFFu >> (31u - lane))) - 1u;
-		begun += __popc(starts);
-		const uint32_t k = base + lane;
-		if (k >= total_rows) break;
-		const SmallTri& o = sm.small[rec];
-		const float4 box = o.q[0];
-		const uint32_t bx = __float_as_uint(box.x), by = __float_as_uint(box.y), bz = __float_as_uint(box.z);
-		// row r = dy + dz * ny of the triangle, r and ny at most kLocalRows: the approximate quotient is more than
-		// 1e-3 away from the next integer and truncates exactly
-		const uint32_t r = k - __float_as_uint(box.w), ny = (by >> 24) + 1u;
-		const uint32_t dz = (uint32_t)__fdividef((float)r + 0.5f, (float)ny);
-		const int y = (int)((by & 0xFFFFFFu) + r - dz * ny), z = (int)((bz & 0xFFFFFFu) + dz);
-		const float py = __fmul_rn(__int2float_rn(y), unit[1]);
-		const float pz = __fmul_rn(__int2float_rn(z), unit[2]);
-		if (!row_in_yz<P>(o, py, pz)) continue;
+	auto test_row = [&](const SmallTri& o, const float4& box, int y, int z) {
+		const uint32_t bx = __float_as_uint(box.x);
 		const int x0 = (int)(bx & 0xFFFFFFu);
-		const uint32_t pm = row_mask<P>(o, unit[0], py, pz, x0, (bx >> 24) + 1u);
-		if (!pm) continue;
+		const uint32_t pm = row_mask<P>(o, unit[0], __fmul_rn(__int2float_rn(y), unit[1]), __fmul_rn(__int2float_rn(z), unit[2]),
+		                                x0, (bx >> 24) + 1u);
+		if (!pm) return;
 		if (kDense && (jflags & JOB_DENSE))
 			write_row_mask<true>(table, (jflags & JOB_MORTON) != 0, (jflags & JOB_NARROW) != 0, grid, y, z, x0, pm);
 		else
 			write_row_mask<false>(table, (jflags & JOB_MORTON) != 0, (jflags & JOB_NARROW) != 0, grid, y, z, x0, pm);
+	};
+	uint32_t begun = 0;  // triangles that start before this step's rows
+	// Row k's triangle and its row of it, y and z; whether the row passes the YZ tests.  Every lane calls it.
+	auto find_row = [&](uint32_t base, uint32_t& rec, uint32_t& r, float4& box, int& y, int& z) {
+		const uint32_t at = start - base;
+		const uint32_t starts = __reduce_or_sync(FULL, n_rows && at < 32u ? 1u << at : 0u);
+		rec = begun + __popc(starts & (0xFFFFFFFFu >> (31u - lane))) - 1u;
+		begun += __popc(starts);
+		const uint32_t k = base + lane;
+		if (k >= total_rows) return false;
+		const SmallTri& o = sm.small[rec];
+		box = o.q[0];
+		r = k - __float_as_uint(box.w);
+		row_place(box, r, y, z);
+		return row_in_yz<P>(o, __fmul_rn(__int2float_rn(y), unit[1]), __fmul_rn(__int2float_rn(z), unit[2]));
+	};
+	uint32_t rec, r;
+	float4 box;
+	int y, z;
+	if (total_rows < kCollectRows) {
+		for (uint32_t base = 0; base < total_rows; base += 32)
+			if (find_row(base, rec, r, box, y, z)) test_row(sm.small[rec], box, y, z);
+		return;
+	}
+	uint16_t* queue = s_queue[wid];      // a ring of rows that passed
+	uint32_t filled = 0, done = 0;       // rows put into it and taken out
+	for (uint32_t base = 0; base < total_rows || done < filled;) {
+		while (base < total_rows && filled - done < 32u) {
+			const bool pass = find_row(base, rec, r, box, y, z);
+			const uint32_t passed = __ballot_sync(FULL, pass);
+			if (pass) queue[(filled + __popc(passed & lt)) % kQueueRows] = (uint16_t)(rec | r << 5);
+			filled += __popc(passed);
+			base += 32;
+		}
+		__syncwarp();
+		if (done + lane < filled) {
+			const uint32_t e = queue[(done + lane) % kQueueRows];
+			const SmallTri& o = sm.small[e & 31u];
+			box = o.q[0];
+			row_place(box, e >> 5, y, z);
+			test_row(o, box, y, z);
+		}
+		done = min(done + 32u, filled);
+		__syncwarp();  // read before the places are filled again
 	}
 }
 

@@ -94,6 +94,14 @@ def test_mixed_sizes(rsqrt, n):
     _check(rsqrt, t, 256, False)
 
 
+@pytest.mark.parametrize("ext,morton", [((3, 2.4, 2.4), False), ((3, 2.6, 2.6), True), ((14, 7, 7), False), ((2, 61, 0.3), True)])
+def test_collected_rows(rsqrt, ext, morton):
+    """Warps of 32 triangles with about 384 rows, where rows that pass are collected, and with up to 64 rows each."""
+    t = _triangles(13, 120_003, ext, 256)
+    t[40_000:80_000] = _triangles(14, 40_000, (2, 1.2, 1.2), 256)  # warps with few rows
+    _check(rsqrt, t, 256, morton)
+
+
 def test_grid_aligned_triangles(rsqrt):
     """Vertices on voxel corners: plane offsets that are exactly zero, and degenerate triangles."""
     rng = np.random.default_rng(11)
