@@ -723,7 +723,8 @@ def main():
     tbytes = 36 * T
     table_bytes = W * 4
     alg = {"surf_classify": tbytes + table_bytes, "solid_classify": tbytes, "surf_rows": 0, "solid_cols": 0,
-           "solid_resolve": 2 * table_bytes, "solid_morton": 2 * table_bytes, "solid_zero": table_bytes}
+           "solid_resolve": 2 * table_bytes, "solid_morton_cols": 2 * table_bytes, "solid_morton_small": 2 * table_bytes,
+           "solid_zero": table_bytes}
     per_launch_ms = kernel_ms[dom] / max(1, launches[dom])
     achieved = alg.get(dom, 0) / (per_launch_ms / 1e3) / 1e9
     peak, peak_kind = peaks()

@@ -296,9 +296,10 @@ class HostPipeline:
     """Round trips back to back: ``len(slots)`` host plans, each over its own device buffers and
     host tables (``slots[i]`` is slot i's list of HostJob), launched on their own streams in turn,
     so that one round trip's upload and kernels run while the previous one's tables are still
-    going down; a round trip's upload follows the previous one's (cvx_plan_wait_uploads).  ``submit()`` launches the next slot and returns its index; that slot's host tables
-    are complete once ``wait(slot)`` returns.  A slot's next launch rewrites its host tables, so
-    read them before the rotation comes back to it (after ``len(slots)`` more submits)."""
+    going down; a round trip's upload follows the previous one's (cvx_plan_wait_uploads).
+    ``submit()`` launches the next slot and returns its index; that slot's host tables are complete
+    once ``wait(slot)`` returns.  A slot's next launch rewrites its host tables, so read them before
+    the rotation comes back to it (after ``len(slots)`` more submits)."""
 
     def __init__(self, slots: Sequence[Sequence[HostJob]], n_chunks: int = 0):
         import torch

@@ -44,10 +44,10 @@ __device__ __forceinline__ void row_place(const float4& box, uint32_t r, int& y,
 // rows that passed at a time: the 512^3 meshes of a 256-mesh mix 546 -> 507 us, its 256^3 meshes 356 ->
 // 343.  With few rows most pass: the icosphere at 512^3 (125 rows a warp) takes 77 us that way, and 74 with
 // one loop for both.
-// Bound by instructions (82% of issue slots busy on the icosphere at 512^3, 50 per triangle).  There
+// Bound by instructions (82% of issue slots busy on the icosphere at 512^3, 45 per triangle).  There
 // 71 us; 90 us with the rows listed in shared memory and dealt over the CTA behind three barriers, the
 // tests combined with short-circuit branches (15% of all instructions) and the edge sums added up
-// before they are compared.  Nine CTAs per SM at 54 registers; ten at 48 are 1% slower.
+// before they are compared.  Nine CTAs per SM at 56 registers; ten at 48 are 1% slower.
 // Triangles with longer rows, or more, cost less in surf_rows, which shares one setup over a warp: with
 // up to 256 rows of any length kept here, the soup of 300,000 at 300^3 took 148 + 642 us in the two
 // kernels, 44 + 701 with this rule.  A warp keeps all such triangles, also in a launch of few CTAs:
