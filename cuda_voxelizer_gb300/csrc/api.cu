@@ -325,6 +325,8 @@ struct Group {
 	uint64_t mwords = 0, mwarps = 0;
 	uint32_t bricks = 0;  // 64^3 bricks of the group's JOB_BRICKS jobs
 	bool dense = false;   // whether one is JOB_DENSE
+	uint64_t coarse_tri = 0;   // triangles, and voxel columns of the grids' faces, of the jobs with kCoarseFaces
+	double coarse_faces = 0.0; // or more of these per triangle
 };
 
 // Voxel columns of the grid's faces per triangle: how much larger than a voxel a mesh's triangles are.
@@ -332,6 +334,10 @@ double faces_per_triangle(const JobDesc& j) {
 	const double x = j.grid[0], y = j.grid[1], z = j.grid[2];
 	return j.n_tri ? (x * y + y * z + z * x) / (double)j.n_tri : 0.0;
 }
+
+// On a closed mesh with 4 or more, an edge spans 3 voxels or more on average and surf_rows gets a good part
+// of the triangles.
+constexpr double kCoarseFaces = 4.0;
 
 // Jobs in the order of falling faces_per_triangle: the CTAs of meshes with the largest triangles have the
 // most rows and columns to walk, and the last ones of a launch are its tail (a tenth of the classify
@@ -344,8 +350,15 @@ void finish_group(Group& g, bool solid) {
 	uint64_t mw = 0, mc = 0;
 	g.tris = 0;
 	g.dense = false;
+	g.coarse_tri = 0;
+	g.coarse_faces = 0.0;
 	for (JobDesc& j : g.jobs) {
 		g.dense |= (j.flags & JOB_DENSE) != 0;
+		const double f = faces_per_triangle(j);
+		if (f >= kCoarseFaces) {
+			g.coarse_tri += j.n_tri;
+			g.coarse_faces += f * (double)j.n_tri;
+		}
 		j.tile_begin = tile;
 		tile += tiles_of(j.n_tri);
 		g.tris += j.n_tri;
@@ -443,6 +456,8 @@ struct Runner {
 		if (g.bricks > bricks) return fail(CVX_ERR_INVALID_VALUE, "brick scratch too small");
 		L.n_bricks = g.bricks;
 		L.any_dense = g.dense;
+		L.coarse_tri = (uint32_t)g.coarse_tri;
+		L.coarse_faces = (uint32_t)std::min(g.coarse_faces, 4e9);
 		bind_scratch(L, rec, cap, bricks, dev.tune, block);
 		if (alternate) {  // an earlier sequence of this call may have left an error there: keep it
 			const RecLayout l = rec_layout(0, 0);
@@ -904,6 +919,8 @@ static cudaError_t capture_group(const Group& g, bool solid, bool resolve, bool 
 	L.n_mwarps = g.mwarps;
 	L.n_bricks = g.bricks;
 	L.any_dense = g.dense;
+	L.coarse_tri = (uint32_t)g.coarse_tri;
+	L.coarse_faces = (uint32_t)std::min(g.coarse_faces, 4e9);
 	bind_scratch(L, static_cast<char*>(rec), cap, bricks, dev.tune);
 	if (g.jobs.size() == 1)
 		L.single = g.jobs[0];

@@ -177,8 +177,9 @@ constexpr size_t kTicketBytes = kTicketQueues * kTicketStride * sizeof(unsigned 
 struct SpreadTickets {
 	unsigned long long next, end;   // claimed positions of queue q not yet taken
 	uint32_t q, K, warp0, n_warps;  // warp0: the warp's own queue
-	__device__ SpreadTickets(uint64_t total, uint32_t warp, uint32_t n_warps_) : n_warps(n_warps_) {
-		const uint64_t per = total / ((uint64_t)n_warps * 8u);
+	// A warp claims about `turns` times.
+	__device__ SpreadTickets(uint64_t total, uint32_t warp, uint32_t n_warps_, uint32_t turns) : n_warps(n_warps_) {
+		const uint64_t per = total / ((uint64_t)n_warps * turns);
 		K = (uint32_t)(per < 1 ? 1 : (per > 16 ? 16 : per));
 		warp0 = q = warp % kTicketQueues;
 		next = (unsigned long long)(warp / kTicketQueues) * K;
@@ -187,6 +188,17 @@ struct SpreadTickets {
 	// Positions of queue i that belong to warps by their number.
 	__device__ __forceinline__ unsigned long long own(uint32_t i) const {
 		return (unsigned long long)((n_warps + kTicketQueues - 1u - i) / kTicketQueues) * K;
+	}
+	// The next tickets of this warp, first, first + kTicketQueues, ...: `count` of them, at most `most` (the same
+	// in every lane); false once every ticket is claimed.
+	__device__ __forceinline__ bool claim(unsigned long long* ctr, uint64_t total, uint32_t lane, uint32_t most,
+	                                      unsigned long long& first, uint32_t& count) {
+		if (!take(ctr, total, lane, first)) return false;
+		const unsigned long long left = (total - first + kTicketQueues - 1u) / kTicketQueues;  // of the queue, from `first` on
+		const unsigned long long n = end - next + 1u < left ? end - next + 1u : left;
+		count = (uint32_t)(n < most ? n : most);
+		next += count - 1u;
+		return true;
 	}
 	// Next ticket of this warp (the same in every lane); false once every ticket is claimed.
 	__device__ __forceinline__ bool take(unsigned long long* ctr, uint64_t total, uint32_t lane,
@@ -255,6 +267,8 @@ struct LaunchDesc {
 	uint64_t n_mwarps;     // warps of solid_morton_cols: solid Morton jobs with g >= 32
 	uint32_t n_bricks;     // 32^3 bricks of the launch's JOB_BRICKS jobs
 	uint32_t any_dense;    // whether a job of the launch is JOB_DENSE
+	uint32_t coarse_tri;   // triangles, and voxel columns of the grid's faces (saturating), of its jobs that
+	uint32_t coarse_faces; // surf_rows gets many triangles of
 	Scratch scr;
 };
 

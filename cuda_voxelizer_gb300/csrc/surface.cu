@@ -223,16 +223,30 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 // Then the item's rows, 32 at a time, one per lane: the row's slice is found by counting the slices that
 // start at or before it, its bounds on x are read from both tables, the plane test narrows them to
 // the row's exact interval, and the interval is ORed into the table.
+// kGrouped: a warp claims up to kRowsGroup items and sets their triangles up at once, one per lane, in shared
+// memory: the setup, a third of the instructions of an item of 100 rows, is paid once per group, and the
+// loads it waits for come together.  An item alone costs 1 - 2 us more that way, so launches whose warps
+// would claim one at a time do without.  Grouped / not: the 512^3 surface meshes of a 256-mesh mix 252 /
+// 300 us, its 256^3 ones 83 / 95, icosphere 6 at 1000^3 68 / 80, 7 at 1000^3 39 / 45; icosphere 5 at 600^3
+// (20,480 triangles) 35 / 33, 4 at 512^3 25 / 24.
 // Bound by the L2's scattered atomics on large tables (issue slots 53% busy), by instructions and, with
 // few items, by the latency of one item elsewhere.  The soup of 2 M triangles at 1024^3: 26.9 ms for
 // 3.36 G word updates (125 G/s); 39.8 ms with all eight x-dependent tests evaluated per row (41 G warp
-// instructions).  The soup of 300,000 at 300^3 390 us / 697 us.  Six CTAs per SM at 80 registers; five
+// instructions).  The soup of 300,000 at 300^3 384 us / 697 us.  Six CTAs per SM at 80 registers; five
 // are 2% faster on the first soup and 3% slower on the second, seven spill.  Reading a word before the
 // atomic, to skip it where its bits are set, cost as many L2 requests as it saved (27.4 - 28.2 ms, and
 // 30% to 90% more where the table fits the L2), and walking the items twice or four times, each time for
 // a half or quarter of the table that stays in the L2, was 2% to 7% slower.
 constexpr uint32_t kRowsCtaThreads = 128;
 constexpr int kRowsWindow = 128;
+
+constexpr uint32_t kRowsGroup = 8;  // items that a warp of the grouped kernel sets up at once
+
+struct __align__(16) RowsTri {
+	SurfTri S;             // bz0: the item's first slice
+	uint32_t job, slices;
+};
+static_assert(sizeof(RowsTri) == 160, "RowsTri is ten 16-byte vectors");
 
 struct RowsWarp {
 	float4 xy[kRowsWindow];  // per y of the window: bounds of x from the XY tests, ny * py, its part of the row's place
@@ -285,13 +299,15 @@ __device__ __forceinline__ void write_morton_warp(uint32_t* table, uint32_t plac
 		write_morton_group(table, spread3_narrow((uint32_t)(k << 2)) | place, k, xl, xh);
 }
 
-template <class P>
+template <class P, bool kGrouped>
 __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_constant__ LaunchDesc L) {
 	static_assert(P::plane == 2 && P::edge_xy == 1 && P::edge_yz == 1 && P::edge_zx == 2,
 	              "the one-test bounds follow the pinned fused-multiply-add pattern");
 	__shared__ RowsWarp s_warp[kRowsCtaThreads / 32];
 	const uint32_t lane = threadIdx.x & 31u;
 	RowsWarp& W = s_warp[threadIdx.x >> 5];
+	__shared__ RowsTri s_group[kGrouped ? kRowsCtaThreads / 32 : 1][kGrouped ? kRowsGroup : 1];
+	RowsTri* group = s_group[kGrouped ? threadIdx.x >> 5 : 0];
 	Counters* C = L.scr.ctr;
 	clear_next_counters(L);
 	// One thread per CTA reads the queue counters (thousands of warps reading one line would
@@ -311,128 +327,184 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 	// Warps beyond the number of queued items have nothing to claim (all of them when only small
 	// triangles were queued).
 	if ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) >= total) return;
-	SpreadTickets wt(total, blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), gridDim.x * (blockDim.x >> 5));
+	// Where few items are parts of big triangles the items are of like size, and longer claims set up more
+	// triangles together (icosphere 6 at 1000^3 68 us, 86 with eight turns); the others differ more (the
+	// soup of 30,000 at 600^3 152 us, 191 with two turns).
+	const uint32_t turns = kGrouped && 4 * n_big_items < total ? 2u : 8u;
+	SpreadTickets wt(total, blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), gridDim.x * (blockDim.x >> 5), turns);
 	for (;;) {
-		unsigned long long tk = 0;
-		if (!wt.take(L.scr.tickets, total, lane, tk)) break;
-		uint32_t job, tri, chunk, slices;
-		if (!queue_item(L, tk, n_big, n_big_items, lane, job, tri, chunk, slices)) continue;
-		const JobDesc& J = job_at(L, job);
-		const float unit[3] = {J.unit[0], J.unit[1], J.unit[2]};
-		const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
-		const bool morton = (J.flags & JOB_MORTON) != 0;
-		const bool narrow = (J.flags & JOB_NARROW) != 0;
-		uint32_t* table = J.table;
-		float tv = lane < 9 ? J.tris[(uint64_t)tri * 9 + lane] : 0.0f;
-		float t[9];
-#pragma unroll
-		for (int k = 0; k < 9; k++) t[k] = __shfl_sync(FULL, tv, k);
 		SurfTri S;
-		surf_setup<P>(t, J.bmin, unit, J.inv_unit, grid, S);
-		const bool product = plane_underflows(S);
-		float lo, hi;
-		plane_bounds(S, lo, hi);
-		const float plane_m = fmaxf(fabsf(lo), fabsf(hi)), plane_inv = __fdividef(-1.0f, S.nx * unit[0]);
-		const float bx0 = (float)S.bx0, bx1 = (float)S.bx1;
-
-		// this lane's z-slice
-		const int z0 = S.bz0 + (int)(chunk * slices), z = z0 + (int)lane;
-		float fy0 = (float)S.by0, fy1 = (float)S.by1, zx0 = bx0, zx1 = bx1, kz;
-		{
-			const float pz = __fmul_rn(__int2float_rn(z), unit[2]);
-			kz = __fmul_rn(S.nz, pz);
-			const float b0 = fy0, b1 = fy1;
+		uint32_t job = 0, tri = 0, chunk = 0, slices = kZch;  // (grouped: of lane i, item i's at first)
+		uint32_t items = 1u;
+		unsigned long long first;
+		float t[9];
+		if constexpr (kGrouped) {
+			uint32_t count;
+			if (!wt.claim(L.scr.tickets, total, lane, kRowsGroup, first, count)) break;
+			bool found = false;
+			for (uint32_t i = 0; i < count && first + i * kTicketQueues < n_big_items; i++) {
+				uint32_t a, b, c, e;
+				const bool ok = queue_item(L, first + i * kTicketQueues, n_big, n_big_items, lane, a, b, c, e);
+				if (lane == i) {
+					found = ok;
+					job = a;
+					tri = b;
+					chunk = c;
+					slices = e;
+				}
+			}
+			const unsigned long long mine = first + lane * kTicketQueues;
+			if (lane < count && mine >= n_big_items) {
+				const MidRec m = L.scr.mid[mine - n_big_items];
+				job = m.job;
+				tri = m.tri;
+				found = job < L.n_jobs && tri < job_at(L, job).n_tri;
+			}
+			if (found) {
+				const float* v = job_at(L, job).tris + (uint64_t)tri * 9;
 #pragma unroll
-			for (int i = 0; i < 3; i++) {
-				clip_test(S.eyz[i][0], __fmul_rn(S.eyz[i][1], pz), S.dyz[i], unit[1], b0, b1, fy0, fy1);
-				clip_test(S.ezx[i][1], __fmul_rn(S.ezx[i][0], pz), S.dzx[i], unit[0], bx0, bx1, zx0, zx1);
+				for (int k = 0; k < 9; k++) t[k] = v[k];
+				const JobDesc& J = job_at(L, job);
+				const float unit[3] = {J.unit[0], J.unit[1], J.unit[2]};
+				const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
+				RowsTri g;
+				surf_setup<P>(t, J.bmin, unit, J.inv_unit, grid, g.S);
+				g.S.bz0 += (int)(chunk * slices);
+				g.job = job;
+				g.slices = slices;
+				group[lane] = g;
 			}
-		}
-		const bool rows = lane < slices && z <= S.bz1 && fy0 <= fy1 && zx0 <= zx1;
-		const int ya = rows ? (int)fy0 : 0x7FFFFFFF, yb = rows ? (int)fy1 : -1;
-		const int y_begin = __reduce_min_sync(FULL, ya), y_last = __reduce_max_sync(FULL, yb);
-		for (int yw = y_begin; yw <= y_last; yw += kRowsWindow) {
-			const int yw1 = min(yw + kRowsWindow - 1, y_last);
-			for (int y = yw + (int)lane; y <= yw1; y += 32) {
-				const float py = __fmul_rn(__int2float_rn(y), unit[1]);
-				float x0 = bx0, x1 = bx1;
-#pragma unroll
-				for (int i = 0; i < 3; i++)
-					clip_test(S.exy[i][0], __fmul_rn(S.exy[i][1], py), S.dxy[i], unit[0], bx0, bx1, x0, x1);
-				W.xy[y - yw] = make_float4(x0, x1, __fmul_rn(S.ny, py), __uint_as_float(y_part(grid, morton, narrow, y)));
-			}
-			const int first = max(ya, yw);
-			const uint32_t cnt = rows ? (uint32_t)max(min(yb, yw1) - first + 1, 0) : 0u;
-			uint32_t incl = cnt;
-#pragma unroll
-			for (int d = 1; d < 32; d <<= 1) {
-				const uint32_t v = __shfl_up_sync(FULL, incl, d);
-				if (lane >= (uint32_t)d) incl += v;
-			}
-			const uint32_t R = __shfl_sync(FULL, incl, 31), start = incl - cnt;
-			const uint32_t slot = __popc(__ballot_sync(FULL, cnt != 0u) & ((1u << lane) - 1u));
-			if (cnt) {
-				W.slice[slot] = make_float4(__int_as_float((int)start - first), __uint_as_float(z_part(grid, morton, narrow, z)),
-				                            zx0, zx1);
-				W.kz[slot] = kz;
-			}
+			items = __ballot_sync(FULL, found);
 			__syncwarp();
-			uint32_t begun = 0;  // slices that start before this step's rows
-			for (uint32_t base = 0; base < R; base += 32) {
-				const uint32_t at = start - base;
-				const uint32_t starts = __reduce_or_sync(FULL, cnt && at < 32u ? 1u << at : 0u);
-				const uint32_t rec = begun + __popc(starts & (0xFFFFFFFFu >> (31u - lane))) - 1u;
-				begun += __popc(starts);
-				const uint32_t k = base + lane;
-				uint32_t yp = 0, zp = 0;  // the row's place
-				int xl = 0, xh = -1;
-				if (k < R) {
-					const float4 q = W.slice[rec];
-					const int y = (int)k - __float_as_int(q.x);
-					const float4 e = W.xy[y - yw];
-					yp = __float_as_uint(e.w);
-					zp = __float_as_uint(q.y);
-					float x0 = fmaxf(q.z, e.x), x1 = fminf(q.w, e.y);
-					if (!product) {
-						clip_plane(S.nx, e.z, W.kz[rec], lo, hi, plane_m, plane_inv, unit[0], bx0, bx1, x0, x1);
-						if (x0 <= x1) {  // integers of [0, 2^22]: their bits after adding 2^23
-							xl = __float_as_int(__fadd_rn(x0, 8388608.0f)) & 0x7FFFFF;
-							xh = __float_as_int(__fadd_rn(x1, 8388608.0f)) & 0x7FFFFF;
+		} else {
+			if (!wt.take(L.scr.tickets, total, lane, first)) break;
+			if (!queue_item(L, first, n_big, n_big_items, lane, job, tri, chunk, slices)) continue;
+		}
+		for (; items; items &= items - 1u) {
+			if constexpr (kGrouped) {
+				const RowsTri g = group[__ffs(items) - 1];
+				S = g.S;
+				job = g.job;
+				slices = g.slices;
+			}
+			const JobDesc& J = job_at(L, job);
+			const float unit[3] = {J.unit[0], J.unit[1], J.unit[2]};
+			const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
+			const bool morton = (J.flags & JOB_MORTON) != 0;
+			const bool narrow = (J.flags & JOB_NARROW) != 0;
+			uint32_t* table = J.table;
+			if constexpr (!kGrouped) {
+				float tv = lane < 9 ? J.tris[(uint64_t)tri * 9 + lane] : 0.0f;
+#pragma unroll
+				for (int k = 0; k < 9; k++) t[k] = __shfl_sync(FULL, tv, k);
+				surf_setup<P>(t, J.bmin, unit, J.inv_unit, grid, S);
+			}
+			const bool product = plane_underflows(S);
+			float lo, hi;
+			plane_bounds(S, lo, hi);
+			const float plane_m = fmaxf(fabsf(lo), fabsf(hi)), plane_inv = __fdividef(-1.0f, S.nx * unit[0]);
+			const float bx0 = (float)S.bx0, bx1 = (float)S.bx1;
+
+			// this lane's z-slice
+			const int z0 = kGrouped ? S.bz0 : S.bz0 + (int)(chunk * slices), z = z0 + (int)lane;
+			float fy0 = (float)S.by0, fy1 = (float)S.by1, zx0 = bx0, zx1 = bx1, kz;
+			{
+				const float pz = __fmul_rn(__int2float_rn(z), unit[2]);
+				kz = __fmul_rn(S.nz, pz);
+				const float b0 = fy0, b1 = fy1;
+	#pragma unroll
+				for (int i = 0; i < 3; i++) {
+					clip_test(S.eyz[i][0], __fmul_rn(S.eyz[i][1], pz), S.dyz[i], unit[1], b0, b1, fy0, fy1);
+					clip_test(S.ezx[i][1], __fmul_rn(S.ezx[i][0], pz), S.dzx[i], unit[0], bx0, bx1, zx0, zx1);
+				}
+			}
+			const bool rows = lane < slices && z <= S.bz1 && fy0 <= fy1 && zx0 <= zx1;
+			const int ya = rows ? (int)fy0 : 0x7FFFFFFF, yb = rows ? (int)fy1 : -1;
+			const int y_begin = __reduce_min_sync(FULL, ya), y_last = __reduce_max_sync(FULL, yb);
+			for (int yw = y_begin; yw <= y_last; yw += kRowsWindow) {
+				const int yw1 = min(yw + kRowsWindow - 1, y_last);
+				for (int y = yw + (int)lane; y <= yw1; y += 32) {
+					const float py = __fmul_rn(__int2float_rn(y), unit[1]);
+					float x0 = bx0, x1 = bx1;
+	#pragma unroll
+					for (int i = 0; i < 3; i++)
+						clip_test(S.exy[i][0], __fmul_rn(S.exy[i][1], py), S.dxy[i], unit[0], bx0, bx1, x0, x1);
+					W.xy[y - yw] = make_float4(x0, x1, __fmul_rn(S.ny, py), __uint_as_float(y_part(grid, morton, narrow, y)));
+				}
+				const int first = max(ya, yw);
+				const uint32_t cnt = rows ? (uint32_t)max(min(yb, yw1) - first + 1, 0) : 0u;
+				uint32_t incl = cnt;
+	#pragma unroll
+				for (int d = 1; d < 32; d <<= 1) {
+					const uint32_t v = __shfl_up_sync(FULL, incl, d);
+					if (lane >= (uint32_t)d) incl += v;
+				}
+				const uint32_t R = __shfl_sync(FULL, incl, 31), start = incl - cnt;
+				const uint32_t slot = __popc(__ballot_sync(FULL, cnt != 0u) & ((1u << lane) - 1u));
+				if (cnt) {
+					W.slice[slot] = make_float4(__int_as_float((int)start - first), __uint_as_float(z_part(grid, morton, narrow, z)),
+					                            zx0, zx1);
+					W.kz[slot] = kz;
+				}
+				__syncwarp();
+				uint32_t begun = 0;  // slices that start before this step's rows
+				for (uint32_t base = 0; base < R; base += 32) {
+					const uint32_t at = start - base;
+					const uint32_t starts = __reduce_or_sync(FULL, cnt && at < 32u ? 1u << at : 0u);
+					const uint32_t rec = begun + __popc(starts & (0xFFFFFFFFu >> (31u - lane))) - 1u;
+					begun += __popc(starts);
+					const uint32_t k = base + lane;
+					uint32_t yp = 0, zp = 0;  // the row's place
+					int xl = 0, xh = -1;
+					if (k < R) {
+						const float4 q = W.slice[rec];
+						const int y = (int)k - __float_as_int(q.x);
+						const float4 e = W.xy[y - yw];
+						yp = __float_as_uint(e.w);
+						zp = __float_as_uint(q.y);
+						float x0 = fmaxf(q.z, e.x), x1 = fminf(q.w, e.y);
+						if (!product) {
+							clip_plane(S.nx, e.z, W.kz[rec], lo, hi, plane_m, plane_inv, unit[0], bx0, bx1, x0, x1);
+							if (x0 <= x1) {  // integers of [0, 2^22]: their bits after adding 2^23
+								xl = __float_as_int(__fadd_rn(x0, 8388608.0f)) & 0x7FFFFF;
+								xh = __float_as_int(__fadd_rn(x1, 8388608.0f)) & 0x7FFFFF;
+							}
+						} else {  // a plane offset so small that the test's product may underflow: all tests together
+							int z = z0;
+							for (uint32_t i = 0; i < slices; i++)
+								if (z_part(grid, morton, narrow, z0 + (int)i) == zp) z = z0 + (int)i;
+							RowK K;
+							row_consts<P>(S, __fmul_rn(__int2float_rn(y), unit[1]), __fmul_rn(__int2float_rn(z), unit[2]), K);
+							RowDirs D;
+							row_dirs(S, unit[0], D);
+							if (!row_interval<P>(S, D, K, unit[0], xl, xh)) xh = -1;
 						}
-					} else {  // a plane offset so small that the test's product may underflow: all tests together
-						int z = z0;
-						for (uint32_t i = 0; i < slices; i++)
-							if (z_part(grid, morton, narrow, z0 + (int)i) == zp) z = z0 + (int)i;
-						RowK K;
-						row_consts<P>(S, __fmul_rn(__int2float_rn(y), unit[1]), __fmul_rn(__int2float_rn(z), unit[2]), K);
-						RowDirs D;
-						row_dirs(S, unit[0], D);
-						if (!row_interval<P>(S, D, K, unit[0], xl, xh)) xh = -1;
+					}
+					// Short rows are written by their own lane, long ones by the whole warp.
+					const bool has = xh >= xl;
+					const bool wide = has && (morton ? (xh >> 2) - (xl >> 2) >= 4 : (xh >> 5) - (xl >> 5) >= 2);
+					uint32_t todo = __ballot_sync(FULL, wide);
+					if (narrow && !morton) {
+						if (has && !wide) write_linear(table, yp + zp, (uint32_t)xl, (uint32_t)xh);
+					} else if (narrow) {
+						if (has && !wide) write_morton(table, yp | zp, xl, xh);
+					} else {
+						if (has && !wide) write_row_t<uint64_t>(table, morton, grid, (int)yp, (int)zp, xl, xh);
+					}
+					while (todo) {
+						const int src = __ffs(todo) - 1;
+						todo &= todo - 1u;
+						const uint32_t wy = __shfl_sync(FULL, yp, src), wz = __shfl_sync(FULL, zp, src);
+						const int wl = __shfl_sync(FULL, xl, src), wh = __shfl_sync(FULL, xh, src);
+						if (narrow && !morton) write_linear_warp(table, wy + wz, (uint32_t)wl, (uint32_t)wh, lane);
+						else if (narrow) write_morton_warp(table, wy | wz, wl, wh, lane);
+						else write_row_warp_t<uint64_t>(table, morton, grid, (int)wy, (int)wz, wl, wh, lane);
 					}
 				}
-				// Short rows are written by their own lane, long ones by the whole warp.
-				const bool has = xh >= xl;
-				const bool wide = has && (morton ? (xh >> 2) - (xl >> 2) >= 4 : (xh >> 5) - (xl >> 5) >= 2);
-				uint32_t todo = __ballot_sync(FULL, wide);
-				if (narrow && !morton) {
-					if (has && !wide) write_linear(table, yp + zp, (uint32_t)xl, (uint32_t)xh);
-				} else if (narrow) {
-					if (has && !wide) write_morton(table, yp | zp, xl, xh);
-				} else {
-					if (has && !wide) write_row_t<uint64_t>(table, morton, grid, (int)yp, (int)zp, xl, xh);
-				}
-				while (todo) {
-					const int src = __ffs(todo) - 1;
-					todo &= todo - 1u;
-					const uint32_t wy = __shfl_sync(FULL, yp, src), wz = __shfl_sync(FULL, zp, src);
-					const int wl = __shfl_sync(FULL, xl, src), wh = __shfl_sync(FULL, xh, src);
-					if (narrow && !morton) write_linear_warp(table, wy + wz, (uint32_t)wl, (uint32_t)wh, lane);
-					else if (narrow) write_morton_warp(table, wy | wz, wl, wh, lane);
-					else write_row_warp_t<uint64_t>(table, morton, grid, (int)wy, (int)wz, wl, wh, lane);
-				}
+				__syncwarp();  // the tables are rewritten for the next window or item
 			}
-			__syncwarp();  // the tables are rewritten for the next window or item
 		}
+		if constexpr (kGrouped) __syncwarp();  // and the triangles for the next group
 	}
 }
 
@@ -463,7 +535,11 @@ static cudaError_t launch_surface_t(const LaunchDesc& L, const Tune& tune, int r
 		e = launch_bricks(L, rows_grid, raster_grid, s, prof);
 		if (e != cudaSuccess) return e;
 	}
-	e = launch_k(surf_rows<P>, (unsigned)rows_grid, kRowsCtaThreads, 0, s, L);
+	// Grouped where the warps can expect to claim several items at a time: many triangles in meshes whose
+	// triangles are larger than a few voxels (both sides at surf_rows; icosphere 6 at 500^3, 205 faces a warp,
+	// 20 us grouped and 19 not, at 700^3, 403 a warp, 35 and 37).
+	const bool grouped = L.coarse_tri >= 16 * warps && L.coarse_faces >= 256 * warps;
+	e = launch_k(grouped ? surf_rows<P, true> : surf_rows<P, false>, (unsigned)rows_grid, kRowsCtaThreads, 0, s, L);
 	if (e != cudaSuccess) return e;
 	if (prof) (*prof)("surf_rows", s);
 	return cudaGetLastError();
@@ -476,7 +552,7 @@ cudaError_t launch_surface(const LaunchDesc& L, const Tune& tune, int rows_grid,
 
 int surf_rows_blocks_per_sm() {
 	int n = 0;
-	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, surf_rows<RefFma>, kRowsCtaThreads, 0);
+	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, surf_rows<RefFma, true>, kRowsCtaThreads, 0);
 	return n > 0 ? n : 1;
 }
 

@@ -102,6 +102,24 @@ def test_collected_rows(rsqrt, ext, morton):
     _check(rsqrt, t, 256, morton)
 
 
+@pytest.mark.parametrize("n_large,g", [(1, 640), (31, 640), (3_000, 640), (60_000, 640), (60_000, 200), (61_000, 448)])
+def test_queued_items_in_a_large_launch(rsqrt, n_large, g):
+    """Queues from less than one item per warp to several per claim, of triangles with one item and with more, on
+    both sides of the rule on the grid's faces."""
+    t = _triangles(21, 70_001, (1, 1, 1), g)
+    t[:n_large] = _triangles(22, n_large, (12, 9, 9), g)
+    t[:n_large:7] = _triangles(23, len(t[:n_large:7]), (5, 4, 70), g)
+    _check(rsqrt, t, g, False)
+
+
+@pytest.mark.parametrize("n", [400, 60_000])
+def test_large_queued_items_in_a_large_launch(rsqrt, n):
+    """The same with more items of large triangles than of others."""
+    t = _triangles(24, 60_001, (1, 1, 1), 512)
+    t[:n] = _triangles(25, n, (4, 9, 140), 512)
+    _check(rsqrt, t, 512, True)
+
+
 def test_grid_aligned_triangles(rsqrt):
     """Vertices on voxel corners: plane offsets that are exactly zero, and degenerate triangles."""
     rng = np.random.default_rng(11)
