@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 		const uint64_t rows = (uint64_t)(ey + 1) * (uint64_t)(ez + 1);
 		while (slices > kMinSlices && (uint64_t)(ey + 1) * slices > item_rows) slices >>= 1;
 		n_items = ez / slices + 1u;
-		if (ex < kMaskRowVoxels && rows <= local_rows && !plane_underflows(S)) n_rows = (uint32_t)rows;
+		if (ex < kMaskRowVoxels && rows <= local_rows && !plane_underflows(S.d1, S.d2)) n_rows = (uint32_t)rows;
 	}
 	uint32_t incl = n_rows;
 #pragma unroll
@@ -399,9 +399,9 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 				for (int k = 0; k < 9; k++) t[k] = __shfl_sync(FULL, tv, k);
 				surf_setup<P>(t, J.bmin, unit, J.inv_unit, grid, S);
 			}
-			const bool product = plane_underflows(S);
 			float lo, hi;
 			plane_bounds(S, lo, hi);
+			plane_widen(lo, hi);
 			const float plane_m = fmaxf(fabsf(lo), fabsf(hi)), plane_inv = __fdividef(-1.0f, S.nx * unit[0]);
 			const float bx0 = (float)S.bx0, bx1 = (float)S.bx1;
 
@@ -463,21 +463,10 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 						yp = __float_as_uint(e.w);
 						zp = __float_as_uint(q.y);
 						float x0 = fmaxf(q.z, e.x), x1 = fminf(q.w, e.y);
-						if (!product) {
-							clip_plane(S.nx, e.z, W.kz[rec], lo, hi, plane_m, plane_inv, unit[0], bx0, bx1, x0, x1);
-							if (x0 <= x1) {  // integers of [0, 2^22]: their bits after adding 2^23
-								xl = __float_as_int(__fadd_rn(x0, 8388608.0f)) & 0x7FFFFF;
-								xh = __float_as_int(__fadd_rn(x1, 8388608.0f)) & 0x7FFFFF;
-							}
-						} else {  // a plane offset so small that the test's product may underflow: all tests together
-							int z = z0;
-							for (uint32_t i = 0; i < slices; i++)
-								if (z_part(grid, morton, narrow, z0 + (int)i) == zp) z = z0 + (int)i;
-							RowK K;
-							row_consts<P>(S, __fmul_rn(__int2float_rn(y), unit[1]), __fmul_rn(__int2float_rn(z), unit[2]), K);
-							RowDirs D;
-							row_dirs(S, unit[0], D);
-							if (!row_interval<P>(S, D, K, unit[0], xl, xh)) xh = -1;
+						clip_plane(S.nx, e.z, W.kz[rec], lo, hi, plane_m, plane_inv, unit[0], bx0, bx1, x0, x1);
+						if (x0 <= x1) {  // integers of [0, 2^22]: their bits after adding 2^23
+							xl = __float_as_int(__fadd_rn(x0, 8388608.0f)) & 0x7FFFFF;
+							xh = __float_as_int(__fadd_rn(x1, 8388608.0f)) & 0x7FFFFF;
 						}
 					}
 					// Short rows are written by their own lane, long ones by the whole warp.

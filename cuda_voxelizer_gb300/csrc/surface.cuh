@@ -180,15 +180,36 @@ __device__ __forceinline__ uint32_t fail_bits(const SurfTri& S, const RowK& K, f
 // sums are positive or both negative: iff s > hi = max(-d1, -d2) or s < lo = min(-d1, -d2) -- unless
 // the product underflows.  It cannot when |d1|, |d2| >= 2^-49: for |s| < 2^-50 both sums are at least
 // 2^-50; otherwise all operands are multiples of 2^-73, so each nonzero sum is at least that and the
-// product at least 2^-146.  plane_underflows() marks a triangle with a smaller d1 or d2.  A NaN in d1
-// or d2 makes the product NaN (never a failure): lo and hi are then both NaN.
-__device__ __forceinline__ bool plane_underflows(const SurfTri& S) {
-	return (fabsf(S.d1) < 0x1p-49f) | (fabsf(S.d2) < 0x1p-49f);
-}
+// product at least 2^-146.  With a smaller d1 or d2 -- a triangle in one of the box's first planes
+// along an axis has a zero -- plane_widen() moves the bounds out to the last s whose product is not
+// positive.  A NaN in d1 or d2 makes the product NaN (never a failure): lo and hi are then both NaN.
 __device__ __forceinline__ void plane_bounds(const SurfTri& S, float& lo, float& hi) {
 	const bool nan = (S.d1 != S.d1) | (S.d2 != S.d2);
 	lo = nan ? __int_as_float(0x7FFFFFFF) : fminf(-S.d1, -S.d2);
 	hi = nan ? __int_as_float(0x7FFFFFFF) : fmaxf(-S.d1, -S.d2);
+}
+__device__ __forceinline__ bool plane_underflows(float lo, float hi) {
+	return (fabsf(lo) < 0x1p-49f) | (fabsf(hi) < 0x1p-49f);
+}
+// The largest float s >= hi at which fl(fl(s - lo) * fl(s - hi)) is not positive (lo <= hi, neither a
+// NaN), by a search over the floats in order: above hi both differences, and so the rounded product,
+// grow with s.
+static __device__ __noinline__ float plane_reach(float lo, float hi) {
+	auto flip = [](int i) { return i ^ ((i >> 31) & 0x7FFFFFFF); };  // float bits <-> an int in the floats' order
+	int l = flip(__float_as_int(hi)), r = 0x7F800000;
+	while (l < r) {
+		const int m = l + (int)(((uint32_t)r - (uint32_t)l + 1u) >> 1);
+		const float s = __int_as_float(flip(m));
+		if (__fmul_rn(__fsub_rn(s, lo), __fsub_rn(s, hi)) > 0.0f) r = m - 1; else l = m;
+	}
+	return __int_as_float(flip(l));
+}
+__device__ __forceinline__ void plane_widen(float& lo, float& hi) {
+	if (plane_underflows(lo, hi)) {
+		const float reach = plane_reach(lo, hi);
+		lo = -plane_reach(-hi, -lo);
+		hi = reach;
+	}
 }
 
 // A small triangle's setup (rows of at most kMaskRowVoxels voxels, plane_underflows() false) parked
@@ -379,13 +400,6 @@ __device__ __forceinline__ uint32_t fail_bits_masked(const SurfTri& S, const Row
 	return f & mask;
 }
 
-// Exact pass interval of row (y, z) within the triangle's bbox [S.bx0, S.bx1].
-template <class P>
-__device__ __forceinline__ bool row_interval(const SurfTri& S, const RowDirs& D, const RowK& K, float ux, int& xl,
-                                             int& xh) {
-	return row_interval_in<P>(S, D, K, ux, S.bx0, S.bx1, xl, xh);
-}
-
 // Certified x-interval of a row, without walking.
 //
 // Each x-dependent test i has the form "fails iff g(x) < 0" (or > 0 for the plane's "above" side)
@@ -492,7 +506,7 @@ __device__ __forceinline__ void clip_test(float a, float k, float d, float u, fl
 }
 
 // The plane test of a row, "fails iff s < lo or s > hi" with s(x) = fl(fl(fma(nx, fl(x * u), kpl)) + kpl2)
-// (plane_bounds; not for plane_underflows() triangles), monotone in x with the sign of nx.
+// (plane_bounds and plane_widen), monotone in x with the sign of nx.
 static __device__ __noinline__ float plane_change(float nx, float kpl, float kpl2, float bound, bool below, float u,
                                                   float b0, float b1) {
 	// below: the side s < bound, else s > bound.  That side fails on a prefix of x iff (nx > 0) == below.

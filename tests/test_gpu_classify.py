@@ -182,3 +182,48 @@ def test_dense_and_sparse_jobs_in_one_plan():
     torch.cuda.synchronize()
     for one, job in zip(alone, jobs):
         assert torch.equal(one, job.table)
+
+
+def _check_info(rsqrt, tris, info, morton=False):
+    d = torch.from_numpy(np.ascontiguousarray(tris).reshape(-1)).cuda()
+    table = torch.zeros(cv.table_words(info) + GUARD, dtype=torch.int32, device="cuda")
+    cv.voxelize(info, d, table, morton)
+    cv.device_status()
+    inv = rsqrt(oracle.len2(bytes(info), tris, oracle.gpu_mode(morton)))
+    want = oracle.voxelize(bytes(info), tris, morton, mode=oracle.gpu_mode(morton, inv_len=inv))
+    got = table.cpu().numpy().view(np.uint32)
+    assert not got[len(want):].any()
+    bad = np.nonzero(got[:len(want)] != want)[0]
+    assert bad.size == 0, f"{bad.size} words differ, first {bad[:5]}"
+
+
+def _floor(seed, n, ext, g, height, tilt=0.0):
+    """n random triangles of about ext voxels along x and y in the plane z = height + tilt * x."""
+    t = _triangles(seed, n, (ext, ext, 0.0 if ext < 1 else 1.0), g).reshape(n, 3, 3).astype(np.float64)
+    t[:, :, 2] = height + tilt * t[:, :, 0]
+    return t.reshape(n, 9).astype(np.float32)
+
+
+@pytest.mark.parametrize("height", [0.0, 1e-16])
+@pytest.mark.parametrize("n", [300, 70_001])
+def test_floor_of_a_wide_flat_grid(rsqrt, n, height):
+    """Offsets of the plane test that are zero or tiny, where 32 bits hold a row's place but not that of 16 slices on."""
+    t = _floor(n, n, 2.5, 16384, height)
+    t[:150] = _floor(1, 150, 24, 16384, height)   # fewer rows than an item of 32 slices may have in a small launch
+    t[150:300] = _floor(2, 150, 120, 16384, height)
+    _check_info(rsqrt, t, cv.make_info((0, 0, 0), (16384.0, 16384.0, 4.0), (16384, 16384, 4), n))
+
+
+@pytest.mark.parametrize("unit", [1.0, 2.0 ** -10, 2.0 ** -40])
+@pytest.mark.parametrize("height,tilt", [(0, 0), (1, 0), (1e-16, 0), (1e-39, 0), (0, 1e-17), (0, -1e-17), (0, -1e-30),
+                                         (0, -1e-36), (0, -1e-39)])
+def test_products_of_the_plane_test_that_underflow(rsqrt, unit, height, tilt):
+    """Planes through, or next to, the corner of the box's first voxels: the product of the plane test's two sums
+    underflows where they do not cancel."""
+    n, g = 900, 64
+    t = np.concatenate([_floor(3, 300, 40, g, height, tilt), _floor(4, 600, 3, g, height, tilt)]).reshape(n, 3, 3)
+    t = (t.astype(np.float64) * unit).astype(np.float32)
+    for axis in range(3):
+        a = np.roll(t, axis, 2)
+        a[::2] = a[::2, ::-1]  # both orientations
+        _check_info(rsqrt, a.reshape(n, 9), cv.make_info((0, 0, 0), (g * unit,) * 3, g, n), axis == 1)
