@@ -296,11 +296,13 @@ JobDesc make_job(const cvx_voxinfo& v, const float* tris, uint32_t* table, int m
 	j.tris = tris;
 	j.table = table;
 	j.n_tri = v.n_triangles;
+	j.box_near = 1.0f;
 	for (int i = 0; i < 3; i++) {
 		j.bmin[i] = v.bbox_min[i];
 		j.unit[i] = v.unit[i];
 		volatile float one = 1.0f;
 		j.inv_unit[i] = one / v.unit[i];  // IEEE single division: correctly rounded
+		if (!std::isfinite(j.inv_unit[i])) j.box_near = 0.0f;
 		j.grid[i] = v.gridsize[i];
 	}
 	j.flags = (morton ? JOB_MORTON : 0u) | (solid ? JOB_SOLID : 0u);

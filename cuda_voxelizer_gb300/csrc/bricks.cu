@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kBinThreads) brick_bin(const __grid_constant__
 		const float unit[3] = {J.unit[0], J.unit[1], J.unit[2]};
 		const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
 		SurfTri S;
-		surf_setup<P>(t, J.bmin, unit, J.inv_unit, grid, S);
+		surf_setup<P>(t, J.bmin, unit, J.inv_unit, J.box_near, grid, S);
 		const float v0[3] = {__fsub_rn(t[0], J.bmin[0]), __fsub_rn(t[1], J.bmin[1]), __fsub_rn(t[2], J.bmin[2])};
 		const BrickBox B(S);
 		uint32_t cnt = 0;

@@ -97,6 +97,7 @@ struct JobDesc {
 	uint32_t flags;        // JOB_MORTON | JOB_SOLID | JOB_NARROW | JOB_TABLE_OVERWRITE | ...
 	uint32_t tile_begin;   // first triangle tile of this job in the launch's tile space
 	uint32_t unit_begin;   // solid: first resolve unit of this job in the launch's unit space
+	float box_near;        // surface: 1, or 0 where an inv_unit overflowed and only divisions give a grid box
 	uint64_t mword_begin;  // solid Morton, g < 32: first Morton word in the launch's word space
 	uint64_t mwarp_begin;  // solid Morton, g >= 32: first warp of solid_morton_cols in the launch
 	uint32_t brick_begin;  // JOB_BRICKS: first 32^3 brick of this job in the launch's brick space

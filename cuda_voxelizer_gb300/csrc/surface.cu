@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 	if (valid) {
 		const float bmin[3] = {J.bmin[0], J.bmin[1], J.bmin[2]};
 		const float inv[3] = {J.inv_unit[0], J.inv_unit[1], J.inv_unit[2]};
-		surf_setup<P>(t, bmin, unit, inv, grid, S);
+		surf_setup<P>(t, bmin, unit, inv, J.box_near, grid, S);
 		const uint32_t ex = (uint32_t)(S.bx1 - S.bx0), ey = (uint32_t)(S.by1 - S.by0), ez = (uint32_t)(S.bz1 - S.bz0);
 		const uint64_t rows = (uint64_t)(ey + 1) * (uint64_t)(ez + 1);
 		while (slices > kMinSlices && (uint64_t)(ey + 1) * slices > item_rows) slices >>= 1;
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 				const float unit[3] = {J.unit[0], J.unit[1], J.unit[2]};
 				const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
 				RowsTri g;
-				surf_setup<P>(t, J.bmin, unit, J.inv_unit, grid, g.S);
+				surf_setup<P>(t, J.bmin, unit, J.inv_unit, J.box_near, grid, g.S);
 				g.S.bz0 += (int)(chunk * slices);
 				g.job = job;
 				g.slices = slices;
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 				float tv = lane < 9 ? J.tris[(uint64_t)tri * 9 + lane] : 0.0f;
 #pragma unroll
 				for (int k = 0; k < 9; k++) t[k] = __shfl_sync(FULL, tv, k);
-				surf_setup<P>(t, J.bmin, unit, J.inv_unit, grid, S);
+				surf_setup<P>(t, J.bmin, unit, J.inv_unit, J.box_near, grid, S);
 			}
 			float lo, hi;
 			plane_bounds(S, lo, hi);

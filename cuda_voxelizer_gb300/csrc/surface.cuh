@@ -54,7 +54,7 @@ __device__ __forceinline__ void bbox_axis(float lo, float hi, float inv, uint32_
 // Triangle setup, src/voxelize.cu:71-133.  `t` holds v0.xyz, v1.xyz, v2.xyz in world space.
 template <class P>
 __device__ __forceinline__ void surf_setup(const float* t, const float* bmin, const float* unit, const float* inv,
-                                           const uint32_t* grid, SurfTri& S) {
+                                           float box_near, const uint32_t* grid, SurfTri& S) {
 	const float v0x = __fsub_rn(t[0], bmin[0]), v0y = __fsub_rn(t[1], bmin[1]), v0z = __fsub_rn(t[2], bmin[2]);
 	const float v1x = __fsub_rn(t[3], bmin[0]), v1y = __fsub_rn(t[4], bmin[1]), v1z = __fsub_rn(t[5], bmin[2]);
 	const float v2x = __fsub_rn(t[6], bmin[0]), v2y = __fsub_rn(t[7], bmin[1]), v2z = __fsub_rn(t[8], bmin[2]);
@@ -71,8 +71,9 @@ __device__ __forceinline__ void surf_setup(const float* t, const float* bmin, co
 	S.nz = __fmul_rn(cz, rlen);
 
 	// grid bbox: clamp(int(min(v) / unit), 0, g - 1)  (:83-87).  Reciprocal quotients decide it unless
-	// one is within their error of an integer; then all six divide.
-	float near = 1.0f;
+	// one is within their error of an integer, or box_near is 0 (a reciprocal overflowed); then all six
+	// divide.
+	float near = box_near;
 	bbox_axis(fminf(v0x, fminf(v1x, v2x)), fmaxf(v0x, fmaxf(v1x, v2x)), inv[0], grid[0], S.bx0, S.bx1, near);
 	bbox_axis(fminf(v0y, fminf(v1y, v2y)), fmaxf(v0y, fmaxf(v1y, v2y)), inv[1], grid[1], S.by0, S.by1, near);
 	bbox_axis(fminf(v0z, fminf(v1z, v2z)), fmaxf(v0z, fmaxf(v1z, v2z)), inv[2], grid[2], S.bz0, S.bz1, near);

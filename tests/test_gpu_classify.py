@@ -227,3 +227,12 @@ def test_products_of_the_plane_test_that_underflow(rsqrt, unit, height, tilt):
         a = np.roll(t, axis, 2)
         a[::2] = a[::2, ::-1]  # both orientations
         _check_info(rsqrt, a.reshape(n, 9), cv.make_info((0, 0, 0), (g * unit,) * 3, g, n), axis == 1)
+
+
+@pytest.mark.parametrize("unit", [2.0 ** -128, 2.0 ** -129, 1e-37 / 64, 2.0 ** -140])
+def test_unit_whose_reciprocal_overflows(rsqrt, unit):
+    """Boxes so small that 1 / unit is not finite: the grid boxes come from the divisions."""
+    g, n = 64, 400
+    t = np.concatenate([_triangles(31, 300, (3, 3, 3), g), _triangles(32, 100, (20, 20, 20), g)])
+    t = (t.astype(np.float64) * unit).astype(np.float32)
+    _check_info(rsqrt, t, cv.make_info((0, 0, 0), (g * unit,) * 3, g, n))
