@@ -105,26 +105,33 @@ const Prof* prof() { return g_profile ? &g_prof : nullptr; }
 
 // ---- scratch ------------------------------------------------------------------------------------
 
-// Record area of a launch sequence: kCounterBlocks blocks of ticket counters and counters, per-brick pair
-// counts (for up to `bricks` bricks per launch; none without JOB_BRICKS jobs), the queues (cap
-// triangles), the other brick arrays, then `n_jobs` uploaded job descriptors.  [0, big) must be zero
-// before the first launch sequence on the area (the counts are zero again after every sequence).
+// Record area of a launch sequence: two blocks of ticket counters and counters, the error words, a third
+// block, per-brick pair counts (for up to `bricks` bricks per launch; none without JOB_BRICKS jobs), the
+// queues (cap triangles), the other brick arrays, then `n_jobs` uploaded job descriptors.  [0, big)
+// must be zero before the first launch sequence on the area (the counts are zero again after every
+// sequence).
 // Pairs: about 27 per queued triangle on the 1024^3 stress soup; triangles whose pairs do not fit are
 // rasterized by surf_rows instead.
 // The per-stream areas use blocks 0 and 1 in turn, each cleared by the sequence before the one that uses
 // it, and block 2 for calls under capture (a graph may be launched any number of times) and for brick
 // jobs; there, and in the other areas, which use block 0, the host clears the counters.
-constexpr uint32_t kCounterBlocks = 3, kCaptureBlock = 2;
+// An error word belongs to a call, whatever its sequences: words 0 and 1 to the direct calls in turn, each
+// of which clears the other two words; word 2 to calls under capture and with brick jobs, which begin by
+// clearing all.  So the words hold what the last call that ran has set, and nothing else.
+constexpr uint32_t kCaptureBlock = 2, kCaptureError = 2;
 struct RecLayout {
-	size_t tickets, ctr, block, bcnt, big, mid, bq, tri, boff, bcur, ubeg, psorted, jobs, end;
+	size_t tickets, ctr, block, errors, capture, bcnt, big, mid, bq, tri, boff, bcur, ubeg, psorted, jobs, end;
 	uint64_t pair_cap;
+	size_t block_at(uint32_t b) const { return b == kCaptureBlock ? capture : b * block; }
 };
 RecLayout rec_layout(uint64_t cap, uint64_t n_jobs, uint32_t bricks = 0) {
 	RecLayout l;
 	l.tickets = 0;
 	l.ctr = align_up(kTicketBytes);
 	l.block = align_up(l.ctr + sizeof(Counters));
-	l.bcnt = kCounterBlocks * l.block;
+	l.errors = kCaptureBlock * l.block;
+	l.capture = align_up(l.errors + kErrorWords * sizeof(unsigned));
+	l.bcnt = l.capture + l.block;
 	l.big = align_up(l.bcnt + (uint64_t)bricks * 4);
 	l.mid = align_up(l.big + cap * sizeof(BigRec));
 	l.bq = align_up(l.mid + cap * sizeof(MidRec));
@@ -142,10 +149,13 @@ RecLayout rec_layout(uint64_t cap, uint64_t n_jobs, uint32_t bricks = 0) {
 
 // Point a launch descriptor's scratch at a record area laid out by rec_layout(cap, *, bricks); the
 // tuning may use less of the pair area (brick_pairs per triangle; 0 sends every triangle to surf_rows).
-void bind_scratch(LaunchDesc& L, char* rec, uint64_t cap, uint32_t bricks, const Tune& tune, uint32_t block = 0) {
+void bind_scratch(LaunchDesc& L, char* rec, uint64_t cap, uint32_t bricks, const Tune& tune, uint32_t block = 0,
+                  uint32_t error = 0) {
 	const RecLayout l = rec_layout(cap, 0, bricks);
-	L.scr.tickets = reinterpret_cast<unsigned long long*>(rec + block * l.block + l.tickets);
-	L.scr.ctr = reinterpret_cast<Counters*>(rec + block * l.block + l.ctr);
+	L.scr.tickets = reinterpret_cast<unsigned long long*>(rec + l.block_at(block) + l.tickets);
+	L.scr.ctr = reinterpret_cast<Counters*>(rec + l.block_at(block) + l.ctr);
+	L.scr.errors = reinterpret_cast<unsigned*>(rec + l.errors);
+	L.scr.error = L.scr.errors + error;
 	L.scr.big = reinterpret_cast<BigRec*>(rec + l.big);
 	L.scr.mid = reinterpret_cast<MidRec*>(rec + l.mid);
 	L.scr.cap = (uint32_t)cap;
@@ -161,14 +171,15 @@ void bind_scratch(LaunchDesc& L, char* rec, uint64_t cap, uint32_t bricks, const
 	L.scr.pair_sorted = reinterpret_cast<uint32_t*>(rec + l.psorted);
 }
 
-// What is cleared of a block between the launch sequences of a call: everything up to the error word.
-size_t reset_bytes() { return rec_layout(0, 0).ctr + kCountersResetBytes; }
+// What is cleared of a block between the launch sequences of a call.
+size_t reset_bytes() { return rec_layout(0, 0).ctr + sizeof(Counters); }
 
 struct StreamScratch {
 	void* rec = nullptr;
 	size_t rec_bytes = 0;
-	uint32_t block = 0;         // counter block of the next call
-	bool ready = false;         // it is zero: the last call on the stream went through
+	uint32_t block = 0;         // counter block of the next direct call
+	uint32_t error = 0;         // and its error word
+	bool ready = false;         // they are zero: the last direct call on the stream went through
 	uint32_t* flips = nullptr;  // zero between launch sequences
 	size_t flip_bytes = 0;
 	JobDesc* staging = nullptr; // pinned host copy of uploaded job arrays
@@ -207,6 +218,8 @@ cvx_status ensure_scratch(int dev, cudaStream_t s, size_t rec_bytes, size_t flip
 			return fail(CVX_ERR_OUT_OF_MEMORY, "cannot allocate %zu bytes of scratch", b);
 		}
 		w.rec_bytes = b;
+		CVX_CUDA(cudaMemsetAsync(w.rec, 0, rec_layout(0, 0).bcnt, s));  // cvx_device_status reads every error word
+		w.ready = true;
 	}
 	if (grow_flip) {
 		if (w.flips) cudaFree(w.flips);
@@ -445,6 +458,7 @@ struct Runner {
 	bool timed = true;     // per-kernel events for cvx_profile_collect (callers on this thread only)
 	bool fresh = true;     // the counters are zero: the caller cleared the area before run()
 	uint32_t block = 0;    // counter block in use
+	uint32_t error = 0;    // error word of the call
 	bool alternate = false;  // the sequences use blocks 0 and 1 in turn, each clearing the other for the next
 	const Prof* p() const { return timed ? prof() : nullptr; }
 
@@ -460,11 +474,10 @@ struct Runner {
 		L.any_dense = g.dense;
 		L.coarse_tri = (uint32_t)g.coarse_tri;
 		L.coarse_faces = (uint32_t)std::min(g.coarse_faces, 4e9);
-		bind_scratch(L, rec, cap, bricks, dev.tune, block);
-		if (alternate) {  // an earlier sequence of this call may have left an error there: keep it
-			const RecLayout l = rec_layout(0, 0);
-			L.scr.next = reinterpret_cast<uint32_t*>(rec + (block ^ 1u) * l.block);
-			L.scr.next_words = (uint32_t)((reset_bytes() + (fresh ? sizeof(Counters::error) : 0)) / 4);
+		bind_scratch(L, rec, cap, bricks, dev.tune, block, error);
+		if (alternate) {
+			L.scr.next = reinterpret_cast<uint32_t*>(rec + rec_layout(0, 0).block_at(block ^ 1u));
+			L.scr.next_words = (uint32_t)(reset_bytes() / 4);
 		}
 		if (g.jobs.size() == 1) {
 			L.single = g.jobs[0];
@@ -484,7 +497,7 @@ struct Runner {
 
 	// Between two sequences: the first finds the counters cleared.
 	cvx_status reset_counters() {
-		if (!fresh && !alternate) CVX_CUDA(cudaMemsetAsync(rec + block * rec_layout(0, 0).block, 0, reset_bytes(), s));
+		if (!fresh && !alternate) CVX_CUDA(cudaMemsetAsync(rec + rec_layout(0, 0).block_at(block), 0, reset_bytes(), s));
 		fresh = false;
 		return CVX_OK;
 	}
@@ -579,17 +592,19 @@ cvx_status run_internal(std::vector<JobDesc> surf, std::vector<JobDesc> solid, c
 	r.alternate = !bricks && !capturing(s);
 	if (r.alternate) {
 		r.block = w->block;
-		if (!w->ready) CVX_CUDA(cudaMemsetAsync(w->rec, 0, lay.big, s));
+		r.error = w->error;
+		if (!w->ready) CVX_CUDA(cudaMemsetAsync(w->rec, 0, lay.bcnt, s));
 		w->ready = false;  // until the call has gone through
-	} else {
-		r.block = kCaptureBlock;  // the last one, beside the brick counts
-		const size_t at = kCaptureBlock * lay.block;
-		CVX_CUDA(cudaMemsetAsync(static_cast<char*>(w->rec) + at, 0, lay.big - at, s));
+	} else {  // the error words, the last block and the brick counts lie beside each other
+		r.block = kCaptureBlock;
+		r.error = kCaptureError;
+		CVX_CUDA(cudaMemsetAsync(static_cast<char*>(w->rec) + lay.errors, 0, lay.big - lay.errors, s));
 	}
 	st = r.run(surf, solid);
 	if (st != CVX_OK) return st;
 	if (r.alternate) {
 		w->block = r.block;
+		w->error = r.error ^ 1u;
 		w->ready = true;
 	}
 	if (slots) CVX_CUDA(cudaEventRecord(w->staging_done, s));
@@ -839,12 +854,10 @@ cvx_status cvx_device_status(cvx_stream_t stream) {
 		if (it != g_ws.end()) rec = it->second.rec;
 	}
 	if (rec) {
-		const RecLayout l = rec_layout(0, 0);
-		for (uint32_t i = 0; i < kCounterBlocks; i++) {
-			Counters c;
-			CVX_CUDA(cudaMemcpy(&c, static_cast<char*>(rec) + i * l.block + l.ctr, sizeof(c), cudaMemcpyDeviceToHost));
-			if (c.error) return fail(CVX_ERR_DEVICE_CHECK, "device check failed (code %u)", c.error);
-		}
+		unsigned errors[kErrorWords];
+		CVX_CUDA(cudaMemcpy(errors, static_cast<char*>(rec) + rec_layout(0, 0).errors, sizeof(errors), cudaMemcpyDeviceToHost));
+		for (unsigned e : errors)
+			if (e) return fail(CVX_ERR_DEVICE_CHECK, "device check failed (code %u)", e);
 	}
 	// the last cvx_voxelize_solid_noalloc call on this device keeps its counters in the library's
 	// fixed scratch array

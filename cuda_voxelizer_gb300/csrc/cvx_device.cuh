@@ -114,7 +114,7 @@ struct MidRec {            // triangle handled as a single item
 	uint32_t job, tri;
 };
 
-// Device counters; zeroed before every launch sequence.
+// Device counters; zero before every launch sequence.
 // `big` packs (number of BigRec << 40) | (number of big items) so that one 64-bit atomic hands a
 // warp both its record slots and its item range; records are then sorted by item_begin, which
 // the consumer's binary search relies on.  A launch holds fewer than 2^24 triangles (the host
@@ -130,11 +130,8 @@ struct Counters {
 	unsigned int mid;            // number of MidRec
 	unsigned int bq;             // number of triangles in the brick queue
 	unsigned int units;          // raster work units (written by brick_scan)
-	unsigned int error;          // nonzero: a device-side check failed (value says which)
-	unsigned int pad[2];
+	unsigned int pad;
 };
-// Everything before `error` is reset before every launch sequence; `error` persists until read.
-constexpr size_t kCountersResetBytes = offsetof(Counters, error);
 
 // Work tickets of the brick kernels, claimed by a warp K at a time: one atomic on the shared counter
 // per K items instead of per item.  K grows with the items per warp, up to 16, so the tail left when
@@ -240,11 +237,15 @@ struct __align__(16) BrickTri {
 };
 static_assert(sizeof(BrickTri) == 176, "BrickTri is eleven 16-byte vectors");
 
+constexpr uint32_t kErrorWords = 3;
+
 struct Scratch {
 	Counters* ctr;
 	unsigned long long* tickets;  // kTicketBytes: the ticket counters of surf_rows, zero before a launch sequence
 	uint32_t* next;        // the counter block of the next launch sequence: the persistent kernel of this one
 	uint32_t next_words;   // zeroes that many words of it (null: the host clears the counters)
+	unsigned* error;       // the call's error word: nonzero, a device-side check failed (the value says which)
+	unsigned* errors;      // the area's kErrorWords error words; where `next` is set, the others are zeroed with it
 	BigRec* big;
 	MidRec* mid;
 	uint32_t cap;          // capacity of big[], mid[], bq[] and tri[] (>= triangles in the launch)
@@ -416,7 +417,7 @@ __device__ __forceinline__ uint32_t job_search(const LaunchDesc& L, uint64_t idx
 }
 
 __device__ __forceinline__ void set_error(const LaunchDesc& L, unsigned code) {
-	atomicCAS(&L.scr.ctr->error, 0u, code);
+	atomicCAS(L.scr.error, 0u, code);
 }
 
 }  // namespace cvx

@@ -37,7 +37,9 @@ namespace {
 constexpr uint64_t kNoallocMaxVoxels = 1ull << 24;               // flip table: 2 MiB
 constexpr uint64_t kNoallocMaxTriangles = 1ull << 16;            // queue: 65,536 triangles per slice
 constexpr size_t kNoallocFlipBytes = kNoallocMaxVoxels / 8;
-constexpr size_t kNoallocBigOff = 256;                           // counters live in the first 256 bytes
+constexpr size_t kNoallocErrorOff = 192;                         // counters and error word live in the
+constexpr size_t kNoallocBigOff = 256;                           // first 256 bytes
+static_assert(sizeof(Counters) <= kNoallocErrorOff, "the error word follows the counters");
 constexpr size_t kNoallocMidOff = kNoallocBigOff + kNoallocMaxTriangles * sizeof(BigRec);
 constexpr size_t kNoallocFlipOff = kNoallocMidOff + kNoallocMaxTriangles * sizeof(MidRec);
 constexpr size_t kNoallocScratchBytes = kNoallocFlipOff + kNoallocFlipBytes;
@@ -132,13 +134,11 @@ cvx_status noalloc_error(int dev, unsigned* err) {
 		if (current_context_id(&ctx) != CVX_OK || ctx != g_ctx_id[dev]) return CVX_OK;  // none in this context
 		base = g_addr[dev];
 	}
-	Counters c;
-	cudaError_t e = cudaMemcpy(&c, base, sizeof(c), cudaMemcpyDeviceToHost);
+	cudaError_t e = cudaMemcpy(err, static_cast<char*>(base) + kNoallocErrorOff, sizeof(*err), cudaMemcpyDeviceToHost);
 	if (e != cudaSuccess) {
-		set_message(std::string("cudaMemcpy(noalloc counters): ") + cudaGetErrorString(e));
+		set_message(std::string("cudaMemcpy(noalloc error word): ") + cudaGetErrorString(e));
 		return CVX_ERR_CUDA;
 	}
-	*err = c.error;
 	return CVX_OK;
 }
 
@@ -186,7 +186,7 @@ extern "C" cvx_status cvx_voxelize_solid_noalloc(const cvx_voxinfo* info, const 
 	const uint64_t words = (g0 * g1 * g2 + 31) / 32;
 	uint32_t* flips = reinterpret_cast<uint32_t*>(scr + kNoallocFlipOff);
 	if ((st = cuda_status(cudaMemsetAsync(flips, 0, words * 4, s), "cudaMemsetAsync(flips)")) != CVX_OK) return st;
-	if ((st = cuda_status(cudaMemsetAsync(scr, 0, sizeof(Counters), s), "cudaMemsetAsync(counters)")) != CVX_OK)
+	if ((st = cuda_status(cudaMemsetAsync(scr, 0, kNoallocBigOff, s), "cudaMemsetAsync(counters)")) != CVX_OK)
 		return st;
 
 	JobDesc job{};
@@ -207,6 +207,7 @@ extern "C" cvx_status cvx_voxelize_solid_noalloc(const cvx_voxinfo* info, const 
 	LaunchDesc L{};
 	L.n_jobs = 1;
 	L.scr.ctr = reinterpret_cast<Counters*>(scr);
+	L.scr.error = reinterpret_cast<unsigned*>(scr + kNoallocErrorOff);
 	L.scr.big = reinterpret_cast<BigRec*>(scr + kNoallocBigOff);
 	L.scr.mid = reinterpret_cast<MidRec*>(scr + kNoallocMidOff);
 	L.scr.cap = (uint32_t)kNoallocMaxTriangles;
@@ -217,7 +218,7 @@ extern "C" cvx_status cvx_voxelize_solid_noalloc(const cvx_voxinfo* info, const 
 		L.single.tris = d_triangles + off * 9;
 		L.single.n_tri = n;
 		L.n_tiles = (uint32_t)((n + kTile - 1) / kTile);
-		if (off && (st = cuda_status(cudaMemsetAsync(scr, 0, kCountersResetBytes, s), "cudaMemsetAsync(counters)")) != CVX_OK)
+		if (off && (st = cuda_status(cudaMemsetAsync(scr, 0, sizeof(Counters), s), "cudaMemsetAsync(counters)")) != CVX_OK)
 			return st;
 		if ((st = cuda_status(launch_solid(L, tune, cols_grid, s, kSolidToggles, nullptr), "solid toggles")) != CVX_OK)
 			return st;

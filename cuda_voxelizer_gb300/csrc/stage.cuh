@@ -59,10 +59,13 @@ __device__ __forceinline__ bool stage_warp(const LaunchDesc& L, const float* src
 }
 
 // The persistent kernels clear the counters of the next launch sequence (whose kernels follow in the
-// stream), so that it needs no memset: 2 us of a small call.
+// stream), so that it needs no memset: 2 us of a small call.  With them go the error words of other
+// calls: of the one before, and the word that the next one will use.
 __device__ __forceinline__ void clear_next_counters(const LaunchDesc& L) {
-	if (L.scr.next && blockIdx.x + 1 == gridDim.x)
+	if (L.scr.next && blockIdx.x + 1 == gridDim.x) {
 		for (uint32_t i = threadIdx.x; i < L.scr.next_words; i += blockDim.x) L.scr.next[i] = 0u;
+		if (threadIdx.x < kErrorWords && L.scr.errors + threadIdx.x != L.scr.error) L.scr.errors[threadIdx.x] = 0u;
+	}
 }
 
 // The queued item of ticket `tk` of a persistent kernel: big items (n_big records, n_big_items items)
