@@ -436,6 +436,33 @@ Group resolve_group(const std::vector<JobDesc>& jobs) {
 	return g;
 }
 
+// The same in as few groups as it takes for no group to hold two jobs whose tables share words: a resolve
+// reads, XORs and writes the table's words without atomics.
+std::vector<Group> resolve_groups(const std::vector<JobDesc>& jobs) {
+	std::vector<std::pair<uint32_t*, uint64_t>> tables;
+	for (const JobDesc& j : jobs) tables.push_back({j.table, ((uint64_t)j.grid[0] * j.grid[1] * j.grid[2] + 31) / 32});
+	const std::vector<char> shared = overlapping_tables(tables);
+	std::vector<std::vector<size_t>> sets(1);
+	for (size_t i = 0; i < jobs.size(); i++) {
+		size_t k = 0;
+		if (shared[i])
+			while (k < sets.size() && std::any_of(sets[k].begin(), sets[k].end(), [&](size_t o) {
+				       return tables[i].first < tables[o].first + tables[o].second &&
+				              tables[o].first < tables[i].first + tables[i].second;
+			       }))
+				k++;
+		if (k == sets.size()) sets.emplace_back();
+		sets[k].push_back(i);
+	}
+	std::vector<Group> out;
+	for (const std::vector<size_t>& set : sets) {
+		std::vector<JobDesc> of;
+		for (size_t i : set) of.push_back(jobs[i]);
+		out.push_back(resolve_group(of));
+	}
+	return out;
+}
+
 uint64_t flip_bytes_of(const JobDesc& j) {
 	return align_up(((uint64_t)j.grid[0] * j.grid[1] * j.grid[2] + 31) / 32 * 4);
 }
@@ -990,7 +1017,8 @@ cvx_status cvx_plan_create(const cvx_job* jobs, uint32_t n_jobs, uint32_t flags,
 	struct Lane {
 		bool solid = false;
 		std::vector<JobDesc> jobs;
-		std::vector<Group> groups;  // toggles / surface launches; the solid lane's resolve is last
+		std::vector<Group> groups;  // surface launches, or the toggles and then the resolves
+		size_t resolves = 0;         // groups at the end that are resolves
 		uint64_t cap = 1;
 		uint32_t bricks = 0;         // largest brick count of the lane's groups
 		size_t job_off = 0;          // first JobDesc slot of the lane in the job area
@@ -1033,11 +1061,15 @@ cvx_status cvx_plan_create(const cvx_job* jobs, uint32_t n_jobs, uint32_t flags,
 	size_t slots = 0;
 	for (Lane& l : lanes) {
 		l.groups = make_groups(l.jobs, l.solid);
-		if (l.solid) l.groups.push_back(resolve_group(l.jobs));
+		if (l.solid)
+			for (Group& g : resolve_groups(l.jobs)) {
+				l.groups.push_back(std::move(g));
+				l.resolves++;
+			}
 		l.job_off = slots;
 		for (size_t gi = 0; gi < l.groups.size(); gi++) {
 			const Group& g = l.groups[gi];
-			if (!(l.solid && gi + 1 == l.groups.size())) l.cap = std::max<uint64_t>(l.cap, g.tris);
+			if (gi + l.resolves < l.groups.size()) l.cap = std::max<uint64_t>(l.cap, g.tris);
 			if (!l.solid) l.bricks = std::max(l.bricks, g.bricks);
 			if (g.jobs.size() > 1) slots += g.jobs.size();
 		}
@@ -1143,7 +1175,7 @@ cvx_status cvx_plan_create(const cvx_job* jobs, uint32_t n_jobs, uint32_t flags,
 		size_t used = l.job_off;
 		for (size_t gi = 0; gi < l.groups.size() && cst == CVX_OK; gi++) {
 			const Group& g = l.groups[gi];
-			const bool resolve = l.solid && gi + 1 == l.groups.size();
+			const bool resolve = gi + l.resolves >= l.groups.size();
 			const cudaError_t e = capture_group(g, l.solid, resolve, gi == 0, rec, l.cap, l.bricks, p->job_area + used, dev, l.stream);
 			if (g.jobs.size() > 1) used += g.jobs.size();
 			if (e != cudaSuccess) cst = cuda_fail(e, "capture launch");

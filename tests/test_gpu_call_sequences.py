@@ -95,3 +95,32 @@ def test_calls_on_several_streams():
         cv.stream_release(s)
     for k, table in done:
         assert torch.equal(table, work.items[k][3])
+
+
+@pytest.mark.parametrize("morton,g", [(False, 100), (False, 128), (False, 72), (True, 16), (True, 64), (True, 128)])
+@pytest.mark.parametrize("n", [2, 3])
+def test_solid_jobs_of_a_plan_that_share_a_table(morton, g, n):
+    """Each job's bits are XORed into the table, as by one call after another: jobs that flip the same words, jobs
+    in parts of the table of their own, a table that overlaps another one in part, and one of its own."""
+    infos, tris = [], []
+    for k in range(n):
+        t = meshgen.icosphere(k, level=4)
+        infos.append(cv.make_voxinfo(t, g))
+        tris.append(torch.from_numpy(np.ascontiguousarray(t).reshape(-1)).cuda())
+    low = cv.make_info((-1, -1, -1), (3, 3, 3), g, infos[0].n_triangles)  # one corner of the box
+    high = cv.make_info((-3, -3, -3), (1, 1, 1), g, infos[0].n_triangles)
+    unit = tris[0] / tris[0].abs().max()
+    W = cv.table_words(infos[0])
+    jobs = [(i, t, 0) for i, t in zip(infos, tris)]
+    jobs += [(low, unit, 2 * W), (high, unit, 2 * W), (infos[0], tris[0], 3 * W - 5), (infos[0], tris[0], 5 * W)]
+    want, got = (torch.zeros(6 * W, dtype=torch.int32, device="cuda") for _ in range(2))
+    for info, t, at in jobs:
+        cv.voxelize_solid(info, t, want[at:at + W], morton)
+    plan = cv.Plan([cv.Job(info, t, got[at:at + W], morton, True) for info, t, at in jobs], clear_tables=True)
+    for _ in range(20):
+        got.fill_(-1)
+        plan.launch()
+        for at in (0, 2 * W, 5 * W):
+            end = at + W if at != 2 * W else 4 * W - 5
+            assert torch.equal(got[at:end], want[at:end]), at
+    plan.close()
