@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 
 	SurfTri S;
 	uint32_t n_items = 0, n_rows = 0, slices = kZch;
+	bool tiny = false;
 	if (valid) {
 		const float bmin[3] = {J.bmin[0], J.bmin[1], J.bmin[2]};
 		const float inv[3] = {J.inv_unit[0], J.inv_unit[1], J.inv_unit[2]};
@@ -94,7 +95,8 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 		const uint64_t rows = (uint64_t)(ey + 1) * (uint64_t)(ez + 1);
 		while (slices > kMinSlices && (uint64_t)(ey + 1) * slices > item_rows) slices >>= 1;
 		n_items = ez / slices + 1u;
-		if (ex < kMaskRowVoxels && rows <= local_rows && !plane_underflows(S.d1, S.d2)) n_rows = (uint32_t)rows;
+		if (ex < kMaskRowVoxels && rows <= local_rows) n_rows = (uint32_t)rows;
+		tiny = plane_underflows(S.d1, S.d2);
 	}
 	uint32_t incl = n_rows;
 #pragma unroll
@@ -107,6 +109,10 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 	const uint32_t lt = (1u << lane) - 1u;
 	const uint32_t parked = __ballot_sync(FULL, n_rows != 0u);
 	if (n_rows) pack_small(S, start, sm.small[__popc(parked & lt)]);
+	if (n_rows && tiny) {  // bounds of the plane test where its product may underflow
+		SmallTri& o = sm.small[__popc(parked & lt)];
+		plane_widen(S.nx, S.ny, S.nz, unit, o.q[4].z, o.q[4].w);
+	}
 	const bool queued = n_items && !n_rows;
 	const bool is_brick = queued && (jflags & JOB_BRICKS);  // rasterized in shared-memory bricks (bricks.cu)
 	const bool is_mid = queued && !is_brick && n_items == 1, is_big = queued && !is_brick && n_items > 1;
@@ -401,7 +407,7 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 			}
 			float lo, hi;
 			plane_bounds(S, lo, hi);
-			plane_widen(lo, hi);
+			if (plane_underflows(lo, hi)) plane_widen(S.nx, S.ny, S.nz, unit, lo, hi);
 			const float plane_m = fmaxf(fabsf(lo), fabsf(hi)), plane_inv = __fdividef(-1.0f, S.nx * unit[0]);
 			const float bx0 = (float)S.bx0, bx1 = (float)S.bx1;
 

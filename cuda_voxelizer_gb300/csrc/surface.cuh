@@ -192,30 +192,41 @@ __device__ __forceinline__ void plane_bounds(const SurfTri& S, float& lo, float&
 __device__ __forceinline__ bool plane_underflows(float lo, float hi) {
 	return (fabsf(lo) < 0x1p-49f) | (fabsf(hi) < 0x1p-49f);
 }
-// The largest float s >= hi at which fl(fl(s - lo) * fl(s - hi)) is not positive (lo <= hi, neither a
-// NaN), by a search over the floats in order: above hi both differences, and so the rounded product,
-// grow with s.
+// The largest float s >= hi at which fl(fl(s - lo) * fl(s - hi)) is not positive (lo <= hi, at least one
+// within 2^-49 of zero), by a search over the floats in order: above hi both differences, and so the
+// rounded product, grow with s.  From 2^-48 above a hi that small they are large enough, and above a
+// larger hi from the next float on.
 static __device__ __noinline__ float plane_reach(float lo, float hi) {
 	auto flip = [](int i) { return i ^ ((i >> 31) & 0x7FFFFFFF); };  // float bits <-> an int in the floats' order
-	int l = flip(__float_as_int(hi)), r = 0x7F800000;
+	auto fails = [&](int i) {
+		const float s = __int_as_float(flip(i));
+		return __fmul_rn(__fsub_rn(s, lo), __fsub_rn(s, hi)) > 0.0f;
+	};
+	int l = flip(__float_as_int(hi)), r = flip(__float_as_int(fmaxf(hi, 0.0f) + 0x1p-48f));
+	if (fails(l + 1)) return hi;
 	while (l < r) {
 		const int m = l + (int)(((uint32_t)r - (uint32_t)l + 1u) >> 1);
-		const float s = __int_as_float(flip(m));
-		if (__fmul_rn(__fsub_rn(s, lo), __fsub_rn(s, hi)) > 0.0f) r = m - 1; else l = m;
+		if (fails(m)) r = m - 1; else l = m;
 	}
 	return __int_as_float(flip(l));
 }
-__device__ __forceinline__ void plane_widen(float& lo, float& hi) {
-	if (plane_underflows(lo, hi)) {
-		const float reach = plane_reach(lo, hi);
-		lo = -plane_reach(-hi, -lo);
-		hi = reach;
-	}
+// For bounds of which plane_underflows().  Offsets that are exactly zero need no search where every
+// component of the normal is zero or, times the voxel's extent, at least 2^-26: products with a
+// coordinate are then multiples of 2^-73, and so is s; a nonzero sum is at least that, and their
+// product at least 2^-146.
+__device__ __forceinline__ void plane_widen(float nx, float ny, float nz, const float* unit, float& lo, float& hi) {
+	auto large = [&](float n, int k) { return (n == 0.0f) | (fabsf(n) * unit[k] >= 0x1p-26f); };
+	auto offset = [](float d) { return (d == 0.0f) | (fabsf(d) >= 0x1p-49f); };
+	if (!(lo <= hi)) return;  // NaN
+	if (offset(lo) & offset(hi) & large(nx, 0) & large(ny, 1) & large(nz, 2)) return;
+	const float reach = plane_reach(lo, hi);
+	lo = -plane_reach(-hi, -lo);
+	hi = reach;
 }
 
-// A small triangle's setup (rows of at most kMaskRowVoxels voxels, plane_underflows() false) parked
-// in shared memory between the two phases of the classify kernel, with the tests in the form that
-// takes the fewest instructions per voxel: the plane test as above, and an edge test, which fails iff
+// A small triangle's setup (rows of at most kMaskRowVoxels voxels) parked in shared memory between the
+// two phases of the classify kernel, with the tests in the form that takes the fewest instructions per
+// voxel: the plane test as above, and an edge test, which fails iff
 // fl(v + d) < 0, as v < -d.  (Rounding keeps the sign of a sum: the sum of two floats is a multiple of
 // the smallest subnormal, so it never rounds to zero; a NaN or an inf - inf fails neither form.)
 // The record is read as nine 16-byte vectors, those of the YZ tests first; its stride of 36 words
