@@ -129,8 +129,7 @@ using namespace cvx;
 
 extern "C" {
 
-cvx_status cvx_mesh_bbox_device_ws(const float* d_triangles, uint64_t n_triangles, void* d_ws, uint64_t ws_bytes,
-                                   float out_min[3], float out_max[3], cvx_stream_t stream) {
+static cvx_status check_box(const float* d_triangles, uint64_t n_triangles, const float* out_min, const float* out_max) {
 	if (!d_triangles || !out_min || !out_max) {
 		set_message("cvx_mesh_bbox_device: null argument");
 		return CVX_ERR_INVALID_VALUE;
@@ -139,6 +138,13 @@ cvx_status cvx_mesh_bbox_device_ws(const float* d_triangles, uint64_t n_triangle
 		set_message("cvx_mesh_bbox_device: empty mesh has no bounding box");
 		return CVX_ERR_INVALID_VALUE;
 	}
+	return CVX_OK;
+}
+
+cvx_status cvx_mesh_bbox_device_ws(const float* d_triangles, uint64_t n_triangles, void* d_ws, uint64_t ws_bytes,
+                                   float out_min[3], float out_max[3], cvx_stream_t stream) {
+	cvx_status st = check_box(d_triangles, n_triangles, out_min, out_max);
+	if (st != CVX_OK) return st;
 	if (!d_ws || ws_bytes < CVX_BBOX_WORKSPACE || reinterpret_cast<uintptr_t>(d_ws) % 16) {
 		set_message("cvx_mesh_bbox_device_ws: workspace null, too small or not 16-byte aligned");
 		return CVX_ERR_INVALID_VALUE;
@@ -152,7 +158,7 @@ cvx_status cvx_mesh_bbox_device_ws(const float* d_triangles, uint64_t n_triangle
 	const uint64_t nv = 3 * n_triangles;
 	const uint64_t want = (nv + kReduceThreads * 8 - 1) / (kReduceThreads * 8);
 	const uint32_t blocks = (uint32_t)(want < (uint64_t)sms * 8 ? (want ? want : 1) : (uint64_t)sms * 8);
-	cvx_status st = cuda_status(cudaMemsetAsync(d_out, 0, sizeof(keys), s), "cudaMemsetAsync");
+	st = cuda_status(cudaMemsetAsync(d_out, 0, sizeof(keys), s), "cudaMemsetAsync");
 	if (st == CVX_OK) {
 		if (reinterpret_cast<uintptr_t>(d_triangles) % 16 == 0) bbox_reduce<true><<<blocks, kReduceThreads, 0, s>>>(d_triangles, nv, d_out);
 		else bbox_reduce<false><<<blocks, kReduceThreads, 0, s>>>(d_triangles, nv, d_out);
@@ -171,9 +177,11 @@ cvx_status cvx_mesh_bbox_device_ws(const float* d_triangles, uint64_t n_triangle
 
 cvx_status cvx_mesh_bbox_device(const float* d_triangles, uint64_t n_triangles, float out_min[3], float out_max[3],
                                 cvx_stream_t stream) {
+	cvx_status st = check_box(d_triangles, n_triangles, out_min, out_max);
+	if (st != CVX_OK) return st;
 	cudaStream_t s = (cudaStream_t)stream;
 	void* ws = nullptr;
-	cvx_status st = cuda_status(cudaMallocAsync(&ws, CVX_BBOX_WORKSPACE, s), "cudaMallocAsync");
+	st = cuda_status(cudaMallocAsync(&ws, CVX_BBOX_WORKSPACE, s), "cudaMallocAsync");
 	if (st != CVX_OK) return st;
 	st = cvx_mesh_bbox_device_ws(d_triangles, n_triangles, ws, CVX_BBOX_WORKSPACE, out_min, out_max, stream);
 	cudaFreeAsync(ws, s);

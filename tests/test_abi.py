@@ -186,3 +186,16 @@ def test_host_pipeline_refuses_slots_sharing_a_buffer():
             cv.HostPipeline([a, b])
     with pytest.raises(ValueError):
         cv.HostPipeline([])
+
+
+def test_device_box_validation_answers_without_a_gpu():
+    """The box of a device mesh refuses null pointers and empty meshes before any CUDA call."""
+    lo, hi = (ctypes.c_float * 3)(), (ctypes.c_float * 3)()
+    g, out = (ctypes.c_uint32 * 3)(8, 8, 8), cv.VoxInfo()
+    for tris, n, a, b in ((None, 1, lo, hi), (16, 1, None, hi), (16, 1, lo, None), (16, 0, lo, hi)):
+        assert _lib.lib.cvx_mesh_bbox_device(tris, n, a, b, None) == 1
+        assert _lib.lib.cvx_mesh_bbox_device_ws(tris, n, 256, 256, a, b, None) == 1
+    for tris, n in ((None, 1), (16, 0)):
+        assert _lib.lib.cvx_voxinfo_from_device(tris, n, g, ctypes.byref(out), None) == 1
+        assert _lib.lib.cvx_voxinfo_from_device_ws(tris, n, g, 256, 256, ctypes.byref(out), None) == 1
+    assert _lib.lib.cvx_voxinfo_from_device(16, 1, None, ctypes.byref(out), None) == 1
