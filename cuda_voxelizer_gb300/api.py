@@ -518,15 +518,25 @@ class Server:
 _BBOX_WORKSPACE = 256  # CVX_BBOX_WORKSPACE
 
 
-def _scratch(nbytes: int, device, stream):
-    """Temporary device memory from torch's allocator, allocated on the stream that uses it."""
+def _on(stream):
+    """A context with torch's current stream set to `stream` (a torch stream, a raw handle, or an object that has
+    one), for memory that is used there: the allocator only orders a block's next use on the stream it belongs to."""
     import contextlib
 
     import torch
-    on = contextlib.nullcontext()
-    if stream is not None:
-        on = torch.cuda.stream(torch.cuda.ExternalStream(stream) if isinstance(stream, int) else stream)
-    with on:
+    if stream is None:
+        return contextlib.nullcontext()
+    if not isinstance(stream, torch.cuda.Stream):
+        raw = _stream(stream)
+        # handles 0 and 1 are the default stream; ExternalStream(0) would be a new one
+        stream = torch.cuda.default_stream() if raw in (0, 1) else torch.cuda.ExternalStream(raw)
+    return torch.cuda.stream(stream)
+
+
+def _scratch(nbytes: int, device, stream):
+    """Temporary device memory from torch's allocator, allocated on the stream that uses it."""
+    import torch
+    with _on(stream):
         return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 

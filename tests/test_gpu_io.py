@@ -225,3 +225,34 @@ def test_bbox_and_gather_at_odd_sizes(n, offset):
     assert not host[:offset].any() and not host[offset + 9 * n:].any()
     lo, hi = cv.mesh_bbox_device(soup)
     assert np.array_equal(lo, want.reshape(-1, 3).min(0)) and np.array_equal(hi, want.reshape(-1, 3).max(0))
+
+
+class _HasHandle:
+    """A stream of another library: an object with its handle."""
+
+    def __init__(self, stream):
+        self.cuda_stream = stream.cuda_stream
+
+
+def _io_calls(stream):
+    tris = meshgen.torus(1)
+    d = torch.from_numpy(tris.reshape(-1)).cuda()
+    info = cv.make_voxinfo(tris, 64)
+    table = torch.zeros(cv.table_words(info), dtype=torch.int32, device="cuda")
+    cv.voxelize(info, d, table)
+    torch.cuda.synchronize()
+    lo, hi = cv.mesh_bbox_device(d, stream=stream)
+    return (lo.tobytes(), hi.tobytes(), bytes(cv.voxinfo_from_device(d, 64, stream=stream)),
+            cv.encode_binvox(info, table, stream=stream), cv.encode_voxel_list(info, table, stream=stream).cpu().numpy().tobytes())
+
+
+@pytest.mark.parametrize("kind", ["torch", "handle", "object", "default", "legacy handle"])
+def test_stream_arguments(kind):
+    """Every form of a stream argument; the calls' scratch belongs to that stream, and to no other."""
+    want = _io_calls(None)
+    side = torch.cuda.Stream()
+    stream = {"torch": side, "handle": side.cuda_stream, "object": _HasHandle(side), "default": 0, "legacy handle": 1}[kind]
+    owners = lambda: {seg["stream"] for seg in torch.cuda.memory_snapshot()}  # noqa: E731
+    before = owners()
+    assert _io_calls(stream) == want
+    assert owners() - before <= {side.cuda_stream}
