@@ -540,6 +540,14 @@ def _scratch(nbytes: int, device, stream):
         return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
+def _result(t, stream):
+    """A tensor made under _on(stream), for a caller who uses it on the current stream."""
+    import torch
+    if stream is not None:
+        t.record_stream(torch.cuda.current_stream(t.device))
+    return t
+
+
 def mesh_bbox_device(triangles, stream=None):
     """Vertex bounding box of a device triangle soup (CUDA tensor); host float32 arrays."""
     n = triangles.numel() // 9
@@ -568,20 +576,23 @@ def gather_soup(vertices, faces, stream=None):
     number of faces with an index out of range).  Synchronizes to read the count."""
     import torch
     f = faces.reshape(-1, 3)
-    soup = torch.empty(f.shape[0] * 9, dtype=torch.float32, device=vertices.device)
-    bad = torch.zeros(1, dtype=torch.int64, device=vertices.device)
-    check(lib.cvx_gather_soup(_ptr(vertices), vertices.numel() // 3, _ptr(f), f.shape[0], _ptr(soup), _ptr(bad),
-                              _stream(stream)), "cvx_gather_soup")
-    return soup, int(bad.item())
+    with _on(stream):
+        soup = torch.empty(f.shape[0] * 9, dtype=torch.float32, device=vertices.device)
+        bad = torch.zeros(1, dtype=torch.int64, device=vertices.device)
+        check(lib.cvx_gather_soup(_ptr(vertices), vertices.numel() // 3, _ptr(f), f.shape[0], _ptr(soup), _ptr(bad),
+                                  _stream(stream)), "cvx_gather_soup")
+        n_bad = int(bad.item())
+    return _result(soup, stream), n_bad
 
 
 def transcode(table, gridsize: int, to_morton: bool, stream=None):
     """Morton <-> linear copy of a g^3 table (CUDA tensor); returns a new tensor."""
     import torch
-    out = torch.empty_like(table)
+    with _on(stream):
+        out = torch.empty_like(table)
     check(lib.cvx_transcode(_ptr(table), _ptr(out), int(gridsize), int(bool(to_morton)), _stream(stream)),
           "cvx_transcode")
-    return out
+    return _result(out, stream)
 
 
 def _encode_scratch(info: VoxInfo, table, stream):
@@ -608,14 +619,13 @@ def _to_bytes(t) -> bytes:
 
 def encode_binvox(info: VoxInfo, table, stream=None) -> bytes:
     """binvox run-length payload of a linear-order device table (the bytes after the header)."""
-    import torch
     ws = _encode_scratch(info, table, stream)
     n = ctypes.c_uint64()
     # Closed meshes need about 2 bytes per 255 voxels and a few per line along y: a fifth to a third of
     # the table.  A payload that does not fit is encoded again, into a buffer of its size.
     capacity = max(4 * table_words(info), 1 << 16)
     while True:
-        out = torch.empty(capacity, dtype=torch.uint8, device=table.device)
+        out = _scratch(capacity, table.device, stream)
         st = lib.cvx_encode_binvox_ws(ctypes.byref(info), _ptr(table), _ptr(ws), ws.numel(), _ptr(out), capacity,
                                       ctypes.byref(n), _stream(stream))
         if n.value <= capacity:
@@ -644,7 +654,8 @@ def encode_voxel_list(info: VoxInfo, table, stream=None):
     n = ctypes.c_uint64()
     check(lib.cvx_encode_voxel_list_ws(ctypes.byref(info), _ptr(table), _ptr(ws), ws.numel(), None, 0, ctypes.byref(n),
                                        _stream(stream)), "cvx_encode_voxel_list_ws")
-    out = torch.empty((max(1, n.value), 3), dtype=torch.int32, device=table.device)
+    with _on(stream):
+        out = torch.empty((max(1, n.value), 3), dtype=torch.int32, device=table.device)
     check(lib.cvx_encode_voxel_list_ws(ctypes.byref(info), _ptr(table), _ptr(ws), ws.numel(), _ptr(out), n.value,
                                        ctypes.byref(n), _stream(stream)), "cvx_encode_voxel_list_ws")
-    return out[:n.value]
+    return _result(out, stream)[:n.value]

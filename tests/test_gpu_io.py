@@ -256,3 +256,50 @@ def test_stream_arguments(kind):
     before = owners()
     assert _io_calls(stream) == want
     assert owners() - before <= {side.cuda_stream}
+
+
+def test_results_of_calls_on_another_stream():
+    """Memory that the current stream still writes when a call on another stream takes it over: the result is not
+    touched by that write, nor the write's value read."""
+    tris = meshgen.torus(1)
+    info = cv.make_voxinfo(tris, 128)
+    table = torch.zeros(cv.table_words(info), dtype=torch.int32, device="cuda")
+    cv.voxelize(info, torch.from_numpy(tris.reshape(-1)).cuda(), table)
+    rng = np.random.default_rng(2)
+    v = torch.from_numpy(rng.normal(size=(5000, 3)).astype(np.float32)).cuda()
+    f = torch.from_numpy(rng.integers(0, 5002, size=(200_000, 3)).astype(np.int32)).cuda()
+    calls = [lambda s: cv.transcode(table, 128, True, stream=s), lambda s: cv.encode_voxel_list(info, table, stream=s),
+             lambda s: cv.gather_soup(v, f, stream=s)]
+    side = torch.cuda.Stream()
+    for call in calls:
+        torch.cuda.synchronize()
+        want = call(None)
+        n_bad = None
+        if isinstance(want, tuple):
+            want, n_bad = want
+        torch.cuda.synchronize()
+        for stream in (side, side.cuda_stream):
+            torch.cuda._sleep(20_000_000)  # 10 ms on the current stream
+            late = torch.full_like(want, 7)
+            del late
+            got = call(stream)
+            if n_bad is not None:
+                got, k = got
+                assert k == n_bad
+            torch.cuda.synchronize()
+            assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+            del got
+
+
+def test_binvox_on_another_stream():
+    tris = meshgen.icosphere(3, level=4)
+    info = cv.make_voxinfo(tris, 200)
+    table = torch.zeros(cv.table_words(info), dtype=torch.int32, device="cuda")
+    cv.voxelize_solid(info, torch.from_numpy(tris.reshape(-1)).cuda(), table)
+    want = cv.encode_binvox(info, table)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    torch.cuda._sleep(20_000_000)
+    late = torch.full((4 * cv.table_words(info),), 7, dtype=torch.uint8, device="cuda")
+    del late
+    assert cv.encode_binvox(info, table, stream=side) == want
