@@ -433,7 +433,7 @@ __host__ __device__ __forceinline__ bool lane_rows(uint32_t gx) { return gx % 12
 // once 69 us (88 with the warp on consecutive words, 111 with the next load made ahead), forty of 256^3
 // 49 / 70, one of 384^3 8 / 10, of 640^3 16 / 20; of 768^3 39 / 26, of 1024^3 92 / 57, hence kLaneRow.
 __global__ void __launch_bounds__(256, 6) solid_resolve(const __grid_constant__ LaunchDesc L) {
-	const uint32_t unit_id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+	const uint32_t unit_id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
 	if (unit_id >= L.n_units) return;
 	const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
 	const uint32_t j = warp_job(L, unit_id, [](const JobDesc& d) { return (uint64_t)d.unit_begin; });
@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(256) solid_morton_small(const __grid_constant_
 // Morton jobs with g < 32: clear the resolved flip table, one warp per resolve unit
 // (solid_morton_cols clears its own words).
 __global__ void __launch_bounds__(256) solid_zero(const __grid_constant__ LaunchDesc L) {
-	const uint32_t unit_id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+	const uint32_t unit_id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
 	if (unit_id >= L.n_units) return;
 	const uint32_t j = warp_job(L, unit_id, [](const JobDesc& d) { return (uint64_t)d.unit_begin; });
 	const JobDesc& J = job_at(L, j);

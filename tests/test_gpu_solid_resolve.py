@@ -149,3 +149,29 @@ def test_columns_per_triangle(n_boxes, extent):
     cv.voxelize_solid(info, torch.from_numpy(tris.reshape(-1)).cuda(), table, False)
     cv.device_status()
     assert np.array_equal(table.cpu().numpy().view(np.uint32), _want(boxes, (g, g, g), False))
+
+
+def test_more_than_2_to_the_27_resolve_units():
+    """A table of 64 GiB in units of 128 words: the first and the last rows, and nothing else, hold their solids."""
+    g = (128, 1 << 21, (1 << 11) + 4)
+    words = g[0] // 32 * g[1] * g[2]
+    if torch.cuda.mem_get_info()[0] < 2 * 4 * words + (8 << 30):
+        pytest.skip("needs 140 GiB of device memory")
+    tris, rows = [], []
+    for z in (1, g[2] - 3):  # a quad in the plane x = 64 over 10 x 2 columns
+        a, b, c, d = ([64.25, y, w] for y, w in ((10, z), (20, z), (20, z + 2), (10, z + 2)))
+        tris += [a + b + c, a + c + d]
+        rows += [y + (z + k) * g[1] for k in range(2) for y in range(10, 20)]
+    info = cv.make_info((0, 0, 0), [float(n) for n in g], g, len(tris))
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        table = torch.zeros(words, dtype=torch.int32, device="cuda")
+        cv.voxelize_solid(info, torch.tensor(tris, dtype=torch.float32, device="cuda").reshape(-1), table)
+        cv.device_status(stream)
+        got = torch.stack([table[4 * r:4 * r + 4] for r in rows]).cpu().numpy().view(np.uint32)
+        n = sum(int(torch.count_nonzero(part)) for part in table.split(1 << 28))
+    del table
+    cv.stream_release(stream)
+    torch.cuda.empty_cache()
+    assert (got == np.array([0xFFFFFFFF, 0xFFFFFFFF, 0, 0], dtype=np.uint32)).all()
+    assert n == 2 * len(rows)
