@@ -8,9 +8,9 @@ voxels: (brick, triangle) pairs per triangle the shared-memory brick rasterizer 
 every larger triangle to the row-by-row path with global atomics).  ``autotune()`` times a fixed set
 of seeded workloads -- sub-voxel and few-voxel triangles at several grids, surface and solid, linear
 and Morton, and a soup of large triangles at 1024^3 -- for every candidate, keeps the fastest,
-applies it with cvx_set_tuning and stores it in a JSON cache keyed by the device; ``load_cached()``
-applies a cached choice without timing anything.  The package applies the cache once per device
-the first time a Plan or Server is made (``apply_cached_once``).
+applies it with cvx_set_tuning and stores it in a JSON cache keyed by the device and the knobs' units;
+``load_cached()`` applies a cached choice without timing anything.  The package applies the cache once
+per device the first time a Plan or Server is made (``apply_cached_once``).
 
     python -m cuda_voxelizer_gb300.autotune            # tune device 0, print and cache the result
 """
@@ -37,10 +37,15 @@ DEFAULT_CACHE = os.environ.get("CVX_TUNING_CACHE") or os.path.join(os.path.expan
                                                                      "cuda_voxelizer_gb300", "tuning.json")
 
 
+# What the knobs count, part of the cache's keys: a choice made when small_vox counted voxels and
+# small_cols columns means something else now and is not applied.
+KNOB_UNITS = "rows, 8 columns"
+
+
 def _device_key(device: int) -> str:
     import torch
     p = torch.cuda.get_device_properties(device)
-    return f"{p.name} sm_{p.major}{p.minor} {p.multi_processor_count}SM"
+    return f"{p.name} sm_{p.major}{p.minor} {p.multi_processor_count}SM ({KNOB_UNITS})"
 
 
 def _workloads(torch):

@@ -61,3 +61,14 @@ def test_autotune_applies_and_caches(tmp_path):
         assert cv.get_tuning(0) == choice
     finally:
         cv.set_tuning(0, **before)
+
+
+def test_a_cache_of_other_knob_units_is_not_applied(tmp_path):
+    """A choice that was stored before the knobs counted rows and eighths of columns."""
+    p = torch.cuda.get_device_properties(0)
+    path = str(tmp_path / "tuning.json")
+    with open(path, "w") as f:
+        json.dump({f"{p.name} sm_{p.major}{p.minor} {p.multi_processor_count}SM": {"small_vox": 16, "small_cols": 4}}, f)
+    before = cv.get_tuning(0)
+    assert at.load_cached(0, path) is None
+    assert cv.get_tuning(0) == before
