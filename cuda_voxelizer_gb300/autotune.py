@@ -25,7 +25,7 @@ import numpy as np
 from . import api as cv
 from . import meshgen
 
-SMALL_VOX = (16, 32, 64, 128, 255)
+SMALL_VOX = (16, 32, 64)
 SMALL_COLS = (4, 8, 16)
 BRICK_PAIRS = (0, 16)
 KNOBS = ("small_vox", "small_cols", "brick_pairs")

@@ -72,3 +72,8 @@ def test_a_cache_of_other_knob_units_is_not_applied(tmp_path):
     before = cv.get_tuning(0)
     assert at.load_cached(0, path) is None
     assert cv.get_tuning(0) == before
+
+
+def test_candidates_differ():
+    """No candidate is above the value at which the engine caps its knob: those would be timed twice."""
+    assert max(at.SMALL_VOX) <= 64 and max(at.SMALL_COLS) <= 16
