@@ -119,9 +119,10 @@ static inline int f2i(float v, int gpu) {
     if (!(v > -2147483904.0f && v < 2147483648.0f)) return (-2147483647 - 1);
     return (int)v;
 }
-/* int(double) with the device's saturating conversion (cvt.rzi.s32.f64); NaN gives 0. */
-static inline int d2i(double v) {
-    if (v != v) return 0;
+/* int(double) with the device's saturating conversion (cvt.rzi.s32.f64).  NaN -- a zero-area triangle's
+ * column -- gives INT_MIN on the device: the reference kernel leaves such columns alone. */
+static inline int d2i(double v, int gpu) {
+    if (v != v) return gpu ? (-2147483647 - 1) : 0;
     if (v >= 2147483647.0) return 2147483647;
     if (v <= -2147483648.0) return (-2147483647 - 1);
     return (int)v;
@@ -367,7 +368,7 @@ static void solid_triangle(const ovx_info* info, const float* tri, uint64_t t, u
             int checknum = check_point_triangle(pp, v0_yz, v1_yz, v2_yz, point);
             if ((checknum == 1 && top_left_edge(v0_yz, v1_yz)) || (checknum == 2 && top_left_edge(v1_yz, v2_yz)) ||
                 (checknum == 3 && top_left_edge(v2_yz, v0_yz)) || (checknum == 0)) {
-                int xmax = d2i((double)(get_x_coordinate(pg, n, v0, point) / unit.x) - 0.5);
+                int xmax = d2i((double)(get_x_coordinate(pg, n, v0, point) / unit.x) - 0.5, gpu);
                 /* The CPU build stores xmax as unsigned (src/cpu_voxelizer.cpp:296-297); the GPU
                  * kernel keeps it signed (src/voxelize_solid.cu:123-124).  They only differ for
                  * hits left of the grid, where the CPU loop runs away; both stop here. */
