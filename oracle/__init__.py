@@ -10,6 +10,8 @@ baseline leg may import this package; the engine in ``cuda_voxelizer_gb300`` nev
   ``oracle/build_ref.sh`` (only where that build ran: it is host code).
 * :class:`RefGPU` -- the reference's own CUDA kernels (src/voxelize.cu, src/voxelize_solid.cu)
   built for sm_103a by ``oracle/build_ref.sh`` and launched by ``oracle/ref_gpu_runner.cu``.
+* :class:`ModelGPU` -- the restatement in those kernels' arithmetic behind RefGPU's interface, for
+  machines where ``oracle/_ref`` holds no build of them (:func:`ref_gpu_available`).
 """
 from __future__ import annotations
 
@@ -271,6 +273,11 @@ def ref_cpu_voxelize(info: bytes, tris, morton: bool = False, solid: bool = Fals
 
 # --- the reference's own CUDA kernels ------------------------------------------------------------
 
+def ref_gpu_available() -> bool:
+    """Whether the reference's kernels were built here (oracle/build_ref.sh needs its sources)."""
+    return os.path.exists(os.path.join(REF_DIR, "ref_voxelize.cubin"))
+
+
 class RefGPU:
     """Launch the reference kernels (compiled from its sources for sm_103a) on device buffers."""
 
@@ -278,7 +285,7 @@ class RefGPU:
         path = _build.build_gpu_runner()
         if path is None:
             raise RuntimeError("nvcc not available to build the reference kernel runner")
-        if not os.path.exists(os.path.join(REF_DIR, "ref_voxelize.cubin")):
+        if not ref_gpu_available():
             raise RuntimeError("reference cubins missing from oracle/_ref (run oracle/build_ref.sh)")
         L = ctypes.CDLL(path)
         L.refgpu_init.argtypes = [ctypes.c_char_p]
@@ -299,3 +306,58 @@ class RefGPU:
         ib = ctypes.create_string_buffer(bytes(info), 64)
         if self.L.refgpu_voxelize(ctypes.addressof(ib), d_tris, d_table, int(morton), int(solid), stream) != 0:
             raise RuntimeError("refgpu_voxelize: " + self.L.refgpu_last_error().decode())
+
+
+class ModelGPU:
+    """RefGPU's calls answered by the restatement (:func:`gpu_mode`, with the device's own rsqrtf for the
+    normals), on all of the host's threads; the tables are what the reference's kernels write."""
+
+    def __init__(self):
+        path = _build.build_gpu_runner()
+        if path is None:
+            raise RuntimeError("nvcc not available to build the device's rsqrtf")
+        self.L = ctypes.CDLL(path)
+        self.L.refgpu_rsqrt.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p]
+        self.threads = os.cpu_count() or 1
+
+    def rsqrt(self, d_in: int, d_out: int, n: int, stream: int = 0):
+        if self.L.refgpu_rsqrt(d_in, d_out, n, stream) != 0:
+            raise RuntimeError("rsqrtf kernel failed")
+
+    def _inv_len(self, l2: np.ndarray) -> np.ndarray:
+        import torch
+        d_in = torch.from_numpy(l2).cuda()
+        d_out = torch.empty_like(d_in)
+        self.rsqrt(d_in.data_ptr(), d_out.data_ptr(), l2.size, torch.cuda.current_stream().cuda_stream)
+        return np.ascontiguousarray(d_out.cpu().numpy())
+
+    def voxelize(self, info: bytes, d_tris: int, d_table: int, morton: bool, solid: bool, stream: int = 0):
+        import concurrent.futures
+        import torch
+
+        def buffer(ptr, n, kind):  # a device buffer as a tensor
+            class Buf:
+                __cuda_array_interface__ = {"shape": (n,), "typestr": kind, "data": (ptr, False), "version": 3}
+            return torch.as_tensor(Buf(), device="cuda")
+
+        info = bytes(info)
+        n = int.from_bytes(info[40:48], "little")
+        if n == 0:
+            return
+        torch.cuda.synchronize()
+        tris = buffer(d_tris, 9 * n, "<f4").cpu().numpy().reshape(n, 9)
+        out = buffer(d_table, table_words(info), "<i4")
+        inv = self._inv_len(len2(info, tris, gpu_mode(morton)))
+        k = min(self.threads, max(1, n // 64))
+
+        def part(i):  # every k-th triangle, into a table of its own
+            il = np.ascontiguousarray(inv[i::k])
+            t = np.ascontiguousarray(tris[i::k])
+            return voxelize(with_count(info, t.shape[0]), t, morton, solid, mode=gpu_mode(morton, inv_len=il))
+
+        table = out.cpu().numpy().view(np.uint32)
+        with concurrent.futures.ThreadPoolExecutor(k) as ex:
+            for t in ex.map(part, range(k)):
+                (np.bitwise_xor if solid else np.bitwise_or)(table, t, out=table)
+        out.copy_(torch.from_numpy(table.view(np.int32)))
+        torch.cuda.synchronize()

@@ -23,6 +23,15 @@ _ensure_built()
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (GB300 / sm_103a)")
+    import oracle
+    if not oracle.ref_gpu_available():
+        oracle.RefGPU = oracle.ModelGPU
+
+
+def pytest_report_header(config):
+    import oracle
+    if not oracle.ref_gpu_available():
+        return "oracle/_ref holds no build of the reference's kernels: the oracle in their arithmetic stands in"
 
 
 def cuda_available() -> bool:
