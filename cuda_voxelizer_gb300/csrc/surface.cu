@@ -6,10 +6,12 @@
 //                  cp.async.bulk (TMA bulk copy) when aligned.  Each lane sets up its triangle;
 //                  triangles of at most kLocalRows rows of at most kMaskRowVoxels voxels are finished
 //                  by the warp, their rows dealt over its lanes, every voxel tested like in the
-//                  reference; the others are queued, one record per triangle, as one item ("mid")
-//                  or as one item per 32 z-slices ("big").
-//   surf_rows      persistent CTAs; each warp takes work tickets (big items first, then mid
-//                  triangles), finds the bounds that the tests of the three projections put on the
+//                  reference; the others are queued, one record per triangle, as one item ("mid"),
+//                  as one item per 4 to 32 z-slices ("big"), or, of few but long rows, in a queue of
+//                  their own ("long").
+//   surf_rows      persistent CTAs; each warp takes its share of the long triangles, up to 32 at a
+//                  time, their rows dealt over its lanes; then work tickets (big items first, then
+//                  mid triangles): it finds the bounds that the tests of the three projections put on the
 //                  item's slices and rows, one test per slice or row instead of one per voxel row,
 //                  narrows every row to its exact x-interval with the plane test and ORs it into the
 //                  table one word at a time (the whole warp for long rows).  Jobs whose indices fit
@@ -22,6 +24,12 @@ namespace cvx {
 
 namespace {
 
+// Triangles of few rows, each longer than kMaskRowVoxels but of at most kLongVoxels voxels, are queued for
+// long_triangles: those of at most kLongRows rows, or of fewer rows than voxels in a row.  One by one as items of
+// surf_rows 200,000 triangles in boxes of 17 x 3 x 3 voxels took 220 us (50 this way), of 60 x 6 x 6 223 / 140, the
+// icosphere 7 on 4096 x 64 x 64 230 / 40; up to 64 rows whatever their length, icosphere 6 at 1000^3 86 us, 83
+// with this rule.
+constexpr uint32_t kLongRows = 32, kLongVoxels = 512;
 constexpr uint32_t kCollectRows = 384;  // rows of a classify warp from which those that pass the YZ tests are collected
 constexpr uint32_t kQueueRows = 64;     // fewer than 32 rows wait when 32 more are tested
 
@@ -95,7 +103,10 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 		const uint64_t rows = (uint64_t)(ey + 1) * (uint64_t)(ez + 1);
 		while (slices > kMinSlices && (uint64_t)(ey + 1) * slices > item_rows) slices >>= 1;
 		n_items = ez / slices + 1u;
-		if (ex < kMaskRowVoxels && rows <= local_rows) n_rows = (uint32_t)rows;
+		if (rows <= local_rows) {
+			if (ex < kMaskRowVoxels) n_rows = (uint32_t)rows;
+			else if (ex < kLongVoxels && rows <= max(kLongRows, ex)) slices = 0u;  // for long_triangles
+		}
 		tiny = plane_underflows(S.d1, S.d2);
 	}
 	uint32_t incl = n_rows;
@@ -114,53 +125,69 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 		plane_widen(S.nx, S.ny, S.nz, unit, o.q[4].z, o.q[4].w);
 	}
 	const bool queued = n_items && !n_rows;
-	const bool is_brick = queued && (jflags & JOB_BRICKS);  // rasterized in shared-memory bricks (bricks.cu)
-	const bool is_mid = queued && !is_brick && n_items == 1, is_big = queued && !is_brick && n_items > 1;
 	// Queue the other triangles: warp-aggregated appends.
-	const uint32_t brick_ballot = __ballot_sync(FULL, is_brick);
-	if (brick_ballot) {
-		uint32_t base = 0;
-		const uint32_t leader = __ffs(brick_ballot) - 1;
-		if (lane == leader) base = atomicAdd(&L.scr.ctr->bq, (unsigned)__popc(brick_ballot));
-		base = __shfl_sync(FULL, base, leader);
-		const uint32_t slot = base + __popc(brick_ballot & lt);
-		if (is_brick) {
-			if (slot < L.scr.cap) L.scr.bq[slot] = MidRec{j, (uint32_t)(t0 + lane)};
-			else set_error(L, kErrQueueOverflow);
+	if (__any_sync(FULL, queued)) {
+		const bool is_brick = queued && (jflags & JOB_BRICKS);  // rasterized in shared-memory bricks (bricks.cu)
+		const bool is_long = queued && !is_brick && slices == 0u;
+		const bool is_item = queued && !is_brick && slices != 0u;
+		const bool is_mid = is_item && n_items == 1, is_big = is_item && n_items > 1;
+		const uint32_t brick_ballot = __ballot_sync(FULL, is_brick);
+		if (brick_ballot) {
+			uint32_t base = 0;
+			const uint32_t leader = __ffs(brick_ballot) - 1;
+			if (lane == leader) base = atomicAdd(&L.scr.ctr->bq, (unsigned)__popc(brick_ballot));
+			base = __shfl_sync(FULL, base, leader);
+			const uint32_t slot = base + __popc(brick_ballot & lt);
+			if (is_brick) {
+				if (slot < L.scr.cap) L.scr.bq[slot] = MidRec{j, (uint32_t)(t0 + lane)};
+				else set_error(L, kErrQueueOverflow);
+			}
 		}
-	}
-	const uint32_t mid_ballot = __ballot_sync(FULL, is_mid);
-	if (mid_ballot) {
-		uint32_t base = 0;
-		const uint32_t leader = __ffs(mid_ballot) - 1;
-		if (lane == leader) base = atomicAdd(&L.scr.ctr->mid, (unsigned)__popc(mid_ballot));
-		base = __shfl_sync(FULL, base, leader);
-		const uint32_t slot = base + __popc(mid_ballot & lt);
-		if (is_mid) {
-			if (slot < L.scr.cap) L.scr.mid[slot] = MidRec{j, (uint32_t)(t0 + lane)};
-			else set_error(L, kErrQueueOverflow);
+		const uint32_t mid_ballot = __ballot_sync(FULL, is_mid);
+		if (mid_ballot) {
+			uint32_t base = 0;
+			const uint32_t leader = __ffs(mid_ballot) - 1;
+			if (lane == leader) base = atomicAdd(&L.scr.ctr->mid, (unsigned)__popc(mid_ballot));
+			base = __shfl_sync(FULL, base, leader);
+			const uint32_t slot = base + __popc(mid_ballot & lt);
+			if (is_mid) {
+				if (slot < L.scr.cap) L.scr.mid[slot] = MidRec{j, (uint32_t)(t0 + lane)};
+				else set_error(L, kErrQueueOverflow);
+			}
 		}
-	}
-	const uint32_t big_ballot = __ballot_sync(FULL, is_big);
-	if (big_ballot) {
-		uint32_t incl = is_big ? n_items : 0u;
+		const uint32_t long_ballot = __ballot_sync(FULL, is_long);
+		if (long_ballot) {
+			uint32_t base = 0;
+			const uint32_t leader = __ffs(long_ballot) - 1;
+			if (lane == leader) base = atomicAdd(&L.scr.ctr->longs, (unsigned)__popc(long_ballot));
+			base = __shfl_sync(FULL, base, leader);
+			const uint32_t slot = base + __popc(long_ballot & lt);
+			if (is_long) {
+				if (slot < L.scr.cap) L.scr.mid[L.scr.cap - 1u - slot] = MidRec{j, (uint32_t)(t0 + lane)};
+				else set_error(L, kErrQueueOverflow);
+			}
+		}
+		const uint32_t big_ballot = __ballot_sync(FULL, is_big);
+		if (big_ballot) {
+			uint32_t incl = is_big ? n_items : 0u;
 #pragma unroll
-		for (int d = 1; d < 32; d <<= 1) {
-			const uint32_t v = __shfl_up_sync(FULL, incl, d);
-			if (lane >= (uint32_t)d) incl += v;
-		}
-		const uint32_t total = __shfl_sync(FULL, incl, 31);
-		unsigned long long old = 0;
-		if (lane == 0)
-			old = atomicAdd(&L.scr.ctr->big, ((unsigned long long)__popc(big_ballot) << kBigShift) | (unsigned long long)total);
-		old = __shfl_sync(FULL, old, 0);
-		if (is_big) {
-			const uint32_t rec = (uint32_t)(old >> kBigShift) + __popc(big_ballot & lt);
-			const uint64_t first = (old & kBigItemMask) + incl - n_items;
-			if (rec < L.scr.cap && first + n_items <= kBigItemMask)
-				L.scr.big[rec] = BigRec{first, j, (uint32_t)(t0 + lane), n_items, slices};
-			else
-				set_error(L, kErrQueueOverflow);
+			for (int d = 1; d < 32; d <<= 1) {
+				const uint32_t v = __shfl_up_sync(FULL, incl, d);
+				if (lane >= (uint32_t)d) incl += v;
+			}
+			const uint32_t total = __shfl_sync(FULL, incl, 31);
+			unsigned long long old = 0;
+			if (lane == 0)
+				old = atomicAdd(&L.scr.ctr->big, ((unsigned long long)__popc(big_ballot) << kBigShift) | (unsigned long long)total);
+			old = __shfl_sync(FULL, old, 0);
+			if (is_big) {
+				const uint32_t rec = (uint32_t)(old >> kBigShift) + __popc(big_ballot & lt);
+				const uint64_t first = (old & kBigItemMask) + incl - n_items;
+				if (rec < L.scr.cap && first + n_items <= kBigItemMask)
+					L.scr.big[rec] = BigRec{first, j, (uint32_t)(t0 + lane), n_items, slices};
+				else
+					set_error(L, kErrQueueOverflow);
+			}
 		}
 	}
 
@@ -305,13 +332,99 @@ __device__ __forceinline__ void write_morton_warp(uint32_t* table, uint32_t plac
 		write_morton_group(table, spread3_narrow((uint32_t)(k << 2)) | place, k, xl, xh);
 }
 
+// Queued triangles of few rows that are too long to test every voxel.
+struct LongWarp {
+	SmallTri tri[32];  // q[0].w: rows of the warp's triangles before this one | voxels of a row - 1 << 16
+	uint32_t job[32];
+};
+
+// A warp sets up up to 32 of them at a time, one per lane (in a launch with few of them fewer, so that all warps
+// have some), parks them and deals their rows over its lanes: the bounds that the six tests of x and the plane
+// test put on a row are found as in surf_rows, and the row is its lane's to write.
+template <class P>
+static __device__ __noinline__ void long_triangles(const LaunchDesc& L, LongWarp& W, uint32_t n_long, uint32_t warp,
+                                                   uint32_t n_warps) {
+	const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+	const uint32_t turns = (n_long + 32u * n_warps - 1u) / (32u * n_warps), each = (n_long + turns * n_warps - 1u) / (turns * n_warps);
+	for (uint64_t first = (uint64_t)warp * each; first < n_long; first += (uint64_t)n_warps * each) {
+		SurfTri S;
+		uint32_t n_rows = 0, job = 0;
+		if (lane < each && first + lane < n_long) {
+			const MidRec m = L.scr.mid[L.scr.cap - 1u - (uint32_t)(first + lane)];
+			if (m.job < L.n_jobs && m.tri < job_at(L, m.job).n_tri) {  // (not so only after a queue overflow)
+				const JobDesc& J = job_at(L, m.job);
+				const float unit[3] = {J.unit[0], J.unit[1], J.unit[2]};
+				const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
+				float t[9];
+#pragma unroll
+				for (int k = 0; k < 9; k++) t[k] = J.tris[(uint64_t)m.tri * 9 + k];
+				surf_setup<P>(t, J.bmin, unit, J.inv_unit, J.box_near, grid, S);
+				n_rows = (uint32_t)((S.by1 - S.by0 + 1) * (S.bz1 - S.bz0 + 1));
+				job = m.job;
+			}
+		}
+		uint32_t start = n_rows;
+#pragma unroll
+		for (int d = 1; d < 32; d <<= 1) {
+			const uint32_t v = __shfl_up_sync(FULL, start, d);
+			if (lane >= (uint32_t)d) start += v;
+		}
+		const uint32_t total = __shfl_sync(FULL, start, 31);
+		start -= n_rows;
+		const uint32_t slot = __popc(__ballot_sync(FULL, n_rows != 0u) & lt);
+		if (n_rows) {
+			SmallTri& o = W.tri[slot];
+			pack_small(S, start | (uint32_t)(S.bx1 - S.bx0) << 16, o);
+			if (plane_underflows(S.d1, S.d2)) plane_widen(S.nx, S.ny, S.nz, job_at(L, job).unit, o.q[4].z, o.q[4].w);
+			W.job[slot] = job;
+		}
+		__syncwarp();
+		uint32_t begun = 0;  // triangles that start before this step's rows
+		for (uint32_t base = 0; base < total; base += 32) {
+			const uint32_t at = start - base;
+			const uint32_t starts = __reduce_or_sync(FULL, n_rows && at < 32u ? 1u << at : 0u);
+			const uint32_t rec = begun + __popc(starts & (0xFFFFFFFFu >> (31u - lane))) - 1u;
+			begun += __popc(starts);
+			if (base + lane >= total) continue;
+			const SmallTri& o = W.tri[rec];
+			const JobDesc& J = job_at(L, W.job[rec]);
+			const float4 box = o.q[0];
+			const uint32_t w = __float_as_uint(box.w);
+			int y, z;
+			row_place(box, base + lane - (w & 0xFFFFu), y, z);
+			const float ux = J.unit[0], py = __fmul_rn(__int2float_rn(y), J.unit[1]), pz = __fmul_rn(__int2float_rn(z), J.unit[2]);
+			if (!row_in_yz<P>(o, py, pz)) continue;
+			const float4 a = o.q[3], b = o.q[4], c = o.q[5], d = o.q[6], e = o.q[7], f = o.q[8];
+			const float b0 = (float)(__float_as_uint(box.x) & 0xFFFFFFu), b1 = b0 + (float)(w >> 16);
+			float x0 = b0, x1 = b1;
+			clip_test_lane(c.x, __fmul_rn(c.z, py), -e.z, ux, b0, b1, x0, x1);
+			clip_test_lane(c.y, __fmul_rn(c.w, py), -e.w, ux, b0, b1, x0, x1);
+			clip_test_lane(d.x, __fmul_rn(b.x, py), -f.x, ux, b0, b1, x0, x1);
+			clip_test_lane(d.y, __fmul_rn(b.y, pz), -f.y, ux, b0, b1, x0, x1);
+			clip_test_lane(d.z, __fmul_rn(e.x, pz), -f.z, ux, b0, b1, x0, x1);
+			clip_test_lane(d.w, __fmul_rn(e.y, pz), -f.w, ux, b0, b1, x0, x1);
+			clip_plane(a.y, __fmul_rn(a.z, py), __fmul_rn(a.w, pz), b.z, b.w, fmaxf(fabsf(b.z), fabsf(b.w)),
+			           __fdividef(-1.0f, a.y * ux), ux, b0, b1, x0, x1);
+			if (!(x0 <= x1)) continue;
+			const uint32_t grid[3] = {J.grid[0], J.grid[1], J.grid[2]};
+			const bool morton = (J.flags & JOB_MORTON) != 0;
+			if (J.flags & JOB_NARROW) write_row_t<uint32_t>(J.table, morton, grid, y, z, (int)x0, (int)x1);
+			else write_row_t<uint64_t>(J.table, morton, grid, y, z, (int)x0, (int)x1);
+		}
+		__syncwarp();  // the records are written again
+	}
+}
+
 template <class P, bool kGrouped>
 __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_constant__ LaunchDesc L) {
 	static_assert(P::plane == 2 && P::edge_xy == 1 && P::edge_yz == 1 && P::edge_zx == 2,
 	              "the one-test bounds follow the pinned fused-multiply-add pattern");
-	__shared__ RowsWarp s_warp[kRowsCtaThreads / 32];
+	__shared__ __align__(16) union {
+		RowsWarp rows;
+		LongWarp longs;
+	} s_warp[kRowsCtaThreads / 32];
 	const uint32_t lane = threadIdx.x & 31u;
-	RowsWarp& W = s_warp[threadIdx.x >> 5];
+	RowsWarp& W = s_warp[threadIdx.x >> 5].rows;
 	__shared__ RowsTri s_group[kGrouped ? kRowsCtaThreads / 32 : 1][kGrouped ? kRowsGroup : 1];
 	RowsTri* group = s_group[kGrouped ? threadIdx.x >> 5 : 0];
 	Counters* C = L.scr.ctr;
@@ -319,16 +432,20 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 	// One thread per CTA reads the queue counters (thousands of warps reading one line would
 	// serialise on its L2 slice), the CTA shares them through shared memory.
 	__shared__ unsigned long long s_bigc;
-	__shared__ unsigned s_mid;
+	__shared__ uint2 s_mids;
 	if (threadIdx.x == 0) {
 		s_bigc = *reinterpret_cast<volatile unsigned long long*>(&C->big);
-		s_mid = *reinterpret_cast<volatile unsigned*>(&C->mid);
+		const unsigned long long mids = *reinterpret_cast<volatile unsigned long long*>(&C->mid);  // and C->longs
+		s_mids = make_uint2((uint32_t)mids, (uint32_t)(mids >> 32));
 	}
 	__syncthreads();
+	if (s_mids.y)  // (warps of different CTAs first)
+		long_triangles<P>(L, s_warp[threadIdx.x >> 5].longs, min(s_mids.y, L.scr.cap), (threadIdx.x >> 5) * gridDim.x + blockIdx.x,
+		                  gridDim.x * (blockDim.x >> 5));
 	const unsigned long long bigc = s_bigc;
 	const uint32_t n_big = min((uint32_t)(bigc >> kBigShift), L.scr.cap);
 	const uint64_t n_big_items = bigc & kBigItemMask;
-	const uint32_t n_mid = min(s_mid, L.scr.cap);
+	const uint32_t n_mid = min(s_mids.x, L.scr.cap);
 	const uint64_t total = n_big_items + n_mid;
 	// Warps beyond the number of queued items have nothing to claim (all of them when only small
 	// triangles were queued).

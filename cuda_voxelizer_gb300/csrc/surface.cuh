@@ -517,6 +517,21 @@ __device__ __forceinline__ void clip_test(float a, float k, float d, float u, fl
 	}
 }
 
+// The same for lanes of different triangles: without branches on the sign of `a`.
+__device__ __forceinline__ void clip_test_lane(float a, float k, float d, float u, float b0, float b1, float& lo, float& hi) {
+	const bool up = a > 0.0f, down = a < 0.0f;
+	const float inv = __fdividef(-1.0f, a * u);
+	const float xe = __fmul_rn(__fadd_rn(k, d), inv);
+	const float B = 0x1p-20f * fmaf(fabsf(k) + fabsf(d), fabsf(inv), fabsf(xe) + 1.0f);
+	float n = __fsub_rn(__fadd_rn(xe, 12582912.0f), 12582912.0f);
+	const bool fails = __fmaf_rn(a, __fmul_rn(n, u), k) < -d;
+	n = fails ? n + (up ? 1.0f : -1.0f) : n;
+	if (!((B < 0.25f) & (inv != 0.0f)) && (up | down)) n = test_change(a, k, -d, u, b0, b1) - (up ? 0.0f : 1.0f);
+	lo = up ? fmaxf(lo, n) : lo;
+	hi = down ? fminf(hi, n) : hi;
+	if (a == 0.0f && k < -d) hi = lo - 1.0f;  // the test does not depend on x, and fails
+}
+
 // The plane test of a row, "fails iff s < lo or s > hi" with s(x) = fl(fl(fma(nx, fl(x * u), kpl)) + kpl2)
 // (plane_bounds and plane_widen), monotone in x with the sign of nx.
 static __device__ __noinline__ float plane_change(float nx, float kpl, float kpl2, float bound, bool below, float u,

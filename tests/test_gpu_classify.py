@@ -267,3 +267,52 @@ def test_small_triangles_of_the_first_planes_stay_in_the_classify_kernel(height,
         t[:, :, 2] = h + s * t[:, :, 0]
         ms.append(_time(info, torch.from_numpy(t.astype(np.float32).reshape(-1)).cuda()))
     assert ms[0] < 4 * ms[1], ms
+
+
+@pytest.mark.parametrize("morton", [False, True])
+@pytest.mark.parametrize("ext,n", [
+    ((16, 3, 3), 700), ((15.4, 3, 3), 9_000), ((17, 7, 3.5), 9_000), ((17, 8, 3.5), 9_000),  # 16 voxels; around 32 rows
+    ((60, 7, 7), 9_000), ((40, 6.2, 5.2), 9_000), ((200, 63, 0.2), 3_000),                   # around as many rows as voxels, 64 rows
+    ((500, 2, 2), 2_000), ((509, 1, 1), 2_000),                                              # around 512 voxels
+    ((30, 2, 2), 1), ((30, 2, 2), 33), ((30, 2, 2), 130_001),                                # triangles per warp
+])
+def test_triangles_of_few_long_rows(rsqrt, ext, n, morton):
+    _check(rsqrt, _triangles(41, n, ext, 512), 512, morton)
+
+
+def test_long_rows_beside_all_other_kinds(rsqrt):
+    """Queues of all three kinds in one launch, and in a plan of several meshes with different grids."""
+    jobs, alone = [], []
+    for seed, g, morton in ((1, 640, False), (2, 256, True), (3, 400, False)):
+        t = _triangles(seed, 20_011, (1.5, 1.5, 1.5), g)
+        t[::7] = _triangles(seed, len(t[::7]), (40, 2, 2), g)
+        t[::53] = _triangles(seed, len(t[::53]), (30, 20, 4), g)
+        t[::97] = _triangles(seed, len(t[::97]), (20, 30, 90), g)
+        _check(rsqrt, t, g, morton)
+        info = cv.make_info((0, 0, 0), (float(g),) * 3, g, len(t))
+        d = torch.from_numpy(t.reshape(-1)).cuda()
+        one, many = (torch.zeros(cv.table_words(info), dtype=torch.int32, device="cuda") for _ in range(2))
+        cv.voxelize(info, d, one, morton)
+        alone.append(one)
+        jobs.append(cv.Job(info, d, many, morton))
+    plan = cv.Plan(jobs, clear_tables=True)
+    for _ in range(2):
+        plan.launch()
+    torch.cuda.synchronize()
+    for one, job in zip(alone, jobs):
+        assert torch.equal(one, job.table)
+
+
+def test_long_rows_on_a_wide_grid(rsqrt):
+    """A grid with an axis much longer than the others, whose voxels are 64 times shorter along it."""
+    t = _triangles(51, 9_000, (0.6, 1.2, 1.2), 64)
+    _check_info(rsqrt, t, cv.make_info((0, 0, 0), (64.0,) * 3, (4096, 64, 64), len(t)))
+
+
+def test_rows_of_17_voxels_cost_about_as_much_as_rows_of_15():
+    """Many triangles of few rows on both sides of the rule on a row's voxels: as much on both sides where it was
+    measured, 4.4 times as much when those of longer rows were items of their own."""
+    n, g = 200_000, 512
+    info = cv.make_info((0, 0, 0), (float(g),) * 3, g, n)
+    ms = [_time(info, torch.from_numpy(_triangles(10, n, (ext, 2, 2), g).reshape(-1)).cuda()) for ext in (14, 17)]
+    assert ms[1] < 2.5 * ms[0], ms
