@@ -9,6 +9,7 @@ process instead).
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 from dataclasses import dataclass
 from typing import Sequence
@@ -518,14 +519,15 @@ class Server:
 _BBOX_WORKSPACE = 256  # CVX_BBOX_WORKSPACE
 
 
+_here = contextlib.nullcontext()
+
+
 def _on(stream):
     """A context with torch's current stream set to `stream` (a torch stream, a raw handle, or an object that has
     one), for memory that is used there: the allocator only orders a block's next use on the stream it belongs to."""
-    import contextlib
-
     import torch
     if stream is None:
-        return contextlib.nullcontext()
+        return _here
     if not isinstance(stream, torch.cuda.Stream):
         raw = _stream(stream)
         # handles 0 and 1 are the default stream; ExternalStream(0) would be a new one
@@ -540,11 +542,14 @@ def _scratch(nbytes: int, device, stream):
         return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
-def _result(t, stream):
-    """A tensor made under _on(stream), for a caller who uses it on the current stream."""
+def _new(make, stream):
+    """make(): a tensor that a call on `stream` writes and the caller uses on the current stream."""
+    if stream is None:
+        return make()
     import torch
-    if stream is not None:
-        t.record_stream(torch.cuda.current_stream(t.device))
+    with _on(stream):
+        t = make()
+    t.record_stream(torch.cuda.current_stream(t.device))
     return t
 
 
@@ -576,23 +581,21 @@ def gather_soup(vertices, faces, stream=None):
     number of faces with an index out of range).  Synchronizes to read the count."""
     import torch
     f = faces.reshape(-1, 3)
+    soup = _new(lambda: torch.empty(f.shape[0] * 9, dtype=torch.float32, device=vertices.device), stream)
     with _on(stream):
-        soup = torch.empty(f.shape[0] * 9, dtype=torch.float32, device=vertices.device)
         bad = torch.zeros(1, dtype=torch.int64, device=vertices.device)
         check(lib.cvx_gather_soup(_ptr(vertices), vertices.numel() // 3, _ptr(f), f.shape[0], _ptr(soup), _ptr(bad),
                                   _stream(stream)), "cvx_gather_soup")
-        n_bad = int(bad.item())
-    return _result(soup, stream), n_bad
+        return soup, int(bad.item())
 
 
 def transcode(table, gridsize: int, to_morton: bool, stream=None):
     """Morton <-> linear copy of a g^3 table (CUDA tensor); returns a new tensor."""
     import torch
-    with _on(stream):
-        out = torch.empty_like(table)
+    out = _new(lambda: torch.empty_like(table), stream)
     check(lib.cvx_transcode(_ptr(table), _ptr(out), int(gridsize), int(bool(to_morton)), _stream(stream)),
           "cvx_transcode")
-    return _result(out, stream)
+    return out
 
 
 def _encode_scratch(info: VoxInfo, table, stream):
@@ -654,8 +657,7 @@ def encode_voxel_list(info: VoxInfo, table, stream=None):
     n = ctypes.c_uint64()
     check(lib.cvx_encode_voxel_list_ws(ctypes.byref(info), _ptr(table), _ptr(ws), ws.numel(), None, 0, ctypes.byref(n),
                                        _stream(stream)), "cvx_encode_voxel_list_ws")
-    with _on(stream):
-        out = torch.empty((max(1, n.value), 3), dtype=torch.int32, device=table.device)
+    out = _new(lambda: torch.empty((max(1, n.value), 3), dtype=torch.int32, device=table.device), stream)
     check(lib.cvx_encode_voxel_list_ws(ctypes.byref(info), _ptr(table), _ptr(ws), ws.numel(), _ptr(out), n.value,
                                        ctypes.byref(n), _stream(stream)), "cvx_encode_voxel_list_ws")
-    return _result(out, stream)[:n.value]
+    return out[:n.value]
