@@ -404,7 +404,7 @@ __device__ __forceinline__ void or_span_morton(uint32_t* table, int xl, int xh, 
 	}
 }
 
-// Last job whose range [begin, ...) starts at or before idx, for any monotone per-job begin field.
+// The same by one thread, for lanes whose idx differ (solid_morton_small, brick_raster).
 template <class F>
 __device__ __forceinline__ uint32_t job_search(const LaunchDesc& L, uint64_t idx, F begin_of) {
 	if (L.n_jobs == 1) return 0;

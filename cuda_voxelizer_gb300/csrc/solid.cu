@@ -432,6 +432,7 @@ __host__ __device__ __forceinline__ bool lane_rows(uint32_t gx) { return gx % 12
 // the L1 for the rest of its sector, which long rows, or loads made ahead, push out.  Ten jobs of 512^3 at
 // once 69 us (88 with the warp on consecutive words, 111 with the next load made ahead), forty of 256^3
 // 49 / 70, one of 384^3 8 / 10, of 640^3 16 / 20; of 768^3 39 / 26, of 1024^3 92 / 57, hence kLaneRow.
+// Six CTAs per SM at 40 registers with 12 B of spills; seven and eight spill more and are no faster.
 __global__ void __launch_bounds__(256, 6) solid_resolve(const __grid_constant__ LaunchDesc L) {
 	const uint32_t unit_id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
 	if (unit_id >= L.n_units) return;
@@ -702,7 +703,8 @@ static cudaError_t launch_solid_t(const LaunchDesc& L, const Tune& tune, int col
 	cudaError_t e = cudaSuccess;
 	if (prof) (*prof)(nullptr, s);
 	if ((phases & kSolidToggles) && L.n_tiles) {
-		// fewer classify CTAs than the persistent column grid has do not fill the chip
+		// split while there are fewer classify CTAs than solid_cols has (4 per SM; the classify kernel itself
+		// holds 12: a line at its own residency has not been measured)
 		const uint32_t split = classify_split(L.n_tiles, (uint32_t)cols_grid);
 		solid_classify<P><<<L.n_tiles << split, kTile, 0, s>>>(L, std::min(tune.small_cols, kSmallCols), split);
 		if ((e = cudaGetLastError()) != cudaSuccess) return e;

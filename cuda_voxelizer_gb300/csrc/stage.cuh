@@ -102,8 +102,10 @@ __device__ __forceinline__ bool queue_item(const LaunchDesc& L, unsigned long lo
 }
 
 // Triangles of a classify warp: 32, or in a launch with few tiles 32 >> split, so that its warps are
-// spread over the chip and none has many rows or columns to walk.  Splits up to kMaxSplit; a split of
-// s launches 2^s CTAs per tile.  (9,216-triangle torus: surf_classify 64^3 11.7 -> 9.5 us, 128^3 16 ->
+// spread over the chip and none has many rows or columns to walk.  Split while the launch has fewer CTAs
+// than `enough`, those of the persistent kernel that follows (6 per SM for surface jobs, 4 for solid
+// ones; the classify kernels themselves hold 9 and 12), up to kMaxSplit; a split of s launches 2^s CTAs
+// per tile.  (9,216-triangle torus: surf_classify 64^3 11.7 -> 9.5 us, 128^3 16 ->
 // 11.3 us, 256^3 with surf_rows 39 -> 27 us; solid_classify + solid_cols 256^3 28 -> 18 us.)
 constexpr uint32_t kMaxSplit = 3;
 inline uint32_t classify_split(uint32_t n_tiles, uint32_t enough) {

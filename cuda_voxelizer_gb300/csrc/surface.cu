@@ -56,7 +56,8 @@ __device__ __forceinline__ void row_place(const float4& box, uint32_t r, int& y,
 // 71 us; 90 us with the rows listed in shared memory and dealt over the CTA behind three barriers, the
 // tests combined with short-circuit branches (15% of all instructions) and the edge sums added up
 // before they are compared.  Nine CTAs per SM at 56 registers; ten at 48 are 1% slower.
-// Triangles with longer rows, or more, cost less in surf_rows, which shares one setup over a warp: with
+// Triangles with more rows cost less in surf_rows, which shares one setup over a warp, and so do those with
+// longer ones, whose voxels need not all be tested (few such rows: long_triangles): with
 // up to 256 rows of any length kept here, the soup of 300,000 at 300^3 took 148 + 642 us in the two
 // kernels, 44 + 701 with this rule.  A warp keeps all such triangles, also in a launch of few CTAs:
 // leaving those of a warp with more than 384 rows to surf_rows took 31 + 75 us instead of 43 + 37 on
@@ -266,7 +267,8 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 // few items, by the latency of one item elsewhere.  The soup of 2 M triangles at 1024^3: 26.9 ms for
 // 3.36 G word updates (125 G/s); 39.8 ms with all eight x-dependent tests evaluated per row (41 G warp
 // instructions).  The soup of 300,000 at 300^3 384 us / 697 us.  Six CTAs per SM at 80 registers; five
-// are 2% faster on the first soup and 3% slower on the second, seven spill.  Reading a word before the
+// are 2% faster on the first soup and 3% slower on the second, seven spill (at six only the part for long
+// triangles does, 76 B and 108 B).  Reading a word before the
 // atomic, to skip it where its bits are set, cost as many L2 requests as it saved (27.4 - 28.2 ms, and
 // 30% to 90% more where the table fits the L2), and walking the items twice or four times, each time for
 // a half or quarter of the table that stays in the L2, was 2% to 7% slower.

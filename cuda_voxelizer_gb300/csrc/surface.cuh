@@ -4,16 +4,17 @@
 // Reference: voxelize_triangle, src/voxelize.cu:58-190.  Per triangle the reference computes a
 // plane test (:89-95) and nine 2D edge functions (:97-133) once, then tests every voxel of the
 // triangle's grid bbox (:136-181).  Here the per-triangle part is SurfTri/surf_setup; the per-voxel
-// part is fail_bits + yz_pass, which evaluate the very same fp32 expressions for a voxel (x, y, z).
+// part is fail_bits + yz_fail_bits, which evaluate the very same fp32 expressions for a voxel (x, y, z),
+// and the same tests as single comparisons (plane_bounds, row_mask, clip_test, clip_plane).
 //
 // Row intervals.  For a fixed row (y, z) every test depends on x only through p.x = x * unit.x,
 // and each test value is a composition of correctly rounded, monotone operations of p.x.  So each
 // edge test passes on a prefix or a suffix of x, and so does each side of the plane test (see
 // fail_bits).  The voxels of a row that pass all tests therefore form one interval [xl, xh].
-// row_interval finds it: a real-valued estimate of every test's crossing picks the candidate
-// ends, then exact evaluations at the candidates (and a walk if an estimate was off) pin them.
-// The result is identical to testing every voxel of the row; only the number of evaluations
-// changes.
+// row_interval_fast (the brick rasterizer) and clip_test / clip_plane (surf_rows) find it: a
+// real-valued estimate of a test's crossing picks the candidate end, then exact evaluations at the
+// candidate (and a search if the estimate is not good enough) pin it.  The result is identical to
+// testing every voxel of the row; only the number of evaluations changes.
 #pragma once
 #include "cvx_device.cuh"
 
@@ -302,7 +303,7 @@ __device__ __forceinline__ uint32_t yz_fail_bits(const SurfTri& S, float py, flo
 
 // Direction of every x-dependent test for this triangle: lo = passes on a suffix of x (a lower
 // bound), hi = passes on a prefix (an upper bound); tests in neither mask do not depend on x.
-// The reciprocals only steer where the exact walk of row_interval starts, so the fast
+// The reciprocals only steer where the exact walk of row_interval_in starts, so the fast
 // approximate division is enough (an infinite or NaN estimate falls back to the bbox end).
 struct RowDirs {
 	uint32_t lo, hi;

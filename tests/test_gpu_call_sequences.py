@@ -97,6 +97,38 @@ def test_calls_on_several_streams():
         assert torch.equal(table, work.items[k][3])
 
 
+
+def test_calls_from_several_threads():
+    """Threads with a stream each: their calls share nothing."""
+    import threading
+    work = _Work()
+    torch.cuda.synchronize()
+    bad, streams = [], [torch.cuda.Stream() for _ in range(4)]
+
+    def run(i):
+        try:
+            with torch.cuda.stream(streams[i]):
+                done = []
+                for r in range(25):
+                    k = (r + i) % len(work.items)
+                    table = work.table(work.items[k][0])
+                    work.call(k, table)
+                    done.append((k, table))
+                cv.device_status(streams[i])
+                bad.extend(k for k, table in done if not torch.equal(table, work.items[k][3]))
+        except Exception as e:
+            bad.append(e)
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(len(streams))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+    for s in streams:
+        cv.stream_release(s)
+
+
 @pytest.mark.parametrize("morton,g", [(False, 100), (False, 128), (False, 72), (True, 16), (True, 64), (True, 128)])
 @pytest.mark.parametrize("n", [2, 3])
 def test_solid_jobs_of_a_plan_that_share_a_table(morton, g, n):
