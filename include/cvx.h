@@ -110,8 +110,8 @@ cvx_status cvx_voxelize_ws(const cvx_voxinfo* info, const float* d_triangles, ui
 cvx_status cvx_voxelize_solid_noalloc(const cvx_voxinfo* info, const float* d_triangles, uint32_t* d_table,
                                       int morton, cvx_stream_t stream);
 
-/* Synchronizes `stream` and reports device-side checks of the last calls made on it through the
- * library-owned scratch, and of the last cvx_voxelize_solid_noalloc call on the current device:
+/* Synchronizes `stream` and reports device-side checks of the last call that ran on it with the
+ * library-owned scratch (a replay of a captured call among them), and of the last cvx_voxelize_solid_noalloc call on the current device:
  * CVX_OK, or CVX_ERR_DEVICE_CHECK (a queue overflow or a timed-out copy; the call's table is then
  * incomplete). */
 cvx_status cvx_device_status(cvx_stream_t stream);
