@@ -1636,8 +1636,8 @@ cvx_status cvx_set_tuning(int device, const cvx_tuning* in) {
 	if (cur != device) cudaSetDevice(cur);
 	if (st != CVX_OK) return st;
 	std::lock_guard<std::mutex> lk(g_mu);
-	g_dev[device].tune.small_vox = in->small_vox;
-	g_dev[device].tune.small_cols = in->small_cols;
+	g_dev[device].tune.small_vox = std::min(in->small_vox, kLocalRows);
+	g_dev[device].tune.small_cols = std::min(in->small_cols, kSmallCols);
 	g_dev[device].tune.brick_pairs = std::min(in->brick_pairs, kMaxBrickPairs);
 	return CVX_OK;
 }

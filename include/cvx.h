@@ -111,9 +111,9 @@ cvx_status cvx_voxelize_solid_noalloc(const cvx_voxinfo* info, const float* d_tr
                                       int morton, cvx_stream_t stream);
 
 /* Synchronizes `stream` and reports device-side checks of the last call that ran on it with the
- * library-owned scratch (a replay of a captured call among them), and of the last cvx_voxelize_solid_noalloc call on the current device:
- * CVX_OK, or CVX_ERR_DEVICE_CHECK (a queue overflow or a timed-out copy; the call's table is then
- * incomplete). */
+ * library-owned scratch (a replay of a captured call among them), and of the last
+ * cvx_voxelize_solid_noalloc call on the current device: CVX_OK, or CVX_ERR_DEVICE_CHECK (a queue
+ * overflow or a timed-out copy; the call's table is then incomplete). */
 cvx_status cvx_device_status(cvx_stream_t stream);
 
 /* Synchronizes `stream` and frees the scratch the library allocated for it (on the current device).
@@ -302,7 +302,8 @@ typedef struct cvx_tuning {
 	                       * shared-memory brick rasterizer may use, at most 16; 0 (the default)
 	                       * rasterizes every larger triangle row by row with global atomics instead */
 } cvx_tuning;
-/* Per-device tuning used by subsequent calls (results never depend on it). */
+/* Per-device tuning used by subsequent calls (results never depend on it).  Values above a knob's
+ * maximum are taken as the maximum, which cvx_get_tuning then reports. */
 cvx_status cvx_get_tuning(int device, cvx_tuning* out);
 cvx_status cvx_set_tuning(int device, const cvx_tuning* in);
 

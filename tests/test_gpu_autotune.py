@@ -77,3 +77,15 @@ def test_a_cache_of_other_knob_units_is_not_applied(tmp_path):
 def test_candidates_differ():
     """No candidate is above the value at which the engine caps its knob: those would be timed twice."""
     assert max(at.SMALL_VOX) <= 64 and max(at.SMALL_COLS) <= 16
+
+
+def test_tuning_reports_the_values_that_run():
+    """Values above a knob's cap are accepted and reported as the cap, which is what the engine runs with."""
+    before = cv.get_tuning(0)
+    try:
+        cv.set_tuning(0, small_vox=255, small_cols=200, brick_pairs=1000)
+        assert cv.get_tuning(0) == {"small_vox": 64, "small_cols": 16, "brick_pairs": 16}
+        cv.set_tuning(0, small_vox=63, small_cols=0, brick_pairs=0)
+        assert cv.get_tuning(0) == {"small_vox": 63, "small_cols": 0, "brick_pairs": 0}
+    finally:
+        cv.set_tuning(0, **before)
