@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 	}
 }
 
-// Persistent CTAs of four warps; a warp takes one item (a triangle, or 32 z-slices of a larger one) at
+// Persistent CTAs of four warps; a warp takes one item (a triangle, or 4 to 32 z-slices of a larger one) at
 // a time.  Lane = slice: the YZ tests' interval of y and the ZX tests' bounds on x.  Lane = y: the XY
 // tests' bounds on x, into a table of the warp in shared memory (kRowsWindow values of y at a time).
 // Then the item's rows, 32 at a time, one per lane: the row's slice is found by counting the slices that
