@@ -127,7 +127,7 @@ struct Counters {
 	unsigned long long bticket;  // next triangle of the brick queue for brick_bin
 	unsigned long long fticket;  // next triangle of the brick queue for brick_fill
 	unsigned long long rticket;  // next raster work unit for brick_raster
-	unsigned int mid;            // number of MidRec (surf_rows reads it and the next one together)
+	alignas(8) unsigned int mid; // number of MidRec (surf_classify and surf_rows take it and the next one together)
 	unsigned int longs;          // number of triangles queued at the end of mid[], the last one first
 	unsigned int bq;             // number of triangles in the brick queue
 	unsigned int units;          // raster work units (written by brick_scan)

@@ -144,27 +144,16 @@ __global__ void __launch_bounds__(kTile, 9) surf_classify(const __grid_constant_
 				else set_error(L, kErrQueueOverflow);
 			}
 		}
-		const uint32_t mid_ballot = __ballot_sync(FULL, is_mid);
-		if (mid_ballot) {
-			uint32_t base = 0;
-			const uint32_t leader = __ffs(mid_ballot) - 1;
-			if (lane == leader) base = atomicAdd(&L.scr.ctr->mid, (unsigned)__popc(mid_ballot));
-			base = __shfl_sync(FULL, base, leader);
-			const uint32_t slot = base + __popc(mid_ballot & lt);
-			if (is_mid) {
-				if (slot < L.scr.cap) L.scr.mid[slot] = MidRec{j, (uint32_t)(t0 + lane)};
-				else set_error(L, kErrQueueOverflow);
-			}
-		}
-		const uint32_t long_ballot = __ballot_sync(FULL, is_long);
-		if (long_ballot) {
-			uint32_t base = 0;
-			const uint32_t leader = __ffs(long_ballot) - 1;
-			if (lane == leader) base = atomicAdd(&L.scr.ctr->longs, (unsigned)__popc(long_ballot));
-			base = __shfl_sync(FULL, base, leader);
-			const uint32_t slot = base + __popc(long_ballot & lt);
-			if (is_long) {
-				if (slot < L.scr.cap) L.scr.mid[L.scr.cap - 1u - slot] = MidRec{j, (uint32_t)(t0 + lane)};
+		const uint32_t mid_ballot = __ballot_sync(FULL, is_mid), long_ballot = __ballot_sync(FULL, is_long);
+		if (mid_ballot | long_ballot) {  // both counters with one atomic: 68 triangles of all sizes at 128^3 14.4 / 13.1 us
+			unsigned long long base = 0;
+			if (lane == 0)
+				base = atomicAdd(reinterpret_cast<unsigned long long*>(&L.scr.ctr->mid),
+				                 ((unsigned long long)__popc(long_ballot) << 32) | (unsigned long long)__popc(mid_ballot));
+			base = __shfl_sync(FULL, base, 0);
+			if (is_mid || is_long) {
+				const uint32_t slot = is_mid ? (uint32_t)base + __popc(mid_ballot & lt) : (uint32_t)(base >> 32) + __popc(long_ballot & lt);
+				if (slot < L.scr.cap) L.scr.mid[is_mid ? slot : L.scr.cap - 1u - slot] = MidRec{j, (uint32_t)(t0 + lane)};
 				else set_error(L, kErrQueueOverflow);
 			}
 		}
@@ -442,9 +431,11 @@ __global__ void __launch_bounds__(kRowsCtaThreads, 6) surf_rows(const __grid_con
 		s_mids = make_uint2((uint32_t)mids, (uint32_t)(mids >> 32));
 	}
 	__syncthreads();
-	if (s_mids.y)  // (warps of different CTAs first)
-		long_triangles<P>(L, s_warp[threadIdx.x >> 5].longs, min(s_mids.y, L.scr.cap), (threadIdx.x >> 5) * gridDim.x + blockIdx.x,
-		                  gridDim.x * (blockDim.x >> 5));
+	// (Warps of different CTAs first, from the last one on: the first ones have the first items.  In launches of
+	// few triangles, 3,223 of all sizes at 128^3: 18.5 us / 16.4.)
+	if (s_mids.y)
+		long_triangles<P>(L, s_warp[threadIdx.x >> 5].longs, min(s_mids.y, L.scr.cap),
+		                  (threadIdx.x >> 5) * gridDim.x + gridDim.x - 1u - blockIdx.x, gridDim.x * (blockDim.x >> 5));
 	const unsigned long long bigc = s_bigc;
 	const uint32_t n_big = min((uint32_t)(bigc >> kBigShift), L.scr.cap);
 	const uint64_t n_big_items = bigc & kBigItemMask;
